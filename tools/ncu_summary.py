@@ -1,10 +1,10 @@
-"""Turn the raw ncu artefacts a gpurun call brings back into the small summaries kept under profiles/.
+"""Turn raw ncu artefacts into the small summaries kept under profiles/.
 
-  python tools/ncu_summary.py launches gpurun_out/launches.csv            -> per-kernel share table (markdown, stdout)
-  python tools/ncu_summary.py full gpurun_out/prof_attn.ncu-rep OUT.json  -> selected metrics per launch (needs `ncu -i`)
+  python tools/ncu_summary.py launches launches.csv            -> per-kernel share table (markdown, stdout)
+  python tools/ncu_summary.py full prof_attn.ncu-rep OUT.json  -> selected metrics per launch (needs `ncu -i`)
 
 The launch list comes from `ncu --metrics gpu__time_duration.sum --clock-control none` (cold caches, serialised: shares
-only); the full capture from `ncu --set full --clock-control none` (tools/gpu_round.sh).
+only); the full capture from `ncu --set full --clock-control none` on a small case of one kernel, a few GB on the device at most.
 """
 from __future__ import annotations
 
