@@ -179,6 +179,25 @@ def test_gemm_weight_only_256_rows(ops, m, n, k):
         assert torch.equal(amax, a.float().abs().view(m, -1, 16).amax(-1))
 
 
+@pytest.mark.parametrize("m,n,k", [(128, 55296, 5120), (100, 5120, 27648), (65, 7168, 5120), (64, 5120, 27648), (17, 5120, 13824)])
+def test_gemm_weight_only_rings_turn_many_times(ops, m, n, k):
+    """Long K with the automatic split: 5 to 40 stages per CTA, so that every ring turns several times and both widening groups reuse each
+    other's stages.  A stage read before its load has landed would be off by some 4e-3 of the bound's sum; fp32 sums are not by 2e-6."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    x = torch.randn((m, k), generator=g, device="cuda").bfloat16()
+    wq = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int8)
+    ws = torch.rand(n, generator=g, device="cuda") * 0.02
+    ref, size = [], []
+    for w in wq.split(8192):
+        ref.append(x.double() @ w.double().T)
+        size.append(x.double().abs() @ w.double().abs().T)
+    ref, size = torch.cat(ref, 1) * ws.double(), torch.cat(size, 1) * ws.double()
+    first = ops.gemm(x, wq, None, ws, out_dtype=torch.float32)
+    assert ((first.double() - ref).abs() <= 2e-6 * size).all()
+    for _ in range(20):
+        assert torch.equal(ops.gemm(x, wq, None, ws, out_dtype=torch.float32), first)
+
+
 def test_gemm_is_deterministic_and_stream_k_leaves_workspace_clean(ops):
     """Partial sums are added in fixed order (cluster rank / stream-K contributor) -> same bits every launch, with PDL on
     or off; the stream-K counters at the head of a shared workspace are zero again after every call (that is what lets

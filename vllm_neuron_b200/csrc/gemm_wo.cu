@@ -25,6 +25,8 @@ constexpr int WOX_RAW = WOX_ROWS * WOX_BK;    // bytes of raw weights per stage
 constexpr int WOX_CONV = 16;                       // widening / epilogue warps: two groups of one warp per 32 rows
 constexpr int WOX_THREADS = 64 + WOX_CONV * 32 + 32;  // + TMA weights, MMA, TMA activations
 constexpr int WOX_MAX_ST = 5;
+template <int BM>
+constexpr int WOX_STAGES = BM == 128 ? 3 : BM == 64 ? 4 : WOX_MAX_ST;
 
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
   float4 v;
@@ -53,7 +55,8 @@ constexpr float WOX_SCALE = 64.f;
 template <int BM, int EPI>
 __global__ void __launch_bounds__(WOX_THREADS, 1)
     gemm_wo_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap a_map, GemmEpilogue ep, int M, int N,
-                   int num_kb, int nst, int tile0) {
+                   int num_kb, int tile0) {
+  constexpr int nst = WOX_STAGES<BM>;
   constexpr int A_TILE = BM * GEMM_BK_BYTES;  // 64 k of the tokens; a stage holds two
   constexpr int STAGE = WOX_RAW + 2 * A_TILE;
   constexpr uint32_t SLOT_COLS = 64;                     // 64 k of widened rows: 32 columns for each half of the tile
@@ -164,13 +167,21 @@ __global__ void __launch_bounds__(WOX_THREADS, 1)
     if (lane == 0) tc_commit(&tfull);
     __syncwarp();
   } else {
-    // widening: a thread owns one weight row of the tile, the two groups of eight warps alternate between stages
+    // widening: a thread owns one weight row of the tile, the two groups of eight warps alternate between stages.
+    // A parity wait only tells a phase from the one before it.  With an odd number of stages the use of a stage before this one was the
+    // other group's, and nothing this group has seen orders it behind that use's load: were that load still in flight, a wait for full_raw
+    // alone would take the phase before it for its own and read stale bytes.  Hence first the wait for the MMAs of stage i - nst (empty_a):
+    // they follow its widening, which followed its load.  That wait cannot come a phase late, since the MMAs of stage i need this group;
+    // nor a phase early, since the MMAs, which retire in order, are past stage i - 2 nst: in stage i - 2 this group waited for those of slot
+    // use 2 i - 3 - SLOTS.
+    static_assert(4 * nst >= (int)SLOTS + 4, "the MMAs of stage i - 2 nst have retired when a group comes to stage i");
     const int q = warp & 3, half = ((warp - 2) >> 2) & 1, group = (warp - 2) >> 3;
     const int row = half * 128 + q * 32 + lane;
     const uint32_t lanes = (uint32_t)(q * 32) << 16;
     for (int i = group; i < nk; i += 2) {
-      const int s = i % nst;
-      mbar_wait(&full_raw[s], (i / nst) & 1);
+      const int s = i % nst, use = i / nst;
+      if (use) mbar_wait(&empty_a[s], (use - 1) & 1);
+      mbar_wait(&full_raw[s], use & 1);
       const uint8_t* rp = smem + (size_t)s * STAGE + row * WOX_BK;
       uint4 raw[2][4];
 #pragma unroll
@@ -304,10 +315,8 @@ __global__ void __launch_bounds__(WOX_THREADS, 1)
 namespace {
 
 template <int BM>
-constexpr int wox_stages() { return BM == 128 ? 3 : BM == 64 ? 4 : 5; }
-template <int BM>
 constexpr size_t wox_smem() {
-  return 1024 + (size_t)wox_stages<BM>() * (WOX_RAW + 2 * BM * GEMM_BK_BYTES);  // 192 to 200 KB; the partial tile takes BM KB of it
+  return 1024 + (size_t)WOX_STAGES<BM> * (WOX_RAW + 2 * BM * GEMM_BK_BYTES);  // 192 to 200 KB; the partial tile takes BM KB of it
 }
 
 // K splits of `tiles` tiles: whole waves of CTAs (one per SM) of nk stages of 1.2 us each, plus filling and draining a CTA, about 4 us, and
@@ -371,7 +380,7 @@ int launch_wo(const void* a, const void* w, const GemmEpilogue& ep, int M, int N
   }
   auto go = [&](int tile0, int n, int S) -> int {
     B200_CUDA_OK(launch_kernel_cluster(gemm_wo_kernel<BM, EPI>, dim3(n * S), dim3(WOX_THREADS), wox_smem<BM>(), S, stream, wm, am, ep, M, N,
-                                       num_kb, wox_stages<BM>(), tile0));
+                                       num_kb, tile0));
     return B200_OK;
   };
   if (first) {
