@@ -16,7 +16,8 @@ bool ssd_segments_ok(const void* xbc, int x_dtype, int C, const float* state, in
 // every segment's own state (from zero) and summed step size -> scratch; then, once the scratch holds the start states
 // (ssd_seg_combine_kernel), outputs and the slots' new states
 int ssd_segment_states(const void* xbc, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log, const float* dt_bias, int H,
-                       int P, int N, int G, const int32_t* segs, int num_segs, float* seg_state, float* seg_dtsum, cudaStream_t st);
+                       int P, int N, int G, const int32_t* segs, int num_segs, const int32_t* seq_seg0, float* seg_state, float* seg_dtsum,
+                       cudaStream_t st);
 int ssd_segment_outputs(const void* xbc, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log, const float* dt_bias,
                         const float* D, float* state, const int32_t* seq_slot, const int32_t* seq_pos0, float* y, int B, int H, int P, int N,
                         int G, const int32_t* segs, int num_segs, const int32_t* seq_seg0, const float* seg_state, const float* seg_dtsum,

@@ -373,7 +373,8 @@ static int launch_scan(const void* xbc, int C, const float* dt_in, int ld_dt, in
   const int4* sd = reinterpret_cast<const int4*>(segs);
   const bool matrix = segs && ssd_segments_ok(xbc, sizeof(XT) == 2 ? B200_BF16 : B200_F32, C, state, P, N, seg_state);
   if (matrix) {
-    const int rc = ssd_segment_states(xbc, C, dt_in, ld_dt, dt_col0, A_log, dt_bias, H, P, N, G, segs, num_segs, seg_state, seg_dtsum, stream);
+    const int rc = ssd_segment_states(xbc, C, dt_in, ld_dt, dt_col0, A_log, dt_bias, H, P, N, G, segs, num_segs, seq_seg0, seg_state, seg_dtsum,
+                                      stream);
     if (rc) return rc;
   } else if (segs) {
     if (smem > 48 * 1024)

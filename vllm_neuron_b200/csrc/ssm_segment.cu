@@ -112,13 +112,14 @@ __device__ __noinline__ void walk_segment(const __nv_bfloat16* __restrict__ xbc,
   }
 }
 
-// S_loc[p][n] = sum_j exp(cum_end - cum_j) dt_j x_j[p] B_j[n] of one (head, segment) -> scratch entry segment + 1; also the segment's
-// summed step size.  8 warps as P / 32 x 8 / (P / 32) tiles of 32 value columns.
+// S_loc[p][n] = sum_j exp(cum_end - cum_j) dt_j x_j[p] B_j[n] of one (head, segment) -> scratch entry segment + 1, where the chaining pass
+// makes the next segment's start state of it; of a sequence's last segment -> its first entry, which no start state needs (the first segment
+// starts from the slot).  Also the segment's summed step size.  8 warps as P / 32 x 8 / (P / 32) tiles of 32 value columns.
 template <int P, int N>
 __global__ void __launch_bounds__(SEG_THREADS, 2)
     ssd_segment_state_kernel(const __nv_bfloat16* __restrict__ xbc, int C, const float* __restrict__ dt_in, int ld_dt, int dt_col0,
                              const float* __restrict__ A_log, const float* __restrict__ dt_bias, int H, int G, const int4* __restrict__ segs,
-                             float* __restrict__ seg_state, float* __restrict__ seg_dtsum) {
+                             const int32_t* __restrict__ seq_seg0, float* __restrict__ seg_state, float* __restrict__ seg_dtsum) {
   griddep_launch();
   griddep_wait();
   constexpr int WP = P / 32, WN = 8 / WP, NT = N / WN / 8;  // n8 tiles per warp
@@ -132,7 +133,8 @@ __global__ void __launch_bounds__(SEG_THREADS, 2)
   const int t0 = sd.x, n = sd.y - sd.x, h = blockIdx.x;
   if (seg_is_short(sd)) return;
   const int64_t bcol = (int64_t)H * P + (int64_t)(h / (H / G)) * N;
-  float* dst = seg_state + ((int64_t)(blockIdx.y + 1) * H + h) * (P * N);
+  const int entry = (sd.w & SEG_LAST) ? seq_seg0[sd.z] : (int)blockIdx.y + 1;
+  float* dst = seg_state + ((int64_t)entry * H + h) * (P * N);
   if (n > SEG_TOKENS) {
     walk_segment<P, N, false>(xbc, C, dt_in, ld_dt, dt_col0 + h, t0, n, (int64_t)h * P, bcol, 0, -expf(A_log[h]), dt_bias[h], 0.f, nullptr, dst,
                               nullptr, 0, seg_dtsum + (int64_t)blockIdx.y * H + h);
@@ -376,7 +378,7 @@ __global__ void ssd_segment_final_kernel(float* __restrict__ state, const float*
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   if (last > seq_seg0[sq]) s = *reinterpret_cast<const float4*>(seg_state + (int64_t)last * per_seq + e);
   else if (seq_pos0[sq] > 0) s = *slot;
-  const float4 l = *reinterpret_cast<const float4*>(seg_state + (int64_t)(last + 1) * per_seq + e);
+  const float4 l = *reinterpret_cast<const float4*>(seg_state + (int64_t)seq_seg0[sq] * per_seq + e);
   *slot = make_float4(d * s.x + l.x, d * s.y + l.y, d * s.z + l.z, d * s.w + l.w);
 }
 
@@ -384,11 +386,11 @@ namespace {
 
 template <int P, int N>
 int launch_state(const __nv_bfloat16* xbc, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log, const float* dt_bias, int H,
-                 int G, const int4* segs, int num_segs, float* seg_state, float* seg_dtsum, cudaStream_t st) {
+                 int G, const int4* segs, int num_segs, const int32_t* seq_seg0, float* seg_state, float* seg_dtsum, cudaStream_t st) {
   constexpr size_t smem = (size_t)SEG_TOKENS * (P + 8 + N + 8) * 2;
   B200_CUDA_OK(cudaFuncSetAttribute(ssd_segment_state_kernel<P, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   B200_CUDA_OK(launch_kernel(ssd_segment_state_kernel<P, N>, dim3(H, num_segs), dim3(SEG_THREADS), smem, st, xbc, C, dt_in, ld_dt, dt_col0,
-                             A_log, dt_bias, H, G, segs, seg_state, seg_dtsum));
+                             A_log, dt_bias, H, G, segs, seq_seg0, seg_state, seg_dtsum));
   return B200_OK;
 }
 
@@ -417,10 +419,11 @@ bool ssd_segments_ok(const void* xbc, int x_dtype, int C, const float* state, in
   return CALL(64, 64)
 
 int ssd_segment_states(const void* xbc, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log, const float* dt_bias, int H,
-                       int P, int N, int G, const int32_t* segs, int num_segs, float* seg_state, float* seg_dtsum, cudaStream_t st) {
+                       int P, int N, int G, const int32_t* segs, int num_segs, const int32_t* seq_seg0, float* seg_state, float* seg_dtsum,
+                       cudaStream_t st) {
 #define CALL(P_, N_)                                                                                                                  \
   launch_state<P_, N_>((const __nv_bfloat16*)xbc, C, dt_in, ld_dt, dt_col0, A_log, dt_bias, H, G, reinterpret_cast<const int4*>(segs), \
-                       num_segs, seg_state, seg_dtsum, st)
+                       num_segs, seq_seg0, seg_state, seg_dtsum, st)
   SEG_SIZES(CALL);
 #undef CALL
 }

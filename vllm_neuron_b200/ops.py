@@ -709,7 +709,7 @@ def ssd_scan(xbc, dt_src, dt_col0: int, a_log, dt_bias, d_skip, state, meta, hea
     nseg = meta.num_segs if segs is not None else 0
     seg_state = seg_dt = None
     if nseg:
-        seg_state = torch.empty((nseg + 1, heads, vdim, nstate), dtype=torch.float32, device=xbc.device)
+        seg_state = torch.empty((nseg, heads, vdim, nstate), dtype=torch.float32, device=xbc.device)
         seg_dt = torch.empty((nseg, heads), dtype=torch.float32, device=xbc.device)
     with _k("ssd_scan"):
         check(_cabi.load().b200_ssd_scan(_ptr(xbc), _edt(xbc), xbc.shape[1], _ptr(dt_src), dt_src.stride(0), dt_col0, _ptr(a_log),
