@@ -160,6 +160,17 @@ def test_gemm_pairs_silu_residual_bias(ops, m, n, k):
     _assert_close(ga, a.float().abs().view(m, -1, 16).amax(-1).cpu())
 
 
+@pytest.mark.parametrize("m,n,k,cut", [(129, 5120, 27648, True), (300, 1024, 28672, True), (640, 2048, 5632, False), (129, 4096, 14336, False)])
+def test_gemm_prompt_schedule(ops, m, n, k, cut):
+    """Short prompts against a long K go to the schedule that cuts K over all SMs, the others to the pairs, which do not: the same bits as a
+    call that asks for every SM, or others."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x, w = torch.randn((m, k), generator=g, device="cuda").bfloat16(), torch.randn((n, k), generator=g, device="cuda").bfloat16()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    got = ops.gemm(x, w, out_dtype=torch.float32)
+    assert torch.equal(got, ops.gemm(x, w, out_dtype=torch.float32, split_k=sms)) == cut
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 1056, 512), (31, 256, 144), (33, 640, 1152), (64, 992, 256), (65, 256, 128), (128, 1000, 144), (100, 640, 1152), (127, 32, 64), (128, 38144, 256), (96, 5120, 2048)])
 def test_gemm_weight_only_256_rows(ops, m, n, k):
     """256-row schedule of decode-sized weight-only batches: ragged rows, k and tokens, uncut tiles beside cut ones (38144 = 149 tiles), every

@@ -191,7 +191,8 @@ __device__ __forceinline__ void epilogue_chunk_xpose(const GemmEpilogue& ep, con
 
 // Weight-only schedule of decode-sized batches (gemm_wo.cu).
 int launch_gemm_wo(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, cudaStream_t stream);
-// Prompt-sized schedule on CTA pairs (gemm_pair.cu): bf16, fp8 and int8 operands.  pair_tokens: tokens of a tile for this shape.
+// Prompt-sized schedule on CTA pairs (gemm_pair.cu): bf16, fp8 and int8 operands.  pair_tokens: tokens of a tile for this shape, 0 where
+// stream-K is the faster schedule.
 int pair_tokens(int M, int N, int K, int ab_dtype);
 int launch_gemm_pair(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, int bt,
                      cudaStream_t stream);

@@ -237,9 +237,15 @@ int launch_pair(const void* a, const void* w, const GemmEpilogue& ep, int M, int
 // the launch; so the widest tile wins unless a narrower one saves a wave or the padding of the last token tile.  Measured (us, 74 pairs):
 //   4096 x 10272 x 2048 bf16: bt 256 134.8, 224 149.2, 192 160.7, 128 212.6;  3688 x 2048 x 2048: 256 31.2, 192 41.8;
 //   1636 x 2048 x 2048: 192 18.6, 256 19.3, 128 28.5;  333 x 2048 x 2048: 64 15.2, 256 17.8;  777 x 4096 x 4096: 224 29.9, 192 50.8.
+// 0: stream-K (gemm_tcgen05.cu) takes the call.  It cuts K, which pays where few tiles walk a long K or a nearly empty wave follows a full
+// one: about 25 us, 0.52 for each k-block of 128 x 256 of an SM's share, and 8 for every CTA that adds to one tile.  Measured (us, pairs /
+// stream-K, bf16): 129 x 5120 x 27648 152 / 106, 256 158 / 115, 320 158 / 156, 512 164 / 173, 777 327 / 292, 1290 400 / 447;
+// 300 x 1024 x 28672 155 / 123, 1400 157 / 122; 200 x 8192 x 28672 175 / 139, 300 170 / 240; 129 x 4096 x 14336 80 / 85, 1200 161 / 158.
+// Over 700 measured calls (bf16 and fp8, 129 to 4096 tokens) the rule takes the slower side by more than 5 % in seven, by 13 % at most, and
+// never leaves a faster pair schedule.
 int pair_tokens(int M, int N, int K, int ab_dtype) {
-  const int eb = ab_dtype == B200_BF16 ? 2 : 1;
-  const int pairs = sm_count() / 2, num_kb = (K * eb + GEMM_BK_BYTES - 1) / GEMM_BK_BYTES, n_tiles = (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN);
+  const int eb = ab_dtype == B200_BF16 ? 2 : 1, sms = sm_count();
+  const int pairs = sms / 2, num_kb = (K * eb + GEMM_BK_BYTES - 1) / GEMM_BK_BYTES, n_tiles = (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN);
   long long best_cost = 0;
   int best = 0;
   for (int bt = PAIR_MAX_BT; bt >= 64; bt -= 32) {
@@ -250,7 +256,9 @@ int pair_tokens(int M, int N, int K, int ab_dtype) {
       best_cost = cost;
     }
   }
-  return best;
+  const double sk_tiles = (double)((M + 255) / 256) * ((N + GEMM_BN - 1) / GEMM_BN), shared = sms / sk_tiles;
+  const double stream_k_us = 25.0 + 0.52 * sk_tiles * num_kb / sms + 8.0 * (shared > 1.0 ? shared : 1.0);
+  return stream_k_us * 1850.0 < (double)best_cost ? 0 : best;  // clocks at 1.85 GHz
 }
 
 int launch_gemm_pair(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, int bt,
