@@ -391,6 +391,34 @@ def test_ssd_scan_segments_as_matrix_products(H, P, N, G, shift, cut, monkeypatc
         at += n
 
 
+@pytest.mark.parametrize("H,P,N,G", [(2, 128, 128, 1), (2, 64, 64, 2)])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_ssd_scan_segments_keep_what_is_not_finite_in_its_place(H, P, N, G, bad):
+    """One infinite or NaN x in the middle of a block of tokens: earlier tokens, other columns and other heads are those of the clean run
+    (its segment is walked token by token: 1e-6 of the norm), the column from that token on is not finite."""
+    from vllm_neuron_b200.hybrid import StepMeta
+
+    ops = _ops()
+    g = torch.Generator().manual_seed(P)
+    T, at, col, C = 300, 150, P + 3, H * P + 2 * G * N  # token 150: the seventh of a block of 16 in the second segment; head 1
+    xbc = torch.nn.functional.silu(torch.randn(T, C, generator=g)).bfloat16()
+    raw, a_log, bias, D = (torch.randn(*s, generator=g).to(DEV) for s in ((T, H), (H,), (H,), (H,)))
+    meta = StepMeta.build([(0, 0, T)], {0: list(range(1, 11))}, 32, torch.device(DEV))
+
+    def scan(x):
+        state = torch.zeros(1, H, P, N, device=DEV)
+        return ops.ssd_scan(x.to(DEV), raw, 0, a_log, bias, D, state, meta, H, P, N, G), state
+
+    clean, clean_state = scan(xbc)
+    x = xbc.clone()
+    x[at, col] = bad
+    y, state = scan(x)
+    assert not torch.isfinite(y[at:, col]).any() and not torch.isfinite(state[0, 1, 3]).any()
+    y[at:, col] = clean[at:, col]
+    state[0, 1, 3] = clean_state[0, 1, 3]
+    assert (y - clean).norm() <= 1e-6 * clean.norm() and (state - clean_state).norm() <= 1e-6 * clean_state.norm()
+
+
 def test_ssd_scan_keeps_to_its_scratch():
     """Scratch of exactly num_segs entries, as the header asks for, a long portion last: the memory behind it stays as it was, and the
     result is that of the wrapper."""

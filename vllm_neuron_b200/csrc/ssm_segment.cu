@@ -73,6 +73,8 @@ __device__ __forceinline__ float segment_decays(const float* __restrict__ dt_in,
   return (float)s;
 }
 
+__device__ __forceinline__ int nonfinite_bf16x2(uint32_t v) { return (v & 0x7f80u) == 0x7f80u || (v & 0x7f800000u) == 0x7f800000u; }
+
 // rows [t0, t0 + n) x COLS bf16 columns from col -> smem rows of COLS + 8; rows past n are zeros
 template <int COLS, int THREADS>
 __device__ __forceinline__ void load_rows(const __nv_bfloat16* __restrict__ src, int ld, int64_t col, int t0, int n, __nv_bfloat16* dst) {
@@ -83,7 +85,8 @@ __device__ __forceinline__ void load_rows(const __nv_bfloat16* __restrict__ src,
   }
 }
 
-// Segments of more tokens than the matrix form takes (a caller's own cut): the recurrence as it stands, a value column per thread.
+// What the products below cannot do -- segments of more tokens, and infinite or NaN x, which a masked weight of zero would carry into the
+// earlier tokens of its block: the recurrence as it stands, a value column per thread.
 template <int P, int N, bool OUT>
 __device__ __noinline__ void walk_segment(const __nv_bfloat16* __restrict__ xbc, int C, const float* __restrict__ dt_in, int ld_dt, int dt_col,
                                           int t0, int n, int64_t xcol, int64_t bcol, int64_t ccol, float negA, float bias, float dsk,
@@ -226,11 +229,6 @@ __global__ void __launch_bounds__(SEG_OUT_THREADS, 1)
   const int64_t bcol = (int64_t)H * P + (int64_t)(h / (H / G)) * N, ccol = bcol + (int64_t)G * N;
   const float* S_in = (sd.w & SEG_FIRST) ? (seq_pos0[sq] > 0 ? state + ((int64_t)seq_slot[sq] * H + h) * (P * N) : nullptr)
                                          : seg_state + ((int64_t)blockIdx.y * H + h) * (P * N);
-  if (n > SEG_TOKENS) {
-    walk_segment<P, N, true>(xbc, C, dt_in, ld_dt, dt_col0 + h, t0, n, (int64_t)h * P, bcol, ccol, -expf(A_log[h]), dt_bias[h], Dskip[h], S_in,
-                             nullptr, y, H * P, nullptr);
-    return;
-  }
   load_rows<N, SEG_OUT_THREADS>(xbc, C, ccol, t0, n, Cs);
   cp_async_commit();
   load_rows<N, SEG_OUT_THREADS>(xbc, C, bcol, t0, n, Bs);
@@ -299,7 +297,16 @@ __global__ void __launch_bounds__(SEG_OUT_THREADS, 1)
     }
   }
   cp_async_wait<0>();
-  __syncthreads();
+  int odd = n > SEG_TOKENS;  // or an infinite or NaN x among those that this thread copied
+  for (int i = threadIdx.x; i < SEG_TOKENS * P / 8; i += SEG_OUT_THREADS) {
+    const uint4 v = *reinterpret_cast<const uint4*>(Xs + i / (P / 8) * (P + 8) + i % (P / 8) * 8);
+    odd |= nonfinite_bf16x2(v.x) | nonfinite_bf16x2(v.y) | nonfinite_bf16x2(v.z) | nonfinite_bf16x2(v.w);
+  }
+  if (__syncthreads_or(odd)) {
+    walk_segment<P, N, true>(xbc, C, dt_in, ld_dt, dt_col0 + h, t0, n, (int64_t)h * P, bcol, ccol, -expf(A_log[h]), dt_bias[h], dsk, S_in,
+                             nullptr, y, H * P, nullptr);
+    return;
+  }
   if (!live) return;
   const float2 ci0 = cum[i0], ci1 = cum[i1];
   for (int jb = 0; jb <= rb; ++jb) {
