@@ -187,9 +187,11 @@ __global__ void __launch_bounds__(SEG_THREADS, 2)
       for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          mma_bf16_16816(acc[i][2 * jj + u], al[i], b[2 * u], b[2 * u + 1]);
-          mma_bf16_16816(acc[i][2 * jj + u], am[i], b[2 * u], b[2 * u + 1]);
-          mma_bf16_16816(acc[i][2 * jj + u], ah[i], b[2 * u], b[2 * u + 1]);
+          float t[4] = {};
+          mma_bf16_16816(t, al[i], b[2 * u], b[2 * u + 1]);
+          mma_bf16_16816(t, am[i], b[2 * u], b[2 * u + 1]);
+          mma_bf16_16816(t, ah[i], b[2 * u], b[2 * u + 1]);
+          add_to(acc[i][2 * jj + u], t);
         }
     }
   }
