@@ -325,11 +325,17 @@ int b200_causal_conv(const float* in, int ld, int col0, const float* conv_w, con
  * state fp32 [slots][H][P][N], updated; y fp32 [T][H*P].  Head h reads group h / (H / G).  N <= 256.
  * segs (or NULL): int32 [num_segs][4] = {first token, end token, sequence, 1 (first of its sequence) | 2 (last)}, 16-byte
  * aligned, a sequence's segments consecutive; seq_seg0 int32 [B + 1] = first segment of each sequence; scratch seg_state
- * fp32 [num_segs][H][P][N] and seg_dtsum fp32 [num_segs][H].  Segments then run in parallel (three launches). */
+ * fp32 [num_segs][H][P][N] and seg_dtsum fp32 [num_segs][H].  Segments of any length then run in parallel (three launches). */
 int b200_ssd_scan(const void* xbc, int x_dtype, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log,
                   const float* dt_bias, const float* D, float* state, const int32_t* seq_start, const int32_t* seq_slot,
                   const int32_t* seq_pos0, float* y, int B, int H, int P, int N, int G, const int32_t* segs, int num_segs,
                   const int32_t* seq_seg0, float* seg_state, float* seg_dtsum, void* stream);
+/* The same for cuts of at most 128 tokens: bf16 x, B and C with P and N of 64 or 128 run as matrix products on the tensor cores (up to
+ * five launches), anything else as above.  Longer segments are right too, but each is walked by one thread per column. */
+int b200_ssd_scan_mma(const void* xbc, int x_dtype, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log,
+                      const float* dt_bias, const float* D, float* state, const int32_t* seq_start, const int32_t* seq_slot,
+                      const int32_t* seq_pos0, float* y, int B, int H, int P, int N, int G, const int32_t* segs, int num_segs,
+                      const int32_t* seq_seg0, float* seg_state, float* seg_dtsum, void* stream);
 /* Scatter keys [G][D] (columns k_col0..) and values [G][Dv] (columns v_col0..) of the fp32 rows `qkv` into the pools
  * K [num_blocks][G][block_size][D], V [num_blocks][G][block_size][Dv] by slot (slot < 0: skipped).
  * mode 0: plain; 1: also keep the unmixed values in v_first fp32 [T][G*Dv]; 2: cache v + lambda * (v_first - v) instead of v. */

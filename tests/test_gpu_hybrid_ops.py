@@ -419,9 +419,10 @@ def test_ssd_scan_segments_keep_what_is_not_finite_in_its_place(H, P, N, G, bad)
     assert (y - clean).norm() <= 1e-6 * clean.norm() and (state - clean_state).norm() <= 1e-6 * clean_state.norm()
 
 
-def test_ssd_scan_keeps_to_its_scratch():
+@pytest.mark.parametrize("entry", ["b200_ssd_scan", "b200_ssd_scan_mma"])
+def test_ssd_scan_keeps_to_its_scratch(entry):
     """Scratch of exactly num_segs entries, as the header asks for, a long portion last: the memory behind it stays as it was, and the
-    result is that of the wrapper."""
+    result is that of the wrapper, bit for bit from the entry that it calls; the other takes the sequential scan, whatever the cuts."""
     from vllm_neuron_b200 import _cabi
     from vllm_neuron_b200.hybrid import StepMeta
 
@@ -436,15 +437,16 @@ def test_ssd_scan_keeps_to_its_scratch():
     meta = StepMeta.build(entries, {r: list(range(1 + 10 * r, 11 + 10 * r)) for r in range(3)}, 32, torch.device(DEV))
     want_state = state.clone()
     want = ops.ssd_scan(xbc, raw, 0, a_log, bias, D, want_state, meta, H, P, N, G)
-    v, entry = meta.num_segs, H * P * N
-    scratch, dts = torch.full((v * entry + 2 * entry,), 7.5, device=DEV), torch.full((v * H + 64,), 7.5, device=DEV)
+    v, size = meta.num_segs, H * P * N
+    scratch, dts = torch.full(((v + 2) * size,), 7.5, device=DEV), torch.full((v * H + 64,), 7.5, device=DEV)
     y = torch.empty(T, H * P, device=DEV)
-    assert _cabi.load().b200_ssd_scan(xbc.data_ptr(), ops.BF16, C, raw.data_ptr(), H, 0, a_log.data_ptr(), bias.data_ptr(), D.data_ptr(),
-                                      state.data_ptr(), meta.seq_start.data_ptr(), meta.seq_slot.data_ptr(), meta.seq_pos0.data_ptr(),
-                                      y.data_ptr(), 3, H, P, N, G, meta.scan_segs.data_ptr(), v, meta.scan_seq_seg0.data_ptr(),
-                                      scratch.data_ptr(), dts.data_ptr(), ops._stream()) == 0
-    assert (scratch[v * entry:] == 7.5).all() and (dts[v * H:] == 7.5).all()
+    assert getattr(_cabi.load(), entry)(xbc.data_ptr(), ops.BF16, C, raw.data_ptr(), H, 0, a_log.data_ptr(), bias.data_ptr(), D.data_ptr(),
+                                        state.data_ptr(), meta.seq_start.data_ptr(), meta.seq_slot.data_ptr(), meta.seq_pos0.data_ptr(),
+                                        y.data_ptr(), 3, H, P, N, G, meta.scan_segs.data_ptr(), v, meta.scan_seq_seg0.data_ptr(),
+                                        scratch.data_ptr(), dts.data_ptr(), ops._stream()) == 0
+    assert (scratch[v * size:] == 7.5).all() and (dts[v * H:] == 7.5).all()
     assert (y - want).norm() <= 1e-6 * want.norm() and (state - want_state).norm() <= 1e-6 * want_state.norm()
+    assert torch.equal(y, want) == (entry == "b200_ssd_scan_mma")
 
 
 @pytest.mark.parametrize("counts", [(300, 0, 129, 128, 1), (3, 40, 0, 32, 33), (0, 0, 0, 0, 7)])

@@ -165,8 +165,8 @@ __global__ void conv_state_update_kernel(const float* __restrict__ in, int ld, i
 //      + S_loc[k], S_in[0] = the slot's state (zero at position 0), and stores S_in[k] over the scratch;
 //   3. the full launch starts every segment from its S_in, writes y, and the last segment writes the slot's new state.
 // The recurrence is linear in S, so this is the sequential result up to fp32 rounding; everything stays fp32.  With bf16 x, B and C and
-// heads of 64 or 128 by 64 or 128, steps 1 and 3 are matrix products instead (ssm_segment.cu), and this kernel only walks the short
-// sequences of the step.
+// heads of 64 or 128 by 64 or 128, and a caller that cut for it (b200_ssd_scan_mma), steps 1 and 3 are matrix products instead
+// (ssm_segment.cu), and this kernel only walks the short sequences of the step.
 
 constexpr int SCAN_PLANES = 32;
 constexpr int SCAN_SLICES = 8;
@@ -366,12 +366,12 @@ template <typename XT, int NPT, int PP>
 static int launch_scan(const void* xbc, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log,
                        const float* dt_bias, const float* Dskip, float* state, const int32_t* seq_start, const int32_t* seq_slot,
                        const int32_t* seq_pos0, float* y, int B, int H, int P, int N, int G, const int32_t* segs, int num_segs,
-                       const int32_t* seq_seg0, float* seg_state, float* seg_dtsum, cudaStream_t stream) {
+                       const int32_t* seq_seg0, float* seg_state, float* seg_dtsum, bool mma, cudaStream_t stream) {
   constexpr int PC = SCAN_PLANES * PP;
   dim3 grid((P + PC - 1) / PC, H, segs ? num_segs : B);
   const size_t smem = (size_t)(SCAN_CHUNK * (2 * NPT * SCAN_SLICES + PC + 2)) * sizeof(float);
   const int4* sd = reinterpret_cast<const int4*>(segs);
-  const bool matrix = segs && ssd_segments_ok(xbc, sizeof(XT) == 2 ? B200_BF16 : B200_F32, C, state, P, N, seg_state);
+  const bool matrix = segs && mma && ssd_segments_ok(xbc, sizeof(XT) == 2 ? B200_BF16 : B200_F32, C, state, P, N, seg_state);
   if (matrix) {
     const int rc = ssd_segment_states(xbc, C, dt_in, ld_dt, dt_col0, A_log, dt_bias, H, P, N, G, segs, num_segs, seq_seg0, seg_state, seg_dtsum,
                                       stream);
@@ -407,10 +407,10 @@ template <typename XT, int NPT>
 static int pick_scan(const void* xbc, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log, const float* dt_bias,
                      const float* Dskip, float* state, const int32_t* seq_start, const int32_t* seq_slot, const int32_t* seq_pos0,
                      float* y, int B, int H, int P, int N, int G, const int32_t* segs, int num_segs, const int32_t* seq_seg0,
-                     float* seg_state, float* seg_dtsum, cudaStream_t stream) {
+                     float* seg_state, float* seg_dtsum, bool mma, cudaStream_t stream) {
 #define PICK_ARGS                                                                                                             \
   xbc, C, dt_in, ld_dt, dt_col0, A_log, dt_bias, Dskip, state, seq_start, seq_slot, seq_pos0, y, B, H, P, N, G, segs, num_segs, \
-      seq_seg0, seg_state, seg_dtsum, stream
+      seq_seg0, seg_state, seg_dtsum, mma, stream
   if constexpr (NPT * 4 <= 32) {
     if (P > 64) return launch_scan<XT, NPT, 4>(PICK_ARGS);
   }
@@ -467,10 +467,10 @@ int b200_causal_conv_silu(const float* in, int ld, int col0, const float* conv_w
                           out_dtype, T, B, C, taps, stream);
 }
 
-int b200_ssd_scan(const void* xbc, int x_dtype, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log,
-                  const float* dt_bias, const float* D, float* state, const int32_t* seq_start, const int32_t* seq_slot,
-                  const int32_t* seq_pos0, float* y, int B, int H, int P, int N, int G, const int32_t* segs, int num_segs,
-                  const int32_t* seq_seg0, float* seg_state, float* seg_dtsum, void* stream) {
+static int ssd_scan(const void* xbc, int x_dtype, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log,
+                    const float* dt_bias, const float* D, float* state, const int32_t* seq_start, const int32_t* seq_slot,
+                    const int32_t* seq_pos0, float* y, int B, int H, int P, int N, int G, const int32_t* segs, int num_segs,
+                    const int32_t* seq_seg0, float* seg_state, float* seg_dtsum, bool mma, void* stream) {
   B200_REQUIRE(xbc && dt_in && A_log && dt_bias && D && state && seq_start && seq_slot && seq_pos0 && y, "ssd_scan: null pointer");
   B200_REQUIRE(H > 0 && G > 0 && H % G == 0, "ssd_scan: %d heads do not split into %d groups", H, G);
   B200_REQUIRE(N >= 1 && N <= 256, "ssd_scan: state size %d (1..256 supported)", N);
@@ -481,7 +481,7 @@ int b200_ssd_scan(const void* xbc, int x_dtype, int C, const float* dt_in, int l
   cudaStream_t st = (cudaStream_t)stream;
 #define SCAN_ARGS                                                                                                          \
   xbc, C, dt_in, ld_dt, dt_col0, A_log, dt_bias, D, state, seq_start, seq_slot, seq_pos0, y, B, H, P, N, G, segs, num_segs, \
-      seq_seg0, seg_state, seg_dtsum, st
+      seq_seg0, seg_state, seg_dtsum, mma, st
   B200_DISPATCH_ELEM(x_dtype, XT, {
     if (N <= 32) return pick_scan<XT, 4>(SCAN_ARGS);
     if (N <= 64) return pick_scan<XT, 8>(SCAN_ARGS);
@@ -490,6 +490,22 @@ int b200_ssd_scan(const void* xbc, int x_dtype, int C, const float* dt_in, int l
   });
 #undef SCAN_ARGS
   return B200_OK;
+}
+
+int b200_ssd_scan(const void* xbc, int x_dtype, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log,
+                  const float* dt_bias, const float* D, float* state, const int32_t* seq_start, const int32_t* seq_slot,
+                  const int32_t* seq_pos0, float* y, int B, int H, int P, int N, int G, const int32_t* segs, int num_segs,
+                  const int32_t* seq_seg0, float* seg_state, float* seg_dtsum, void* stream) {
+  return ssd_scan(xbc, x_dtype, C, dt_in, ld_dt, dt_col0, A_log, dt_bias, D, state, seq_start, seq_slot, seq_pos0, y, B, H, P, N, G, segs,
+                  num_segs, seq_seg0, seg_state, seg_dtsum, false, stream);
+}
+
+int b200_ssd_scan_mma(const void* xbc, int x_dtype, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log,
+                      const float* dt_bias, const float* D, float* state, const int32_t* seq_start, const int32_t* seq_slot,
+                      const int32_t* seq_pos0, float* y, int B, int H, int P, int N, int G, const int32_t* segs, int num_segs,
+                      const int32_t* seq_seg0, float* seg_state, float* seg_dtsum, void* stream) {
+  return ssd_scan(xbc, x_dtype, C, dt_in, ld_dt, dt_col0, A_log, dt_bias, D, state, seq_start, seq_slot, seq_pos0, y, B, H, P, N, G, segs,
+                  num_segs, seq_seg0, seg_state, seg_dtsum, true, stream);
 }
 
 }  // extern "C"

@@ -85,8 +85,8 @@ __device__ __forceinline__ void load_rows(const __nv_bfloat16* __restrict__ src,
   }
 }
 
-// What the products below cannot do -- segments of more tokens, and infinite or NaN x, which a masked weight of zero would carry into the
-// earlier tokens of its block: the recurrence as it stands, a value column per thread.
+// What the products below cannot do -- infinite or NaN x, which a masked weight of zero would carry into the earlier tokens of its block, and
+// segments of more tokens, which no caller cuts for this form: the recurrence as it stands, a value column per thread.
 template <int P, int N, bool OUT>
 __device__ __noinline__ void walk_segment(const __nv_bfloat16* __restrict__ xbc, int C, const float* __restrict__ dt_in, int ld_dt, int dt_col,
                                           int t0, int n, int64_t xcol, int64_t bcol, int64_t ccol, float negA, float bias, float dsk,

@@ -712,11 +712,11 @@ def ssd_scan(xbc, dt_src, dt_col0: int, a_log, dt_bias, d_skip, state, meta, hea
         seg_state = torch.empty((nseg, heads, vdim, nstate), dtype=torch.float32, device=xbc.device)
         seg_dt = torch.empty((nseg, heads), dtype=torch.float32, device=xbc.device)
     with _k("ssd_scan"):
-        check(_cabi.load().b200_ssd_scan(_ptr(xbc), _edt(xbc), xbc.shape[1], _ptr(dt_src), dt_src.stride(0), dt_col0, _ptr(a_log),
+        check(_cabi.load().b200_ssd_scan_mma(_ptr(xbc), _edt(xbc), xbc.shape[1], _ptr(dt_src), dt_src.stride(0), dt_col0, _ptr(a_log),
                                          _ptr(dt_bias), _ptr(d_skip), _ptr(state), _ptr(meta.seq_start), _ptr(meta.seq_slot),
                                          _ptr(meta.seq_pos0), _ptr(y), meta.num_seqs, heads, vdim, nstate, groups,
                                          _ptr(segs) if nseg else 0, nseg, _ptr(meta.scan_seq_seg0) if nseg else 0,
-                                         _ptr(seg_state), _ptr(seg_dt), _stream()), "b200_ssd_scan")
+                                         _ptr(seg_state), _ptr(seg_dt), _stream()), "b200_ssd_scan_mma")
     return y
 
 
