@@ -160,6 +160,37 @@ def test_gemm_pairs_silu_residual_bias(ops, m, n, k):
     _assert_close(ga, a.float().abs().view(m, -1, 16).amax(-1).cpu())
 
 
+@pytest.mark.parametrize("kind", ["bf16", "wo"])
+@pytest.mark.parametrize("m,n,k", [(33, 640, 1152), (64, 4096, 2048), (300, 1056, 640)])
+def test_gemm_outputs_on_any_boundary(ops, kind, m, n, k):
+    """Outputs that start one, two or four elements after a 16-byte boundary: the bits of the aligned call on the schedule that they take
+    (decode batches in bf16: the one that does not cut K, where vectors of four would not lie on their size), nothing written around them."""
+    from vllm_neuron_b200 import _cabi
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn((m, k), generator=g, device="cuda").bfloat16()
+    w = (torch.randn((n, k), generator=g, device="cuda") * k**-0.5).bfloat16() if kind == "bf16" else torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int8)
+    ws = None if kind == "bf16" else torch.rand(n, generator=g, device="cuda") * 0.01
+    dt = ops.BF16 if kind == "bf16" else ops.INT8_WO
+    work = ops.gemm_workspace(m, n, k, dt, x.device)
+    nw = 0 if work is None else work.numel()
+    for odt in (torch.bfloat16, torch.float32):
+        for off in (1, 2, 4):
+            want = ops.gemm(x, w, None, ws, out_dtype=odt, split_k=1 if kind == "bf16" and m <= 128 and off < 4 else 0)
+            buf = torch.full((m * n + 16,), 7.0, dtype=odt, device="cuda")
+            ops.gemm(x, w, None, ws, out=buf[off:off + m * n].view(m, n), workspace=work)
+            assert torch.equal(buf[off:off + m * n].view(m, n), want)
+            assert (buf[:off] == 7).all() and (buf[off + m * n:] == 7).all()
+    for off in (1, 2, 4):
+        act, amax = ops.gemm_silu_mul(x, w, None, ws, split_k=1 if kind == "bf16" and m <= 128 and off < 4 else 0)
+        buf, am = torch.full((m * n // 2 + 16,), 7.0, dtype=torch.bfloat16, device="cuda"), torch.empty_like(amax)
+        out = buf[off:off + m * n // 2]
+        assert _cabi.load().b200_gemm_silu_mul(x.data_ptr(), w.data_ptr(), out.data_ptr(), 0, 0 if ws is None else ws.data_ptr(), 0, am.data_ptr(),
+                                               m, n, k, dt, 0, 0 if work is None else work.data_ptr(), nw, ops._stream()) == 0
+        assert torch.equal(out.view(m, -1), act) and torch.equal(am, amax)
+        assert (buf[:off] == 7).all() and (buf[off + m * n // 2:] == 7).all()
+
+
 @pytest.mark.parametrize("m,n,k,cut", [(129, 5120, 27648, True), (300, 1024, 28672, True), (640, 2048, 5632, False), (129, 4096, 14336, False)])
 def test_gemm_prompt_schedule(ops, m, n, k, cut):
     """Short prompts against a long K go to the schedule that cuts K over all SMs, the others to the pairs, which do not: the same bits as a

@@ -1282,6 +1282,9 @@ int gemm_common(const void* a, const void* w, const GemmEpilogue& ep, int epi, i
     set_last_error("gemm: workspace %zu < %zu bytes", workspace_bytes, p.ws_bytes);
     return B200_ERR_WORKSPACE;
   }
+  // the cut decode schedule writes vectors of four: an output that is not aligned to them keeps the uncut one, which writes single values
+  const uintptr_t vec_bytes = ep.out_f32 ? 16 : 8;
+  if (p.decode && epi != EPI_ROPE && ((uintptr_t)ep.out & (vec_bytes - 1)) && !(wo && split_k == 0)) split_k = 1;
   // decode-sized batches of the weight-only kind: 256 weight rows per CTA (calls that name their K splits keep the 128-row schedule)
   if (p.decode && wo && split_k == 0 && epi != EPI_ROPE) return launch_gemm_wo(a, w, ep, epi, M, N, K, (cudaStream_t)stream);
   // prompt-sized batches run on CTA pairs; stream-K keeps the shapes where cutting K is faster, the weight-only kind, whose tiles are widened

@@ -298,8 +298,13 @@ __global__ void __launch_bounds__(WOX_THREADS, 1)
         x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
         if (ok && is_gate) {
           const int ch = (n0 >> 5) * 16 + (lane & 3) * 4;
-          *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(ep.out) + (int64_t)m * I + ch) =
-              make_uint2(pack_bf16(act[0], act[1]), pack_bf16(act[2], act[3]));
+          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(ep.out) + (int64_t)m * I + ch;
+          if ((reinterpret_cast<uintptr_t>(ep.out) & 7) == 0) {
+            *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(act[0], act[1]), pack_bf16(act[2], act[3]));
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dst[e] = __float2bfloat16_rn(act[e]);
+          }
           if ((lane & 7) == 0) ep.group_amax[(int64_t)m * n_groups + (n0 >> 5)] = x;
         }
       }
