@@ -449,6 +449,29 @@ def test_ssd_scan_keeps_to_its_scratch(entry):
     assert torch.equal(y, want) == (entry == "b200_ssd_scan_mma")
 
 
+def test_ssd_scan_writes_outputs_on_any_boundary():
+    """Outputs that start one float after a 16-byte boundary: those of the wrapper's aligned ones, and nothing beside them."""
+    from vllm_neuron_b200 import _cabi
+    from vllm_neuron_b200.hybrid import StepMeta
+
+    ops = _ops()
+    H, P, N, G, T = 2, 64, 64, 1, 300
+    g = torch.Generator().manual_seed(6)
+    C = H * P + 2 * G * N
+    xbc = torch.nn.functional.silu(torch.randn(T, C, generator=g)).bfloat16().to(DEV)
+    raw, a_log, bias, D = (torch.randn(*s, generator=g).to(DEV) for s in ((T, H), (H,), (H,), (H,)))
+    meta = StepMeta.build([(0, 0, T)], {0: list(range(1, 11))}, 32, torch.device(DEV))
+    states = torch.zeros(2, 1, H, P, N, device=DEV)
+    want = ops.ssd_scan(xbc, raw, 0, a_log, bias, D, states[0], meta, H, P, N, G)
+    scratch, dts, buf = torch.empty(meta.num_segs, H, P, N, device=DEV), torch.empty(meta.num_segs, H, device=DEV), torch.full((T * H * P + 2,), 7.0, device=DEV)
+    assert _cabi.load().b200_ssd_scan_mma(xbc.data_ptr(), ops.BF16, C, raw.data_ptr(), H, 0, a_log.data_ptr(), bias.data_ptr(), D.data_ptr(),
+                                          states[1].data_ptr(), meta.seq_start.data_ptr(), meta.seq_slot.data_ptr(), meta.seq_pos0.data_ptr(),
+                                          buf[1:].data_ptr(), 1, H, P, N, G, meta.scan_segs.data_ptr(), meta.num_segs,
+                                          meta.scan_seq_seg0.data_ptr(), scratch.data_ptr(), dts.data_ptr(), ops._stream()) == 0
+    y = buf[1:-1].view(T, H * P)
+    assert (y - want).norm() <= 1e-6 * want.norm() and (states[1] - states[0]).norm() <= 1e-6 * states[0].norm() and buf[0] == 7 and buf[-1] == 7
+
+
 @pytest.mark.parametrize("counts", [(300, 0, 129, 128, 1), (3, 40, 0, 32, 33), (0, 0, 0, 0, 7)])
 @pytest.mark.parametrize("wide", [False, True])
 @pytest.mark.parametrize("act", ["clamped", "silu"])

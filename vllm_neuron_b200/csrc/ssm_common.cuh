@@ -12,7 +12,7 @@ constexpr int SEG_SHORT = 32;
 __device__ __forceinline__ bool seg_is_short(int4 sd) { return (sd.w & (SEG_FIRST | SEG_LAST)) == (SEG_FIRST | SEG_LAST) && sd.y - sd.x <= SEG_SHORT; }
 
 // whether the matrix form takes these operands
-bool ssd_segments_ok(const void* xbc, int x_dtype, int C, const float* state, int P, int N, const float* seg_state);
+bool ssd_segments_ok(const void* xbc, int x_dtype, int C, const float* state, int P, int N, const float* seg_state, const float* y);
 // every segment's own state (from zero) and summed step size -> scratch; then, once the scratch holds the start states
 // (ssd_seg_combine_kernel), outputs and the slots' new states
 int ssd_segment_states(const void* xbc, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log, const float* dt_bias, int H,

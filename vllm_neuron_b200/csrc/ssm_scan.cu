@@ -371,7 +371,7 @@ static int launch_scan(const void* xbc, int C, const float* dt_in, int ld_dt, in
   dim3 grid((P + PC - 1) / PC, H, segs ? num_segs : B);
   const size_t smem = (size_t)(SCAN_CHUNK * (2 * NPT * SCAN_SLICES + PC + 2)) * sizeof(float);
   const int4* sd = reinterpret_cast<const int4*>(segs);
-  const bool matrix = segs && mma && ssd_segments_ok(xbc, sizeof(XT) == 2 ? B200_BF16 : B200_F32, C, state, P, N, seg_state);
+  const bool matrix = segs && mma && ssd_segments_ok(xbc, sizeof(XT) == 2 ? B200_BF16 : B200_F32, C, state, P, N, seg_state, y);
   if (matrix) {
     const int rc = ssd_segment_states(xbc, C, dt_in, ld_dt, dt_col0, A_log, dt_bias, H, P, N, G, segs, num_segs, seq_seg0, seg_state, seg_dtsum,
                                       stream);

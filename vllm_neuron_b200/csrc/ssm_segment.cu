@@ -416,9 +416,9 @@ int launch_out(const __nv_bfloat16* xbc, int C, const float* dt_in, int ld_dt, i
 
 }  // namespace
 
-bool ssd_segments_ok(const void* xbc, int x_dtype, int C, const float* state, int P, int N, const float* seg_state) {
+bool ssd_segments_ok(const void* xbc, int x_dtype, int C, const float* state, int P, int N, const float* seg_state, const float* y) {
   return x_dtype == B200_BF16 && (P == 64 || P == 128) && (N == 64 || N == 128) && C % 8 == 0 && !((uintptr_t)xbc & 15) &&
-         !((uintptr_t)state & 15) && !((uintptr_t)seg_state & 15);
+         !((uintptr_t)state & 15) && !((uintptr_t)seg_state & 15) && !((uintptr_t)y & 7);
 }
 
 #define SEG_SIZES(CALL)                                  \
