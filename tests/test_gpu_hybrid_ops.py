@@ -502,6 +502,19 @@ def test_moe_experts_on_pairs(counts, wide, act):
         assert (got[rows] - want).norm() <= 1e-2 * want.norm() + 1e-9, e
 
 
+def test_moe_experts_on_rows_off_a_16_byte_boundary():
+    """Token rows whose pitch suits the pair kernel but whose first element does not lie on 16 bytes: the experts of the aligned rows."""
+    ops = _ops()
+    E, W, ff, T = 4, 512, 256, 40
+    g = torch.Generator().manual_seed(9)
+    buf = torch.randn(T, W + 8, generator=g).bfloat16().to(DEV)
+    h = buf[:, 1:W + 1]
+    idx, wt = torch.randint(0, E, (T, 1), generator=g).to(torch.int32).to(DEV), torch.rand(T, 1, generator=g).to(DEV)
+    gu, dn = (torch.randn(E, 2 * ff, W, generator=g) * W**-0.5).bfloat16().to(DEV), (torch.randn(E, W, ff, generator=g) * ff**-0.5).bfloat16().to(DEV)
+    got, want = (ops.moe_experts(x, wt, ops.moe_align(idx, E), gu, dn, 1, 7.0) for x in (h, h.contiguous()))
+    assert (got - want).norm() <= 1e-2 * want.norm()  # the hidden activations' rounding to bf16
+
+
 @pytest.mark.parametrize("T,W", [(1, 4), (3, 1028), (2, 4096), (5, 4100), (700, 132), (4, 30)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_row_kernels_in_vectors(T, W, dtype):

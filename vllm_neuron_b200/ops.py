@@ -969,7 +969,7 @@ def moe_experts(h, topk_weight, align, w_gate_up, w_down, top: int, limit: float
     out = torch.empty((h.shape[0] * top, width), dtype=torch.float32, device=h.device)
     lib = _cabi.load()
     # prompt-sized batches, and experts of whole pair-kernel tiles at any size: gather and scale the pairs once, then plain rows
-    pair_tiles = h.dtype == torch.bfloat16 and width % 256 == 0 and ff % 128 == 0 and tiles <= 1024 and h.stride(0) % 8 == 0
+    pair_tiles = h.dtype == torch.bfloat16 and width % 256 == 0 and ff % 128 == 0 and tiles <= 1024 and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0
     if bm > moe_tile_rows() or pair_tiles:
         rows = torch.empty((sorted_ids.numel(), width), dtype=h.dtype, device=h.device)
         with _k("moe_gather_scale"):
