@@ -515,6 +515,22 @@ def test_moe_experts_on_rows_off_a_16_byte_boundary():
     assert (got - want).norm() <= 1e-2 * want.norm()  # the hidden activations' rounding to bf16
 
 
+@pytest.mark.parametrize("rows,tiles", [(0, 1), (33, 1), (40, 2)])
+def test_fp32_linear_writes_the_tiles_it_is_asked_for(rows, tiles):
+    """Dense rows of the C entry: row_tiles tiles of 32 rows or all M rows, whichever is less; none is none."""
+    from vllm_neuron_b200 import _cabi
+
+    ops = _ops()
+    N, K = 40, 64
+    g = torch.Generator().manual_seed(rows)
+    a, w, out = torch.randn(64, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV), torch.full((64, N), 7.0, device=DEV)
+    assert _cabi.load().b200_grouped_linear(a.data_ptr(), K, 0, 0, 0, w.data_ptr(), 0, 0, 0, tiles, rows, N, K, ops.F32, out.data_ptr(), N, 0, 0, 0,
+                                            0.0, ops.moe_tile_rows(), ops._stream()) == 0
+    n = min(rows, 32 * tiles)
+    want = a.double() @ w.double().T
+    assert ((out[:n].double() - want[:n]).abs() <= K * 2.0**-24 * (a.abs().double() @ w.abs().double().T)[:n]).all() and (out[n:] == 7).all()
+
+
 @pytest.mark.parametrize("T,W", [(1, 4), (3, 1028), (2, 4096), (5, 4100), (700, 132), (4, 30)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_row_kernels_in_vectors(T, W, dtype):

@@ -948,6 +948,9 @@ int b200_grouped_linear(const void* a, int lda, const int32_t* sorted_ids, int g
     return B200_OK;
   }
   if (dtype == B200_F32 && fp32_rows_ok(a, lda, 0, w, w_expert_stride, K)) {
+    const long long rows = (long long)row_tiles * tile_rows;
+    if (rows < M) M = (int)rows;
+    if (!sorted_ids && M <= 0) return B200_OK;
     if (!sorted_ids && !glu) return dense_fp32_linear(1, a, lda, w, 0, M, N, K, out, ldo, 0, 0, no_gate, 0, 0, st);
     if (glu)
       return launch_fp32_linear<MOE_BM, 64, 8, 4, 4, GL_EPI_GLU>(row_tiles, 1, a, lda, sorted_ids, gather_div, row_scale, w, w_expert_stride,
