@@ -531,6 +531,54 @@ def test_fp32_linear_writes_the_tiles_it_is_asked_for(rows, tiles):
     assert ((out[:n].double() - want[:n]).abs() <= K * 2.0**-24 * (a.abs().double() @ w.abs().double().T)[:n]).all() and (out[n:] == 7).all()
 
 
+@pytest.mark.parametrize("kind", ["full", "window-sink", "chunk", "softcap", "keep", "pooled", "latent", "maps", "sigmoid", "fp32-out"])
+def test_attention_of_mixed_steps_apart_and_together(kind, monkeypatch):
+    """Prompt portions (one continued, one after decoded tokens) beside decoded ones, through every attention variant in one launch and in
+    one per kind: the prompts' rows bit for bit, the decoded ones up to the two kernels' bf16 roundings (weights and outputs, 2^-8 each)."""
+    from vllm_neuron_b200.hybrid import StepMeta
+
+    ops = _ops()
+    entries = [(0, 0, 140), (1, 200, 1), (2, 77, 3), (3, 500, 1), (4, 60, 40)]
+    H, G, D, Dv, bs, win = 8, 2, 64, 64, 32, 1 << 30
+    kw, sink, latent = {}, None, 0
+    g = torch.Generator(device=DEV).manual_seed(3)
+    r = lambda *s: torch.randn(s, generator=g, device=DEV)  # noqa: E731
+    rows = {e[0]: list(range(1 + 20 * e[0], 21 + 20 * e[0])) for e in entries}
+    if kind in ("window-sink", "keep", "pooled"):
+        win = 96
+    if kind == "window-sink":
+        sink = r(H)
+    if kind == "latent":
+        G, D, latent = 1, 192, 128
+    k_pool = r(101, G, bs, D).bfloat16()
+    v_pool = k_pool if latent else r(101, G // 2 if kind == "maps" else G, bs, Dv).bfloat16()
+    if kind == "chunk":
+        kw["chunk"] = 128
+    elif kind == "softcap":
+        kw["softcap"] = 20.0
+    elif kind == "keep":
+        kw["keep"] = 4
+    elif kind == "pooled":
+        kw["pooled"] = (r(101, G, 2, D).bfloat16(), r(101, G, 2, Dv).bfloat16(), 16)
+    elif kind == "sigmoid":
+        kw["sigmoid_bias"] = r(H)
+    elif kind == "fp32-out":
+        kw["out_f32"] = True
+    meta = StepMeta.build(entries, rows, bs, torch.device(DEV))
+    assert len(meta.parts) == 3
+    table = torch.tensor([rows[i] for i in range(5)], dtype=torch.int32, device=DEV)
+    q = r(meta.num_tokens, H * D)
+    outs = []
+    for apart in (False, True):
+        monkeypatch.setattr(ops, "_split_pays", lambda *a, apart=apart: apart)
+        outs.append(ops.swa_sink_attn(q, H, k_pool, v_pool, table, meta, sink, D**-0.5, win, latent, **kw).float())
+    short = torch.zeros(meta.num_tokens, dtype=torch.bool, device=DEV)
+    short[140:145] = True
+    assert (outs[0][short] - outs[1][short]).norm() <= 2.0**-7 * outs[0][short].norm()
+    # the 40 tokens of the last portion may meet another prompt kernel than the step's longest portion does
+    assert torch.equal(outs[0][:140], outs[1][:140]) and (outs[0][145:] - outs[1][145:]).norm() <= 2.0**-7 * outs[0][145:].norm()
+
+
 @pytest.mark.parametrize("T,W", [(1, 4), (3, 1028), (2, 4096), (5, 4100), (700, 132), (4, 30)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_row_kernels_in_vectors(T, W, dtype):

@@ -157,3 +157,20 @@ def test_step_parts_keep_prompt_portions_and_decoded_tokens_apart():
     assert StepMeta.build(entries[:1], rows, 32, "cpu").parts is None
     often = [(i, 0, 40 if i % 2 else 1) for i in range(MAX_STEP_PARTS + 1)]
     assert StepMeta.build(often, rows, 32, "cpu").parts is None
+
+
+def test_step_parts_are_split_only_where_the_decoded_tokens_are_worth_a_launch():
+    """Apart where many tokens walk long contexts, or one of them more than the prompts beside it; together where the prompts hide them."""
+    from vllm_neuron_b200 import ops
+    from vllm_neuron_b200.hybrid import StepMeta
+
+    def pays(prompts, tokens, ctx, h, g, d, dv, window=1 << 30, latent=False, tc=False):
+        entries = [(i, 0, p) for i, p in enumerate(prompts)] + [(len(prompts) + i, ctx, 1) for i in range(tokens)]
+        m = StepMeta.build(entries, {e[0]: list(range(1, 201)) for e in entries}, 32, "cpu")
+        return ops._split_pays(m.parts, h, g, d, dv, latent, tc, [ops._span(p.max_end, window, 0, 0, 0) for p in m.parts])
+
+    assert pays((1600,), 29, 1800, 16, 1, 320, 256, latent=True) and not pays((3000,), 29, 300, 16, 1, 320, 256, latent=True)
+    assert pays((1600,), 29, 1800, 16, 4, 128, 128, 512) and not pays((1600,), 4, 1800, 16, 4, 128, 128, 512)
+    assert pays((1600,), 60, 1800, 16, 4, 128, 128, tc=True) and not pays((1600,), 4, 300, 16, 4, 128, 128, tc=True)
+    assert pays((200,), 1, 1800, 12, 4, 80, 80) and not pays((200,), 1, 300, 12, 4, 80, 80)
+    assert ops._span(900, 256, 0, 32, 4) == 256 + 644 // 32 + 4 and ops._span(900, 1 << 30, 128, 0, 0) == 128

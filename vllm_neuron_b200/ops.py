@@ -738,6 +738,39 @@ PREFILL_TC_MIN_TOKENS = 128   # ... and from which the tcgen05 kernel with its 1
 _SWA_PREFILL_LEGACY = bool(os.environ.get("B200_SWA_PREFILL_LEGACY"))
 
 
+def _span(max_end: int, window: int, chunk: int, pool: int, keep: int) -> int:
+    """Keys that a query sees at most in a step whose sequences reach max_end tokens (the pooled blocks before its window count as keys)."""
+    return min(max_end, window, chunk or 1 << 30) + (max(max_end - window, 0) // pool if pool else 0) + keep
+
+
+def _split_pays(parts, num_heads: int, g: int, d: int, dv: int, latent: bool, tc: bool, spans) -> bool:
+    """Whether the decoded tokens of a mixed step are worth launches of their own.  spans: per part, the keys its queries see at most.
+    In the prompt kernel each of them is a row tile per head (the tcgen05 kernel: per two heads) that walks its keys behind the prompts' own
+    tiles; apart they cost a launch behind the prompts', 14 us, and the decode kernel's time.  The estimate of the first is a list of tiles
+    over the chip's slots: `us` per key and 5 per tile, the last tile's walk on top where there are more tiles than slots, a fifth for
+    sharing the SMs.  Measured, apart / together, us, 16 heads: prompts of 1600, over latents 29 tokens at 1800 366 / 695, 2 356 / 360, 29 at
+    300 317 / 298; window of 512 with sinks, 29 at 1800 111 / 144, 4 97 / 78; full context on tcgen05, 29 at 1800 133 / 143, 4 78 / 56,
+    4 at 300 64 / 46; a prompt of 200 beside one token at 1800, window of 512 43 / 51, 12 heads of 80 45 / 132, at 300 35 / 28.  Over 300 such
+    steps the rule's choice costs 1.6 % more than the better one on average, always apart 8 %, always together 29 %."""
+    us, rows, heads, slots = (0.026, 128, g * -(-num_heads // (2 * g)), 148) if tc else \
+        (0.045 + 0.00014 * (d + dv), 64, num_heads, 148 * (4 if dv <= 128 else 2))
+    n, keys, tiles, work, walk = 0, 0, 0, 0.0, 0.0
+    for p, span in zip(parts, spans):
+        if p.max_new < PREFILL_ATTN_MIN_TOKENS:
+            n, keys = n + p.num_tokens, max(keys, span)
+        else:
+            t = (-(-p.num_tokens // rows) + p.num_seqs - 1) * heads
+            tiles, work, walk = tiles + t, work + t * (5 + us * min(span, p.max_end - p.max_new / 2)), max(walk, 5 + us * span)
+    last = 5 + us * keys
+
+    def makespan(tiles, work):
+        return max(walk, last, work / slots + last * max(0.0, 1 - slots / tiles))
+
+    alone = max(walk, work / slots + walk * max(0.0, 1 - slots / tiles))
+    decode = 0.035 * keys * max(1.0, n / 32) if latent else keys * (n * g / 4000 + 0.008)
+    return 1.2 * makespan(tiles + n * heads, work + n * heads * last) > alone + 14 * (len(parts) - 1) + decode
+
+
 def swa_sink_attn(q_src, num_heads: int, k_pool, v_pool, block_table, meta, sink, scale: float, window: int,
                   latent_values: int = 0, *, chunk: int = 0, softcap: float = 0.0, sigmoid_bias=None, out_f32: bool = False,
                   split_p: bool = False, pooled=None, keep: int = 0):
@@ -774,12 +807,32 @@ def swa_sink_attn(q_src, num_heads: int, k_pool, v_pool, block_table, meta, sink
     v_div = g // v_pool.shape[1]
     assert v_pool.shape[1] * v_div == g and v_pool.shape[2] == bs
     out = torch.empty((q_src.shape[0], num_heads * dv), dtype=torch.float32 if out_f32 else k_pool.dtype, device=q_src.device)
-    # decoded tokens beside prompt portions: each kind runs on its own kernel.  A prompt kernel would give every one of them a row tile of
-    # its own, 64 or 128 rows for a single one (29 decoded tokens at 1 800 positions beside 1 607 prompt tokens, 16 heads over latents: 497 -> 285 us)
-    for part in (getattr(meta, "parts", None) or [meta]) if k_pool.dtype == torch.bfloat16 else [meta]:
+    # decoded tokens beside prompt portions: each kind on its own kernel where that pays, in one launch of the prompt kernel otherwise
+    parts = getattr(meta, "parts", None)
+    if parts:
+        tc = _prompt_tc(q_src, k_pool, meta, sink, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool)
+        spans = [_span(p.max_end, int(window), int(chunk), pool, int(keep)) for p in parts]
+        if not (tc or _prompt_mma(q_src, k_pool, meta, d, dv)) or not _split_pays(parts, num_heads, g, d, dv, bool(latent_values), tc, spans):
+            parts = None
+    for part in parts or [meta]:
         _swa_part(q_src, num_heads, k_pool, v_pool, block_table, part, sink, scale, window, latent_values, chunk, softcap, sigmoid_bias,
                   out_f32, split_p, pool, pool_args, keep, out, g, bs, d, dv, v_pitch, v_div)
     return out
+
+
+def _prompt_tc(q, k_pool, meta, sink, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool) -> bool:
+    """Long prompt portions in bf16 serving (a sliding window only without pooled blocks), head sizes of 64 / 128 with pages of 32 tokens: the
+    tcgen05 kernel (128-row query tiles, accumulators in tensor memory); B200_SWA_PREFILL_LEGACY=1 keeps the mma.sync kernel (A/B aid)."""
+    return bool(k_pool.dtype == torch.bfloat16 and meta.max_new >= PREFILL_TC_MIN_TOKENS and sink is None and not pool
+                and not latent_values and q.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0 and not _SWA_PREFILL_LEGACY
+                and _cabi.load().b200_swa_sink_attn_prefill_tc_supported(d, dv, bs, v_div, 1 if softcap else 0,
+                                                                         0 if sigmoid_bias is None else 1))
+
+
+def _prompt_mma(q, k_pool, meta, d, dv) -> bool:
+    """Shorter prompt portions in bf16 serving: the mma.sync kernel."""
+    return (k_pool.dtype == torch.bfloat16 and meta.max_new >= PREFILL_ATTN_MIN_TOKENS and d % 16 == 0 and dv % 16 == 0
+            and d <= 512 and dv <= 256 and q.stride(0) % 2 == 0)
 
 
 def _swa_part(q_src, num_heads, k_pool, v_pool, block_table, meta, sink, scale, window, latent_values, chunk, softcap, sigmoid_bias, out_f32,
@@ -795,12 +848,7 @@ def _swa_part(q_src, num_heads, k_pool, v_pool, block_table, meta, sink, scale, 
     # the per-launch timer tells the variants apart (their floors differ)
     tag = "[latent]" if plain and latent_values else "" if plain and not pool and not keep else "[" + "+".join(n for n, on in (("chunk", chunk), ("cap", softcap), ("sigmoid", sigmoid_bias is not None),
                                                                        ("maps", v_div > 1), ("pool", pool), ("keep", keep)) if on) + "]"
-    # long prompt portions in bf16 serving (a sliding window only without pooled blocks), head sizes of 64 / 128 with pages of 32 tokens: the tcgen05 kernel (128-row query
-    # tiles, accumulators in tensor memory); B200_SWA_PREFILL_LEGACY=1 keeps the mma.sync kernel (A/B aid)
-    if (k_pool.dtype == torch.bfloat16 and meta.max_new >= PREFILL_TC_MIN_TOKENS and sink is None and not pool
-            and not latent_values and q_all.stride(0) % 4 == 0 and q_all.data_ptr() % 16 == 0 and not _SWA_PREFILL_LEGACY
-            and _cabi.load().b200_swa_sink_attn_prefill_tc_supported(d, dv, bs, v_div, 1 if softcap else 0,
-                                                                     0 if sigmoid_bias is None else 1)):
+    if _prompt_tc(q_all, k_pool, meta, sink, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool):
         with _k("swa_sink_attn_prefill_tc" + tag):
             check(_cabi.load().b200_swa_sink_attn_prefill_tc(_ptr(q_all), q_all.stride(0), _ptr(k_pool), _ptr(v_pool), k_pool.shape[0],
                                                              _ptr(block_table), block_table.stride(0), _ptr(meta.seq_start),
@@ -810,10 +858,7 @@ def _swa_part(q_src, num_heads, k_pool, v_pool, block_table, meta, sink, scale, 
                                                              int(keep), _stream()),
                   "b200_swa_sink_attn_prefill_tc")
         return
-    # shorter prompt portions in bf16 serving: the mma.sync kernel; decode-sized steps, fp32 pools and odd head sizes: one CTA
-    # per (token, head) on the CUDA cores
-    if (k_pool.dtype == torch.bfloat16 and meta.max_new >= PREFILL_ATTN_MIN_TOKENS and d % 16 == 0 and dv % 16 == 0
-            and d <= 512 and dv <= 256 and q_all.stride(0) % 2 == 0):
+    if _prompt_mma(q_all, k_pool, meta, d, dv):
         with _k("swa_sink_attn_prefill" + tag):
             check(_cabi.load().b200_swa_sink_attn_prefill(_ptr(q_all), q_all.stride(0), _ptr(k_pool), _ptr(v_pool), _ptr(block_table),
                                                           block_table.stride(0), _ptr(meta.seq_start), _ptr(meta.seq_slot),
@@ -831,11 +876,9 @@ def _swa_part(q_src, num_heads, k_pool, v_pool, block_table, meta, sink, scale, 
                                                        float(scale), int(window), _ptr(out), t, num_heads, d, dv, bs, _stream()),
                   "b200_latent_attn_decode")
         return
-    # long contexts at small batch: several CTAs share a (token, kv head)'s keys, so that every SM has its CTAs
-    span = min(getattr(meta, "max_end", 0) or 0, int(window), int(chunk) if chunk else 1 << 30)
-    if pool:  # the blocks before the window count as keys too
-        span += max((getattr(meta, "max_end", 0) or 0) - int(window), 0) // pool
-    span += int(keep)
+    # decode-sized steps, fp32 pools and odd head sizes.  Long contexts at small batch: several CTAs share a (token, kv head)'s keys, so that
+    # every SM has its CTAs
+    span = _span(getattr(meta, "max_end", 0) or 0, int(window), int(chunk), pool, int(keep))
     tc = (k_pool.dtype == torch.bfloat16 and not latent_values and d % 16 == 0 and dv % 16 == 0 and d * v_div <= 512 and dv <= 256
           and q_src.stride(0) % 2 == 0)
     gv = g // v_div
