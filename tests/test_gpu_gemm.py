@@ -164,7 +164,7 @@ def test_gemm_pairs_silu_residual_bias(ops, m, n, k):
 @pytest.mark.parametrize("m,n,k", [(33, 640, 1152), (64, 4096, 2048), (300, 1056, 640)])
 def test_gemm_outputs_on_any_boundary(ops, kind, m, n, k):
     """Outputs that start one, two or four elements after a 16-byte boundary: the bits of the aligned call on the schedule that they take
-    (decode batches in bf16: the one that does not cut K, where vectors of four would not lie on their size), nothing written around them."""
+    (decode batches in bf16 and narrow weight-only ones: the one that does not cut K, where vectors of four would not lie on their size), nothing written around them."""
     from vllm_neuron_b200 import _cabi
 
     g = torch.Generator(device="cuda").manual_seed(n)
@@ -174,15 +174,16 @@ def test_gemm_outputs_on_any_boundary(ops, kind, m, n, k):
     dt = ops.BF16 if kind == "bf16" else ops.INT8_WO
     work = ops.gemm_workspace(m, n, k, dt, x.device)
     nw = 0 if work is None else work.numel()
+    single = m <= 128 and (kind == "bf16" or n < 2048)  # decode schedules that write vectors where K is cut
     for odt in (torch.bfloat16, torch.float32):
         for off in (1, 2, 4):
-            want = ops.gemm(x, w, None, ws, out_dtype=odt, split_k=1 if kind == "bf16" and m <= 128 and off < 4 else 0)
+            want = ops.gemm(x, w, None, ws, out_dtype=odt, split_k=1 if single and off < 4 else 0)
             buf = torch.full((m * n + 16,), 7.0, dtype=odt, device="cuda")
             ops.gemm(x, w, None, ws, out=buf[off:off + m * n].view(m, n), workspace=work)
             assert torch.equal(buf[off:off + m * n].view(m, n), want)
             assert (buf[:off] == 7).all() and (buf[off + m * n:] == 7).all()
     for off in (1, 2, 4):
-        act, amax = ops.gemm_silu_mul(x, w, None, ws, split_k=1 if kind == "bf16" and m <= 128 and off < 4 else 0)
+        act, amax = ops.gemm_silu_mul(x, w, None, ws, split_k=1 if single and off < 4 else 0)
         buf, am = torch.full((m * n // 2 + 16,), 7.0, dtype=torch.bfloat16, device="cuda"), torch.empty_like(amax)
         out = buf[off:off + m * n // 2]
         assert _cabi.load().b200_gemm_silu_mul(x.data_ptr(), w.data_ptr(), out.data_ptr(), 0, 0 if ws is None else ws.data_ptr(), 0, am.data_ptr(),
@@ -202,10 +203,11 @@ def test_gemm_prompt_schedule(ops, m, n, k, cut):
     assert torch.equal(got, ops.gemm(x, w, out_dtype=torch.float32, split_k=sms)) == cut
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 1056, 512), (31, 256, 144), (33, 640, 1152), (64, 992, 256), (65, 256, 128), (128, 1000, 144), (100, 640, 1152), (127, 32, 64), (128, 38144, 256), (96, 5120, 2048)])
+@pytest.mark.parametrize("m,n,k", [(1, 1056, 512), (31, 256, 144), (33, 640, 1152), (64, 992, 256), (65, 256, 128), (128, 1000, 144), (100, 640, 1152), (127, 32, 64), (128, 38144, 256), (96, 5120, 2048),
+                                   (1, 3104, 512), (31, 3072, 144), (33, 3220, 1152), (64, 4064, 256), (65, 3328, 128), (128, 4072, 144), (127, 3072, 64), (100, 3104, 1152)])
 def test_gemm_weight_only_256_rows(ops, m, n, k):
-    """256-row schedule of decode-sized weight-only batches: ragged rows, k and tokens, uncut tiles beside cut ones (38144 = 149 tiles), every
-    epilogue operand.  bf16 operands are exact on both sides: fp32 sums in another order, one bf16 rounding."""
+    """Decode-sized weight-only batches: ragged rows, k and tokens, every epilogue operand; narrow weights on the 128-row schedule, from 3072
+    rows on the one of 256.  bf16 operands are exact on both sides: fp32 sums in another order, one bf16 rounding."""
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
     r = lambda *s: torch.randn(s, generator=g, device="cuda").bfloat16()  # noqa: E731
     x, bias, res, ws = r(m, k), r(n), r(m, n), torch.rand(n, generator=g, device="cuda") * 0.02
@@ -219,6 +221,43 @@ def test_gemm_weight_only_256_rows(ops, m, n, k):
         want = torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]
         _assert_close(a, want.reshape(m, -1).cpu())
         assert torch.equal(amax, a.float().abs().view(m, -1, 16).amax(-1))
+
+
+@pytest.mark.parametrize("m,n,k,launches", [(128, 38144, 1024, 2), (100, 38100, 1040, 2), (128, 38144, 256, 1), (64, 7168, 5120, 1)])
+def test_gemm_weight_only_whole_waves_and_a_cut_rest(ops, m, n, k, launches):
+    """More tiles than whole waves hold, K long enough: uncut tiles in one launch, the rest cut along K over a cluster in a second (a ragged
+    last tile in one case).  Both epilogues against 64 bits, fp32 sums up to 2e-6 of the sum of magnitudes."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn((m, k), generator=g, device="cuda").bfloat16()
+    wq, ws = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int8), torch.rand(n, generator=g, device="cuda") * 0.02
+    ops.gemm(x, wq, None, ws)
+    before = ops.launch_count()
+    got = ops.gemm(x, wq, None, ws, out_dtype=torch.float32)
+    assert ops.launch_count() - before == launches
+    ref = torch.cat([x.double() @ w.double().T for w in wq.split(8192)], 1) * ws.double()
+    size = torch.cat([x.double().abs() @ w.double().abs().T for w in wq.split(8192)], 1) * ws.double()
+    assert ((got.double() - ref).abs() <= 2e-6 * size).all()
+    if n % 32 == 0:
+        a, amax = ops.gemm_silu_mul(x, wq, None, ws)
+        z = ref.bfloat16().double().view(m, -1, 2, 16)
+        want = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(m, -1)
+        _assert_close(a, want.cpu())
+        assert torch.equal(amax, a.float().abs().view(m, -1, 16).amax(-1))
+
+
+@pytest.mark.parametrize("n,k,wide", [(1024, 2048, False), (896, 4864, False), (4096, 2048, True), (7168, 5120, True)])
+def test_gemm_weight_only_plan_is_the_one_that_runs(ops, n, k, wide):
+    """Narrow weights keep the 128-row schedule: a call without K splits gives the bits of the one that names the plan's; wide ones leave it."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.randn((48, k), generator=g, device="cuda").bfloat16()
+    wq = torch.randint(-127, 128, (n, k), generator=g, device="cuda", dtype=torch.int8)
+    ws = torch.rand(n, generator=g, device="cuda")
+    plan = ops.gemm_decode_plan(48, n, k, ops.INT8_WO)
+    got = ops.gemm(x, wq, None, ws, out_dtype=torch.float32)
+    if wide:
+        assert plan["ctas_per_sm"] == 1 and 1 <= plan["split"] <= 8 and plan["w_stages"] == 4
+    else:
+        assert torch.equal(got, ops.gemm(x, wq, None, ws, out_dtype=torch.float32, split_k=plan["split"]))
 
 
 @pytest.mark.parametrize("m,n,k", [(128, 55296, 5120), (100, 5120, 27648), (65, 7168, 5120), (64, 5120, 27648), (17, 5120, 13824)])

@@ -190,6 +190,9 @@ __device__ __forceinline__ void epilogue_chunk_xpose(const GemmEpilogue& ep, con
 }
 
 // Weight-only schedule of decode-sized batches (gemm_wo.cu).
+// gemm_wo_wide: whether it takes a call that names no K splits.  gemm_wo_plan: its K splits and the CTAs that clusters of them hold at once.
+bool gemm_wo_wide(int epi, int M, int N, int K);
+int gemm_wo_plan(int epi, int M, int N, int K, int& splits, int& cap_ctas, int& stages, size_t& smem);
 int launch_gemm_wo(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, cudaStream_t stream);
 // Prompt-sized schedule on CTA pairs (gemm_pair.cu): bf16, fp8 and int8 operands.  pair_tokens: tokens of a tile for this shape, 0 where
 // stream-K is the faster schedule.

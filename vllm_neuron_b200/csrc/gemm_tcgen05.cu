@@ -1283,10 +1283,12 @@ int gemm_common(const void* a, const void* w, const GemmEpilogue& ep, int epi, i
     return B200_ERR_WORKSPACE;
   }
   // the cut decode schedule writes vectors of four: an output that is not aligned to them keeps the uncut one, which writes single values
+  const bool wide = p.decode && wo && split_k == 0 && epi != EPI_ROPE && gemm_wo_wide(epi, M, N, K);
   const uintptr_t vec_bytes = ep.out_f32 ? 16 : 8;
-  if (p.decode && epi != EPI_ROPE && ((uintptr_t)ep.out & (vec_bytes - 1)) && !(wo && split_k == 0)) split_k = 1;
-  // decode-sized batches of the weight-only kind: 256 weight rows per CTA (calls that name their K splits keep the 128-row schedule)
-  if (p.decode && wo && split_k == 0 && epi != EPI_ROPE) return launch_gemm_wo(a, w, ep, epi, M, N, K, (cudaStream_t)stream);
+  if (p.decode && !wide && epi != EPI_ROPE && ((uintptr_t)ep.out & (vec_bytes - 1))) split_k = 1;
+  // decode-sized batches of the weight-only kind: 256 weight rows per CTA (narrow weights, and calls that name their K splits, keep the
+  // 128-row schedule)
+  if (wide) return launch_gemm_wo(a, w, ep, epi, M, N, K, (cudaStream_t)stream);
   // prompt-sized batches run on CTA pairs; stream-K keeps the shapes where cutting K is faster, the weight-only kind, whose tiles are widened
   // on the way, and calls that cap its CTAs
   if (const int bt = !p.decode && !wo && split_k == 0 ? pair_tokens(M, N, K, ab_dtype) : 0)
@@ -1371,6 +1373,15 @@ int b200_gemm_decode_plan(int M, int N, int K, int ab_dtype, int split_k, int si
   GemmPlan p;
   int rc = plan_gemm(p, M, N, K, ab_dtype, split_k);
   if (rc) return rc;
+  const int epi = silu_mul == 2 ? EPI_ROPE : silu_mul ? EPI_SILU_MUL : EPI_LINEAR;
+  if (ab_dtype == B200_INT8_WO && split_k == 0 && gemm_wo_wide(epi, M, N, K)) {  // the rotation is a launch of its own there
+    size_t smem;
+    rc = gemm_wo_plan(epi, M, N, K, out6[0], out6[4], out6[2], smem);
+    out6[1] = 1;
+    out6[3] = out6[2];
+    out6[5] = (int)smem;
+    return rc;
+  }
   DecodeCfg c{};
   const bool r = has_residual != 0;
   if (silu_mul == 2) {  // the qkv GEMM with the RoPE / KV-write epilogue
@@ -1427,7 +1438,7 @@ int b200_gemm_rope_kv_write(const void* a, const void* w, void* qkv_out, const f
   // other schedule (one CTA per tile, the stream-K prefill kernel, odd head sizes) runs the GEMM, then the RoPE/scatter
   // kernel: same bits either way.
   bool fused = false;
-  const bool wide_wo = ab_dtype == B200_INT8_WO && split_k == 0;  // its own schedule, without the rotation
+  const bool wide_wo = ab_dtype == B200_INT8_WO && split_k == 0 && gemm_wo_wide(EPI_ROPE, M, N, K);  // its own schedule, without the rotation
   if (M <= 128 && !wide_wo && (D == 64 || D == 128) && N % GEMM_BN == 0 && max_pos > 0 &&
       (ab_dtype == B200_BF16 || ab_dtype == B200_FP8_E4M3 || ab_dtype == B200_INT8 || ab_dtype == B200_INT8_WO)) {
     int plan6[6];

@@ -327,7 +327,7 @@ constexpr size_t wox_smem() {
 // K splits of `tiles` tiles: whole waves of CTAs (one per SM) of nk stages of 1.2 us each, plus filling and draining a CTA, about 4 us, and
 // the exchange of the partial tiles, 2.
 struct WoPlan {
-  int S;
+  int S, cap;
   double us;
 };
 template <int BM, int EPI>
@@ -337,7 +337,7 @@ int plan_wo(WoPlan& best, int tiles, int num_kb) {
   std::lock_guard<std::mutex> g(mu);
   auto kern = gemm_wo_kernel<BM, EPI>;
   if (!cap[1]) B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wox_smem<BM>()));
-  best = {0, 0.0};
+  best = {0, 0, 0.0};
   for (int S = 1; S <= 8 && S <= num_kb; ++S) {
     if (!cap[S]) {
       cudaLaunchConfig_t cfg{};
@@ -358,9 +358,25 @@ int plan_wo(WoPlan& best, int tiles, int num_kb) {
     if (cap[S] < 0) continue;
     const int waves = (tiles * S + cap[S] - 1) / cap[S];
     const double us = waves * (((num_kb + S - 1) / S) * 1.2 + 4.0) + (S > 1 ? 2.0 : 0.0);
-    if (!best.S || us < best.us) best = {S, us};
+    if (!best.S || us < best.us) best = {S, cap[S], us};
   }
   B200_REQUIRE(best.S > 0, "gemm: no weight-only configuration fits");
+  return B200_OK;
+}
+
+// One launch (first = 0), or `first` whole waves of uncut tiles and the rest cut along K.
+template <int BM, int EPI>
+int plan_launches(WoPlan& all, WoPlan& rest, int& first, int N, int K) {
+  const int tiles = (N + WOX_ROWS - 1) / WOX_ROWS, num_kb = (K + WOX_BK - 1) / WOX_BK;
+  int rc = plan_wo<BM, EPI>(all, tiles, num_kb);
+  if (rc) return rc;
+  const int main_tiles = tiles / sm_count() * sm_count();
+  first = 0;
+  if (main_tiles && main_tiles < tiles) {
+    rc = plan_wo<BM, EPI>(rest, tiles - main_tiles, num_kb);
+    if (rc) return rc;
+    if (main_tiles / sm_count() * (num_kb * 1.2 + 4.0) + rest.us < all.us) first = main_tiles;
+  }
   return B200_OK;
 }
 
@@ -372,17 +388,10 @@ int launch_wo(const void* a, const void* w, const GemmEpilogue& ep, int M, int N
   rc = make_tmap_2d(&am, a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, 64, BM);
   if (rc) return rc;
   const int tiles = (N + WOX_ROWS - 1) / WOX_ROWS, num_kb = (K + WOX_BK - 1) / WOX_BK;
-  // one launch, or whole waves of uncut tiles and the rest cut along K
-  WoPlan all, rest{0, 0.0};
-  rc = plan_wo<BM, EPI>(all, tiles, num_kb);
+  WoPlan all, rest{};
+  int first;
+  rc = plan_launches<BM, EPI>(all, rest, first, N, K);
   if (rc) return rc;
-  const int main_tiles = tiles / sm_count() * sm_count();
-  int first = 0;
-  if (main_tiles && main_tiles < tiles) {
-    rc = plan_wo<BM, EPI>(rest, tiles - main_tiles, num_kb);
-    if (rc) return rc;
-    if (main_tiles / sm_count() * (num_kb * 1.2 + 4.0) + rest.us < all.us) first = main_tiles;
-  }
   auto go = [&](int tile0, int n, int S) -> int {
     B200_CUDA_OK(launch_kernel_cluster(gemm_wo_kernel<BM, EPI>, dim3(n * S), dim3(WOX_THREADS), wox_smem<BM>(), S, stream, wm, am, ep, M, N,
                                        num_kb, tile0));
@@ -396,6 +405,32 @@ int launch_wo(const void* a, const void* w, const GemmEpilogue& ep, int M, int N
 }
 
 }  // namespace
+
+// Fewer weight rows leave most of the chip without a tile of 256, and the 128-row schedule is the faster one there.  Measured (us, 128 rows ->
+// 256): linear 1024 x 1024, M = 64 6.2 -> 7.8; 2560 x 2048, M = 16 7.5 -> 7.7, 128 11.3 -> 12.3; 896 x 4864, M = 64 9.4 -> 11.7; but 2048 x 4096,
+// M = 1 to 33, 0.94 to 0.99 of the time, 3072 x 2048 0.96 to 1.06, 4096 x 2048 0.97 to 1.01, 7168 x 5120 0.68; with SiLU 2048 x 4096 0.87 to
+// 1.00, 1024 x 8192 0.99 to 1.07, 896 x 4864 1.05 to 1.19.
+bool gemm_wo_wide(int epi, int M, int N, int K) {
+  return epi == EPI_SILU_MUL ? N >= 2048 : epi == EPI_ROPE ? N >= 4096 : N >= 3072 || (N >= 2048 && K >= 4096 && M <= 32);
+}
+
+int gemm_wo_plan(int epi, int M, int N, int K, int& splits, int& cap_ctas, int& stages, size_t& smem) {
+  WoPlan all{}, rest{};
+  int first = 0, rc = B200_OK;
+#define WO_PLAN(BM)                                                                                                                     \
+  do {                                                                                                                                  \
+    rc = epi == EPI_SILU_MUL ? plan_launches<BM, EPI_SILU_MUL>(all, rest, first, N, K) : plan_launches<BM, EPI_LINEAR>(all, rest, first, N, K); \
+    stages = WOX_STAGES<BM>;                                                                                                            \
+    smem = wox_smem<BM>();                                                                                                              \
+  } while (0)
+  if (M <= 32) WO_PLAN(32);
+  else if (M <= 64) WO_PLAN(64);
+  else WO_PLAN(128);
+#undef WO_PLAN
+  splits = first ? rest.S : all.S;
+  cap_ctas = first ? rest.cap : all.cap;
+  return rc;
+}
 
 int launch_gemm_wo(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, cudaStream_t s) {
 #define WO_LAUNCH(BM) \
