@@ -38,6 +38,20 @@ def test_topk_candidates_bit_exact(ops, b, v, off):
     assert np.array_equal(idx.cpu().numpy(), wi)
 
 
+@pytest.mark.parametrize("v", [1, 1023, 1024, 1025, 4097, 63999, 64000, 64003])
+def test_topk_candidates_at_the_ends_of_its_paths(ops, v):
+    """Rows sorted whole, rows that go through the radix select, rows with a threshold and a list; among these a sorted one, one masked but for
+    40 logits, one constant and one with 5000 equal to its largest, which the list gives up."""
+    x = _logits(5, v, v)
+    x[1] = x[1].sort().values
+    x[2, torch.randperm(v, generator=torch.Generator().manual_seed(v))[: max(v - 40, 0)]] = -float("inf")
+    x[3] = 0.25
+    x[4, ::13] = x[4].max()
+    val, idx = ops.topk_candidates(x.cuda())
+    wv, wi = S.topk_candidates_ref(x.numpy())
+    assert np.array_equal(val.cpu().numpy(), wv) and np.array_equal(idx.cpu().numpy(), wi)
+
+
 def test_constant_row_keeps_the_lowest_indices(ops):
     x = torch.zeros(2, 5000)
     val, idx = ops.topk_candidates(x.cuda())

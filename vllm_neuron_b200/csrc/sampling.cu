@@ -14,6 +14,8 @@ constexpr int SAMPLE_K = 256;        // candidates per (row, shard): the referen
 constexpr int TOPK_THREADS = 1024;
 constexpr int EQ_CAP = 1024;
 constexpr int LIST_CAP = 4096;       // elements at or above the threshold that are sorted directly
+constexpr int LIST_ALL = 1024;       // rows of so few logits are sorted whole
+constexpr int LIST_MIN_V = 64000;    // rows from which a threshold and the few that reach it beat the radix select
 
 // monotone map fp32 -> uint32 (larger float <=> larger key); -0 < +0 is irrelevant here
 __device__ __forceinline__ uint32_t f2key(float x) {
@@ -51,6 +53,9 @@ __device__ __forceinline__ unsigned long long pack_cand(uint32_t key, uint32_t i
   return ((unsigned long long)key << 32) | (unsigned long long)(0xffffffffu - idx);
 }
 
+// LIST: with the two passes below (the list's shared memory is L1 that the radix select would keep the row in: 48000 logits 44 us without
+// it, 50 with)
+template <bool LIST>
 __global__ void __launch_bounds__(TOPK_THREADS)
     topk_candidates_kernel(const float* __restrict__ logits, int64_t row_stride, float* __restrict__ cand_val,
                            int64_t* __restrict__ cand_idx, int V, int64_t idx_offset) {
@@ -67,16 +72,17 @@ __global__ void __launch_bounds__(TOPK_THREADS)
 
   // ---- two passes over the row: the least of 256 disjoint groups' maxima is a threshold that at least 256 elements reach (about 1400
   // of a row in no particular order, whatever its length); they are listed and sorted.  Rows that put more than LIST_CAP elements there
-  // (long runs of ties, sorted rows) and only they go through the radix select below, whose first pass counts nearly every element in
-  // the same few bins (119 us for 32 rows of 128256 logits)
-  __shared__ unsigned long long list[LIST_CAP];
-  __shared__ unsigned int group_min[TOPK_THREADS / 32];
-  {
+  // (long runs of ties, sorted rows, rows masked almost everywhere) go through the radix select below, and give the list up when it is
+  // full; so do rows in between: sorting 2048 or 4096 elements takes 25 or 47 us, whatever the length.  Radix select / list (us, 8 rows):
+  // 1000 logits 26 / 13, 2000 26 / 24, 4096 26 / 47, 32000 42 / 30 to 52, 50257 44 / 56, 65536 60 / 34 to 57, 128256 91 / 41 to 64.
+  if constexpr (LIST) {
+    __shared__ unsigned long long list[LIST_CAP];
+    __shared__ unsigned int group_min[TOPK_THREADS / 32];
     const bool vec = (row_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
     const int V4 = vec ? V / 4 : 0;
     const float4* r4 = reinterpret_cast<const float4*>(r);
     uint32_t thr = 0;
-    if (V > LIST_CAP) {
+    if (V > LIST_ALL) {
       uint32_t mx = 0;
 #pragma unroll 4
       for (int i = tid; i < V4; i += TOPK_THREADS) {
@@ -91,7 +97,7 @@ __global__ void __launch_bounds__(TOPK_THREADS)
     }
     if (tid == 0) s_cnt = 0;
     __syncthreads();
-    if (V > LIST_CAP) thr = __reduce_min_sync(0xffffffffu, group_min[tid & 31]);
+    if (V > LIST_ALL) thr = __reduce_min_sync(0xffffffffu, group_min[tid & 31]);
     auto take = [&](float x, int i) {
       const uint32_t k = f2key(x);
       if (k >= thr) {
@@ -99,13 +105,23 @@ __global__ void __launch_bounds__(TOPK_THREADS)
         if (at < LIST_CAP) list[at] = pack_cand(k, (uint32_t)i);
       }
     };
-#pragma unroll 4
-    for (int i = tid; i < V4; i += TOPK_THREADS) {
-      const float4 x = r4[i];
+    auto take4 = [&](float4 x, int i) {
       take(x.x, 4 * i);
       take(x.y, 4 * i + 1);
       take(x.z, 4 * i + 2);
       take(x.w, 4 * i + 3);
+    };
+    int i4 = tid;
+    for (; i4 + 7 * TOPK_THREADS < V4 && *(volatile unsigned int*)&s_cnt <= LIST_CAP; i4 += 8 * TOPK_THREADS) {
+      float4 x[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = r4[i4 + j * TOPK_THREADS];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) take4(x[j], i4 + j * TOPK_THREADS);
+    }
+    if (*(volatile unsigned int*)&s_cnt <= LIST_CAP) {
+#pragma unroll 4
+      for (; i4 < V4; i4 += TOPK_THREADS) take4(r4[i4], i4);
     }
     for (int i = 4 * V4 + tid; i < V; i += TOPK_THREADS) take(r[i], i);
     __syncthreads();
@@ -423,8 +439,9 @@ int b200_topk_candidates(const float* logits, int64_t row_stride, float* cand_va
   B200_REQUIRE(logits && cand_val && cand_idx, "topk_candidates: null pointer");
   B200_REQUIRE(V > 0 && idx_offset >= 0 && idx_offset + V <= 0xffffffffll, "topk_candidates: bad V / idx_offset");
   if (B <= 0) return B200_OK;
-  B200_CUDA_OK(launch_kernel(topk_candidates_kernel, dim3(B), dim3(TOPK_THREADS), 0, (cudaStream_t)stream, logits, row_stride,
-                             cand_val, cand_idx, V, idx_offset));
+  const bool list = V <= LIST_ALL || V >= LIST_MIN_V;
+  B200_CUDA_OK(launch_kernel(list ? topk_candidates_kernel<true> : topk_candidates_kernel<false>, dim3(B), dim3(TOPK_THREADS), 0,
+                             (cudaStream_t)stream, logits, row_stride, cand_val, cand_idx, V, idx_offset));
   return B200_OK;
 }
 
