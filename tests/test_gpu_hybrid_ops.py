@@ -579,6 +579,20 @@ def test_attention_of_mixed_steps_apart_and_together(kind, monkeypatch):
     assert torch.equal(outs[0][:140], outs[1][:140]) and (outs[0][145:] - outs[1][145:]).norm() <= 2.0**-7 * outs[0][145:].norm()
 
 
+@pytest.mark.parametrize("T,inner,groups", [(1, 1024, 8), (63, 512, 2), (300, 512, 2), (700, 264, 2), (820, 1024, 1), (1640, 1024, 1), (5, 516, 1), (400, 2080, 2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gated_group_rmsnorm_slices(T, inner, groups, dtype):
+    """Slices of a warp's registers and of a CTA, few and many of them, ragged ones: against 64 bits, a few fp32 roundings of the result's size
+    plus the rounding to the output type."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(T + inner)
+    y, z, w = (torch.randn(*s, generator=g) for s in ((T, inner), (T, inner + 12), (inner,)))
+    got = ops.gated_group_rmsnorm(y.to(DEV), z.to(DEV), w.to(DEV), groups, 1e-6, dtype).double().cpu()
+    v = (y.double() * torch.nn.functional.silu(z[:, :inner].double())).view(T, groups, -1)
+    want = (v / torch.sqrt(v.pow(2).mean(-1, keepdim=True) + 1e-6)).reshape(T, inner) * w.double()
+    assert (got - want).abs().max() <= (2.0**-8 if dtype == torch.bfloat16 else 2e-6) * max(1.0, float(want.abs().max()))
+
+
 @pytest.mark.parametrize("T,W", [(1, 4), (3, 1028), (2, 4096), (5, 4100), (700, 132), (4, 30)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_row_kernels_in_vectors(T, W, dtype):

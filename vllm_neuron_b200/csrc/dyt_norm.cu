@@ -118,7 +118,8 @@ __global__ void gated_group_rmsnorm_kernel(const float* __restrict__ y, const fl
 }
 
 // The same with a warp per (token, slice), the slice in its registers: 16-byte accesses, no barrier (4096 x 8 slices of 512: 79 -> 37
-// us).  Slices of up to 128 V.
+// us).  Slices of up to 128 V, and enough of them: a warp alone walks a wide slice more slowly than the CTA above does (CTA / warp, us: slices
+// of 1024, 4 of them 2.9 / 4.8, 1024 5.3 / 5.7, 1600 6.6 / 6.3; of 512, 64 2.2 / 3.1, 800 3.8 / 3.4; of 256, 64 2.0 / 2.3, 400 2.4 / 2.3).
 template <typename OT, int V>
 __global__ void gated_group_rmsnorm_warp_kernel(const float* __restrict__ y, const float* __restrict__ z, int ldz,
                                                 const float* __restrict__ w, OT* __restrict__ out, int inner, int ng, float eps, int T) {
@@ -253,7 +254,8 @@ int b200_gated_group_rmsnorm(const float* y, const float* z, int ldz, const floa
   B200_REQUIRE((size_t)(inner / groups) * 4 <= 160 * 1024, "gated_group_rmsnorm: group of %d too wide", inner / groups);
   if (T <= 0) return B200_OK;
   const int gs = inner / groups, oes = out_dtype == B200_BF16 ? 2 : 4;
-  if (gs % 4 == 0 && gs <= 1024 && groups <= 65535 && ldz % 4 == 0 && vec4_ok(y) && vec4_ok(z) && vec4_ok(w) && vec4_ok(out, oes)) {
+  const bool many = gs <= 128 || 5LL * T * groups >= 8LL * gs;
+  if (many && gs % 4 == 0 && gs <= 1024 && groups <= 65535 && ldz % 4 == 0 && vec4_ok(y) && vec4_ok(z) && vec4_ok(w) && vec4_ok(out, oes)) {
     const int warps = T >= 8 * 148 ? 8 : 2;  // small batches spread over the SMs
 #define GGR(V)                                                                                                                             \
   B200_DISPATCH_ELEM(out_dtype, OT,                                                                                                        \
