@@ -174,3 +174,11 @@ def test_step_parts_are_split_only_where_the_decoded_tokens_are_worth_a_launch()
     assert pays((1600,), 60, 1800, 16, 4, 128, 128, tc=True) and not pays((1600,), 4, 300, 16, 4, 128, 128, tc=True)
     assert pays((200,), 1, 1800, 12, 4, 80, 80) and not pays((200,), 1, 300, 12, 4, 80, 80)
     assert ops._span(900, 256, 0, 32, 4) == 256 + 644 // 32 + 4 and ops._span(900, 1 << 30, 128, 0, 0) == 128
+
+
+def test_delta_rule_rounds_where_a_chain_is_long_or_the_chip_is_free():
+    from vllm_neuron_b200.ops import _delta_rounds
+
+    assert _delta_rounds(4096, 4096, 16, 128, 128) and _delta_rounds(300, 331, 8, 64, 64) and _delta_rounds(17, 4 * 17, 8, 64, 64)
+    assert not _delta_rounds(17, 20 * 17, 8, 64, 64) and not _delta_rounds(130, 32 * 130, 8, 64, 64) and _delta_rounds(300, 6000, 8, 64, 64)
+    assert not _delta_rounds(17, 20 * 17, 8, 128, 128) and _delta_rounds(40, 64 * 40, 8, 128, 128) and _delta_rounds(8, 64 * 8, 8, 128, 128)

@@ -1105,6 +1105,18 @@ def glu(gate_up, act: int, out_dtype):
     return out
 
 
+def _delta_rounds(longest: int, tokens: int, heads: int, dim: int, vdim: int) -> bool:
+    """Whether a step whose longest portion has 8 tokens or more takes the rounds of eight tokens.  They shorten the chain of a portion; where
+    portions of one length already fill the chip, the two-token kernel's smaller CTAs share an SM better.  Two-token / rounds, us, heads of
+    64 x 64: 4 portions of 17 x 8 heads 9.0 / 7.1, 20 12.7 / 15.9; 12 of 40 17.6 / 15.0, 24 21.9 / 24.2, 64 44.5 / 53.0; 20 of 300 121.7 / 112.0,
+    one of 300 beside 31 tokens 71.6 / 30.3.  Of 128 x 128, 20 of 17 x 8 heads 30.9 / 34.0 (rounds of eight pad 17 to 24), of 8 19.7 / 20.4, of 40
+    56.7 / 49.1."""
+    together = tokens / longest * heads * (vdim // 16)  # CTAs of 16 columns, were all portions the longest
+    if dim == 64:
+        return together <= 300 or (together <= 640 and longest >= 32)
+    return together <= 640 or not 16 < longest < 24
+
+
 def delta_rule(qkv, proj, b_col0: int, a_col0: int, a_log, dt_bias, state, meta, heads: int, kv_heads: int, dim: int, vdim: int,
                q_scale: float, unit_eps: float = 1e-6):
     """Gated delta rule over a ragged batch.  qkv fp32 [T, q: G*D | k: G*D | v: H*P] (convolved; q and k are normalised IN
@@ -1123,9 +1135,12 @@ def delta_rule(qkv, proj, b_col0: int, a_col0: int, a_log, dt_bias, state, meta,
         check(lib.b200_delta_prep(_ptr(qkv), qkv.stride(0), _ptr(proj), proj.stride(0), b_col0, a_col0, _ptr(a_log), _ptr(dt_bias),
                                   _ptr(bg), _ptr(kq), t, heads, kv_heads, dim, float(q_scale), float(unit_eps), _stream()),
               "b200_delta_prep")
+    longest = int(meta.max_new)
+    if longest >= 8 and not _delta_rounds(longest, t, heads, dim, vdim):
+        longest = 7  # the two-token kernel
     with _k("delta_scan"):
         check(lib.b200_delta_scan(_ptr(qkv), qkv.stride(0), _ptr(bg), _ptr(kq), _ptr(state), _ptr(meta.seq_start),
-                                  _ptr(meta.seq_slot), _ptr(meta.seq_pos0), _ptr(out), meta.num_seqs, int(meta.max_new), heads, kv_heads, dim, vdim,
+                                  _ptr(meta.seq_slot), _ptr(meta.seq_pos0), _ptr(out), meta.num_seqs, longest, heads, kv_heads, dim, vdim,
                                   _stream()), "b200_delta_scan")
     return out
 
