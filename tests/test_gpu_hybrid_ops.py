@@ -593,6 +593,26 @@ def test_gated_group_rmsnorm_slices(T, inner, groups, dtype):
     assert (got - want).abs().max() <= (2.0**-8 if dtype == torch.bfloat16 else 2e-6) * max(1.0, float(want.abs().max()))
 
 
+@pytest.mark.parametrize("m,n,k,short", [(400, 1024, 64, True), (129, 64, 160, True), (1000, 2048, 128, False), (129, 64, 168, False), (100, 64, 64, False)])
+def test_short_prompt_rows_take_the_small_kernel(m, n, k, short):
+    """Prompts on short rows: the bits of the mma.sync kernel; longer rows, larger products and decode batches leave it.  bf16 products are
+    exact: k roundings of fp32 sums either way (cut short, not rounded, on the tensor cores: 2^-23 each)."""
+    from types import SimpleNamespace
+
+    from vllm_neuron_b200.hybrid import HybridCausalLM
+
+    ops = _ops()
+    g = torch.Generator().manual_seed(m + k)
+    a, w = torch.randn(m, k, generator=g).bfloat16().to(DEV), torch.randn(n, k, generator=g).bfloat16().to(DEV)
+    before = ops.launch_count()
+    got = HybridCausalLM._linear(SimpleNamespace(et=torch.bfloat16, gemm_ws=None, device=DEV), a, w)
+    assert ops.launch_count() == before + 1
+    if short:
+        assert torch.equal(got, ops.linear_simt(a, w))
+    want = a.double() @ w.double().T
+    assert ((got.double() - want).abs() <= k * 2.0**-23 * (a.double().abs() @ w.double().abs().T)).all()
+
+
 @pytest.mark.parametrize("T,W", [(1, 4), (3, 1028), (2, 4096), (5, 4100), (700, 132), (4, 30)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_row_kernels_in_vectors(T, W, dtype):

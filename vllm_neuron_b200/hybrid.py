@@ -1216,11 +1216,13 @@ class HybridCausalLM:
     # ------------------------------------------------------------------ building blocks
     def _linear(self, a, w):
         """fp32 [M, N] = a @ w^T.  bf16 serving: the tcgen05 GEMM (TMA needs K * 2 bytes to be a multiple of 16), narrow weights
-        and short rows included (us against the mma.sync kernel: 4096 x 16 x 2048 17 / 31, 4096 x 160 x 4096 29 / 133, 4096 x 4096 x
-        128 25 / 53, 400 x 160 x 4096 27 / 46); anything else, and all of 32-bit serving, runs on the CUDA cores with true fp32
-        arithmetic."""
+        included (us against the mma.sync kernel: 4096 x 16 x 2048 17 / 31, 4096 x 160 x 4096 29 / 133, 4096 x 4096 x 128 25 / 53,
+        400 x 160 x 4096 27 / 46).  Prompts on rows so short that a GEMM is all prologue and epilogue stay with the mma.sync kernel
+        (2000 x 64 x 16 3.6 / 2.6, 400 x 1024 x 64 4.1 / 3.7, 700 x 256 x 128 4.3 / 3.7; 1000 x 512 x 128 4.4 / 4.5).  Anything else, and
+        all of 32-bit serving, runs on the CUDA cores with true fp32 arithmetic."""
         m, (n, k) = a.shape[0], w.shape
-        if self.et == torch.bfloat16 and k % 8 == 0:
+        short = m > 128 and k <= 160 and m * n * (k + 64) <= 1 << 26
+        if self.et == torch.bfloat16 and k % 8 == 0 and not short:
             need = ops.gemm_workspace_bytes(m, n, k, ops.BF16, 0)
             if need and (self.gemm_ws is None or self.gemm_ws.numel() < need):
                 self.gemm_ws = torch.zeros(need, dtype=torch.uint8, device=self.device)  # stream-K counters start at zero
