@@ -203,6 +203,20 @@ def test_gemm_prompt_schedule(ops, m, n, k, cut):
     assert torch.equal(got, ops.gemm(x, w, out_dtype=torch.float32, split_k=sms)) == cut
 
 
+@pytest.mark.parametrize("m,n,k", PAIR_SHAPES + [(300, 1056, 640), (2048, 4096, 4096)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_gemm_pairs_bf16_against_64_bits(ops, m, n, k, f32):
+    """bf16 operands, every epilogue operand.  Products are exact; the tensor cores cut the low bits of every sum of 16 of them: 2^-23 of the
+    magnitudes summed so far, k / 16 times at most; then the epilogue's roundings and the one to bf16."""
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda").bfloat16()  # noqa: E731
+    x, w, bias, res = r(m, k), r(n, k), r(n), r(m, n)
+    want = x.double() @ w.double().T + bias.double() + res.double()
+    size = x.double().abs() @ w.double().abs().T + bias.double().abs() + res.double().abs()
+    got = ops.gemm(x, w, None, None, bias, res, out_dtype=torch.float32 if f32 else torch.bfloat16).double()
+    assert ((got - want).abs() <= (k / 16 + 3) * 2.0**-23 * size + (0.0 if f32 else 2.0**-8) * want.abs()).all()
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 1056, 512), (31, 256, 144), (33, 640, 1152), (64, 992, 256), (65, 256, 128), (128, 1000, 144), (100, 640, 1152), (127, 32, 64), (128, 38144, 256), (96, 5120, 2048),
                                    (1, 3104, 512), (31, 3072, 144), (33, 3220, 1152), (64, 4064, 256), (65, 3328, 128), (128, 4072, 144), (127, 3072, 64), (100, 3104, 1152)])
 def test_gemm_weight_only_256_rows(ops, m, n, k):
