@@ -156,15 +156,18 @@ int b200_paged_attn_prefill(const void* q, int64_t q_token_stride, const void* k
  *   Weights stream through a deep TMA ring (up to 176 KB per SM in flight, issued before the previous kernel of the
  *   stream has finished), activations through a shallow one; the schedule (S, CTAs per SM, ring depths) is picked per
  *   shape from occupancy queries and a latency/bandwidth model (b200_gemm_decode_plan reports it).
- * M > 128 (prefill): persistent stream-K over min(split_k, #SM) CTAs (0 = one per SM), each an equal share of the
- *   (tile, k-block) space; tiles cut by a share boundary are summed in fixed order by the last contributor.
- *   `workspace` (b200_gemm_workspace_bytes) holds the fix-up counters in its first 4 KiB: it must be ZERO-FILLED before
- *   its first use and is left zeroed by every call; one workspace may serve all GEMMs issued on one stream. */
+ *   Weight-only batches (INT8_WO) of wide weights take 256 weight rows per CTA instead where split_k is 0.
+ * M > 128 (prefill), split_k = 0: CTA pairs, each on whole tiles of 256 weight rows x 64 to 256 tokens; where few tiles walk a long K, and for
+ *   INT8_WO, the schedule of an explicit split_k:
+ *   persistent stream-K over min(split_k, #SM) CTAs (0 = one per SM), each an equal share of the (tile, k-block) space; tiles cut by a share
+ *   boundary are summed in fixed order by the last contributor.
+ *   `workspace` (b200_gemm_workspace_bytes; asked for whichever schedule a call takes) holds the fix-up counters in its first 4 KiB: it must
+ *   be ZERO-FILLED before its first use and is left zeroed by every call; one workspace may serve all GEMMs issued on one stream. */
 size_t b200_gemm_workspace_bytes(int M, int N, int K, int ab_dtype, int split_k);
 /* The decode schedule (M <= 128) chosen on the current device for a shape: out6 = {cluster size S, CTAs per SM, weight
  * ring depth, activation ring depth, CTAs the chip holds at once, dynamic shared memory bytes}.  Needs a device.
  * silu_mul selects the epilogue variant planned for: 0 linear, 1 SiLU*mul (b200_gemm_silu_mul), 2 RoPE + KV write
- * (b200_gemm_rope_kv_write). */
+ * (b200_gemm_rope_kv_write).  Weight-only batches on 256 weight rows: the cluster size of the cut tiles; both rings have one depth. */
 int b200_gemm_decode_plan(int M, int N, int K, int ab_dtype, int split_k, int silu_mul, int has_residual, int* out6);
 /* Profiling aid: with a non-NULL device buffer ([#CTAs][8] uint64) every decode-schedule GEMM CTA records %globaltimer
  * at its phase boundaries (tools/gemm_trace.py); NULL (default) switches it off. */
@@ -174,8 +177,8 @@ int b200_gemm(const void* a, const void* w, void* out, const float* a_scale, con
               size_t workspace_bytes, void* stream);
 /* INT8 weight-only linear (SURVEY 8(b) `b200_gemm_int8_wo`; reference config keys quantized / quantization_dtype=int8 with
  * bf16 activations, model_loader.py:885-898): out = (a_bf16 . w_int8^T) * w_scale[n] + bias + residual.  The int8 rows are
- * streamed from HBM as int8 (half the bytes of bf16) and widened to bf16 operand tiles in shared memory by the CTA's
- * epilogue warps (exact), then multiplied with kind::f16.  Same as b200_gemm with ab_dtype = B200_INT8_WO. */
+ * streamed from HBM as int8 (half the bytes of bf16) and widened to bf16 (exactly) by warps of their own -- into tensor memory by the 256-row
+ * decode schedule, into shared memory by the others -- then multiplied with kind::f16.  Same as b200_gemm with ab_dtype = B200_INT8_WO. */
 int b200_gemm_int8_wo(const void* a_bf16, const void* w_int8, void* out, const float* w_scale, const void* bias,
                       const void* residual, int M, int N, int K, int out_dtype, int split_k, void* workspace,
                       size_t workspace_bytes, void* stream);

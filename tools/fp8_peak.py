@@ -3,9 +3,9 @@
 Same protocol as the driver's bf16 figure in MEASURED_PEAKS.json (torch.matmul 8192^3: best of 10 = burst, back to back for
 4 s = sustained), with cuBLASLt's FP8 GEMM (torch._scaled_mm, e4m3 x e4m3 -> bf16, per-tensor scales, fp32 accumulate) in
 place of the bf16 matmul; bf16 is re-measured beside it so the two come from one box and one clock state.  LIBRARY code, used
-only as a yardstick -- nothing on the product path calls it.  Writes one JSON object (default gpurun_out/fp8_peak.json).
+only as a yardstick -- nothing on the product path calls it.  Writes one JSON object (default fp8_peak.json).
 
-    python tools/fp8_peak.py [--out gpurun_out/fp8_peak.json]
+    python tools/fp8_peak.py [--out fp8_peak.json]
 """
 import argparse
 import json
@@ -38,7 +38,7 @@ def measure(fn, flops):
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("--out", default="gpurun_out/fp8_peak.json")
+    ap.add_argument("--out", default="fp8_peak.json")
     a = ap.parse_args()
     dev = torch.device("cuda:0")
     res = {"gpu": torch.cuda.get_device_name(0), "torch": torch.__version__, "shapes": []}

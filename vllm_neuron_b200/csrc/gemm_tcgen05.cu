@@ -16,7 +16,8 @@
 //    then each CTA adds the slices in fixed rank order (bit-reproducible) and runs the epilogue for its 128/S rows.
 //    No global workspace, no atomics, no second kernel.  CTAs are sized (<= 105 KB smem, <= 64 TMEM columns) so that
 //    two are resident per SM: the prologue/epilogue of one overlaps the streaming of the other.
-//  * PREFILL (M > 128): CTA pairs (gemm_pair.cu) for bf16, fp8 and int8 operands; for the weight-only kind persistent stream-K, one CTA per SM; the flattened (tile, k-block) space is cut into equal
+//  * PREFILL (M > 128): CTA pairs (gemm_pair.cu) for bf16, fp8 and int8 operands.  For the weight-only kind, long K against few tiles and
+//    calls that cap the CTAs persistent stream-K, one CTA per SM; the flattened (tile, k-block) space is cut into equal
 //    contiguous spans; a tile cut by a span boundary is finished by whichever contributor arrives last (partials parked
 //    in the workspace, summed in fixed contributor order).
 // Both use programmatic dependent launch: the grid becomes resident while the previous kernel drains and the TMA
@@ -652,7 +653,7 @@ __global__ void __launch_bounds__(KIND == KIND_WO8 ? WO_THREADS : DEC_THREADS, K
         for (int i = npre; i < pf_end; ++i) tma_prefetch_l2_2d(&w_map, (kb0 + i) * BK_ELEMS, n_tile * GEMM_BN);
       }
       // refills: weights only -- the activation tiles come from their own producer warp (AP_WARP).  One issuing thread
-      // sustains about one TMA box row per 5.5 cycles (tools/tma_ingest.cu: 128x64B boxes 21 GB/s per SM from one
+      // sustains about one TMA box row per 5.5 cycles (profiles/r02_tma_ingest_v1.txt: 128x64B boxes 21 GB/s per SM from one
       // producer warp, 40 GB/s from two), so W and A boxes issued by the same thread queue behind each other.
       int s = 0, ph = 0;  // stage / parity of the empty barriers for refills
       for (int i = npre; i < nk; ++i) {

@@ -5,14 +5,14 @@
 //   S_out = exp(cum_end) S_in    +  sum_j exp(cum_end - cum_j) dt_j x_j B_j^T
 // which is the recurrence with its sums regrouped.  One operand of every product is exact in bf16 (x, B or C); the other (the weighted
 // scores, the state, the weighted x) is fp32 and enters as THREE bf16 terms that together hold its 24 mantissa bits, so products are
-// exact and sums are fp32 as on the CUDA cores.  The cumulated log decays are summed in 64 bits and kept as a pair of floats: the
+// exact; their sums, 16 tokens or state elements at a time, are the tensor cores' (below).  The cumulated log decays are summed in 64 bits and kept as a pair of floats: the
 // difference of two of them is good to fp32 wherever in the segment it is taken.
 //
 // Why: the sequential kernel walks tokens at ~0.19 us each (two passes over a segmented portion) and issues 5 fp32 operations per state
 // element and token on the FMA pipe; mma.sync does the regrouped sums, three terms included, in a seventh of the issue slots.  Per
 // (head, segment) the output kernel runs 5 400 m16n8k16 products (about 6 us of tensor pipe) on 160 KB of operands, one CTA per SM: load,
 // split and products follow one another, which is what bounds it now (18 us).  One portion of 4096 tokens, 32 heads of 128 x 128: 843 us
-// sequential, 219 us here (states 55, chaining 35, outputs 120).
+// sequential, 217 us here; the outputs are more than half of it.
 #include "ssm_common.cuh"
 
 namespace b200 {
@@ -31,10 +31,11 @@ __device__ __forceinline__ void split3(float2 v, uint32_t& h, uint32_t& m, uint3
   l = *reinterpret_cast<const uint32_t*>(&c);
 }
 
-// The tensor cores cut a sum's low bits where the CUDA cores round; sums over more than 16 products are therefore made of fresh MMA
-// results with rounded additions.  Against 64 bits (2-norm of the
-// difference over that of the result; sequential kernel in brackets): outputs 0.9 - 1.0e-7 (0.8 - 0.95e-7) with fast decays, 1.0 -
-// 2.2e-7 (2.5 - 5.9e-7) with slow ones, states 0.6 - 2.9e-7 (0.6 - 6.3e-7).
+// The tensor cores cut a sum's low bits where the CUDA cores round; longer sums are therefore made of fresh MMA results -- one for 16 exact
+// products, three in a chain where an operand has its three terms -- with rounded additions.  Against 64 bits (2-norm of the difference
+// over that of the result, 4096 and 8192 tokens; sequential kernel in brackets): step sizes of a tenth and more: outputs 0.9 - 1.0e-7 (0.8 -
+// 0.97e-7), states 0.5 - 0.9e-7 (0.5 - 0.98e-7); of a few thousandths: outputs 0.7 - 0.98e-7 (3.8 - 6.5e-7), states 1.0 - 1.1e-7 (4.1 -
+// 9.0e-7); of a few ten-thousandths: outputs 1.1 - 1.5e-7 (1.0 - 6.9e-6), states 1.9 - 3.0e-7 (1.9 - 17e-6).
 __device__ __forceinline__ void add_to(float (&a)[4], const float (&b)[4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) a[i] += b[i];

@@ -20,7 +20,7 @@ _DTN = {BF16: "bf16", FP8_E4M3: "fp8", INT8: "int8", INT8_WO: "int8wo"}
 
 
 def _stream():
-    # the raw handle of the current stream: torch.cuda.current_stream() builds a Stream object on every launch (4 us of host time)
+    # the raw handle of the current stream: torch.cuda.current_stream() builds a Stream object on every launch (3 us of host time)
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
