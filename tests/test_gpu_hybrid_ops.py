@@ -579,6 +579,26 @@ def test_attention_of_mixed_steps_apart_and_together(kind, monkeypatch):
     assert torch.equal(outs[0][:140], outs[1][:140]) and (outs[0][145:] - outs[1][145:]).norm() <= 2.0**-7 * outs[0][145:].norm()
 
 
+def test_dyt_residual_sees_weights_that_the_kernel_ahead_wrote():
+    """Weight rows that come straight out of another kernel of the library, whose blocks let the next one start early: the last row that it
+    writes is the weight, a new one each time."""
+    ops = _ops()
+    W = 1024
+    g = torch.Generator().manual_seed(2)
+    src, one, zero = torch.randn(8, 3000, W, generator=g).to(DEV), torch.ones(W, device=DEV), torch.zeros(W, device=DEV)
+    y = torch.randn(4, W, generator=g).to(DEV)
+    got = []
+    for i in range(8):
+        w = ops.dyt_norm(src[i], one, zero, 1.0, torch.float32)[-1]
+        x = torch.zeros(4, W, device=DEV)
+        w2 = ops.dyt_norm(src[i], one, zero, 0.5, torch.float32)[-1]
+        got.append((ops.dyt_residual(x, y, (w, zero, 0.7), (w2, zero, 0.4), torch.float32), x))
+    for i, (out, x) in enumerate(got):
+        want = torch.tanh(0.7 * y.double()) * torch.tanh(src[i, -1].double())
+        assert (x.double() - want).abs().max() <= 2e-6
+        assert (out.double() - torch.tanh(0.4 * want) * torch.tanh(0.5 * src[i, -1].double())).abs().max() <= 2e-6
+
+
 @pytest.mark.parametrize("T,inner,groups", [(1, 1024, 8), (63, 512, 2), (300, 512, 2), (700, 264, 2), (820, 1024, 1), (1640, 1024, 1), (5, 516, 1), (400, 2080, 2)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_gated_group_rmsnorm_slices(T, inner, groups, dtype):

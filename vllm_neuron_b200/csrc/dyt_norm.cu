@@ -57,11 +57,11 @@ __global__ void dyt_residual_vec_kernel(float* __restrict__ x, const float* __re
                                         int W, int T) {
   griddep_launch();
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  griddep_wait();  // before the weights too: they may be what the kernel ahead has written
   if (c >= W) return;
   const float4 u1 = ldf4(w1, c), v1 = ldf4(b1, c);
   float4 u2 = make_float4(0.f, 0.f, 0.f, 0.f), v2 = u2;
   if (out2) u2 = ldf4(w2, c), v2 = ldf4(b2, c);
-  griddep_wait();
 #pragma unroll 2
   for (int t = blockIdx.y; t < T; t += gridDim.y) {
     const int64_t i = (int64_t)t * W + c;
