@@ -163,6 +163,17 @@ def load():
     return lib
 
 
+def native():
+    """The functions that take tensors (csrc/bind.cpp), over the same library."""
+    load()
+    try:
+        from . import _b200_bind
+    except ImportError as e:
+        raise B200Error(f"the Python binding is missing or does not load ({e}): build it with `python -m vllm_neuron_b200.build`") from e
+    _b200_bind.set_error(B200Error)
+    return _b200_bind
+
+
 def check(rc: int, what: str):
     if rc != OK:
         msg = load().b200_last_error().decode(errors="replace")

@@ -15,6 +15,8 @@ SOURCES = ["host.cu", "kv_ops.cu", "paged_attn.cu", "paged_attn_prefill_tc.cu", 
            "dyt_norm.cu", "ssm_scan.cu", "ssm_segment.cu", "swa_attn.cu", "swa_attn_prefill.cu", "swa_attn_prefill_tc.cu", "moe.cu", "rms_norm.cu", "delta_rule.cu",
            "latent_attn.cu", "gated_scan.cu", "selective_scan.cu", "hyper_conn.cu"]
 HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "gemm_common.cuh"), os.path.join(CSRC, "gemm_pair.cuh"), os.path.join(CSRC, "gemm_group.cuh"), os.path.join(CSRC, "hybrid_common.cuh"), os.path.join(CSRC, "ssm_common.cuh"), os.path.join(os.path.dirname(HERE), "include", "b200_paged.h")]
+BIND = os.path.join(HERE, "_b200_bind.so")  # the library's functions on torch tensors, for ops.py
+BIND_SOURCES = [os.path.join(CSRC, "bind.cpp"), os.path.join(os.path.dirname(HERE), "include", "b200_paged.h")]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-std=c++17", "-lineinfo",
@@ -38,7 +40,30 @@ def needs_build() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_bind(force: bool = False) -> str:
+    """The extension module beside the library (host code only)."""
+    if not force and os.path.exists(BIND) and all(os.path.getmtime(d) <= os.path.getmtime(BIND) for d in BIND_SOURCES):
+        return BIND
+    import sysconfig
+
+    import torch
+
+    t = os.path.dirname(torch.__file__)
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", sysconfig.get_paths()["include"], "-I", f"{t}/include",
+           "-I", f"{t}/include/torch/csrc/api/include", "-I", os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include"), BIND_SOURCES[0],
+           "-o", BIND, "-L", f"{t}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-L", HERE, "-l:libb200_paged.so", "-Wl,-rpath,$ORIGIN"]
+    subprocess.check_call(cmd)
+    return BIND
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    _build_lib(force, verbose)
+    build_bind(force)
+    return LIB
+
+
+def _build_lib(force: bool, verbose: bool) -> str:
     if not force and not needs_build():
         return LIB
     objs = []

@@ -902,10 +902,14 @@ class StepMeta:
         tok_seq = np.repeat(np.arange(b, dtype=np.int64), n)
         tok_pos = np.arange(t, dtype=np.int64) - start[tok_seq] + pos0[tok_seq]
         slots = np.empty(t, dtype=np.int64)
+        at = start.tolist()
         for s, (row, p0, k) in enumerate(entries):
+            if k == 1:  # a decoded token: one page number, not an array of the row's
+                slots[at[s]] = block_rows[row][p0 // block_size] * block_size + p0 % block_size
+                continue
             blocks = np.asarray(block_rows[row], dtype=np.int64)
             p = np.arange(p0, p0 + k)
-            slots[start[s]:start[s + 1]] = blocks[p // block_size] * block_size + p % block_size
+            slots[at[s]:at[s + 1]] = blocks[p // block_size] * block_size + p % block_size
         parts = [start, rows, pos0, tok_seq, rows[tok_seq], tok_pos]
         i32 = np.concatenate(parts).astype(np.int32)
         if i32.size % 2:  # the int64 slots that follow must start on an 8-byte boundary
