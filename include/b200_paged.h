@@ -339,6 +339,10 @@ int b200_ssd_scan_mma(const void* xbc, int x_dtype, int C, const float* dt_in, i
                       const float* dt_bias, const float* D, float* state, const int32_t* seq_start, const int32_t* seq_slot,
                       const int32_t* seq_pos0, float* y, int B, int H, int P, int N, int G, const int32_t* segs, int num_segs,
                       const int32_t* seq_seg0, float* seg_state, float* seg_dtsum, void* stream);
+/* The same where every sequence brings one token (a decode step).  N of 32, 64 or 128 takes the kernel for it, anything else the scan. */
+int b200_ssd_step(const void* xbc, int x_dtype, int C, const float* dt_in, int ld_dt, int dt_col0, const float* A_log, const float* dt_bias,
+                  const float* D, float* state, const int32_t* seq_start, const int32_t* seq_slot, const int32_t* seq_pos0, float* y, int B,
+                  int H, int P, int N, int G, void* stream);
 /* Scatter keys [G][D] (columns k_col0..) and values [G][Dv] (columns v_col0..) of the fp32 rows `qkv` into the pools
  * K [num_blocks][G][block_size][D], V [num_blocks][G][block_size][Dv] by slot (slot < 0: skipped).
  * mode 0: plain; 1: also keep the unmixed values in v_first fp32 [T][G*Dv]; 2: cache v + lambda * (v_first - v) instead of v. */

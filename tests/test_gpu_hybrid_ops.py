@@ -673,3 +673,31 @@ def test_row_kernels_in_vectors(T, W, dtype):
     gu = 4 * r(T, 2 * W)
     a, b = gu[:, :W].double().clamp(max=7.0), gu[:, W:].double().clamp(-7.0, 7.0)
     close(ops.clamped_glu(d(gu), 7.0, dtype), a * torch.sigmoid(1.702 * a) * (b + 1))
+
+
+@pytest.mark.parametrize("H,P,N,G", [(4, 128, 128, 2), (2, 70, 64, 1), (3, 5, 32, 3), (2, 257, 128, 2), (2, 12, 40, 1)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_ssd_step_of_one_token_each(H, P, N, G, dtype):
+    """Decode steps: value columns that end inside a warp's rows, every state size with a kernel of its own and one without, a sequence at
+    position 0 over a used slot.  The state is that of the scan bit for bit; y within N roundings of an fp32 sum of N products (one more for D x)."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(H * P + N)
+    entries = [(3, 5, 1), (0, 0, 1), (2, 90, 1)]
+    C, slots = H * P + 2 * G * N, 4
+    xbc = torch.randn(3, C, generator=g).to(dtype)
+    raw = torch.randn(3, H + 2, generator=g)
+    a_log, bias, D = 0.5 * torch.randn(H, generator=g), torch.randn(H, generator=g), torch.randn(H, generator=g)
+    state = torch.randn(slots, H, P, N, generator=g)
+    meta = _meta(entries, {r: [1] * 40 for r in range(slots)})
+    args = [t.to(DEV) for t in (xbc, raw)] + [2] + [t.to(DEV) for t in (a_log, bias, D)]
+    got, want = state.to(DEV), state.to(DEV)
+    y = ops.ssd_scan(*args, got, meta, H, P, N, G)
+    meta.max_new = 2
+    ops.ssd_scan(*args, want, meta, H, P, N, G)
+    assert torch.equal(got, want) and torch.equal(got[1].cpu(), state[1])
+    S = got[torch.tensor([3, 0, 2], device=DEV)].double().cpu()
+    Cm = xbc[:, H * P + G * N:].double().view(3, G, N).repeat_interleave(H // G, 1)
+    skip = D.double()[:, None] * xbc[:, :H * P].double().view(3, H, P)
+    terms = S * Cm[:, :, None, :]
+    bound = (N + 1) * 2.0**-24 * (terms.abs().sum(-1) + skip.abs())
+    assert ((y.double().cpu().view(3, H, P) - terms.sum(-1) - skip).abs() <= bound).all()

@@ -694,6 +694,12 @@ def ssd_scan(xbc, dt_src, dt_col0: int, a_log, dt_bias, d_skip, state, meta, hea
     assert xbc.is_contiguous() and state.shape[1:] == (heads, vdim, nstate)
     t = xbc.shape[0]
     y = _new(xbc, torch.float32, t, heads * vdim)
+    if getattr(meta, "max_new", 0) == 1:  # one token of every sequence: the state passes once, nothing is walked
+        with _k("ssd_step"):
+            check(_lib().b200_ssd_step(xbc, _edt(xbc), xbc.shape[1], dt_src, dt_src.stride(0), dt_col0, a_log,
+                                             dt_bias, d_skip, state, meta.seq_start, meta.seq_slot,
+                                             meta.seq_pos0, y, meta.num_seqs, heads, vdim, nstate, groups), "b200_ssd_step")
+        return y
     segs = getattr(meta, "scan_segs", None)
     nseg = meta.num_segs if segs is not None else 0
     seg_state = seg_dt = None
