@@ -448,3 +448,52 @@ def test_gemm_silu_mul_quant_fused_equals_two_calls(ops, kind, m, i, k):
             continue
         assert torch.equal(got[1], want_s)
         assert torch.equal(got[0].view(torch.uint8), want_q.view(torch.uint8))
+
+
+SMALL_SHAPES = [(1, 16, 16), (8, 24, 48), (3, 40, 528), (7, 2000, 144), (5, 2416, 1040), (2, 4808, 272), (1, 9600, 80), (8, 2048, 5632), (4, 2320, 2048)]
+
+
+@pytest.mark.parametrize("m,n,k", SMALL_SHAPES)
+@pytest.mark.parametrize("kind", ["bf16", "fp8", "int8", "int8_wo", "int8_wo_16"])
+def test_gemm_of_a_few_tokens(ops, m, n, k, kind):
+    """Rows that end inside a tile of 16 and 32, k inside a piece of 64 bytes, fewer k-blocks than warps, every CTA size, up to 16 tokens where the
+    weights are widened; scale, bias and residual, both output types.  Bound: the roundings of fp32 sums of k products (none for integers),
+    tensor cores cutting each of them, then one ulp of the output type per epilogue step."""
+    g = torch.Generator().manual_seed(m * n + k)
+    if kind == "int8_wo_16":
+        m += 8
+    x = torch.randn(m, k, generator=g)
+    w = torch.randn(n, k, generator=g)
+    if kind in ("bf16", "int8_wo", "int8_wo_16"):
+        x = x.bfloat16()
+        xs = None
+    else:
+        x = x.clamp(-4, 4).to(torch.float8_e4m3fn) if kind == "fp8" else (20 * x).round().clamp(-127, 127).to(torch.int8)
+        xs = torch.rand(m, generator=g) + 0.5
+    if kind == "bf16":
+        w, ws = w.bfloat16(), None
+    else:
+        w = w.clamp(-4, 4).to(torch.float8_e4m3fn) if kind == "fp8" else (40 * w).round().clamp(-127, 127).to(torch.int8)
+        ws = torch.rand(n, generator=g) + 0.5
+    bias, res = torch.randn(n, generator=g).bfloat16(), torch.randn(m, n, generator=g).bfloat16()
+    dev = lambda t: None if t is None else t.cuda()  # noqa: E731
+    a64, w64 = x.double(), w.double()
+    scale = (1 if xs is None else xs.double()[:, None]) * (1 if ws is None else ws.double())
+    want = a64 @ w64.T * scale + bias.double() + res.double()
+    size = a64.abs() @ w64.abs().T * scale + bias.double().abs() + res.double().abs()
+    steps = 4 if kind == "int8" else 2 * k + 4
+    for dtype, ulp in ((torch.float32, 2.0**-24), (torch.bfloat16, 2.0**-8)):
+        out = ops.gemm(dev(x), dev(w), dev(xs), dev(ws), dev(bias), dev(res), out_dtype=dtype).double().cpu()
+        assert ((out - want).abs() <= steps * 2.0**-24 * size + ulp * want.abs() * 1.01).all()
+    again = ops.gemm(dev(x), dev(w), dev(xs), dev(ws), dev(bias), dev(res), out_dtype=torch.bfloat16)
+    assert torch.equal(again.double().cpu(), out)
+
+
+def test_gemm_of_a_few_tokens_on_any_boundary(ops):
+    """An output that starts on no 4-byte boundary."""
+    from vllm_neuron_b200 import _cabi
+
+    x, w = torch.randn(3, 256).bfloat16().cuda(), torch.randn(40, 256).bfloat16().cuda()
+    buf = torch.zeros(3 * 40 + 8, dtype=torch.bfloat16, device="cuda")
+    assert _cabi.load().b200_gemm(x.data_ptr(), w.data_ptr(), buf.data_ptr() + 2, 0, 0, 0, 0, 3, 40, 256, ops.BF16, ops.BF16, 0, 0, 0, 0) == 0
+    assert torch.equal(buf[1:121].view(3, 40), ops.gemm(x, w)) and not buf[121:].any() and not buf[0]

@@ -11,10 +11,10 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200_paged.so")
-SOURCES = ["host.cu", "kv_ops.cu", "paged_attn.cu", "paged_attn_prefill_tc.cu", "gemm_tcgen05.cu", "gemm_pair.cu", "gemm_group.cu", "gemm_wo.cu", "tp_allreduce.cu", "sampling.cu",
+SOURCES = ["host.cu", "kv_ops.cu", "paged_attn.cu", "paged_attn_prefill_tc.cu", "gemm_tcgen05.cu", "gemm_pair.cu", "gemm_group.cu", "gemm_wo.cu", "gemm_small.cu", "tp_allreduce.cu", "sampling.cu",
            "dyt_norm.cu", "ssm_scan.cu", "ssm_segment.cu", "swa_attn.cu", "swa_attn_prefill.cu", "swa_attn_prefill_tc.cu", "moe.cu", "rms_norm.cu", "delta_rule.cu",
            "latent_attn.cu", "gated_scan.cu", "selective_scan.cu", "hyper_conn.cu"]
-HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "gemm_common.cuh"), os.path.join(CSRC, "gemm_pair.cuh"), os.path.join(CSRC, "gemm_group.cuh"), os.path.join(CSRC, "hybrid_common.cuh"), os.path.join(CSRC, "ssm_common.cuh"), os.path.join(os.path.dirname(HERE), "include", "b200_paged.h")]
+HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "gemm_common.cuh"), os.path.join(CSRC, "gemm_pair.cuh"), os.path.join(CSRC, "gemm_group.cuh"), os.path.join(CSRC, "gemm_small.cuh"), os.path.join(CSRC, "hybrid_common.cuh"), os.path.join(CSRC, "ssm_common.cuh"), os.path.join(os.path.dirname(HERE), "include", "b200_paged.h")]
 BIND = os.path.join(HERE, "_b200_bind.so")  # the library's functions on torch tensors, for ops.py
 BIND_SOURCES = [os.path.join(CSRC, "bind.cpp"), os.path.join(os.path.dirname(HERE), "include", "b200_paged.h")]
 NVCC_FLAGS = [

@@ -7,6 +7,7 @@ namespace b200 {
 
 constexpr int GEMM_BN = 128;        // weight rows per tile  (UMMA M)
 constexpr int GEMM_BK_BYTES = 128;  // one 128B swizzle row of K per stage
+constexpr int KIND_WO8 = 3;         // beside UmmaKind: bf16 activations, int8 weights
 template <int KIND>
 struct KindTraits;
 template <>

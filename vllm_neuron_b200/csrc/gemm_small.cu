@@ -1,0 +1,303 @@
+// The weight GEMM for a few tokens: out[M, N] = epilogue(a[M, K] . w[N, K]^T), all operand kinds.
+//
+// At a few tokens a GEMM is its weights' bytes and a chain of latencies, and the decode schedule (gemm_tcgen05.cu) pays the chain: barrier set-up,
+// TMA round trips, tensor-memory allocation, partial tiles through a cluster.  Here a weight byte goes from memory into the register that
+// mma.sync reads it from: a lane loads 16 contiguous bytes of its row (four lanes a 64-byte piece, two loads a 128-byte line) and takes them
+// as the k slots of its fragments -- a sum does not care which k a slot holds, as long as the tokens' fragments are loaded alike.  No
+// shared memory before the sums meet, no barrier in the loop, and the first PF k-blocks of every warp are in flight BEFORE
+// griddepcontrol.wait: with 16 warps an SM the chip holds 19 MB of the next GEMM's weights while the kernel ahead finishes.
+//   * a CTA takes 16 MT weight rows (MT = 2: gate and up rows of a group, or the two halves of a head, which the epilogue needs together),
+//     its eight warps the k-blocks of 128 bytes in turn; partial sums meet in shared memory in warp order, so results do not depend on timing;
+//   * two accumulators per tile, so a chain of tensor-core sums is a sixteenth of K.
+#include "gemm_small.cuh"
+
+#include <limits.h>
+
+namespace b200 {
+
+__device__ __forceinline__ uint4 ldg_stream(const uint8_t* p) {  // weights are read once: they pass L1
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+template <int KIND>
+__device__ __forceinline__ void mma_small(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  if constexpr (KIND == KIND_F8F6F4)
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  else if constexpr (KIND == KIND_I8)
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  else
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// four int8 -> two bf16 pairs, in order (exact: 2^23 + 128 + w as a float, less 2^23 + 128)
+__device__ __forceinline__ uint2 widen4(uint32_t w) {
+  const uint32_t x = w ^ 0x80808080u;
+  const float f0 = __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7440)) - 8388736.f, f1 = __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7441)) - 8388736.f;
+  const float f2 = __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7442)) - 8388736.f, f3 = __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7443)) - 8388736.f;
+  return make_uint2(__byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632), __byte_perm(__float_as_uint(f2), __float_as_uint(f3), 0x7632));
+}
+
+// one 64-byte piece of 16 weight rows (lo: row g, hi: row g + 8) against the tokens' piece
+template <int KIND>
+__device__ __forceinline__ void mma_piece(uint32_t (&d)[4], const uint4& lo, const uint4& hi, const uint4 (&x)[KIND == KIND_WO8 ? 2 : 1]) {
+  if constexpr (KIND == KIND_WO8) {
+    const uint32_t l[4] = {lo.x, lo.y, lo.z, lo.w}, h[4] = {hi.x, hi.y, hi.z, hi.w};
+    const uint32_t b[8] = {x[0].x, x[0].y, x[0].z, x[0].w, x[1].x, x[1].y, x[1].z, x[1].w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint2 a = widen4(l[j]), c = widen4(h[j]);
+      mma_small<KIND>(d, a.x, c.x, a.y, c.y, b[2 * j], b[2 * j + 1]);
+    }
+  } else {
+    mma_small<KIND>(d, lo.x, hi.x, lo.y, hi.y, x[0].x, x[0].y);
+    mma_small<KIND>(d, lo.z, hi.z, lo.w, hi.w, x[0].z, x[0].w);
+  }
+}
+
+// NT: eights of tokens; MT: 16-row weight tiles; 16 warps on an SM, in CTAs of WARPS
+template <int KIND, int EPI, int NT, int MT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
+    gemm_small_kernel(const uint8_t* __restrict__ w, const uint8_t* __restrict__ a, const GemmEpilogue ep, int M, int N, int K) {
+  constexpr bool WO = KIND == KIND_WO8;
+  constexpr int THREADS = WARPS * 32;
+  constexpr int XE = WO ? 2 : 1;                                            // activation bytes per weight byte
+  constexpr int PF = MT * NT == 4 ? 1 : MT * NT == 2 ? 2 : WO ? 3 : 4;     // k-blocks of a warp in flight: what 128 registers hold
+  constexpr int ROWS = 16 * MT, TOK = 8 * NT, PITCH = TOK + 1;
+  constexpr int SIDES = EPI == EPI_LINEAR ? 1 : 2;                          // sums that an epilogue item takes
+  constexpr int ITEM_ROWS = ROWS / SIDES, ITEMS = ITEM_ROWS * TOK, PER = (ITEMS + THREADS - 1) / THREADS;
+  __shared__ float red[WARPS][ROWS * PITCH];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+  // first weight row of tile mt
+  int row0[MT];
+  if constexpr (EPI == EPI_ROPE) {
+    const int per = ep.rope.D / 32, head = blockIdx.x / per, j = blockIdx.x - head * per;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) row0[mt] = head * ep.rope.D + j * 16 + mt * (ep.rope.D >> 1);
+  } else {
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) row0[mt] = blockIdx.x * ROWS + mt * 16;
+  }
+  const int wrow = K * (KIND == KIND_F16 ? 2 : 1);  // bytes
+  const int nkb = (wrow + 127) >> 7;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  uint4 wb[PF][MT][4], xb[PF][2][NT][XE];
+  const uint8_t* wp[MT][2];
+  bool wok[MT][2];
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int hi = 0; hi < 2; ++hi) {
+      const int r = row0[mt] + g + 8 * hi;
+      wok[mt][hi] = r < N;
+      wp[mt][hi] = w + (int64_t)(r < N ? r : 0) * wrow + c * 16;
+    }
+  auto load_w = [&](uint4 (&b)[MT][4], int kb) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const int off = kb * 128 + p * 64;
+      const bool in = off + c * 16 < wrow;  // rows are whole 16-byte pieces
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int hi = 0; hi < 2; ++hi) b[mt][p * 2 + hi] = in && wok[mt][hi] ? ldg_stream(wp[mt][hi] + off) : zero;
+    }
+  };
+  auto load_x = [&](uint4 (&b)[2][NT][XE], int kb) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const int off = kb * 128 + p * 64 + c * 16;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int m = nt * 8 + g;
+#pragma unroll
+        for (int e = 0; e < XE; ++e)
+          b[p][nt][e] = off < wrow && m < M ? *reinterpret_cast<const uint4*>(a + ((int64_t)m * wrow + off) * XE + e * 16) : zero;
+      }
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < PF; ++s)
+    if (warp + s * WARPS < nkb) load_w(wb[s], warp + s * WARPS);
+  // the epilogue's operands of this thread's items: weights' side now, tokens' side while the products are taken
+  float wsc[PER][SIDES], bia[PER][SIDES], asc[PER], res[PER];
+  long long pos[PER], slot[PER];
+  const bool hb = ep.bias != nullptr, hr = EPI == EPI_LINEAR && ep.residual != nullptr;
+#pragma unroll
+  for (int q = 0; q < PER; ++q)
+#pragma unroll
+    for (int sd = 0; sd < SIDES; ++sd) {
+      const int i = threadIdx.x + q * THREADS, n = (SIDES == 1 ? row0[0] : row0[sd % MT]) + i % ITEM_ROWS;
+      wsc[q][sd] = i < ITEMS && n < N && ep.w_scale ? ep.w_scale[n] : 1.f;
+      bia[q][sd] = i < ITEMS && n < N && hb ? __bfloat162float(ep.bias[n]) : 0.f;
+    }
+  griddep_wait();
+#pragma unroll
+  for (int s = 0; s < PF; ++s)
+    if (warp + s * WARPS < nkb) load_x(xb[s], warp + s * WARPS);
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int i = threadIdx.x + q * THREADS, m = i / ITEM_ROWS, n = row0[0] + i % ITEM_ROWS;
+    const bool ok = i < ITEMS && m < M;
+    asc[q] = ok && ep.a_scale ? ep.a_scale[m] : 1.f;
+    res[q] = ok && hr && n < N ? __bfloat162float(ep.residual[(int64_t)m * N + n]) : 0.f;
+    if constexpr (EPI == EPI_ROPE) {
+      pos[q] = ok ? ep.rope.positions[m] : 0;
+      slot[q] = ok ? ep.rope.slot_mapping[m] : -1;
+      pos[q] = pos[q] < 0 ? 0 : pos[q] >= ep.rope.max_pos ? ep.rope.max_pos - 1 : pos[q];
+    }
+  }
+  uint32_t acc[2][MT][NT][4];
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[p][mt][nt][e] = 0u;
+  for (int kb = warp; kb < nkb; kb += PF * WARPS) {
+#pragma unroll
+    for (int s = 0; s < PF; ++s) {
+      const int k = kb + s * WARPS;
+      if (k < nkb) {
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) mma_piece<KIND>(acc[p][mt][nt], wb[s][mt][p * 2], wb[s][mt][p * 2 + 1], xb[s][p][nt]);
+        if (k + PF * WARPS < nkb) {
+          load_w(wb[s], k + PF * WARPS);
+          load_x(xb[s], k + PF * WARPS);
+        }
+      }
+    }
+  }
+  // Not earlier: CTAs of the next kernels that wait for this one hold registers that its own CTAs still need (a step of TinyLlama, one
+  // sequence, 1071 us with this at the top, 776 here; Llama 3.1 8B fp8, 6 layers, 520 and 510)
+  griddep_launch();
+  // ---- the warps' sums meet
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int r = mt * 16 + g + (e >= 2 ? 8 : 0), t = nt * 8 + 2 * c + (e & 1);
+        red[warp][r * PITCH + t] = KIND == KIND_I8 ? __int_as_float((int)(acc[0][mt][nt][e] + acc[1][mt][nt][e]))
+                                                   : __uint_as_float(acc[0][mt][nt][e]) + __uint_as_float(acc[1][mt][nt][e]);
+      }
+  __syncthreads();
+  auto total = [&](int r, int t) {
+    if constexpr (KIND == KIND_I8) {
+      int v = 0;
+#pragma unroll
+      for (int k = 0; k < WARPS; ++k) v += __float_as_int(red[k][r * PITCH + t]);
+      return (float)v;
+    } else {
+      float v[WARPS];  // by halves: log2 roundings
+#pragma unroll
+      for (int k = 0; k < WARPS; ++k) v[k] = red[k][r * PITCH + t];
+#pragma unroll
+      for (int o = WARPS / 2; o >= 1; o /= 2)
+#pragma unroll
+        for (int k = 0; k < o; ++k) v[k] += v[k + o];
+      return v[0];
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int i = threadIdx.x + q * THREADS, m = i / ITEM_ROWS, r = i % ITEM_ROWS;
+    const bool ok = i < ITEMS && m < M;
+    if constexpr (EPI == EPI_LINEAR) {
+      const int n = row0[0] + r;
+      if (!ok || n >= N) continue;
+      const float y = scaled_value(total(r, m), asc[q], wsc[q][0], hb, bia[q][0], hr, res[q]);
+      if (ep.out_f32) reinterpret_cast<float*>(ep.out)[(int64_t)m * N + n] = y;
+      else reinterpret_cast<__nv_bfloat16*>(ep.out)[(int64_t)m * N + n] = __float2bfloat16_rn(y);
+    } else {
+      const int mm = i < ITEMS ? m : 0;
+      const float lo = __bfloat162float(__float2bfloat16_rn(scaled_value(total(r, mm), asc[q], wsc[q][0], hb, bia[q][0], false, 0.f)));
+      const float hi = __bfloat162float(__float2bfloat16_rn(scaled_value(total(16 + r, mm), asc[q], wsc[q][1], hb, bia[q][1], false, 0.f)));
+      if constexpr (EPI == EPI_SILU_MUL) {  // whole groups of 32 rows: N is a multiple of 32
+        const float v = silu_mul_bf16(lo, hi);
+        float x = fabsf(v);
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+        if (!ok) continue;
+        reinterpret_cast<__nv_bfloat16*>(ep.out)[(int64_t)m * (N >> 1) + blockIdx.x * 16 + r] = __float2bfloat16_rn(v);
+        if (r == 0) ep.group_amax[(int64_t)m * (N >> 5) + blockIdx.x] = x;
+      } else {
+        if (!ok) continue;
+        const auto& rp = ep.rope;
+        const int half = rp.D >> 1, head = row0[0] / rp.D, d = row0[0] - head * rp.D + r;
+        const bool is_q = head < rp.Hq, roped = head < rp.Hq + rp.Hkv;
+        float o1 = lo, o2 = hi;
+        if (roped) {
+          const float cc = rp.cos_t[pos[q] * half + d], ss = rp.sin_t[pos[q] * half + d];
+          o1 = __fsub_rn(__fmul_rn(lo, cc), __fmul_rn(hi, ss));
+          o2 = __fadd_rn(__fmul_rn(hi, cc), __fmul_rn(lo, ss));
+        }
+        // the row keeps what the GEMM and the rotation kernel leave there: rotated q, k and v as they are
+        __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(ep.out) + (int64_t)m * N + row0[0] + r;
+        orow[0] = __float2bfloat16_rn(is_q ? o1 : lo);
+        orow[half] = __float2bfloat16_rn(is_q ? o2 : hi);
+        if (!is_q && slot[q] >= 0 && slot[q] < rp.num_slots) {
+          const long long blk = slot[q] / rp.bs;
+          const int off = (int)(slot[q] - blk * rp.bs);
+          __nv_bfloat16* dst = (roped ? rp.k_pool : rp.v_pool) + ((blk * rp.Hkv + head - rp.Hq - (roped ? 0 : rp.Hkv)) * rp.bs + off) * rp.D + d;
+          dst[0] = __float2bfloat16_rn(o1);
+          dst[half] = __float2bfloat16_rn(o2);
+        }
+      }
+    }
+  }
+}
+
+// Which calls the kernel takes: up to 8 tokens all of them, 9 to 16 the weight-only ones.  Chained launches over weights larger than L2, us, decode
+// schedule / here, one token: bf16 2048 x 2048 4.7 / 2.5, 2048 x 5632 8.3 / 5.1, 11264 x 2048 gate and up 12.6 / 9.8, 4096 x 14336 25.7 / 19.4, 28672 x 4096
+// gate and up 48.8 / 41.5; fp8 4.0 / 2.3, 5.8 / 3.6, 7.8 / 7.1, 14.9 / 11.0, 25.5 / 25.7; weight-only 7.1 / 2.8, 11.3 / 4.4, 12.5 / 9.6, 26.1 / 18.8, 39.4 / 33.7.
+// Decode steps at 500 tokens of context, one token: TinyLlama bf16 1026 / 776; Llama 3.1 8B, 6 layers, bf16 813 / 727, fp8 550 / 510, 8 tokens weight-only
+// 823 / 680; Qwen2.5 32B, 2 layers, 4 tokens, bf16 673 / 610 -- with all of a layer's GEMMs on one schedule: a decode-schedule GEMM behind one of these
+// finds no room for its rings (Qwen 883 where only its 5120 x 27648 stayed, which alone is 55 there and 57 here).
+// 9 to 16 tokens load twice the fragments a weight: 16 tokens, 8B bf16 820 / 898, fp8 572 / 667; weight-only, whose decode schedule
+// widens in a pass of its own, 858 / 742, TinyLlama 1235 / 908, Qwen 598 / 596.
+bool gemm_small_ok(const void* a, const void* w, int epi, int M, int N, int K, int ab_dtype, int head_dim) {
+  const int64_t row = (int64_t)K * (ab_dtype == B200_BF16 ? 2 : 1);
+  if (M > (ab_dtype == B200_INT8_WO ? 16 : 8) || row % 16 || (((uintptr_t)a | (uintptr_t)w) & 15) || row * 2 > INT_MAX) return false;
+  return epi == EPI_LINEAR || epi == EPI_SILU_MUL || (epi == EPI_ROPE && head_dim % 32 == 0);
+}
+
+template <int KIND, int EPI, int NT, int MT, int WARPS>
+static int launch_small(const void* a, const void* w, const GemmEpilogue& ep, int M, int N, int K, cudaStream_t s) {
+  B200_CUDA_OK(launch_kernel(gemm_small_kernel<KIND, EPI, NT, MT, WARPS>, dim3((N + 16 * MT - 1) / (16 * MT)), dim3(WARPS * 32), 0, s,
+                             (const uint8_t*)w, (const uint8_t*)a, ep, M, N, K));
+  return B200_OK;
+}
+// CTAs of 16 rows while they fit the chip once (16 warps of one SM share a long row, or 8), then of 32 rows; where those are many, four warps
+// each, so that more of them are in flight and the last wave is short.  Measured, bf16, one token, us: 2048 x 5632 with 16 / 8 warps 5.1 / 6.2,
+// 2048 x 2048 2.6 / 2.5, 4096 x 4096 7.4 / 6.4; 6144 x 4096 16 / 32 rows 11.3 / 10.2; 10272 x 2048 8 / 4 warps 10.2 / 9.2, 32000 x 2048 22.8 / 21.8.
+template <int KIND, int NT>
+static int pick_small(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, cudaStream_t s) {
+  if (epi == EPI_SILU_MUL) return launch_small<KIND, EPI_SILU_MUL, NT, 2, 4>(a, w, ep, M, N, K, s);
+  if (epi == EPI_ROPE) return launch_small<KIND, EPI_ROPE, NT, 2, 8>(a, w, ep, M, N, K, s);
+  const int tiles = (N + 15) / 16, sms = sm_count(), row = K * (KIND == KIND_F16 ? 2 : 1);
+  if (tiles <= sms && row > 4096) return launch_small<KIND, EPI_LINEAR, NT, 1, 16>(a, w, ep, M, N, K, s);
+  if (tiles <= 2 * sms) return launch_small<KIND, EPI_LINEAR, NT, 1, 8>(a, w, ep, M, N, K, s);
+  if (tiles <= 4 * sms) return launch_small<KIND, EPI_LINEAR, NT, 2, 8>(a, w, ep, M, N, K, s);
+  return launch_small<KIND, EPI_LINEAR, NT, 2, 4>(a, w, ep, M, N, K, s);
+}
+
+int launch_gemm_small(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, cudaStream_t s) {
+  if (ab_dtype == B200_BF16) return pick_small<KIND_F16, 1>(a, w, ep, epi, M, N, K, s);
+  if (ab_dtype == B200_FP8_E4M3) return pick_small<KIND_F8F6F4, 1>(a, w, ep, epi, M, N, K, s);
+  if (ab_dtype == B200_INT8) return pick_small<KIND_I8, 1>(a, w, ep, epi, M, N, K, s);
+  return M <= 8 ? pick_small<KIND_WO8, 1>(a, w, ep, epi, M, N, K, s) : pick_small<KIND_WO8, 2>(a, w, ep, epi, M, N, K, s);
+}
+
+}  // namespace b200

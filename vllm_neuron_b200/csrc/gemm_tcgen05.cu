@@ -30,6 +30,7 @@
 #include <tuple>
 
 #include "gemm_common.cuh"
+#include "gemm_small.cuh"
 
 namespace b200 {
 
@@ -38,7 +39,6 @@ constexpr int GEMM_CNT_INTS = 1024;  // fix-up counters at the head of the works
 
 // INT8 weight-only (W8A16): bf16 activations, int8 weights streamed from HBM as int8 and widened to bf16 inside the
 // kernel (exact: |w| <= 127), then kind::f16.  The per-channel scale is applied in the epilogue like the other kinds.
-constexpr int KIND_WO8 = 3;
 template <>
 struct KindTraits<KIND_WO8> {
   static constexpr int ELEM = 2, CFMT = 1, ABFMT = 1;
@@ -1283,6 +1283,8 @@ int gemm_common(const void* a, const void* w, const GemmEpilogue& ep, int epi, i
     set_last_error("gemm: workspace %zu < %zu bytes", workspace_bytes, p.ws_bytes);
     return B200_ERR_WORKSPACE;
   }
+  if (split_k == 0 && gemm_small_ok(a, w, epi, M, N, K, ab_dtype, ep.rope.D))
+    return launch_gemm_small(a, w, ep, epi, M, N, K, ab_dtype, (cudaStream_t)stream);
   // the cut decode schedule writes vectors of four: an output that is not aligned to them keeps the uncut one, which writes single values
   const bool wide = p.decode && wo && split_k == 0 && epi != EPI_ROPE && gemm_wo_wide(epi, M, N, K);
   const uintptr_t vec_bytes = ep.out_f32 ? 16 : 8;
@@ -1375,6 +1377,14 @@ int b200_gemm_decode_plan(int M, int N, int K, int ab_dtype, int split_k, int si
   int rc = plan_gemm(p, M, N, K, ab_dtype, split_k);
   if (rc) return rc;
   const int epi = silu_mul == 2 ? EPI_ROPE : silu_mul ? EPI_SILU_MUL : EPI_LINEAR;
+  if (split_k == 0 && gemm_small_ok(nullptr, nullptr, epi, M, N, K, ab_dtype, 64)) {  // no cluster, no shared-memory rings
+    out6[0] = 1;
+    out6[1] = 2;
+    out6[2] = out6[3] = 2;  // k-blocks of a warp in flight, at least
+    out6[4] = 2 * sm_count();  // at 8 warps
+    out6[5] = 0;
+    return B200_OK;
+  }
   if (ab_dtype == B200_INT8_WO && split_k == 0 && gemm_wo_wide(epi, M, N, K)) {  // the rotation is a launch of its own there
     size_t smem;
     rc = gemm_wo_plan(epi, M, N, K, out6[0], out6[4], out6[2], smem);
@@ -1445,6 +1455,7 @@ int b200_gemm_rope_kv_write(const void* a, const void* w, void* qkv_out, const f
     int plan6[6];
     if (b200_gemm_decode_plan(M, N, K, ab_dtype, split_k, 2, 0, plan6) == B200_OK && plan6[0] > 1) fused = true;
   }
+  if (split_k == 0 && max_pos > 0 && gemm_small_ok(a, w, EPI_ROPE, M, N, K, ab_dtype, D)) fused = true;
   static const bool no_fuse = getenv("B200_NO_ROPE_FUSION") != nullptr;  // A/B aid
   if (fused && !no_fuse) {
     ep.rope = {positions, slot_mapping, cos_table, sin_table, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool,
