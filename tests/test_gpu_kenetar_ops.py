@@ -236,6 +236,40 @@ def test_delta_rule_in_rounds_of_eight_tokens(H, G, D, P):
     test_delta_rule_portions_slots_and_sizes(H, G, D, P)
 
 
+@pytest.mark.parametrize("H,G,D,P", [(4, 2, 128, 128), (2, 1, 128, 40), (3, 3, 64, 64), (2, 1, 64, 70), (1, 1, 128, 3)])
+@pytest.mark.parametrize("longest", [1, 2])
+def test_delta_rule_of_one_token_each(H, G, D, P, longest):
+    """Decode steps: value columns that end inside a warp's rows, a sequence at position 0 over a used slot, slots in any order; `longest` 1 may be
+    said of a portion of three tokens too.  Bound: the roundings of fp32 sums of D products, a few of them behind one another."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(D + P)
+    n = [1, 1, 3] if longest == 1 else [1, 2, 1]
+    entries = [(2, 7, n[0]), (0, 0, n[1]), (3, 30, n[2])]
+    T, C = sum(n), 2 * G * D + H * P
+    qkv, proj = torch.randn(T, C, generator=g), torch.randn(T, 2 * H, generator=g)
+    A_log, dt_bias, state = torch.log(0.5 + torch.rand(H, generator=g)), torch.randn(H, generator=g), torch.randn(5, H, P, D, generator=g)
+    meta = _meta(entries, {r: list(range(1, 40)) for r in range(5)})
+    meta.max_new = longest
+    got = state.to(DEV)
+    o = ops.delta_rule(qkv.to(DEV), proj.to(DEV), 0, H, A_log.to(DEV), dt_bias.to(DEV), got, meta, H, G, D, P, D ** -0.5).double().cpu().view(T, H, P)
+    q, k, v = (x.view(T, -1, c) for x, c in zip(qkv.double().split([G * D, G * D, H * P], -1), (D, D, P)))
+    unit = lambda a: (a / torch.sqrt(a.pow(2).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(H // G, 1)  # noqa: E731
+    q, k = unit(q) * D ** -0.5, unit(k)
+    beta, gd = torch.sigmoid(proj[:, :H].double()), torch.exp(-torch.exp(A_log.double()) * F.softplus(proj[:, H:].double() + dt_bias.double()))
+    at = 0
+    for r, pos0, c in entries:
+        S = state[r].double() if pos0 else torch.zeros(H, P, D, dtype=torch.float64)
+        size = S.abs().amax() + v.abs().amax()
+        for t in range(at, at + c):
+            S = gd[t, :, None, None] * S
+            u = beta[t, :, None] * (v[t] - (S @ k[t, :, :, None]).squeeze(-1))
+            S = S + u[:, :, None] * k[t, :, None]
+            assert ((o[t] - (S @ q[t, :, :, None]).squeeze(-1)).abs() <= 3 * c * D * 2.0**-24 * size).all()
+        assert ((got[r].double().cpu() - S).abs() <= 3 * c * D * 2.0**-24 * size).all()
+        at += c
+    assert torch.equal(got[[1, 4]].cpu(), state[[1, 4]])
+
+
 def test_delta_rule_write_is_visible_to_its_own_readout_and_decay_comes_first():
     """One head, hand-made numbers: with S = 0, o_1 = beta (k.q) v (the read-out sees the token's own write); the second
     token's prediction uses the DECAYED state."""

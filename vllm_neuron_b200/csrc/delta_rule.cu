@@ -570,6 +570,74 @@ __global__ void __launch_bounds__(DR_MAIN + DR_AUX, 2)
           make_float4(S[c][2 * r].x, S[c][2 * r].y, S[c][2 * r + 1].x, S[c][2 * r + 1].y);
 }
 
+// Steps of one token per sequence: nothing is walked, so the state rows [P][D] pass through registers once as 16-byte pieces, D / 4 lanes a row,
+// 8 rows a warp, whose 16 sums are reduced together by halving.  Bound by the state's bytes, read and written: 64 sequences, 16 heads of
+// 128 x 128 (134 MB, 20 us), with delta_prep in front, L2 flushed, 64.5 us by the kernel above (staged tokens, two barriers), 27.6 by this one;
+// 33 sequences 39.8 / 21.5, 4 sequences 17.4 / 13.3; heads of 64 x 64, 64 sequences 33.6 / 17.3.  Errors as before (o 1.0e-7, S 5.8e-8).
+constexpr int DSTEP_ROWS = 8, DSTEP_WARPS = 4;
+template <int LANES>
+__global__ void __launch_bounds__(DSTEP_WARPS * 32)
+    delta_step_kernel(const float* __restrict__ qkv, int ldc, const float* __restrict__ bg, const float* __restrict__ kq,
+                      float* __restrict__ state, const int32_t* __restrict__ seq_start, const int32_t* __restrict__ seq_slot,
+                      const int32_t* __restrict__ seq_pos0, float* __restrict__ out, int H, int G, int P) {
+  constexpr int D = 4 * LANES, PER = 32 / LANES;
+  griddep_launch();
+  griddep_wait();
+  const int sq = blockIdx.z, h = blockIdx.y, t0 = seq_start[sq], t1 = seq_start[sq + 1];
+  if (t0 >= t1) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / LANES, l = lane % LANES, gh = h / (H / G);
+  const int row0 = (blockIdx.x * DSTEP_WARPS + warp) * DSTEP_ROWS * PER;  // rows row0 + i PER + sub
+  if (row0 >= P) return;
+  float* sp = state + (((int64_t)seq_slot[sq] * H + h) * P + row0 + sub) * D + l * 4;
+  const bool old = seq_pos0[sq] > 0;
+  float4 S[DSTEP_ROWS];
+#pragma unroll
+  for (int i = 0; i < DSTEP_ROWS; ++i)
+    S[i] = old && row0 + i * PER + sub < P ? *reinterpret_cast<const float4*>(sp + (int64_t)i * PER * D) : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int t = t0; t < t1; ++t) {  // one turn in a decode step; a longer portion is only slower
+    const float* row = qkv + (int64_t)t * ldc;
+    const float4 q = *reinterpret_cast<const float4*>(row + (int64_t)gh * D + l * 4), k = *reinterpret_cast<const float4*>(row + (int64_t)(G + gh) * D + l * 4);
+    const float beta = bg[(int64_t)t * 2 * H + h], gd = bg[(int64_t)t * 2 * H + H + h], kqd = kq[(int64_t)t * G + gh];
+    float v[2 * DSTEP_ROWS];
+#pragma unroll
+    for (int i = 0; i < DSTEP_ROWS; ++i) {
+      v[i] = (S[i].x * k.x + S[i].y * k.y) + (S[i].z * k.z + S[i].w * k.w);
+      v[DSTEP_ROWS + i] = (S[i].x * q.x + S[i].y * q.y) + (S[i].z * q.z + S[i].w * q.w);
+    }
+    int mine = 0, off = LANES / 2;  // mine: the row whose two sums this lane ends up with
+#pragma unroll
+    for (int m = DSTEP_ROWS / 2; m >= 1; m /= 2, off /= 2) {
+      const bool up = l & off;
+      mine += up ? m : 0;
+#pragma unroll
+      for (int i = 0; i < m; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          float* b = v + e * DSTEP_ROWS;
+          const float keep = up ? b[i + m] : b[i], give = up ? b[i] : b[i + m];
+          b[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+    }
+#pragma unroll
+    for (int o = LANES / 2 / DSTEP_ROWS; o >= 1; o /= 2) {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+      v[DSTEP_ROWS] += __shfl_xor_sync(0xffffffffu, v[DSTEP_ROWS], o);
+    }
+    const int p = row0 + mine * PER + sub;
+    const float u = p < P ? beta * (row[2 * (int64_t)G * D + (int64_t)h * P + p] - gd * v[0]) : 0.f;
+    if (l % (LANES / DSTEP_ROWS) == 0 && p < P) out[((int64_t)t * H + h) * P + p] = gd * v[DSTEP_ROWS] + u * kqd;
+#pragma unroll
+    for (int i = 0; i < DSTEP_ROWS; ++i) {
+      // row i's value sits in the lanes whose bits spell i
+      const float w = __shfl_sync(0xffffffffu, u, sub * LANES + ((i & 4) ? LANES / 2 : 0) + ((i & 2) ? LANES / 4 : 0) + ((i & 1) ? LANES / 8 : 0));
+      S[i] = make_float4(fmaf(gd, S[i].x, k.x * w), fmaf(gd, S[i].y, k.y * w), fmaf(gd, S[i].z, k.z * w), fmaf(gd, S[i].w, k.w * w));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < DSTEP_ROWS; ++i)
+    if (row0 + i * PER + sub < P) *reinterpret_cast<float4*>(sp + (int64_t)i * PER * D) = S[i];
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -594,6 +662,18 @@ int b200_delta_scan(const float* qkv, int ldc, const float* beta_decay, const fl
   B200_REQUIRE(H > 0 && G > 0 && H % G == 0, "delta_scan: %d heads over %d key heads", H, G);
   B200_REQUIRE(D >= 1 && D <= 1024 && P >= 1, "delta_scan: key size %d (1..1024 supported)", D);
   if (B <= 0) return B200_OK;
+  // decode steps on rows of whole 16-byte pieces (the kernel's own condition)
+  if (max_new == 1 && (D == 64 || D == 128) && ldc % 4 == 0 && H <= 65535 && B <= 65535 && !(((uintptr_t)qkv | (uintptr_t)state) & 15)) {
+    const int rows = DSTEP_WARPS * DSTEP_ROWS * (128 / D);
+    const dim3 grid((P + rows - 1) / rows, H, B);
+#define DSTEP_LAUNCH(LANES)                                                                                                               \
+  B200_CUDA_OK(launch_kernel(delta_step_kernel<LANES>, grid, dim3(DSTEP_WARPS * 32), 0, (cudaStream_t)stream, qkv, ldc, beta_decay, kq,   \
+                             state, seq_start, seq_slot, seq_pos0, out, H, G, P))
+    if (D == 128) DSTEP_LAUNCH(32);
+    else DSTEP_LAUNCH(16);
+#undef DSTEP_LAUNCH
+    return B200_OK;
+  }
   // Rounds of eight tokens once a portion fills one; shorter steps stay with the kernel that lets more CTAs share an SM.  Two-token
   // rounds -> rounds of eight at 16 heads of 128 x 128: one portion of 8 tokens 10.2 -> 9.6 us, of 4096 936 -> 522, eight of 512
   // 503 -> 367, 32 of 8 61 -> 59, one of 8 beside 31 decoded tokens 37 -> 31, 1210 and 333 beside 29 decoded tokens 392 -> 246; 8 heads of
