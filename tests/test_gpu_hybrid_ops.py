@@ -352,6 +352,12 @@ def test_fp32_linear_tiles(m, n, k):
     assert ((got - a.double() @ w.double().T).abs() <= k * 2.0**-24 * (a.abs().double() @ w.abs().double().T)).all()
 
 
+@pytest.mark.parametrize("m,n,k", [(97, 7233, 68), (33, 8, 36), (10, 13, 132), (301, 16, 1024), (7, 40, 100), (64, 64, 96)])
+def test_fp32_linear_many_tiles_and_narrow_rows(m, n, k):
+    """Batches of many tiles (64 x 32), fewer slices than stages, and a few outputs per row (a warp per two rows, an odd row left)."""
+    test_fp32_linear_tiles(m, n, k)
+
+
 @pytest.mark.parametrize("H,P,N,G", [(4, 128, 128, 2), (4, 64, 64, 4), (2, 64, 128, 1), (2, 128, 64, 2)])
 @pytest.mark.parametrize("shift", [-2.0, -6.0])
 @pytest.mark.parametrize("cut", [128, 150])

@@ -276,16 +276,15 @@ __global__ void __launch_bounds__(GL_THREADS)
 }
 
 // ---------------------------------------------------------------- fp32 operands: the same contract at the rate of the FMA pipes
-// True fp32 products and sums, so the ceiling is the chip's 74 TFLOP/s of fp32 FMAs; the kernel above stood at 4: scalar loads, 8 FMAs for
-// 6 shared-memory reads, no copy in flight.  Here a thread owns TM rows x TN outputs as packed fp32 pairs (fma.rn.f32x2: two rows per
-// instruction), operands go through two K = 32 slices in shared memory laid out [k][row] -- 4-row chunks exchanged by k so that the
-// transposing stores and the 16-byte reads are both free of bank conflicts -- and the next slice's global loads are in flight under the
-// FMAs.  With batches of a few hundred rows a tile per SM is all there is, and one warp per scheduler cannot hide its own latencies: KG
-// groups of threads take every KG-th k of a slice each and add their sums at the end, in order.
-// Tiles: 64 x 32 (8 x 4 per thread: 16 FMA instructions for 3 reads) for dense batches, 32 x 32 where those leave half the SMs idle; 32 x
-// 64 for expert tiles, whose rows come in 32s; 8 x 32 (8 x 1) for a handful of rows, where reading the weights is all there is.
+// True fp32 products and sums, so the ceiling is the chip's 74 TFLOP/s of fp32 FMAs.  With batches of a few hundred rows a tile or two per SM is
+// all there is, so what bounds it is the latency of a K slice: one slice ahead in registers, transposed into shared memory, cost 0.65 us per
+// 32 k whatever the tile.  Here FL_STAGES slices of 32 k are on their way by cp.async, rows as they lie (128 bytes, 16-byte pieces exchanged by
+// row so that eight rows' pieces of one k are conflict-free), and a thread multiplies k pairs: both factors are the pairs that a 16-byte read
+// holds (fma.rn.f32x2), a sum's two halves meet at the end.  Thread rows and columns are dealt round-robin (ty + RY i, tx + CX j).
+// KG groups of threads take every KG-th piece of a slice each and add their sums at the end, in order.
 // Needs K % 4 == 0 and 16-byte aligned rows; anything else stays on the kernel above.
 constexpr int FL_BK = 32;
+constexpr int FL_STAGES = 4;
 
 template <int BM, int BN, int TM, int TN, int KG, int EPI>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN) * KG)
@@ -296,15 +295,14 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN) * KG)
                        const float* __restrict__ gate, int gate_ld, int gate_cols) {
   griddep_launch();
   griddep_wait();
-  constexpr int NG = (BM / TM) * (BN / TN), NT = NG * KG, CX = BN / TN;  // threads of a k group, of the CTA
-  constexpr int AV = BM * FL_BK / 4, WV = BN * FL_BK / 4;                 // 16-byte pieces of a slice
-  constexpr int AL = (AV + NT - 1) / NT, WL = (WV + NT - 1) / NT;         // per thread
-  constexpr int OUTS = EPI == GL_EPI_GLU ? BN / 2 : BN;                   // GLU: a thread's 4 columns are 2 gates and their 2 ups
-  static_assert(EPI != GL_EPI_GLU || TN == 4, "gate / up columns come in fours");
-  __shared__ __align__(16) float slices[2 * FL_BK * (BM + BN)];
-  float (*As)[FL_BK][BM] = reinterpret_cast<float (*)[FL_BK][BM]>(slices);
-  float (*Ws)[FL_BK][BN] = reinterpret_cast<float (*)[FL_BK][BN]>(slices + 2 * FL_BK * BM);
-  static_assert((KG - 1) * BM * BN <= 2 * FL_BK * (BM + BN), "the groups' sums meet where the slices were");
+  constexpr int RY = BM / TM, CX = BN / TN, NG = RY * CX, NT = NG * KG;   // threads of a k group, of the CTA
+  constexpr int PIECES = FL_BK / 4;                                       // 16-byte pieces of a row's slice
+  constexpr int AL = (BM * PIECES + NT - 1) / NT, WL = (BN * PIECES + NT - 1) / NT;
+  constexpr int OUTS = EPI == GL_EPI_GLU ? BN / 2 : BN;                   // GLU: a thread's columns are gates and their ups in turn
+  static_assert(EPI != GL_EPI_GLU || TN % 2 == 0, "gate and up columns of an output belong to one thread");
+  constexpr int STAGE = (BM + BN) * FL_BK;  // floats: A rows, then W rows
+  __shared__ __align__(128) float slices[FL_STAGES * STAGE];
+  static_assert((KG - 1) * BM * BN <= FL_STAGES * STAGE, "the groups' sums meet where the slices were");
   const int tile = blockIdx.x;
   if (num_tiles && tile >= *num_tiles) return;
   const int e = tile_expert ? tile_expert[tile] : blockIdx.z;
@@ -312,161 +310,130 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN) * KG)
   a += (int64_t)blockIdx.z * a_zs;
   const int n0 = blockIdx.y * OUTS;
   const int tid = threadIdx.x, kg = tid / NG, tx = tid % CX, ty = tid % NG / CX;
-  // (source row, destination row, scale) of tile row r
-  auto src_of = [&](int r, float& sc) -> int {
-    const int row = tile * BM + r;
-    sc = 1.0f;
-    if (!sorted_ids) return row < M ? row : -1;
-    const int id = sorted_ids[row];
-    if (id < 0) return -1;
-    if (row_scale) sc = row_scale[id];
-    return gather_div > 0 ? id / gather_div : row;
-  };
-  const float* ap[AL];
-  float as[AL];
+  const float *ap[AL], *wp[WL];  // this thread's pieces of a slice (NULL: zeros)
 #pragma unroll
   for (int i = 0; i < AL; ++i) {
     const int id = tid + i * NT;
     ap[i] = nullptr;
-    as[i] = 1.0f;
-    if (id < AV) {
-      const int r = src_of(id / (FL_BK / 4), as[i]);
-      if (r >= 0) ap[i] = a + (int64_t)r * lda + (id % (FL_BK / 4)) * 4;
+    if (id < BM * PIECES) {
+      const int row = tile * BM + id / PIECES;
+      int src = row < M ? row : -1;
+      if (sorted_ids) {
+        const int pair = sorted_ids[row];
+        src = pair < 0 ? -1 : gather_div > 0 ? pair / gather_div : row;
+      }
+      if (src >= 0) ap[i] = a + (int64_t)src * lda + id % PIECES * 4;
     }
   }
-  const float* wp[WL];
 #pragma unroll
   for (int i = 0; i < WL; ++i) {
-    const int id = tid + i * NT, c = id / (FL_BK / 4);
-    const int n = EPI == GL_EPI_GLU ? n0 + (c >> 2) * 2 + (c & 1) : n0 + c;
-    wp[i] = id < WV && n < N ? we + ((int64_t)((EPI == GL_EPI_GLU && (c & 2)) ? N : 0) + n) * K + (id % (FL_BK / 4)) * 4 : nullptr;
+    const int id = tid + i * NT, c = id / PIECES;
+    const int n = EPI == GL_EPI_GLU ? n0 + c / CX / 2 * CX + c % CX : n0 + c;
+    wp[i] = id < BN * PIECES && n < N ? we + ((int64_t)(EPI == GL_EPI_GLU && (c / CX & 1) ? N : 0) + n) * K + id % PIECES * 4 : nullptr;
   }
-  float4 ra[AL], rw[WL];
-  auto fetch = [&](int k0) {
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+  const uint32_t sm0 = smem_u32(slices);
+  auto issue = [&](int it) {
+    const int k0 = it * FL_BK;
+    if (k0 < K) {
+      const uint32_t dst = sm0 + (uint32_t)(it % FL_STAGES) * STAGE * 4;
 #pragma unroll
-    for (int i = 0; i < AL; ++i) {
-      const int k4 = (tid + i * NT) % (FL_BK / 4);
-      ra[i] = ap[i] && k0 + 4 * k4 < K ? *reinterpret_cast<const float4*>(ap[i] + k0) : z;
-      ra[i] = make_float4(ra[i].x * as[i], ra[i].y * as[i], ra[i].z * as[i], ra[i].w * as[i]);
-    }
+      for (int i = 0; i < AL; ++i) {
+        const int id = tid + i * NT, r = id / PIECES, p = id % PIECES;
+        const bool ok = ap[i] && k0 + p * 4 < K;
+        if (AL * NT == BM * PIECES || id < BM * PIECES) cp_async16(dst + r * 128 + ((p ^ (r & 7)) << 4), ok ? ap[i] + k0 : a, ok);
+      }
 #pragma unroll
-    for (int i = 0; i < WL; ++i) {
-      const int k4 = (tid + i * NT) % (FL_BK / 4);
-      rw[i] = wp[i] && k0 + 4 * k4 < K ? *reinterpret_cast<const float4*>(wp[i] + k0) : z;
+      for (int i = 0; i < WL; ++i) {
+        const int id = tid + i * NT, r = id / PIECES, p = id % PIECES;
+        const bool ok = wp[i] && k0 + p * 4 < K;
+        if (WL * NT == BN * PIECES || id < BN * PIECES) cp_async16(dst + (BM + r) * 128 + ((p ^ (r & 7)) << 4), ok ? wp[i] + k0 : w, ok);
+      }
     }
+    cp_async_commit();  // an empty group past the end keeps the wait counts uniform
   };
-  // column of row r in the slice row of k: its 4-row chunk exchanged by k (chunks of 8-row tiles: two only)
-  auto swz = [](int r, int k, int rows) { return r ^ ((((k >> 3) & 3) << 2) & (rows - 1)); };
-  auto park = [&](int b) {
+  float2 acc[TM][TN];  // sums over even and over odd k
 #pragma unroll
-    for (int i = 0; i < AL; ++i) {
-      const int id = tid + i * NT, r = id / (FL_BK / 4), k = (id % (FL_BK / 4)) * 4;
-      if (AV % NT && id >= AV) continue;
-      const int c = swz(r, k, BM);
-      As[b][k][c] = ra[i].x;
-      As[b][k + 1][c] = ra[i].y;
-      As[b][k + 2][c] = ra[i].z;
-      As[b][k + 3][c] = ra[i].w;
-    }
-#pragma unroll
-    for (int i = 0; i < WL; ++i) {
-      const int id = tid + i * NT, r = id / (FL_BK / 4), k = (id % (FL_BK / 4)) * 4;
-      if (WV % NT && id >= WV) continue;
-      const int c = swz(r, k, BN);
-      Ws[b][k][c] = rw[i].x;
-      Ws[b][k + 1][c] = rw[i].y;
-      Ws[b][k + 2][c] = rw[i].z;
-      Ws[b][k + 3][c] = rw[i].w;
-    }
-  };
-  float2 acc[TM / 2][TN];  // rows 2 i, 2 i + 1 of this thread
-#pragma unroll
-  for (int i = 0; i < TM / 2; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
-  fetch(0);
-  park(0);
-  __syncthreads();
-  int b = 0;
-  for (int k0 = 0; k0 < K; k0 += FL_BK, b ^= 1) {
-    const bool more = k0 + FL_BK < K;
-    if (more) fetch(k0 + FL_BK);
 #pragma unroll
-    for (int kk = 0; kk < FL_BK / KG; ++kk) {
-      const int k = kk * KG + kg;
-      float4 af[TM / 4];
+  for (int i = 0; i < FL_STAGES - 1; ++i) issue(i);
+  const int its = (K + FL_BK - 1) / FL_BK;
+  for (int it = 0; it < its; ++it) {
+    cp_async_wait<FL_STAGES - 2>();
+    __syncthreads();  // slice `it` is there for everyone, and everyone has left the one before it
+    issue(it + FL_STAGES - 1);
+    const float* As = slices + it % FL_STAGES * STAGE;
+    const float* Ws = As + BM * FL_BK;
 #pragma unroll
-      for (int i = 0; i < TM / 4; ++i) af[i] = *reinterpret_cast<const float4*>(&As[b][k][swz(ty * TM + 4 * i, k, BM)]);
-      float wf[TN];
-      if constexpr (TN == 4) {
-        const float4 v = *reinterpret_cast<const float4*>(&Ws[b][k][swz(tx * 4, k, BN)]);
-        wf[0] = v.x, wf[1] = v.y, wf[2] = v.z, wf[3] = v.w;
-      } else {
-        wf[0] = Ws[b][k][swz(tx, k, BN)];
+    for (int q = 0; q < PIECES / KG; ++q) {
+      const int p = q * KG + kg;
+      float4 af[TM];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const int r = ty + RY * i;
+        af[i] = *reinterpret_cast<const float4*>(As + r * FL_BK + ((p ^ (r & 7)) << 2));
       }
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
-        const float2 ww = make_float2(wf[j], wf[j]);
+        const int c = tx + CX * j;
+        const float4 wf = *reinterpret_cast<const float4*>(Ws + c * FL_BK + ((p ^ (c & 7)) << 2));
 #pragma unroll
-        for (int i = 0; i < TM / 4; ++i) {
-          acc[2 * i][j] = ffma2(make_float2(af[i].x, af[i].y), ww, acc[2 * i][j]);
-          acc[2 * i + 1][j] = ffma2(make_float2(af[i].z, af[i].w), ww, acc[2 * i + 1][j]);
+        for (int i = 0; i < TM; ++i) {
+          acc[i][j] = ffma2(make_float2(af[i].x, af[i].y), make_float2(wf.x, wf.y), acc[i][j]);
+          acc[i][j] = ffma2(make_float2(af[i].z, af[i].w), make_float2(wf.z, wf.w), acc[i][j]);
         }
       }
     }
-    if (more) park(b ^ 1);
-    __syncthreads();
   }
-  if constexpr (KG > 1) {  // the groups' sums, added in order
-    float* sums = slices + (kg - 1) * BM * BN + tid % NG;
+  float sum[TM][TN];
 #pragma unroll
-    for (int i = 0; i < TM / 2; ++i)
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) sum[i][j] = acc[i][j].x + acc[i][j].y;
+  if constexpr (KG > 1) {  // the groups' sums, added in order
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
       for (int j = 0; j < TN; ++j)
-        if (kg > 0) {
-          sums[(2 * i * TN + j) * NG] = acc[i][j].x;
-          sums[((2 * i + 1) * TN + j) * NG] = acc[i][j].y;
-        }
+        if (kg > 0) slices[(kg - 1) * BM * BN + (i * TN + j) * NG + tid % NG] = sum[i][j];
     __syncthreads();
     if (kg > 0) return;
 #pragma unroll
     for (int q = 1; q < KG; ++q)
 #pragma unroll
-      for (int i = 0; i < TM / 2; ++i)
+      for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-          acc[i][j].x += slices[(q - 1) * BM * BN + (2 * i * TN + j) * NG + tid];
-          acc[i][j].y += slices[(q - 1) * BM * BN + ((2 * i + 1) * TN + j) * NG + tid];
-        }
+        for (int j = 0; j < TN; ++j) sum[i][j] += slices[(q - 1) * BM * BN + (i * TN + j) * NG + tid];
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
-    const int row = tile * BM + ty * TM + i;
+    const int row = tile * BM + ty + RY * i;
     int dst = row;
+    float sc = 1.f;  // the pair's routing weight, ahead of the nonlinearity
     if (sorted_ids) {
       const int id = sorted_ids[row];
       dst = id < 0 ? -1 : scatter ? id : row;
+      if (id >= 0 && row_scale) sc = row_scale[id];
     } else if (row >= M) {
       dst = -1;
     }
     if (dst < 0) continue;
-    float v[TN];
-#pragma unroll
-    for (int j = 0; j < TN; ++j) v[j] = (i & 1) ? acc[i / 2][j].y : acc[i / 2][j].x;
     if constexpr (EPI == GL_EPI_GLU) {
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int n = n0 + 2 * tx + j;
-        if (n < N) out[(int64_t)blockIdx.z * o_zs + (int64_t)dst * ldo + n] = glu_act(v[j], v[j + TN / 2], act, limit);
+      for (int j = 0; j < TN / 2; ++j) {
+        const int n = n0 + tx + CX * j;
+        if (n < N) out[(int64_t)blockIdx.z * o_zs + (int64_t)dst * ldo + n] = glu_act(sc * sum[i][2 * j], sc * sum[i][2 * j + 1], act, limit);
       }
     } else {
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
-        const int n = n0 + TN * tx + j;
+        const int n = n0 + tx + CX * j;
         if (n >= N) continue;
-        if (gate) v[j] *= 1.0f / (1.0f + expf(-gate[(int64_t)dst * gate_ld + (gate_cols ? blockIdx.z * N + n : blockIdx.z)]));
-        out[(int64_t)blockIdx.z * o_zs + (int64_t)dst * ldo + n] = v[j];
+        float v = sc * sum[i][j];
+        if (gate) v *= 1.0f / (1.0f + expf(-gate[(int64_t)dst * gate_ld + (gate_cols ? blockIdx.z * N + n : blockIdx.z)]));
+        out[(int64_t)blockIdx.z * o_zs + (int64_t)dst * ldo + n] = v;
       }
     }
   }
@@ -802,6 +769,46 @@ __global__ void __launch_bounds__(GP_THREADS)
     }
 }
 
+// A few outputs per row (a router): a warp takes two rows, its lanes every 32nd 16-byte piece of k, and the 2 NW sums are reduced together by
+// halving.  Tiles of 32 x 32 walk all of k in a dozen CTAs: 304 x 8 x 1024 23.3 us, here 11.9; 304 x 16 23.5 / 13.5.
+template <int NW>
+__global__ void __launch_bounds__(32) fp32_narrow_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int M, int N, int K,
+                                                         float* __restrict__ out, int ldo) {
+  griddep_launch();
+  griddep_wait();
+  const int lane = threadIdx.x, r0 = blockIdx.x * 2;
+  const float* a0 = a + (int64_t)r0 * lda;
+  const float* a1 = a + (int64_t)(r0 + 1 < M ? r0 + 1 : r0) * lda;
+  float v[2 * NW];
+#pragma unroll
+  for (int i = 0; i < 2 * NW; ++i) v[i] = 0.f;
+#pragma unroll 2
+  for (int k = lane * 4; k < K; k += 128) {
+    const float4 x = ldf4(a0, k), y = ldf4(a1, k);
+#pragma unroll
+    for (int n = 0; n < NW; ++n) {
+      const float4 c = n < N ? ldf4(w, (int64_t)n * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[n] = fmaf(x.w, c.w, fmaf(x.z, c.z, fmaf(x.y, c.y, fmaf(x.x, c.x, v[n]))));
+      v[NW + n] = fmaf(y.w, c.w, fmaf(y.z, c.z, fmaf(y.y, c.y, fmaf(y.x, c.x, v[NW + n]))));
+    }
+  }
+  int mine = 0, off = 16;  // mine: the sum that this lane ends up with
+#pragma unroll
+  for (int m = NW; m >= 1; m /= 2, off /= 2) {
+    const bool up = lane & off;
+    mine += up ? m : 0;
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      const float keep = up ? v[i + m] : v[i], give = up ? v[i] : v[i + m];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+    }
+  }
+#pragma unroll
+  for (int o = 16 / (2 * NW); o >= 1; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  const int row = r0 + mine / NW, n = mine % NW;
+  if (lane % (32 / (2 * NW)) == 0 && row < M && n < N) out[(int64_t)row * ldo + n] = v[0];
+}
+
 namespace {
 
 // fp32 operands that the packed-pair kernel takes: rows of whole, aligned 16-byte pieces
@@ -828,13 +835,17 @@ int dense_fp32_linear(int batch, const void* a, int lda, const void* w, int64_t 
 #define FL_DENSE(BM, BN, TM, TN, KG)                                                                                                      \
   return launch_fp32_linear<BM, BN, TM, TN, KG, GL_EPI_STORE>((M + BM - 1) / BM, batch, a, lda, nullptr, 0, nullptr, w, w_stride, nullptr, \
                                                           nullptr, M, N, K, out, ldo, 0, 0.f, 0, a_zs, o_zs, gate, gate_ld, gate_cols, st)
-  // Measured (us; 64 x 64 tiles in one k group before): 304 x 2048 x 1024 80 -> 51 (KG 2; 58 with 4), 304 x 4640 x 1024 88 -> 87,
-  // 304 x 1536 x 1024 64 -> 38 (KG 4; 50 with 2), 304 x 1024 x 2048 99 -> 72 (90 with 2), 40 x 2048 x 1024 43 -> 24, 304 x 8 x 1024 43 -> 20,
-  // 4 x 2048 x 1024 42 -> 15, 4 x 32000 x 1024 115 -> 49.
+  // Measured, us, one register slice ahead (64 x 32 tiles, or 32 x 32 of 4 x 4 per thread) / here: 304 x 1024 x 1024 41.5 / 30.4, 304 x 1024 x 2048
+  // 75.8 / 54.8, 304 x 2048 x 1024 55.4 / 46.9, 400 x 1024 x 2048 75.9 / 54.4, 100 x 1024 x 1024 23.4 / 16.0, 4 x 2048 x 1024 19.9 / 12.8, 4 x 32000 x 1024
+  // 52.6 / 31.1.  Many tiles: 304 x 4640 x 1024 85.3, in tiles of 32 x 32 86.8, of 64 x 32 78.1; 150 x 4640 47.0 and 49.7; 400 x 4640 110 and 106.
   if (M <= 8) FL_DENSE(8, 32, 8, 1, 4);
-  const long long tiles = (long long)((M + 63) / 64) * ((N + 31) / 32) * batch;
-  if (M <= 32 || 2 * tiles <= sm_count()) FL_DENSE(32, 32, 4, 4, 4);
-  if (tiles <= 2LL * sm_count()) FL_DENSE(64, 32, 8, 4, 4);
+  if (N <= 16 && batch == 1 && !gate) {
+    auto kern = N <= 8 ? fp32_narrow_kernel<8> : fp32_narrow_kernel<16>;
+    B200_CUDA_OK(launch_kernel(kern, dim3((M + 1) / 2), dim3(32), 0, st, (const float*)a, lda, (const float*)w, M, N, K, (float*)out, ldo));
+    return B200_OK;
+  }
+  const long long tiles = (long long)((M + 31) / 32) * ((N + 31) / 32) * batch;
+  if (tiles <= 6LL * sm_count()) FL_DENSE(32, 32, 8, 4, 4);
   FL_DENSE(64, 32, 8, 4, 2);
 #undef FL_DENSE
 }
@@ -952,13 +963,18 @@ int b200_grouped_linear(const void* a, int lda, const int32_t* sorted_ids, int g
     if (rows < M) M = (int)rows;
     if (!sorted_ids && M <= 0) return B200_OK;
     if (!sorted_ids && !glu) return dense_fp32_linear(1, a, lda, w, 0, M, N, K, out, ldo, 0, 0, no_gate, 0, 0, st);
-    if (glu)
-      return launch_fp32_linear<MOE_BM, 64, 8, 4, 4, GL_EPI_GLU>(row_tiles, 1, a, lda, sorted_ids, gather_div, row_scale, w, w_expert_stride,
-                                                              tile_expert, num_tiles, M, N, K, out, ldo, scatter, limit, act, 0, 0, no_gate,
-                                                              0, 0, st);
-    return launch_fp32_linear<MOE_BM, 64, 8, 4, 4, GL_EPI_STORE>(row_tiles, 1, a, lda, sorted_ids, gather_div, row_scale, w, w_expert_stride,
-                                                              tile_expert, num_tiles, M, N, K, out, ldo, scatter, limit, act, 0, 0, no_gate,
-                                                              0, 0, st);
+    // Expert tiles come in 32 rows.  512 x 1024 gate, up and down of 8 experts, two of them a token, us, tiles of 32 x 64 from registers / here:
+    // 304 tokens 118 / 80, 400 121 / 106, 100 66 / 41, 30 63 / 39; twice the threads a tile pay while the tiles leave SMs idle (100 tokens 41 and 52,
+    // 304 tokens 104 and 80).
+#define FL_EXPERT(EPI, TM, COLS)                                                                                                              \
+  return launch_fp32_linear<MOE_BM, COLS, TM, 4, 4, EPI>(row_tiles, 1, a, lda, sorted_ids, gather_div, row_scale, w, w_expert_stride,         \
+                                                         tile_expert, num_tiles, M, N, K, out, ldo, scatter, limit, act, 0, 0, no_gate, 0, 0, st)
+    const bool few = (long long)row_tiles * ((N + (glu ? 15 : 31)) / (glu ? 16 : 32)) <= 4LL * sm_count();
+    if (glu && few) FL_EXPERT(GL_EPI_GLU, 4, 32);
+    if (glu) FL_EXPERT(GL_EPI_GLU, 8, 32);
+    if (few) FL_EXPERT(GL_EPI_STORE, 4, 32);
+    FL_EXPERT(GL_EPI_STORE, 8, 32);
+#undef FL_EXPERT
   }
   dim3 grid(row_tiles, (N + GL_BN - 1) / GL_BN);
   B200_DISPATCH_ELEM(dtype, ET, {
