@@ -163,6 +163,13 @@ def test_prefill_matches_oracle(ops, s_new, computed, hq, hkv, d):
     _check(got.cpu(), want)
 
 
+@pytest.mark.parametrize("s_new,computed,hq,hkv,d", [(1, 0, 8, 8, 64), (5, 3, 4, 2, 128), (63, 0, 32, 4, 64), (33, 95, 8, 1, 128), (41, 511, 32, 8, 128),
+                                                     (17, 900, 40, 8, 64), (20, 1503, 4, 4, 128)])
+def test_prefill_of_a_few_tokens(ops, s_new, computed, hq, hkv, d):
+    """Fewer blocks than groups, rows that end inside a warp's, groups whose blocks no row sees, one, two and four CTAs a tile."""
+    test_prefill_matches_oracle(ops, s_new, computed, hq, hkv, d)
+
+
 def test_prefill_last_row_equals_decode(ops):
     """Size-independent property: the last query row of a prefill equals a decode step at the same context."""
     g = torch.Generator().manual_seed(23)
