@@ -64,6 +64,38 @@ def test_decode_matches_oracle(ops, b, hq, hkv, d, ctxs, quota):
     _check(got.cpu(), want)
 
 
+@pytest.mark.parametrize("b,hq,hkv,d,ctxs,blocks", [
+    (1, 32, 4, 64, [161], 8),                       # a block a warp, idle warps
+    (4, 8, 8, 128, [0, 1, 32, 33], 2),              # no keys, one key, both sides of a block's end; one head a group
+    (3, 10, 2, 64, [512, 513, 300], 17),            # two CTAs of a cluster; five heads a group
+    (2, 16, 2, 128, [1000, 1024], 32),              # two CTAs
+    (2, 8, 1, 64, [2047, 40], 64),                  # four
+    (1, 8, 1, 128, [8192], 256),                    # eight, four blocks a warp
+    (18, 8, 8, 128, [70 + i for i in range(18)], 4),  # 144 pairs
+])
+def test_decode_of_few_blocks(ops, b, hq, hkv, d, ctxs, blocks):
+    """One cluster per (sequence, kv head), rows through row_ids; quantised outputs are the codes of the bf16 ones."""
+    from oracle import quant_ref
+
+    g = torch.Generator().manual_seed(b + d)
+    nb = sum(-(-c // 32) for c in ctxs) + 2
+    kp, vp = _pools(nb, 32, hkv, d, g)
+    small = make_block_tables(b, ctxs, 32, nb, blocks, g)
+    rows = torch.randperm(b + 2, generator=g)[:b].int()
+    bt = torch.zeros((b + 2, blocks), dtype=torch.int32)
+    bt[rows.long()] = small
+    q, ctx = torch.randn(b, hq, d, generator=g).bfloat16(), torch.tensor(ctxs, dtype=torch.int32)
+    args = (q.cuda(), logical_to_device_pool(kp).cuda(), logical_to_device_pool(vp).cuda(), bt.cuda(), ctx.cuda(), 0.11)
+    got = ops.paged_attn_decode(*args, row_ids=rows.cuda())
+    _check(got.cpu(), attn_ref.paged_attention_decode_ref(q, kp, vp, small, ctx, 0.11))
+    split = ops.paged_attn_decode(*args, row_ids=rows.cuda(), min_quota=1)
+    assert rel_err(got.cpu(), split.cpu()) <= 4e-3  # bf16 rounding of sums in another order
+    for kind in ("fp8", "int8"):
+        yq, ys = ops.paged_attn_decode(*args, row_ids=rows.cuda(), quant=kind)
+        qw, sw = quant_ref.quantize_act_per_token(got.cpu().reshape(b, hq * d), kind)
+        assert torch.equal(ys.cpu(), sw) and torch.equal(yq.cpu().view(torch.uint8), qw.view(torch.uint8))
+
+
 def test_decode_row_ids_and_strided_q(ops):
     """Persistent block-table rows addressed through row_ids; q taken as a strided view of a packed qkv row."""
     g = torch.Generator().manual_seed(3)

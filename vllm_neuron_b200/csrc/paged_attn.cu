@@ -446,6 +446,182 @@ __global__ void __launch_bounds__(COMB_THREADS)
   }
 }
 
+// ---- decode of few blocks, bf16 output: one cluster per (sequence, kv head), its result in one launch
+// With few sequences of short context the balanced split above leaves a block or two to a warp, and what is left is latency: the prefix sum, the
+// search, the trip of the partials through memory and the merge kernel's launch.  Here the pair's 32-token blocks are dealt to the eight warps
+// of the S CTAs of a cluster, and the warps' (m, l, O) meet in shared memory.  Same products and roundings per block as above.
+// Decode steps, us, by the split above and its merge / here: TinyLlama, one sequence at 161, 779 / 666 (8.6 us a layer for the two launches, 3.5
+// here).
+constexpr int FEW_WARPS = 8;
+
+__device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+
+template <int D>
+__global__ void __launch_bounds__(FEW_WARPS * 32, 1)
+    paged_attn_decode_few_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
+                                 const __nv_bfloat16* __restrict__ q, int64_t q_stride, const int32_t* __restrict__ block_table,
+                                 int64_t bt_stride, const int32_t* __restrict__ row_ids, const int32_t* __restrict__ ctx_lens,
+                                 __nv_bfloat16* __restrict__ out, int Hq, int Hkv, int max_blocks, float scale_log2) {
+  constexpr int TILE = BS * D * 2, KSTEPS = D / 16, NST = 128 / D;  // 16 KB of ring a warp
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  float* O = reinterpret_cast<float*>(smem + FEW_WARPS * NST * 2 * TILE);   // [warps][8][D]
+  float* ml = O + FEW_WARPS * 8 * D;                                        // [warps][8][2]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ml + FEW_WARPS * 16) + (threadIdx.x >> 5) * NST;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int S = (int)cluster_nctarank(), rank = (int)cluster_ctarank();
+  const int kvh = blockIdx.y, b = blockIdx.z, G = Hq / Hkv;
+  uint8_t* ring = smem + (size_t)warp * NST * 2 * TILE;
+  if (lane == 0) {
+#pragma unroll
+    for (int s = 0; s < NST; ++s) mbar_init(&bars[s], 1);
+    fence_mbar_init();
+    fence_proxy_async();
+  }
+  __syncwarp();
+  griddep_wait();
+  const int row = row_ids ? row_ids[b] : b, ctx = ctx_lens[b];
+  const int h0 = (lane & 3) * 2, qn = lane >> 2;
+  uint32_t qb[KSTEPS][2];
+  {
+    const __nv_bfloat16* qp = q + (int64_t)b * q_stride + (int64_t)(kvh * G + (qn < G ? qn : 0)) * D + h0;
+#pragma unroll
+    for (int ks = 0; ks < KSTEPS; ++ks) {
+      qb[ks][0] = qn < G ? *reinterpret_cast<const uint32_t*>(qp + ks * 16) : 0u;
+      qb[ks][1] = qn < G ? *reinterpret_cast<const uint32_t*>(qp + ks * 16 + 8) : 0u;
+    }
+  }
+  const int nblk = blocks_of(ctx, max_blocks), first = rank * FEW_WARPS + warp, step = S * FEW_WARPS;
+  const int32_t* bt = block_table + (int64_t)row * bt_stride;
+  // lane l: tile row of this warp's block number 32 n + l
+  auto rows_from = [&](int i) { return first + (i + lane) * step < nblk ? (bt[first + (i + lane) * step] * Hkv + kvh) * BS : 0; };
+  int tr = rows_from(0);
+  auto issue = [&](int i) {
+    if ((i & 31) == 0 && i > 0) tr = rows_from(i);
+    const int t = __shfl_sync(0xffffffffu, tr, i & 31), s = i % NST;
+    if (lane == 0) issue_tile_pair<D>(&k_map, &v_map, 0, ring + s * 2 * TILE, ring + s * 2 * TILE + TILE, &bars[s], t);
+  };
+#pragma unroll
+  for (int s = 0; s < NST; ++s)
+    if (first + s * step < nblk) issue(s);
+  griddep_launch();
+  float oacc[KSTEPS][4];
+#pragma unroll
+  for (int i = 0; i < KSTEPS; ++i) oacc[i][0] = oacc[i][1] = oacc[i][2] = oacc[i][3] = 0.f;
+  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+  for (int i = 0, j = first; j < nblk; ++i, j += step) {
+    const int s = i % NST;
+    mbar_wait(&bars[s], (i / NST) & 1);
+    const uint32_t kbase = smem_u32(ring + s * 2 * TILE), vbase = kbase + TILE;
+    const int nvalid = ctx - j * BS;
+    float sacc[2][4];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt) {
+      sacc[mt][0] = sacc[mt][1] = sacc[mt][2] = sacc[mt][3] = 0.f;
+#pragma unroll
+      for (int ks = 0; ks < KSTEPS; ++ks) {
+        uint32_t a[4];
+        ldmatrix_x4(a, tile_addr(kbase, mt * 16 + (lane & 15), ks * 2 + (lane >> 4)));
+        mma_bf16_16816(sacc[mt], a, qb[ks][0], qb[ks][1]);
+      }
+    }
+    float bm0 = -INFINITY, bm1 = -INFINITY;
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const bool ok = mt * 16 + hf * 8 + (lane >> 2) < nvalid;
+        sacc[mt][hf * 2] = ok ? sacc[mt][hf * 2] * scale_log2 : -INFINITY;
+        sacc[mt][hf * 2 + 1] = ok ? sacc[mt][hf * 2 + 1] * scale_log2 : -INFINITY;
+        bm0 = fmaxf(bm0, sacc[mt][hf * 2]);
+        bm1 = fmaxf(bm1, sacc[mt][hf * 2 + 1]);
+      }
+#pragma unroll
+    for (int o = 4; o <= 16; o <<= 1) {
+      bm0 = fmaxf(bm0, __shfl_xor_sync(0xffffffffu, bm0, o));
+      bm1 = fmaxf(bm1, __shfl_xor_sync(0xffffffffu, bm1, o));
+    }
+    const float mn0 = fmaxf(m0, bm0), mn1 = fmaxf(m1, bm1);
+    const float r0 = mn0 == -INFINITY ? 0.f : mn0, r1 = mn1 == -INFINITY ? 0.f : mn1;
+    const float al0 = exp2f(m0 - r0), al1 = exp2f(m1 - r1);
+    m0 = mn0;
+    m1 = mn1;
+    float ps0 = 0.f, ps1 = 0.f;
+    uint32_t pb[2][2];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const float p0 = exp2f(sacc[mt][hf * 2] - r0), p1 = exp2f(sacc[mt][hf * 2 + 1] - r1);
+        ps0 += p0;
+        ps1 += p1;
+        pb[mt][hf] = movmatrix_trans(pack_bf16(p0, p1));
+      }
+    l0 = l0 * al0 + ps0;
+    l1 = l1 * al1 + ps1;
+#pragma unroll
+    for (int dm = 0; dm < KSTEPS; ++dm) {
+      oacc[dm][0] *= al0;
+      oacc[dm][1] *= al1;
+      oacc[dm][2] *= al0;
+      oacc[dm][3] *= al1;
+#pragma unroll
+      for (int ks = 0; ks < 2; ++ks) {
+        uint32_t a[4];
+        ldmatrix_x4_trans(a, tile_addr(vbase, ks * 16 + (lane & 7) + ((lane >> 4) & 1) * 8, dm * 2 + ((lane >> 3) & 1)));
+        mma_bf16_16816(oacc[dm], a, pb[ks][0], pb[ks][1]);
+      }
+    }
+    __syncwarp();
+    if (j + NST * step < nblk) issue(i + NST);
+  }
+#pragma unroll
+  for (int o = 4; o <= 16; o <<= 1) {
+    l0 += __shfl_xor_sync(0xffffffffu, l0, o);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+  }
+  float* mine = O + warp * 8 * D;
+#pragma unroll
+  for (int dm = 0; dm < KSTEPS; ++dm) {
+    const int d = dm * 16 + qn;
+    mine[h0 * D + d] = oacc[dm][0];
+    mine[(h0 + 1) * D + d] = oacc[dm][1];
+    mine[h0 * D + d + 8] = oacc[dm][2];
+    mine[(h0 + 1) * D + d + 8] = oacc[dm][3];
+  }
+  if (qn == 0) {
+    *reinterpret_cast<float4*>(ml + (warp * 8 + h0) * 2) = make_float4(m0, l0, m1, l1);
+  }
+  if (S > 1) cluster_sync_all();
+  else __syncthreads();
+  // ---- the heads' column pairs rank, rank + S, .. from all the warps, in order
+  for (int i = threadIdx.x * S + rank; i < G * (D / 2); i += FEW_WARPS * 32 * S) {
+    const int h = i / (D / 2), c = i % (D / 2) * 2;
+    const uint32_t o_at = smem_u32(O) + (h * D + c) * 4, ml_at = smem_u32(ml) + h * 8;
+    float M = -INFINITY, L = 0.f;
+    float2 acc = make_float2(0.f, 0.f);
+    for (int r = 0; r < S; ++r)
+#pragma unroll
+      for (int w = 0; w < FEW_WARPS; ++w) M = fmaxf(M, ld_cluster_f2(mapa_shared(ml_at + w * 64, r)).x);
+    for (int r = 0; r < S; ++r)
+#pragma unroll
+      for (int w = 0; w < FEW_WARPS; ++w) {
+        const float2 p = ld_cluster_f2(mapa_shared(ml_at + w * 64, r)), o = ld_cluster_f2(mapa_shared(o_at + w * 8 * D * 4, r));
+        const float f = p.x == -INFINITY ? 0.f : exp2f(p.x - M);  // a warp without a block
+        L += f * p.y;
+        acc.x += f * o.x;
+        acc.y += f * o.y;
+      }
+    const bool any = L > 0.f;
+    *reinterpret_cast<uint32_t*>(out + ((int64_t)b * Hq + kvh * G + h) * D + c) = pack_bf16(any ? acc.x / L : 0.f, any ? acc.y / L : 0.f);
+  }
+  if (S > 1) cluster_sync_all();  // nobody leaves while a peer still reads its parts
+}
+
 // ============================================================ prefix-cached prefill (one sequence)
 // A few new tokens over a cached prefix are one tile of 64 query rows per head: 32 or 40 CTAs that would walk all the keys, a microsecond a
 // block of 32.  So the blocks are dealt to PF_GROUPS groups of four warps (16 query rows a warp, a double-buffered TMA ring a group) in each
@@ -453,12 +629,6 @@ __global__ void __launch_bounds__(COMB_THREADS)
 // between them.  us, one group / here: 41 tokens after 512, 32 heads of 64 21.8 / 12.8, after 4096, 32 heads of 128
 // 135.9 / 35.3, 17 tokens after 32 16.1 / 11.8.
 constexpr int PF_GROUPS = 4;
-
-__device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
-  return v;
-}
 
 template <int D>
 __global__ void __launch_bounds__(PF_GROUPS * 128, 1)
@@ -741,6 +911,26 @@ int launch_decode(const CUtensorMap& km, const CUtensorMap& vm, const void* q, i
   return B200_OK;
 }
 
+// CTAs of a cluster that give every warp at most FEW_BLOCKS blocks, or 0 where the chip does not hold them all at once
+int few_split(int B, int Hkv, int max_blocks) {
+  for (int S = 1; S <= 8; S <<= 1) {
+    if ((int64_t)B * Hkv * S > sm_count()) return 0;
+    if (max_blocks <= 2 * FEW_WARPS * S || (S == 8 && max_blocks <= 4 * FEW_WARPS * S)) return S;
+  }
+  return 0;
+}
+template <int D>
+int launch_few(const CUtensorMap& km, const CUtensorMap& vm, const void* q, int64_t q_stride, const int32_t* bt, int64_t bt_stride,
+               const int32_t* row_ids, const int32_t* ctx_lens, void* out, int B, int Hq, int Hkv, int max_blocks, int S, float scale,
+               cudaStream_t stream) {
+  auto kern = paged_attn_decode_few_kernel<D>;
+  constexpr size_t smem = (size_t)FEW_WARPS * (128 / D * 2 * BS * D * 2 + 8 * D * 4 + 64 + 16) + 1024;
+  B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  B200_CUDA_OK(launch_kernel_cluster(kern, dim3(S, Hkv, B), dim3(FEW_WARPS * 32), smem, S, stream, km, vm, (const __nv_bfloat16*)q, q_stride, bt,
+                                     bt_stride, row_ids, ctx_lens, (__nv_bfloat16*)out, Hq, Hkv, max_blocks, scale * 1.4426950408889634f));
+  return B200_OK;
+}
+
 template <int D>
 int launch_prefill(const CUtensorMap& km, const CUtensorMap& vm, const void* q, int64_t q_stride, const int32_t* bt_row,
                    void* out, int S_new, int computed_len, int Hq, int Hkv, float scale, cudaStream_t stream) {
@@ -803,6 +993,17 @@ int b200_paged_attn_decode(const void* q, int64_t q_token_stride, const void* k_
   if (rc) return rc;
   rc = pool_tmap(v_pool, num_blocks, Hkv, D, &vm);
   if (rc) return rc;
+  // a call that names its quota asks for the split above; a quantised result takes its row's maximum over all heads, in a launch of its own
+  const int few = min_quota == 0 && ((uintptr_t)out & 15) == 0 && ((uintptr_t)workspace & 15) == 0 && (Hq * D) % 8 == 0 ? few_split(B, Hkv, max_blocks) : 0;
+  if (few) {
+    void* rows = out ? out : workspace;
+    rc = D == 128 ? launch_few<128>(km, vm, q, q_token_stride, block_table, bt_row_stride, row_ids, ctx_lens, rows, B, Hq, Hkv, max_blocks, few, scale,
+                                    (cudaStream_t)stream)
+                  : launch_few<64>(km, vm, q, q_token_stride, block_table, bt_row_stride, row_ids, ctx_lens, rows, B, Hq, Hkv, max_blocks, few, scale,
+                                   (cudaStream_t)stream);
+    if (rc || q_dtype == B200_BF16) return rc;
+    return b200_quantize_per_token(rows, out_q, out_scale, nullptr, 0, B, Hq * D, q_dtype, stream);
+  }
   float* part_o = (float*)workspace;
   float* part_ml = part_o + (size_t)B * Hq * p.max_parts * D;
   int32_t* part_cnt = reinterpret_cast<int32_t*>(part_ml + (size_t)B * Hq * p.max_parts * 2);
