@@ -221,6 +221,33 @@ def test_warp_attention_shares_key_rows_between_query_heads(H, G, D, Dv):
         _close(_run_attn(q, k, v, sink, window, bs, [T], torch.bfloat16), want, 3e-2)
 
 
+@pytest.mark.parametrize("H,G,D,Dv", [(8, 2, 128, 128), (4, 4, 64, 64), (5, 1, 128, 64)])
+@pytest.mark.parametrize("window", [100, 128, 1 << 30])
+def test_long_prompts_with_a_sink_on_tcgen05(H, G, D, Dv, window):
+    """Portions of 128 tokens and more (one of them the second part, one short) in tiles of 128 rows: the sink joins every row's denominator once,
+    whether it lies above or below all scores, and a dominant key counts just inside the window and not just outside."""
+    from oracle.pumopel_ref import sink_window_attention
+
+    ops = _ops()
+    T, scale = 420, 1 / math.sqrt(D)
+    bf = lambda t: t.bfloat16().float()  # noqa: E731
+    for sink_val in (None, 4.0, -60.0, 60.0):
+        q, k, v, sink = _attn_case(T, H, G, D, Dv, window, 32, sink_val=sink_val)
+        with ops.kernel_timer() as kt:
+            got = _run_attn(bf(q), bf(k), bf(v), sink, window, 32, [150, 200, 70], torch.bfloat16)
+        assert any(n.startswith("swa_sink_attn_prefill_tc") for n in kt.summary())
+        if sink_val == 60.0:
+            assert got.abs().max() < 1e-6
+            continue
+        want = sink_window_attention(bf(q).double(), bf(k).double(), bf(v).double(), sink.double(), scale, window)
+        _close(got, want, 2.0**-8)  # weights in two bf16 terms: the output's rounding is what is left
+    if window < T:
+        for j, inside in ((T - window, True), (T - 1 - window, False)):
+            q, k, v, sink = _attn_case(T, H, G, D, Dv, window, 32, spike=(T - 1, j, H - 1))
+            head = _run_attn(bf(q), bf(k), bf(v), sink, window, 32, [T], torch.bfloat16)[T - 1].view(H, Dv)[H - 1].float().cpu()
+            assert ((head - bf(v)[j, (H - 1) // (H // G)]).abs().max() < 1e-2) == inside
+
+
 @pytest.mark.parametrize("chunks", [[150], [16, 64, 3, 67], [33, 1, 1, 17, 98]])
 def test_tensor_core_prompt_attention_edges(chunks):
     """bf16 pools, head sizes 32 / 48: portions of 16 tokens or more run on the mma.sync kernel (64-row tiles, 32-key tiles

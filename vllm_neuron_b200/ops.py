@@ -804,7 +804,7 @@ def swa_sink_attn(q_src, num_heads: int, k_pool, v_pool, block_table, meta, sink
     # decoded tokens beside prompt portions: each kind on its own kernel where that pays, in one launch of the prompt kernel otherwise
     parts = getattr(meta, "parts", None)
     if parts:
-        tc = _prompt_tc(q_src, k_pool, meta, sink, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool)
+        tc = _prompt_tc(q_src, k_pool, meta, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool)
         spans = [_span(p.max_end, int(window), int(chunk), pool, int(keep)) for p in parts]
         if not (tc or _prompt_mma(q_src, k_pool, meta, d, dv)) or not _split_pays(parts, num_heads, g, d, dv, bool(latent_values), tc, spans):
             parts = None
@@ -814,10 +814,10 @@ def swa_sink_attn(q_src, num_heads: int, k_pool, v_pool, block_table, meta, sink
     return out
 
 
-def _prompt_tc(q, k_pool, meta, sink, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool) -> bool:
-    """Long prompt portions in bf16 serving (a sliding window only without pooled blocks), head sizes of 64 / 128 with pages of 32 tokens: the
+def _prompt_tc(q, k_pool, meta, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool) -> bool:
+    """Long prompt portions in bf16 serving (with or without a sink; a sliding window only without pooled blocks), head sizes of 64 / 128 with pages of 32 tokens: the
     tcgen05 kernel (128-row query tiles, accumulators in tensor memory); B200_SWA_PREFILL_LEGACY=1 keeps the mma.sync kernel (A/B aid)."""
-    return bool(k_pool.dtype == torch.bfloat16 and meta.max_new >= PREFILL_TC_MIN_TOKENS and sink is None and not pool
+    return bool(k_pool.dtype == torch.bfloat16 and meta.max_new >= PREFILL_TC_MIN_TOKENS and not pool
                 and not latent_values and q.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0 and not _SWA_PREFILL_LEGACY
                 and _lib().b200_swa_sink_attn_prefill_tc_supported(d, dv, bs, v_div, 1 if softcap else 0,
                                                                          0 if sigmoid_bias is None else 1))
@@ -842,15 +842,15 @@ def _swa_part(q_src, num_heads, k_pool, v_pool, block_table, meta, sink, scale, 
     # the per-launch timer tells the variants apart (their floors differ)
     tag = "[latent]" if plain and latent_values else "" if plain and not pool and not keep else "[" + "+".join(n for n, on in (("chunk", chunk), ("cap", softcap), ("sigmoid", sigmoid_bias is not None),
                                                                        ("maps", v_div > 1), ("pool", pool), ("keep", keep)) if on) + "]"
-    if _prompt_tc(q_all, k_pool, meta, sink, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool):
+    if _prompt_tc(q_all, k_pool, meta, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool):
         with _k("swa_sink_attn_prefill_tc" + tag):
-            check(_lib().b200_swa_sink_attn_prefill_tc(q_all, q_all.stride(0), k_pool, v_pool, k_pool.shape[0],
+            check(_lib().b200_swa_attn_prefill_tc_sink(q_all, q_all.stride(0), k_pool, v_pool, k_pool.shape[0],
                                                              block_table, block_table.stride(0), meta.seq_start,
                                                              meta.seq_slot, meta.seq_pos0, meta.num_seqs, meta.max_new,
                                                              float(scale), out_all, num_heads, g, d, dv, bs, *variant,
                                                              1 if split_p else 0, int(window) if window < (1 << 30) else 0,
-                                                             int(keep)),
-                  "b200_swa_sink_attn_prefill_tc")
+                                                             int(keep), sink),
+                  "b200_swa_attn_prefill_tc_sink")
         return
     if _prompt_mma(q_all, k_pool, meta, d, dv):
         with _k("swa_sink_attn_prefill" + tag):
