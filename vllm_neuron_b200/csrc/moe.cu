@@ -838,12 +838,14 @@ int dense_fp32_linear(int batch, const void* a, int lda, const void* w, int64_t 
   // Measured, us, one register slice ahead (64 x 32 tiles, or 32 x 32 of 4 x 4 per thread) / here: 304 x 1024 x 1024 41.5 / 30.4, 304 x 1024 x 2048
   // 75.8 / 54.8, 304 x 2048 x 1024 55.4 / 46.9, 400 x 1024 x 2048 75.9 / 54.4, 100 x 1024 x 1024 23.4 / 16.0, 4 x 2048 x 1024 19.9 / 12.8, 4 x 32000 x 1024
   // 52.6 / 31.1.  Many tiles: 304 x 4640 x 1024 85.3, in tiles of 32 x 32 86.8, of 64 x 32 78.1; 150 x 4640 47.0 and 49.7; 400 x 4640 110 and 106.
-  if (M <= 8) FL_DENSE(8, 32, 8, 1, 4);
+  // A row's sums run alike in the two smaller tiles and, where a row has few outputs, in batches of any size: how a prompt is cut changes
+  // nothing below the tiles of 64 rows.
   if (N <= 16 && batch == 1 && !gate) {
     auto kern = N <= 8 ? fp32_narrow_kernel<8> : fp32_narrow_kernel<16>;
     B200_CUDA_OK(launch_kernel(kern, dim3((M + 1) / 2), dim3(32), 0, st, (const float*)a, lda, (const float*)w, M, N, K, (float*)out, ldo));
     return B200_OK;
   }
+  if (M <= 8) FL_DENSE(8, 32, 8, 1, 4);
   const long long tiles = (long long)((M + 31) / 32) * ((N + 31) / 32) * batch;
   if (tiles <= 6LL * sm_count()) FL_DENSE(32, 32, 8, 4, 4);
   FL_DENSE(64, 32, 8, 4, 2);
