@@ -267,6 +267,26 @@ def test_tensor_core_prompt_attention_edges(chunks):
             assert ((head - vb[j, 3 // (H // G)]).abs().max() < 3e-2) == inside, (i, j)
 
 
+@pytest.mark.parametrize("bs", [32, 64, 8])
+@pytest.mark.parametrize("window", [37, 64, 96, 1])
+def test_decoded_token_window_over_pages(window, bs):
+    """Decoded tokens, window tiles that start on pages (32 and 64 rows) and at the window's first key (8): windows that begin at a page's
+    first row, one to either side of it and inside it, a dominant key just inside and just outside.  Weights and outputs are rounded to
+    bf16 (2^-9 each) and the weights sum to at most 1: 2^-8 of the largest value."""
+    from oracle.pumopel_ref import sink_window_attention
+
+    H, G, D, Dv = 4, 2, 32, 48
+    for T in (132, window + 63, window + 64, window + 65):
+        i = T - 2
+        for j, inside in ((i - window + 1, True), (i - window, False)):
+            q, k, v, sink = _attn_case(T, H, G, D, Dv, window, bs, spike=(i, j, 3), seed=T)
+            q, k, v = (x.bfloat16().float() for x in (q, k, v))
+            want = sink_window_attention(q.double(), k.double(), v.double(), sink.double(), 1 / math.sqrt(D), window)[-4:]
+            got = _run_attn(q, k, v, sink, window, bs, [T - 4, 1, 1, 1, 1], torch.bfloat16)[-4:]
+            assert (got.double().cpu().view(4, H, Dv) - want.view(4, H, Dv)).abs().max() <= 2.0**-8 * v.abs().max()
+            assert ((got[2].float().view(H, Dv)[3].cpu() - v[j, 1]).abs().max() < 3e-2) == inside, (T, j)
+
+
 def test_far_key_among_hundreds_without_window():
     """No window: key 3 of 400 must still decide the last query (pages of 32)."""
     from oracle.pumopel_ref import sink_window_attention

@@ -384,33 +384,54 @@ __global__ void __launch_bounds__(DT_WARPS * 32)
   // b pool + pool - 1 <= pos - window.  Kept tokens (keep > 0, no pooled blocks): positions 0 .. keep - 1 before the window.  The
   // tile list is these early entries (32 per tile), then the window's keys
   const int nb = pool > 0 ? (pos - window + 1 > 0 ? (pos - window + 1) / pool : 0) : min(keep, lo);
-  const int npt = (nb + LDT_KEYS - 1) / LDT_KEYS, ntt = (pos - lo) / LDT_KEYS + 1;
+  // Pages of whole tiles: the window's tiles start where a page's 32 rows do (keys before lo are masked like those behind the token), so a tile
+  // is one page number and rows that follow one another.  Looking up and broadcasting a page and an offset for every row cost more than the
+  // copies: 64 tokens, 16 heads over 4 kv heads of 128, context 2048, L2 flushed, events around the call: window 1024 69.6 us (20.5 of bytes),
+  // 49.2 with tiles on pages; no window 122.9 / 77.8; 64 tokens, heads of 64, window 512 34.8 / 22.6; 64 at 200 26.6 / 22.5.
+  const bool paged = bs % LDT_KEYS == 0;
+  const int lo_t = paged ? lo / LDT_KEYS * LDT_KEYS : lo;
+  const int npt = (nb + LDT_KEYS - 1) / LDT_KEYS, ntt = (pos - lo_t) / LDT_KEYS + 1;
   for (int ti = warp + DT_WARPS * split; ti < npt + ntt; ti += DT_WARPS * splits) {
     // ---- this warp's 32 key and value rows -> its buffer (rows past the token's position / the last seen block are zeros)
     const bool early = ti < npt, ptile = early && pool > 0;
-    const int j0 = early ? ti * LDT_KEYS : lo + (ti - npt) * LDT_KEYS;  // first pooled block / first key position of the tile
-    const int j_end = early ? nb - 1 : pos;                            // last visible one
-    const int jm = j0 + lane;
-    int my_blk = -1, my_off = 0;
-    if (jm <= j_end) {
-      if (ptile) {
-        const int e = jm * pool + pool - 1;
-        my_blk = bt[e / bs];
-        my_off = (e % bs) / pool;
-      } else {
-        my_blk = bt[jm / bs];
-        my_off = jm % bs;
-      }
-    }
-    for (int r = 0; r < LDT_KEYS; ++r) {
-      const int blk = __shfl_sync(0xffffffffu, my_blk, r), off = __shfl_sync(0xffffffffu, my_off, r);
-      const bool ok = blk >= 0;
+    const int j0 = early ? ti * LDT_KEYS : lo_t + (ti - npt) * LDT_KEYS;  // first pooled block / first key position of the tile
+    const int j_end = early ? nb - 1 : pos;                              // last visible one
+    const int j_lo = early ? 0 : lo;
+    if (paged && !early) {
+      const int64_t blk = bt[j0 / bs];
+      const int r_lo_k = max(lo - j0, 0), r_hi_k = min(pos - j0, LDT_KEYS - 1);  // visible rows
 #pragma unroll
       for (int sl = 0; sl < DT_SLOTS; ++sl) {
         if (ch_on[sl]) {
-          const __nv_bfloat16* src = ptile ? pc_pool[sl] + ((int64_t)(ok ? blk : 0) * pc_blk[sl] + (off * pc_row[sl] + pc_src[sl]))
-                                           : ch_pool[sl] + ((int64_t)(ok ? blk : 0) * ch_blk[sl] + (off * ch_row[sl] + ch_src[sl]));
-          cp_async16(ch_dst[sl] + r * ch_pitch[sl], src, ok);
+          const __nv_bfloat16* src = ch_pool[sl] + (blk * ch_blk[sl] + (j0 % bs * ch_row[sl] + ch_src[sl]));
+          uint32_t dst = ch_dst[sl];
+#pragma unroll 8
+          for (int r = 0; r < LDT_KEYS; ++r, src += ch_row[sl], dst += ch_pitch[sl]) cp_async16(dst, src, r >= r_lo_k && r <= r_hi_k);
+        }
+      }
+    } else {
+      const int jm = j0 + lane;
+      int my_blk = -1, my_off = 0;
+      if (jm <= j_end) {
+        if (ptile) {
+          const int e = jm * pool + pool - 1;
+          my_blk = bt[e / bs];
+          my_off = (e % bs) / pool;
+        } else {
+          my_blk = bt[jm / bs];
+          my_off = jm % bs;
+        }
+      }
+      for (int r = 0; r < LDT_KEYS; ++r) {
+        const int blk = __shfl_sync(0xffffffffu, my_blk, r), off = __shfl_sync(0xffffffffu, my_off, r);
+        const bool ok = blk >= 0;
+#pragma unroll
+        for (int sl = 0; sl < DT_SLOTS; ++sl) {
+          if (ch_on[sl]) {
+            const __nv_bfloat16* src = ptile ? pc_pool[sl] + ((int64_t)(ok ? blk : 0) * pc_blk[sl] + (off * pc_row[sl] + pc_src[sl]))
+                                             : ch_pool[sl] + ((int64_t)(ok ? blk : 0) * ch_blk[sl] + (off * ch_row[sl] + ch_src[sl]));
+            cp_async16(ch_dst[sl] + r * ch_pitch[sl], src, ok);
+          }
         }
       }
     }
@@ -436,14 +457,14 @@ __global__ void __launch_bounds__(DT_WARPS * 32)
         mma_bf16_16816(s[2 * jp + 1], af, bf[2], bf[3]);
       }
     }
-    // ---- mask (every row is the same token: keys lo .. pos are visible), weights in fp32
+    // ---- mask (every row is the same token: keys lo .. pos are visible, one of them in every tile), weights in fp32
     float mx_lo = -INFINITY, mx_hi = -INFINITY;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int key = j0 + 8 * j + 2 * (lane & 3) + (c & 1);
-        const bool hi = c >= 2, seen = key <= j_end;
+        const bool hi = c >= 2, seen = key <= j_end && key >= j_lo;
         float v = s[j][c] * scale;
         if (softcap > 0.f) v = softcap * (1.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * v * inv_cap)));
         if (sig) v = seen ? __fdividef(1.0f, 1.0f + __expf(-(v + (hi ? sb_hi : sb_lo)))) : 0.f;
@@ -455,7 +476,7 @@ __global__ void __launch_bounds__(DT_WARPS * 32)
     mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
     mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
     mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
-    const float mn_lo = sig ? 0.f : fmaxf(m_lo, mx_lo), mn_hi = sig ? 0.f : fmaxf(m_hi, mx_hi);  // finite: key j0 is visible
+    const float mn_lo = sig ? 0.f : fmaxf(m_lo, mx_lo), mn_hi = sig ? 0.f : fmaxf(m_hi, mx_hi);  // finite: a key of the tile is visible
     const float c_lo = __expf(m_lo - mn_lo), c_hi = __expf(m_hi - mn_hi);
     m_lo = mn_lo;
     m_hi = mn_hi;
