@@ -401,7 +401,8 @@ int b200_swa_sink_attn_prefill_tc(const float* q, int ldq, const void* k_pool, c
                                   const int32_t* seq_slot, const int32_t* seq_pos0, int B, int max_new, float scale, void* out,
                                   int H, int G, int D, int Dv, int block_size, int chunk, float softcap,
                                   const float* sigmoid_bias, int v_div, int out_f32, int split_p, int window, int keep, void* stream);
-/* The same with a sink logit per query head (or NULL) in every softmax: its weight joins the denominator once, it has no value and is not scaled. */
+/* The same with a sink logit per query head (or NULL) in every softmax: its weight joins the denominator once, it has no value and is not scaled.
+ * With a sink the weights are always carried as two bf16 terms (split_p). */
 int b200_swa_attn_prefill_tc_sink(const float* q, int ldq, const void* k_pool, const void* v_pool, int num_blocks,
                                   const int32_t* block_table, int64_t bt_stride, const int32_t* seq_start,
                                   const int32_t* seq_slot, const int32_t* seq_pos0, int B, int max_new, float scale, void* out,

@@ -248,6 +248,25 @@ def test_long_prompts_with_a_sink_on_tcgen05(H, G, D, Dv, window):
             assert ((head - bf(v)[j, (H - 1) // (H // G)]).abs().max() < 1e-2) == inside
 
 
+@pytest.mark.parametrize("D,window", [(128, 100), (64, 1 << 30)])
+def test_sink_on_tcgen05_keeps_the_weights_precision(D, window):
+    """fp32 outputs of bf16 operands, against 64 bits: weights in two bf16 terms leave 2^-17 of a weight, exponentials and fp32 sums the rest;
+    2^-13 of the largest value, where one term leaves up to 2^-9."""
+    from oracle.pumopel_ref import sink_window_attention
+
+    ops = _ops()
+    T, H, G, bs = 420, 4, 2, 32
+    q, k, v, sink = _attn_case(T, H, G, D, D, window, bs, seed=9)
+    q, k, v = (x.bfloat16() for x in (q, k, v))
+    nb = -(-T // bs)
+    pages = lambda x: torch.cat([x, x.new_zeros(nb * bs - T, G, D)]).view(nb, bs, G, D).transpose(1, 2).contiguous().to(DEV)  # noqa: E731
+    meta = _meta([(0, 0, T)], {0: list(range(nb))}, bs)
+    table = torch.arange(nb, dtype=torch.int32, device=DEV)[None]
+    got = ops.swa_sink_attn(q.float().reshape(T, H * D).to(DEV), H, pages(k), pages(v), table, meta, sink.to(DEV), D**-0.5, window, out_f32=True)
+    want = sink_window_attention(q.double(), k.double(), v.double(), sink.double(), D**-0.5, window)
+    assert (got.double().cpu() - want).abs().max() <= 2.0**-13 * v.double().abs().max()
+
+
 @pytest.mark.parametrize("chunks", [[150], [16, 64, 3, 67], [33, 1, 1, 17, 98]])
 def test_tensor_core_prompt_attention_edges(chunks):
     """bf16 pools, head sizes 32 / 48: portions of 16 tokens or more run on the mma.sync kernel (64-row tiles, 32-key tiles

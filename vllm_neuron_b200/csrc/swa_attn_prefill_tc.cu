@@ -499,6 +499,11 @@ int b200_swa_attn_prefill_tc_sink(const float* q, int ldq, const void* k_pool, c
     return B200_ERR_UNSUPPORTED;
   }
   if (B <= 0 || max_new <= 0) return B200_OK;
+  // With a sink the weights go as two bf16 terms: the maximum starts at the sink and moves in steps of 2^8, so the largest weight is no longer
+  // exactly 1 and one rounding costs more than in the mma.sync kernel, which long prompts with a sink would take otherwise.  Difference from
+  // 64 bits, fp32 outputs, 16 heads of 128, window 1024, 4096 tokens: mma.sync 2.04e-3 (276 us), here 2.27e-3 with one term (92 us),
+  // 1.56e-3 with two (94 us).
+  split_p = split_p || sink;
   CUtensorMap km, vm;
   // key rows of 32 columns are 64 bytes: boxes of 32 columns x 32 rows under the 64B swizzle
   int rc = D == 32 ? make_tmap_2d_sw64(&km, k_pool, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 32, (uint64_t)num_blocks * G * TP_BLK, 64, 32,
