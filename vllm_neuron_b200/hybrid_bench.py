@@ -395,12 +395,13 @@ def _floors(cfg, sz, t, keys_per_query, kv_tokens, nseq):
     used = min(m["experts"], pairs)
     att = (2.0 * t * a["heads"] * keys_per_query * (a["dim"] + a["vdim"]),
            2.0 * kv_tokens * a["kv_heads"] * (a["dim"] + a["vdim"]) + t * a["heads"] * (4 * a["dim"] + 2 * a["vdim"]))
+    ssd = (6.0 * t * s["heads"] * s["state"] * s["vdim"],
+           t * (2 * c + 4 * s["heads"] + 4 * inner) + 8.0 * nseq * s["heads"] * s["state"] * s["vdim"])
     return {
-        "swa_sink_attn_prefill": att, "swa_sink_attn_decode_tc": att,
+        "swa_sink_attn_prefill": att, "swa_sink_attn_prefill_tc": att, "swa_sink_attn_decode_tc": att,
         "swa_sink_attn": (2.0 * t * a["heads"] * keys_per_query * (a["dim"] + a["vdim"]),
                           2.0 * kv_tokens * a["kv_heads"] * (a["dim"] + a["vdim"]) + t * a["heads"] * (4 * a["dim"] + 2 * a["vdim"])),
-        "ssd_scan": (6.0 * t * s["heads"] * s["state"] * s["vdim"],
-                     t * (2 * c + 4 * s["heads"] + 4 * inner) + 8.0 * nseq * s["heads"] * s["state"] * s["vdim"]),
+        "ssd_scan": ssd, "ssd_step": ssd,
         "moe_gate_up_glu": (4.0 * pairs * m["ff"] * w, used * 4.0 * m["ff"] * w + t * 2 * w + pairs * 2 * m["ff"]),
         "moe_down": (2.0 * pairs * m["ff"] * w, used * 2.0 * m["ff"] * w + pairs * (2 * m["ff"] + 4 * w)),
         "moe_gather_scale": (0.0, pairs * w * 4.0),
