@@ -773,3 +773,23 @@ def test_ssd_step_of_one_token_each(H, P, N, G, dtype):
     terms = S * Cm[:, :, None, :]
     bound = (N + 1) * 2.0**-24 * (terms.abs().sum(-1) + skip.abs())
     assert ((y.double().cpu().view(3, H, P) - terms.sum(-1) - skip).abs() <= bound).all()
+
+
+def test_ssd_step_sees_parameters_that_the_kernel_ahead_wrote():
+    """Decay, bias and skip rows that come straight out of another kernel of the library, whose blocks let the next one start early: the same
+    call on the same rows, once they are there, gives the same bits."""
+    ops = _ops()
+    H, P, N, G, W = 8, 64, 64, 2, 1024
+    g = torch.Generator().manual_seed(4)
+    src, one, zero = torch.randn(8, 3000, W, generator=g).to(DEV), torch.ones(W, device=DEV), torch.zeros(W, device=DEV)
+    xbc, raw, state = torch.randn(2, H * P + 2 * G * N, generator=g).to(DEV), torch.randn(2, H, generator=g).to(DEV), torch.randn(2, H, P, N, generator=g).to(DEV)
+    meta = _meta([(0, 5, 1), (1, 9, 1)], {0: [1] * 40, 1: [2] * 40})
+    runs = []
+    for i in range(8):
+        s = state.clone()
+        p = ops.dyt_norm(src[i], one, zero, 1.0, torch.float32)[-1]
+        runs.append((p, s, ops.ssd_scan(xbc, raw, 0, p[:H], p[H:2 * H], p[2 * H:3 * H], s, meta, H, P, N, G)))
+    torch.cuda.synchronize()
+    for p, s, y in runs:
+        want = state.clone()
+        assert torch.equal(y, ops.ssd_scan(xbc, raw, 0, p[:H], p[H:2 * H], p[2 * H:3 * H], want, meta, H, P, N, G)) and torch.equal(s, want)

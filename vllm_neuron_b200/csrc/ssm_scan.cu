@@ -343,9 +343,9 @@ __global__ void __launch_bounds__(STEP_WARPS * 32)
   constexpr int N = 4 * LANES, PER = 32 / LANES;  // state size; rows a warp reads with one load per lane
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane / LANES, c4 = lane % LANES * 4;
   const int h = blockIdx.y, sq = blockIdx.z;
-  const float negA = -expf(A_log[h]), bias = dt_bias[h], dsk = Dskip[h];  // weights
   griddep_launch();
-  griddep_wait();
+  griddep_wait();  // before the parameters too: they may be what the kernel ahead has written
+  const float negA = -expf(A_log[h]), bias = dt_bias[h], dsk = Dskip[h];
   const int t = seq_start[sq];
   if (t >= seq_start[sq + 1]) return;
   const int row0 = (blockIdx.x * STEP_WARPS + warp) * STEP_ROWS * PER;  // rows row0 + i PER + sub
