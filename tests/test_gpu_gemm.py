@@ -497,3 +497,21 @@ def test_gemm_of_a_few_tokens_on_any_boundary(ops):
     buf = torch.zeros(3 * 40 + 8, dtype=torch.bfloat16, device="cuda")
     assert _cabi.load().b200_gemm(x.data_ptr(), w.data_ptr(), buf.data_ptr() + 2, 0, 0, 0, 0, 3, 40, 256, ops.BF16, ops.BF16, 0, 0, 0, 0) == 0
     assert torch.equal(buf[1:121].view(3, 40), ops.gemm(x, w)) and not buf[121:].any() and not buf[0]
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1024, 512), (8, 512, 4096)])
+def test_gemm_of_a_few_tokens_sees_scales_and_biases_that_the_kernel_ahead_wrote(ops, m, n, k):
+    """Scale and bias rows that come straight out of another kernel of the library, whose blocks let the next one start early: the same call
+    on the same rows, once they are there, gives the same bits."""
+    g = torch.Generator().manual_seed(m)
+    src, one, zero = torch.randn(8, 3000, n, generator=g).cuda(), torch.ones(n).cuda(), torch.zeros(n).cuda()
+    x, w = torch.randn(m, k, generator=g).bfloat16().cuda(), torch.randint(-127, 128, (n, k), generator=g).to(torch.int8).cuda()
+    runs = []
+    for i in range(8):
+        scale = ops.dyt_norm(src[i], one, zero, 1.0, torch.float32)[-1]
+        first = ops.gemm(x, w, None, scale)
+        bias = ops.dyt_norm(src[i], one, zero, 0.5, torch.bfloat16)[-1]
+        runs.append((scale, bias, first, ops.gemm(x, w, None, scale, bias)))
+    torch.cuda.synchronize()
+    for scale, bias, first, both in runs:
+        assert torch.equal(first, ops.gemm(x, w, None, scale)) and torch.equal(both, ops.gemm(x, w, None, scale, bias))

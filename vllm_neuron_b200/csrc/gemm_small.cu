@@ -123,7 +123,11 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
 #pragma unroll
   for (int s = 0; s < PF; ++s)
     if (warp + s * WARPS < nkb) load_w(wb[s], warp + s * WARPS);
-  // the epilogue's operands of this thread's items: weights' side now, tokens' side while the products are taken
+  griddep_wait();  // before everything but the weights: scales and biases may be what the kernel ahead has written
+#pragma unroll
+  for (int s = 0; s < PF; ++s)
+    if (warp + s * WARPS < nkb) load_x(xb[s], warp + s * WARPS);
+  // the epilogue's operands of this thread's items, while the products are taken
   float wsc[PER][SIDES], bia[PER][SIDES], asc[PER], res[PER];
   long long pos[PER], slot[PER];
   const bool hb = ep.bias != nullptr, hr = EPI == EPI_LINEAR && ep.residual != nullptr;
@@ -135,10 +139,6 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
       wsc[q][sd] = i < ITEMS && n < N && ep.w_scale ? ep.w_scale[n] : 1.f;
       bia[q][sd] = i < ITEMS && n < N && hb ? __bfloat162float(ep.bias[n]) : 0.f;
     }
-  griddep_wait();
-#pragma unroll
-  for (int s = 0; s < PF; ++s)
-    if (warp + s * WARPS < nkb) load_x(xb[s], warp + s * WARPS);
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
     const int i = threadIdx.x + q * THREADS, m = i / ITEM_ROWS, n = row0[0] + i % ITEM_ROWS;
