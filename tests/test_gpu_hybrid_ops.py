@@ -793,3 +793,20 @@ def test_ssd_step_sees_parameters_that_the_kernel_ahead_wrote():
     for p, s, y in runs:
         want = state.clone()
         assert torch.equal(y, ops.ssd_scan(xbc, raw, 0, p[:H], p[H:2 * H], p[2 * H:3 * H], want, meta, H, P, N, G)) and torch.equal(s, want)
+
+
+@pytest.mark.parametrize("window", [100, 1 << 30])
+def test_decode_attention_over_a_page_that_is_not_there(window):
+    """A page number below 0 stands for rows of zeros, inside the window too."""
+    from vllm_neuron_b200.hybrid import StepMeta
+
+    ops = _ops()
+    g = torch.Generator(device=DEV).manual_seed(3)
+    G, D, H = 2, 64, 8
+    kp, vp = (torch.randn(10, G, 32, D, generator=g, device=DEV).bfloat16() for _ in range(2))
+    kp[9], vp[9] = 0, 0
+    meta = StepMeta.build([(0, 200, 1), (1, 130, 1)], {0: list(range(1, 8)), 1: list(range(1, 8))}, 32, torch.device(DEV))
+    table = torch.tensor([[1, 2, 3, 4, 5, 9, 7], [2, 9, 1, 9, 3, 4, 5]], dtype=torch.int32, device=DEV)
+    q, sink = torch.randn(2, H * D, generator=g, device=DEV), torch.randn(H, generator=g, device=DEV)
+    want = ops.swa_sink_attn(q, H, kp, vp, table, meta, sink, 0.1, window)
+    assert torch.equal(ops.swa_sink_attn(q, H, kp, vp, torch.where(table == 9, -1, table), meta, sink, 0.1, window), want)

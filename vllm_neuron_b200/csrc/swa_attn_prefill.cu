@@ -398,8 +398,9 @@ __global__ void __launch_bounds__(DT_WARPS * 32)
     const int j_end = early ? nb - 1 : pos;                              // last visible one
     const int j_lo = early ? 0 : lo;
     if (paged && !early) {
-      const int64_t blk = bt[j0 / bs];
-      const int r_lo_k = max(lo - j0, 0), r_hi_k = min(pos - j0, LDT_KEYS - 1);  // visible rows
+      const int page = bt[j0 / bs];
+      const int64_t blk = max(page, 0);
+      const int r_lo_k = max(lo - j0, 0), r_hi_k = page < 0 ? -1 : min(pos - j0, LDT_KEYS - 1);  // visible rows; a page below 0 is zeros
 #pragma unroll
       for (int sl = 0; sl < DT_SLOTS; ++sl) {
         if (ch_on[sl]) {
