@@ -810,3 +810,24 @@ def test_decode_attention_over_a_page_that_is_not_there(window):
     q, sink = torch.randn(2, H * D, generator=g, device=DEV), torch.randn(H, generator=g, device=DEV)
     want = ops.swa_sink_attn(q, H, kp, vp, table, meta, sink, 0.1, window)
     assert torch.equal(ops.swa_sink_attn(q, H, kp, vp, torch.where(table == 9, -1, table), meta, sink, 0.1, window), want)
+
+
+def _one_sequence(T, G, Gv, D, Dv, g):
+    """bf16 pools of one sequence on pages in reverse, and the same rows in 64 bits: (meta, table, key pool, value pool, keys, values)."""
+    from vllm_neuron_b200.hybrid import StepMeta
+
+    nb = -(-T // 32)
+    pages = list(range(nb, 0, -1))
+    kp, vp = (torch.randn(nb + 1, n, 32, d, generator=g, device=DEV).bfloat16() for n, d in ((G, D), (Gv, Dv)))
+    meta = StepMeta.build([(0, 0, T)], {0: pages}, 32, torch.device(DEV))
+    k, v = (p[pages].transpose(1, 2).reshape(nb * 32, -1, p.shape[3])[:T].double() for p in (kp, vp))
+    return meta, torch.tensor([pages], dtype=torch.int32, device=DEV), kp, vp, k, v
+
+
+def test_a_window_of_no_tokens_beside_a_sink_is_refused():
+    ops = _ops()
+    g = torch.Generator(device=DEV).manual_seed(1)
+    for T in (40, 200):
+        meta, table, kp, vp, _, _ = _one_sequence(T, 2, 2, 64, 64, g)
+        with pytest.raises(RuntimeError):
+            ops.swa_sink_attn(torch.randn(T, 4 * 64, generator=g, device=DEV), 4, kp, vp, table, meta, torch.zeros(4, device=DEV), 0.1, 0)

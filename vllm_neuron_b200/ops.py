@@ -843,6 +843,8 @@ def _swa_part(q_src, num_heads, k_pool, v_pool, block_table, meta, sink, scale, 
     tag = "[latent]" if plain and latent_values else "" if plain and not pool and not keep else "[" + "+".join(n for n, on in (("chunk", chunk), ("cap", softcap), ("sigmoid", sigmoid_bias is not None),
                                                                        ("maps", v_div > 1), ("pool", pool), ("keep", keep)) if on) + "]"
     if _prompt_tc(q_all, k_pool, meta, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool):
+        if sink is not None and window < 1:
+            raise _cabi.B200Error(f"swa_sink_attn: a window of {window}")
         with _k("swa_sink_attn_prefill_tc" + tag):
             check(_lib().b200_swa_attn_prefill_tc_sink(q_all, q_all.stride(0), k_pool, v_pool, k_pool.shape[0],
                                                              block_table, block_table.stride(0), meta.seq_start,
