@@ -824,6 +824,46 @@ def _one_sequence(T, G, Gv, D, Dv, g):
     return meta, torch.tensor([pages], dtype=torch.int32, device=DEV), kp, vp, k, v
 
 
+@pytest.mark.parametrize("kind,D,Dv,G", [("cap", 128, 128, 2), ("cap", 128, 64, 4), ("chunk", 64, 64, 2), ("chunk+cap", 64, 64, 2), ("keep", 128, 128, 2),
+                                         ("keep", 128, 64, 2), ("maps", 32, 64, 4), ("maps", 64, 128, 2), ("maps+window", 64, 64, 2), ("none", 64, 64, 2)])
+def test_sink_of_prompts_beside_the_other_options(kind, D, Dv, G):
+    """A sink with a soft cap (which it does not pass), chunks, kept tokens and two score maps, and sinks of -inf, against 64 bits.  Weights in two
+    bf16 terms and fp32 rows: 2^-15 of a row's weighted values, and the query's rounding to bf16, which the reference shares."""
+    ops = _ops()
+    g = torch.Generator(device=DEV).manual_seed(D + G)
+    T, H, maps = 300, 8, kind.startswith("maps")
+    meta, table, kp, vp, k, v = _one_sequence(T, G, G // 2 if maps else G, D, Dv, g)
+    q = torch.randn(T, H * D, generator=g, device=DEV).bfloat16().float()
+    sink = 2 * torch.randn(H, generator=g, device=DEV) + 2
+    if kind == "none":
+        sink[:] = -math.inf
+    kw, window, scale = {}, 1 << 30, 2 * D**-0.5
+    if "cap" in kind:
+        kw["softcap"] = 2.0
+    if "chunk" in kind:
+        kw["chunk"] = 130
+    if kind == "keep":
+        kw["keep"], window = 70, 90
+    if "window" in kind:
+        window = 100
+    with ops.kernel_timer() as kt:
+        got = ops.swa_sink_attn(q, H, kp, vp, table, meta, sink, scale, window, out_f32=True, **kw)
+    assert any(n.startswith("swa_sink_attn_prefill_tc") for n in kt.summary())
+    i = torch.arange(T, device=DEV)
+    seen = (i[None] <= i[:, None]) & ((i[None] > i[:, None] - window) | (i[None] < kw.get("keep", 0)))
+    if "chunk" in kind:
+        seen &= i[None] // 130 == i[:, None] // 130
+    of = torch.arange(H, device=DEV) // (H // G)
+    s = torch.einsum("thd,lhd->htl", q.double().view(T, H, D), k[:, of]) * scale
+    if "cap" in kind:
+        s = 2.0 * torch.tanh(s / 2.0)
+    s = torch.cat([s.masked_fill(~seen, -math.inf), sink.double()[:, None, None].expand(H, T, 1)], 2)
+    p, vh = torch.softmax(s, 2)[..., :T], v[:, of // 2 if maps else of]
+    want, size = torch.einsum("htl,lhd->thd", p, vh), torch.einsum("htl,lhd->thd", p, vh.abs())
+    # scores in fp32 and exponents by the fast exponential: 2^-17 of a weight each, beside the two terms' 2^-16
+    assert ((got.double().view(T, H, Dv) - want).abs() <= 2.0**-13 * size).all()
+
+
 def test_a_window_of_no_tokens_beside_a_sink_is_refused():
     ops = _ops()
     g = torch.Generator(device=DEV).manual_seed(1)
