@@ -73,3 +73,24 @@ def test_product_does_not_import_oracle():
         ["grep", "-rnE", r"^\s*(from|import)\s+oracle", os.path.join(ROOT, "vllm_neuron_b200")], capture_output=True, text=True
     )
     assert out.stdout == "", out.stdout
+
+
+def test_kernel_timer_closed_during_a_launch(monkeypatch):
+    """A launch that another thread's timer was open for when it began ends in that timer's list, not in an error."""
+    import torch
+
+    from vllm_neuron_b200 import ops
+
+    class Event:
+        def __init__(self, **kw):
+            pass
+
+        def record(self):
+            pass
+
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    timer = ops.kernel_timer()
+    timer.__enter__()
+    with ops._k("gemm[{}]", 3):
+        timer.__exit__()
+    assert [r[0] for r in timer.records] == ["gemm[3]"] and ops._PROF is None

@@ -51,10 +51,10 @@ class kernel_timer:
 
 
 class _Timed:
-    __slots__ = ("name", "e0")
+    __slots__ = ("name", "to", "e0")
 
-    def __init__(self, name):
-        self.name = name
+    def __init__(self, name, to):
+        self.name, self.to = name, to  # the timer may be closed by another thread before the launch is over
 
     def __enter__(self):
         self.e0 = torch.cuda.Event(enable_timing=True)
@@ -63,7 +63,7 @@ class _Timed:
     def __exit__(self, *exc):
         e1 = torch.cuda.Event(enable_timing=True)
         e1.record()
-        _PROF.append((self.name, self.e0, e1))
+        self.to.append((self.name, self.e0, e1))
         return False
 
 
@@ -80,7 +80,8 @@ _UNTIMED = _Untimed()
 
 def _k(name, *sizes):
     """Context of one launch: timed under its name (a format of the sizes) while a kernel_timer is open."""
-    return _UNTIMED if _PROF is None else _Timed(name.format(*sizes))
+    to = _PROF
+    return _UNTIMED if to is None else _Timed(name.format(*sizes), to)
 
 
 def _lib():
