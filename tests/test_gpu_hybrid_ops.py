@@ -812,6 +812,40 @@ def test_decode_attention_over_a_page_that_is_not_there(window):
     assert torch.equal(ops.swa_sink_attn(q, H, kp, vp, torch.where(table == 9, -1, table), meta, sink, 0.1, window), want)
 
 
+def test_allocations_leave_the_interpreter_to_other_threads():
+    """A result that has to wait for the device, because cached memory is given back for it, does not hold up other threads' Python."""
+    import threading
+    import time
+
+    ops = _ops()
+    like, held, over = torch.zeros(1, device=DEV), [0.0], threading.Event()
+
+    def work():
+        last = time.perf_counter()
+        while not over.is_set():
+            now = time.perf_counter()
+            held[0], last = max(held[0], now - last), now
+
+    thread = threading.Thread(target=work)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    cached = torch.empty(1 << 30, dtype=torch.uint8, device=DEV)
+    del cached
+    room = torch.cuda.memory_reserved() + (64 << 20)
+    torch.cuda.set_per_process_memory_fraction(room / torch.cuda.get_device_properties(0).total_memory)
+    try:
+        torch.cuda._sleep(1 << 29)  # a quarter of a second or more
+        thread.start()
+        t0 = time.perf_counter()
+        made = ops._new(like, torch.uint8, (1 << 30) + (16 << 20))
+        took = time.perf_counter() - t0
+    finally:
+        over.set()
+        thread.join()
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert made.numel() > 1 << 30 and took > 0.1 and held[0] < took / 2
+
+
 def _one_sequence(T, G, Gv, D, Dv, g):
     """bf16 pools of one sequence on pages in reverse, and the same rows in 64 bits: (meta, table, key pool, value pool, keys, values)."""
     from vllm_neuron_b200.hybrid import StepMeta

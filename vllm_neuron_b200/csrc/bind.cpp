@@ -24,6 +24,11 @@ PyObject* g_error = nullptr;  // vllm_neuron_b200._cabi.B200Error
 
 struct Raised {};  // a Python exception is set
 
+struct Unlocked {  // other threads run Python meanwhile; taken back also where a C++ exception passes
+  PyThreadState* state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 template <typename T>
 T arg(PyObject* o) {
   if constexpr (std::is_pointer_v<T>) {
@@ -66,11 +71,8 @@ struct Call<Fn> {
     if constexpr (streamed) {
       if (n == N - 1) std::get<N - 1>(v) = (void*)c10::cuda::getCurrentCUDAStream().stream();
     }
-    R r;
-    Py_BEGIN_ALLOW_THREADS  // a full launch queue blocks here
-    r = std::apply(Fn, v);
-    Py_END_ALLOW_THREADS
-    return r;
+    Unlocked u;  // a full launch queue blocks here
+    return std::apply(Fn, v);
   }
   static PyObject* call(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
@@ -103,7 +105,13 @@ PyObject* new_tensor(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (shape[i - 2] == -1 && PyErr_Occurred()) return nullptr;
   }
   const at::ScalarType type = args[1] == Py_None ? like.scalar_type() : reinterpret_cast<THPDtype*>(args[1])->scalar_type;
-  return THPVariable_Wrap(at::empty(at::IntArrayRef(shape, n - 2), at::TensorOptions().dtype(type).device(like.device())));
+  const auto options = at::TensorOptions().dtype(type).device(like.device());
+  at::Tensor made;
+  {
+    Unlocked u;  // an allocation that gives cached blocks back waits for the device
+    made = at::empty(at::IntArrayRef(shape, n - 2), options);
+  }
+  return THPVariable_Wrap(std::move(made));
   END_HANDLE_TH_ERRORS
 }
 
