@@ -75,6 +75,37 @@ def test_product_does_not_import_oracle():
     assert out.stdout == "", out.stdout
 
 
+def test_binding_is_made_anew_for_another_torch(lib, monkeypatch):
+    """An up-to-date module is left alone; one that another torch was there for is compiled again, whatever the files' times say."""
+    import torch
+
+    from vllm_neuron_b200 import build
+
+    calls = []
+    monkeypatch.setattr(build.subprocess, "check_call", lambda cmd: calls.append(cmd))
+    build.build_bind()
+    assert not calls
+    stamp = os.path.join(build.HERE, "build", "bind_command.txt")
+    kept = open(stamp).read()
+    try:
+        monkeypatch.setattr(torch, "__version__", "0.0.1")
+        build.build_bind()
+        assert len(calls) == 1 and '-DB200_BIND_TORCH="0.0.1"' in calls[0]
+    finally:
+        open(stamp, "w").write(kept)
+
+
+def test_binding_of_another_torch_is_refused(lib, monkeypatch):
+    import torch
+
+    from vllm_neuron_b200 import _cabi
+
+    assert _cabi.native().torch == torch.__version__
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    with pytest.raises(_cabi.B200Error, match="built for torch"):
+        _cabi.native()
+
+
 def test_kernel_timer_closed_during_a_launch(monkeypatch):
     """A launch that another thread's timer was open for when it began ends in that timer's list, not in an error."""
     import torch

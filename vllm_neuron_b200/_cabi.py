@@ -169,10 +169,15 @@ def load():
 def native():
     """The functions that take tensors (csrc/bind.cpp), over the same library."""
     load()
+    import torch
+
+    remedy = "build it with `python -m vllm_neuron_b200.build`"
     try:
         from . import _b200_bind
     except ImportError as e:
-        raise B200Error(f"the Python binding is missing or does not load ({e}): build it with `python -m vllm_neuron_b200.build`") from e
+        raise B200Error(f"the Python binding is missing or does not load ({e}): {remedy}") from e
+    if _b200_bind.torch != torch.__version__:  # it reads tensors by that version's layout
+        raise B200Error(f"the Python binding was built for torch {_b200_bind.torch}, this is {torch.__version__}: {remedy}")
     _b200_bind.set_error(B200Error)
     return _b200_bind
 

@@ -7,6 +7,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -15,7 +16,8 @@ SOURCES = ["host.cu", "kv_ops.cu", "paged_attn.cu", "paged_attn_prefill_tc.cu", 
            "dyt_norm.cu", "ssm_scan.cu", "ssm_segment.cu", "swa_attn.cu", "swa_attn_prefill.cu", "swa_attn_prefill_tc.cu", "moe.cu", "rms_norm.cu", "delta_rule.cu",
            "latent_attn.cu", "gated_scan.cu", "selective_scan.cu", "hyper_conn.cu"]
 HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "gemm_common.cuh"), os.path.join(CSRC, "gemm_pair.cuh"), os.path.join(CSRC, "gemm_group.cuh"), os.path.join(CSRC, "gemm_small.cuh"), os.path.join(CSRC, "hybrid_common.cuh"), os.path.join(CSRC, "ssm_common.cuh"), os.path.join(os.path.dirname(HERE), "include", "b200_paged.h")]
-BIND = os.path.join(HERE, "_b200_bind.so")  # the library's functions on torch tensors, for ops.py
+# the library's functions on torch tensors, for ops.py: good for the Python in its name and the torch that its attribute `torch` names
+BIND = os.path.join(HERE, "_b200_bind" + sysconfig.get_config_var("EXT_SUFFIX"))
 BIND_SOURCES = [os.path.join(CSRC, "bind.cpp"), os.path.join(os.path.dirname(HERE), "include", "b200_paged.h")]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -40,20 +42,29 @@ def needs_build() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
-def build_bind(force: bool = False) -> str:
-    """The extension module beside the library (host code only)."""
-    if not force and os.path.exists(BIND) and all(os.path.getmtime(d) <= os.path.getmtime(BIND) for d in BIND_SOURCES):
-        return BIND
-    import sysconfig
-
+def _bind_command() -> list:
     import torch
 
     t = os.path.dirname(torch.__file__)
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", sysconfig.get_paths()["include"], "-I", f"{t}/include",
-           "-I", f"{t}/include/torch/csrc/api/include", "-I", os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include"), BIND_SOURCES[0],
-           "-o", BIND, "-L", f"{t}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-L", HERE, "-l:libb200_paged.so", "-Wl,-rpath,$ORIGIN"]
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DB200_BIND_TORCH="{torch.__version__}"',
+            "-I", sysconfig.get_paths()["include"], "-I", f"{t}/include", "-I", f"{t}/include/torch/csrc/api/include",
+            "-I", os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include"), BIND_SOURCES[0],
+            "-o", BIND, "-L", f"{t}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-L", HERE, "-l:libb200_paged.so", "-Wl,-rpath,$ORIGIN"]
+
+
+def build_bind(force: bool = False) -> str:
+    """The extension module beside the library (host code only).  Another torch, Python or compiler flag makes it anew."""
+    cmd = _bind_command()
+    stamp = os.path.join(HERE, "build", "bind_command.txt")
+    made = " ".join([sys.version, *cmd])
+    if not force and os.path.exists(BIND) and all(os.path.getmtime(d) <= os.path.getmtime(BIND) for d in BIND_SOURCES):
+        if os.path.exists(stamp) and open(stamp).read() == made:
+            return BIND
     subprocess.check_call(cmd)
+    os.makedirs(os.path.dirname(stamp), exist_ok=True)
+    with open(stamp, "w") as f:
+        f.write(made)
     return BIND
 
 

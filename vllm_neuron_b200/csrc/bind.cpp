@@ -147,4 +147,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_b200_bind", nullptr, -1, methods,
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__b200_bind(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__b200_bind(void) {
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "torch", B200_BIND_TORCH) < 0) Py_CLEAR(m);
+  return m;
+}
