@@ -11,6 +11,7 @@
 //
 // Prefix-cached prefill (batch 1, q_len > 1) is a flash-attention-2 style kernel over the same TMA tiles with
 // the causal mask shifted by the cached prefix length.
+#include <array>
 #include <mutex>
 #include <unordered_map>
 
@@ -449,9 +450,10 @@ __global__ void __launch_bounds__(COMB_THREADS)
 // ---- decode of few blocks, bf16 output: one cluster per (sequence, kv head), its result in one launch
 // With few sequences of short context the balanced split above leaves a block or two to a warp, and what is left is latency: the prefix sum, the
 // search, the trip of the partials through memory and the merge kernel's launch.  Here the pair's 32-token blocks are dealt to the eight warps
-// of the S CTAs of a cluster, and the warps' (m, l, O) meet in shared memory.  Same products and roundings per block as above.
-// Decode steps, us, by the split above and its merge / here: TinyLlama, one sequence at 161, 779 / 666 (8.6 us a layer for the two launches, 3.5
-// here).
+// of the S CTAs of a cluster, and the warps' (m, l, O) meet in shared memory: a CTA's eight first, then the cluster's S.  Same products and
+// roundings per block as above.  Decode steps, us, by the split above and its merge / here: TinyLlama, one sequence at 161, 779 / 666 (8.6 us a
+// layer for the two launches, 3.5 here).  All 8 S parts read over the cluster in one go took 18.6 for one sequence at 8192, 8 kv heads of 128, where
+// the split takes 36.8 and this 11.9, and 15.4, 8.2 and 5.8 for one kv head at 600 of a table of 96 blocks.
 constexpr int FEW_WARPS = 8;
 
 __device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
@@ -471,7 +473,8 @@ __global__ void __launch_bounds__(FEW_WARPS * 32, 1)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* O = reinterpret_cast<float*>(smem + FEW_WARPS * NST * 2 * TILE);   // [warps][8][D]
   float* ml = O + FEW_WARPS * 8 * D;                                        // [warps][8][2]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ml + FEW_WARPS * 16) + (threadIdx.x >> 5) * NST;
+  float2* cml = reinterpret_cast<float2*>(ml + FEW_WARPS * 16);             // [8]: (m, l) of the CTA
+  uint64_t* bars = reinterpret_cast<uint64_t*>(cml + 8) + (threadIdx.x >> 5) * NST;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = (int)cluster_nctarank(), rank = (int)cluster_ctarank();
   const int kvh = blockIdx.y, b = blockIdx.z, G = Hq / Hkv;
@@ -596,30 +599,62 @@ __global__ void __launch_bounds__(FEW_WARPS * 32, 1)
   if (qn == 0) {
     *reinterpret_cast<float4*>(ml + (warp * 8 + h0) * 2) = make_float4(m0, l0, m1, l1);
   }
-  if (S > 1) cluster_sync_all();
-  else __syncthreads();
-  // ---- the heads' column pairs rank, rank + S, .. from all the warps, in order
-  for (int i = threadIdx.x * S + rank; i < G * (D / 2); i += FEW_WARPS * 32 * S) {
+  __syncthreads();
+  auto store = [&](int h, int c, float L, float2 v) {
+    const bool any = L > 0.f;
+    *reinterpret_cast<uint32_t*>(out + ((int64_t)b * Hq + kvh * G + h) * D + c) = pack_bf16(any ? v.x / L : 0.f, any ? v.y / L : 0.f);
+  };
+  // ---- the heads' column pairs from the CTA's warps, in order
+  for (int i = threadIdx.x; i < G * (D / 2); i += FEW_WARPS * 32) {
     const int h = i / (D / 2), c = i % (D / 2) * 2;
-    const uint32_t o_at = smem_u32(O) + (h * D + c) * 4, ml_at = smem_u32(ml) + h * 8;
     float M = -INFINITY, L = 0.f;
     float2 acc = make_float2(0.f, 0.f);
-    for (int r = 0; r < S; ++r)
 #pragma unroll
-      for (int w = 0; w < FEW_WARPS; ++w) M = fmaxf(M, ld_cluster_f2(mapa_shared(ml_at + w * 64, r)).x);
-    for (int r = 0; r < S; ++r)
+    for (int w = 0; w < FEW_WARPS; ++w) M = fmaxf(M, ml[(w * 8 + h) * 2]);
 #pragma unroll
-      for (int w = 0; w < FEW_WARPS; ++w) {
-        const float2 p = ld_cluster_f2(mapa_shared(ml_at + w * 64, r)), o = ld_cluster_f2(mapa_shared(o_at + w * 8 * D * 4, r));
-        const float f = p.x == -INFINITY ? 0.f : exp2f(p.x - M);  // a warp without a block
-        L += f * p.y;
-        acc.x += f * o.x;
-        acc.y += f * o.y;
-      }
-    const bool any = L > 0.f;
-    *reinterpret_cast<uint32_t*>(out + ((int64_t)b * Hq + kvh * G + h) * D + c) = pack_bf16(any ? acc.x / L : 0.f, any ? acc.y / L : 0.f);
+    for (int w = 0; w < FEW_WARPS; ++w) {
+      const float2 p = *reinterpret_cast<const float2*>(ml + (w * 8 + h) * 2), o = *reinterpret_cast<const float2*>(O + (w * 8 + h) * D + c);
+      const float f = p.x == -INFINITY ? 0.f : exp2f(p.x - M);  // a warp without a block
+      L += f * p.y;
+      acc.x += f * o.x;
+      acc.y += f * o.y;
+    }
+    if (S == 1) {
+      store(h, c, L, acc);
+    } else {
+      *reinterpret_cast<float2*>(O + h * D + c) = acc;  // the first warp's part, which no other thread reads
+      if (c == 0) cml[h] = make_float2(M, L);
+    }
   }
-  if (S > 1) cluster_sync_all();  // nobody leaves while a peer still reads its parts
+  if (S == 1) return;
+  // ---- then the pairs rank, rank + S, .. from the cluster's CTAs, in order: S loads over the cluster, not 8 S
+  cluster_sync_all();
+  for (int i = threadIdx.x * S + rank; i < G * (D / 2); i += FEW_WARPS * 32 * S) {
+    const int h = i / (D / 2), c = i % (D / 2) * 2;
+    const uint32_t o_at = smem_u32(O) + (h * D + c) * 4, ml_at = smem_u32(cml) + h * 8;
+    float2 p[8], o[8];
+    float M = -INFINITY, L = 0.f;
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (r < S) {
+        p[r] = ld_cluster_f2(mapa_shared(ml_at, r));
+        o[r] = ld_cluster_f2(mapa_shared(o_at, r));
+      }
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (r < S) M = fmaxf(M, p[r].x);
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (r < S) {
+        const float f = p[r].x == -INFINITY ? 0.f : exp2f(p[r].x - M);
+        L += f * p[r].y;
+        acc.x += f * o[r].x;
+        acc.y += f * o[r].y;
+      }
+    store(h, c, L, acc);
+  }
+  cluster_sync_all();  // nobody leaves while a peer still reads its parts
 }
 
 // ============================================================ prefix-cached prefill (one sequence)
@@ -911,11 +946,49 @@ int launch_decode(const CUtensorMap& km, const CUtensorMap& vm, const void* q, i
   return B200_OK;
 }
 
-// CTAs of a cluster that give every warp at most FEW_BLOCKS blocks, or 0 where the chip does not hold them all at once
+template <int D>
+constexpr size_t few_smem() {
+  return (size_t)FEW_WARPS * (128 / D * 2 * BS * D * 2 + 8 * D * 4 + 64 + 16) + 64 + 1024;
+}
+// Clusters of S = 1, 2, 4, 8 CTAs that the chip holds at once
+template <int D>
+const int* few_clusters() {
+  static const std::array<int, 4> fit = [] {
+    std::array<int, 4> n{};
+    auto kern = paged_attn_decode_few_kernel<D>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem<D>());
+    for (int i = 0; i < 4; ++i) {
+      cudaLaunchConfig_t cfg{};
+      cudaLaunchAttribute at[1];
+      cfg.gridDim = dim3(1 << i);
+      cfg.blockDim = dim3(FEW_WARPS * 32);
+      cfg.dynamicSmemBytes = few_smem<D>();
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = 1u << i;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&n[i], kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n[i] = 0;
+      }
+    }
+    return n;
+  }();
+  return fit.data();
+}
+// CTAs of a cluster: the fewest that give every warp at most FEW_BLOCKS blocks of a full table (FEW_BLOCKS_MOST with the largest cluster), or 0 --
+// the split above -- where that is too many blocks or the chip does not hold all clusters at once (clusters of four and eight do not fill
+// it: 18 sequences, one kv head of 128, table of 96 blocks, 18 clusters of eight 31.4 us, the split 9.4).  Over 1100 shapes of 1 to 148 sequences, 1 to 8
+// kv heads and tables of 1 to 256 blocks, full and a fifth full, this takes 0.18 to 0.77 of the split's time (quantised 0.38 to 0.91); at the edges, split / here: 18
+// sequences at 512 on 8 kv heads of 128 12.2 / 9.0, 9 at 1024 14.0 / 10.4, 4 at 2048 16.8 / 10.1, 12 at 4096 on one 22.5 / 10.4.
+constexpr int FEW_BLOCKS = 2, FEW_BLOCKS_MOST = 4;
+template <int D>
 int few_split(int B, int Hkv, int max_blocks) {
-  for (int S = 1; S <= 8; S <<= 1) {
-    if ((int64_t)B * Hkv * S > sm_count()) return 0;
-    if (max_blocks <= 2 * FEW_WARPS * S || (S == 8 && max_blocks <= 4 * FEW_WARPS * S)) return S;
+  for (int i = 0; i < 4; ++i) {
+    const int S = 1 << i;
+    if ((int64_t)B * Hkv > few_clusters<D>()[i]) return 0;
+    if (max_blocks <= FEW_WARPS * S * (S == 8 ? FEW_BLOCKS_MOST : FEW_BLOCKS)) return S;
   }
   return 0;
 }
@@ -924,7 +997,7 @@ int launch_few(const CUtensorMap& km, const CUtensorMap& vm, const void* q, int6
                const int32_t* row_ids, const int32_t* ctx_lens, void* out, int B, int Hq, int Hkv, int max_blocks, int S, float scale,
                cudaStream_t stream) {
   auto kern = paged_attn_decode_few_kernel<D>;
-  constexpr size_t smem = (size_t)FEW_WARPS * (128 / D * 2 * BS * D * 2 + 8 * D * 4 + 64 + 16) + 1024;
+  constexpr size_t smem = few_smem<D>();
   B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   B200_CUDA_OK(launch_kernel_cluster(kern, dim3(S, Hkv, B), dim3(FEW_WARPS * 32), smem, S, stream, km, vm, (const __nv_bfloat16*)q, q_stride, bt,
                                      bt_stride, row_ids, ctx_lens, (__nv_bfloat16*)out, Hq, Hkv, max_blocks, scale * 1.4426950408889634f));
@@ -994,7 +1067,9 @@ int b200_paged_attn_decode(const void* q, int64_t q_token_stride, const void* k_
   rc = pool_tmap(v_pool, num_blocks, Hkv, D, &vm);
   if (rc) return rc;
   // a call that names its quota asks for the split above; a quantised result takes its row's maximum over all heads, in a launch of its own
-  const int few = min_quota == 0 && ((uintptr_t)out & 15) == 0 && ((uintptr_t)workspace & 15) == 0 && (Hq * D) % 8 == 0 ? few_split(B, Hkv, max_blocks) : 0;
+  const int few = min_quota == 0 && ((uintptr_t)out & 15) == 0 && ((uintptr_t)workspace & 15) == 0 && (Hq * D) % 8 == 0
+                      ? D == 128 ? few_split<128>(B, Hkv, max_blocks) : few_split<64>(B, Hkv, max_blocks)
+                      : 0;
   if (few) {
     void* rows = out ? out : workspace;
     rc = D == 128 ? launch_few<128>(km, vm, q, q_token_stride, block_table, bt_row_stride, row_ids, ctx_lens, rows, B, Hq, Hkv, max_blocks, few, scale,
