@@ -245,3 +245,23 @@ def test_prefill_prefix_consistency_full_size(ops):
     torch.cuda.synchronize()
     assert torch.equal(full2[: total - bs], full[: total - bs])
     assert not torch.equal(full2[total - bs:], full[total - bs:])
+
+
+@pytest.mark.parametrize("s_new,computed,hq,hkv,d", [(41, 279, 8, 2, 128), (41, 280, 8, 2, 128), (1, 191, 4, 4, 128), (1, 192, 4, 4, 128), (33, 95, 8, 2, 64),
+                                                     (33, 96, 8, 2, 64), (63, 321, 4, 1, 128), (63, 322, 4, 1, 128)])
+def test_prefill_on_both_sides_of_one_group(ops, s_new, computed, hq, hkv, d):
+    """The last table of blocks that one group of warps walks, and the first that four share."""
+    test_prefill_matches_oracle(ops, s_new, computed, hq, hkv, d)
+
+
+@pytest.mark.parametrize("s_new,computed,hq,hkv,d", [(64, 0, 4, 1, 128), (100, 700, 4, 2, 128), (70, 33, 8, 2, 64), (300, 40, 32, 4, 128)])
+def test_prefill_of_rows_off_16_bytes(ops, s_new, computed, hq, hkv, d):
+    """64 rows and more that the tcgen05 kernel cannot read, in tiles of one group and of four, more tiles than SMs among them: the aligned rows'
+    result, which that kernel gives."""
+    g = torch.Generator().manual_seed(s_new)
+    nb = -(-(s_new + computed) // 32) + 1
+    kp, vp = (torch.randn(nb, hkv, 32, d, generator=g).bfloat16().cuda() for _ in range(2))
+    bt = (1 + torch.randperm(nb - 1, generator=g)).int().cuda()
+    buf = torch.randn(s_new * hq * d + 2, generator=g).bfloat16().cuda()
+    q = buf[2:].view(s_new, hq, d)
+    _check(ops.paged_attn_prefill(q, kp, vp, bt, computed, d**-0.5).cpu(), ops.paged_attn_prefill(q.clone(), kp, vp, bt, computed, d**-0.5).cpu())

@@ -660,13 +660,13 @@ __global__ void __launch_bounds__(FEW_WARPS * 32, 1)
 // ============================================================ prefix-cached prefill (one sequence)
 // A few new tokens over a cached prefix are one tile of 64 query rows per head: 32 or 40 CTAs that would walk all the keys, a microsecond a
 // block of 32.  So the blocks are dealt to PF_GROUPS groups of four warps (16 query rows a warp, a double-buffered TMA ring a group) in each
-// of the S CTAs of a cluster; every group leaves its (m, l, O) in shared memory, over its ring, and the cluster's CTAs merge the rows
-// between them.  us, one group / here: 41 tokens after 512, 32 heads of 64 21.8 / 12.8, after 4096, 32 heads of 128
-// 135.9 / 35.3, 17 tokens after 32 16.1 / 11.8.
+// of the S CTAs of a cluster; every group leaves its (m, l, O) in shared memory, over its ring, a CTA's groups meet there, then the cluster's
+// CTAs merge the rows between them.  Chained launches, us, one group / here: 41 tokens after 700, 32 heads of 64 22.8 / 9.1, of 128 25.7 / 15.0, after
+// 4096 131.6 / 29.3.  One group is left where there are few keys (launch_prefill).
 constexpr int PF_GROUPS = 4;
 
-template <int D>
-__global__ void __launch_bounds__(PF_GROUPS * 128, 1)
+template <int D, int GROUPS>
+__global__ void __launch_bounds__(GROUPS * 128)
     paged_attn_prefill_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                               const __nv_bfloat16* __restrict__ q, int64_t q_stride,
                               const int32_t* __restrict__ bt_row, __nv_bfloat16* __restrict__ out, int S_new,
@@ -677,9 +677,10 @@ __global__ void __launch_bounds__(PF_GROUPS * 128, 1)
   static_assert(RING == 64 * D * 4, "a group's O takes its ring");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem0 = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* ml = reinterpret_cast<float*>(smem0 + PF_GROUPS * RING);                        // [groups][64][2]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ml + PF_GROUPS * 128);                     // [groups][full | empty][NST]
-  const int S = (int)cluster_nctarank(), rank = (int)cluster_ctarank();
+  float* ml = reinterpret_cast<float*>(smem0 + GROUPS * RING);                           // [groups][64][2]
+  float2* cml = reinterpret_cast<float2*>(ml + GROUPS * 128);                             // [64]: (m, l) of the CTA
+  uint64_t* bars = reinterpret_cast<uint64_t*>(cml + 64);                                 // [groups][full | empty][NST]
+  const int S = GROUPS > 1 ? (int)cluster_nctarank() : 1, rank = GROUPS > 1 ? (int)cluster_ctarank() : 0;
   const int kg = threadIdx.x >> 7, tid = threadIdx.x & 127, warp = tid >> 5, lane = tid & 31;
   uint8_t* smem = smem0 + kg * RING;
   uint64_t* full = bars + kg * 2 * NST;
@@ -700,7 +701,7 @@ __global__ void __launch_bounds__(PF_GROUPS * 128, 1)
 
   int q_last = q0 + 63 < S_new - 1 ? q0 + 63 : S_new - 1;
   const int nblk = (computed_len + q_last) / BS + 1;
-  const int first = rank * PF_GROUPS + kg, step = S * PF_GROUPS;  // this group's blocks
+  const int first = rank * GROUPS + kg, step = S * GROUPS;  // this group's blocks
   auto issue = [&](int s, int j) {
     issue_tile_pair<D>(&k_map, &v_map, 0, smem + (size_t)s * 2 * TILE, smem + (size_t)s * 2 * TILE + TILE, &full[s],
                        (bt_row[j] * Hkv + kvh) * BS);
@@ -807,12 +808,25 @@ __global__ void __launch_bounds__(PF_GROUPS * 128, 1)
       mbar_wait(&empty[s], (i / NST) & 1);
       issue(s, j + NST * step);
     }
-    __syncwarp();
+    if (GROUPS > 1) __syncwarp();
   }
 #pragma unroll
   for (int o = 1; o <= 2; o <<= 1) {
     l_lo += __shfl_xor_sync(0xffffffffu, l_lo, o);
     l_hi += __shfl_xor_sync(0xffffffffu, l_hi, o);
+  }
+  auto store = [&](int row, int col, float inv, float x, float y) {
+    *reinterpret_cast<uint32_t*>(out + ((int64_t)row * Hq + head) * D + col) = pack_bf16(x * inv, y * inv);
+  };
+  if constexpr (GROUPS == 1) {
+    const float inv_lo = l_lo > 0.f ? 1.f / l_lo : 0.f, inv_hi = l_hi > 0.f ? 1.f / l_hi : 0.f;
+#pragma unroll
+    for (int dn = 0; dn < D / 8; ++dn) {
+      const int col = dn * 8 + (lane & 3) * 2;
+      if (v_lo) store(r_lo, col, inv_lo, oacc[dn][0], oacc[dn][1]);
+      if (v_hi) store(r_hi, col, inv_hi, oacc[dn][2], oacc[dn][3]);
+    }
+    return;
   }
   // ---- this group's rows, over its ring (8-column chunks exchanged by row: no bank conflicts)
   named_bar_sync(1 + kg, 128);
@@ -828,31 +842,59 @@ __global__ void __launch_bounds__(PF_GROUPS * 128, 1)
     *reinterpret_cast<float2*>(ml + (kg * 64 + t_lo) * 2) = make_float2(m_lo, l_lo);
     *reinterpret_cast<float2*>(ml + (kg * 64 + t_hi) * 2) = make_float2(m_hi, l_hi);
   }
-  if (S > 1) cluster_sync_all();
-  else __syncthreads();
-  // ---- rows rank, rank + S, .. of the tile from all the groups, in order
+  __syncthreads();
+  // ---- the tile's rows from the CTA's groups, in order
   const int rows = min(64, S_new - q0);
-  for (int i = threadIdx.x; i < (rows - rank + S - 1) / S * (D / 2); i += PF_GROUPS * 128) {
-    const int row = rank + i / (D / 2) * S, c2 = i % (D / 2);
-    const uint32_t o_at = smem_u32(smem0) + (uint32_t)(row * D + (((c2 >> 2) ^ (row & 7)) << 3) + (c2 & 3) * 2) * 4, ml_at = smem_u32(ml) + row * 8;
+  for (int i = threadIdx.x; i < rows * (D / 2); i += GROUPS * 128) {
+    const int row = i / (D / 2), c2 = i % (D / 2), at = row * D + (((c2 >> 2) ^ (row & 7)) << 3) + (c2 & 3) * 2;
     float M = -INFINITY, L = 0.f;
     float2 acc = make_float2(0.f, 0.f);
-    for (int r = 0; r < S; ++r)
 #pragma unroll
-      for (int k = 0; k < PF_GROUPS; ++k) M = fmaxf(M, ld_cluster_f2(mapa_shared(ml_at + k * 512, r)).x);
-    for (int r = 0; r < S; ++r)
+    for (int k = 0; k < GROUPS; ++k) M = fmaxf(M, ml[(k * 64 + row) * 2]);
 #pragma unroll
-      for (int k = 0; k < PF_GROUPS; ++k) {
-        const float2 p = ld_cluster_f2(mapa_shared(ml_at + k * 512, r)), o = ld_cluster_f2(mapa_shared(o_at + k * RING, r));
-        const float w = p.x == -INFINITY ? 0.f : exp2f(p.x - M);  // a group without visible keys
-        L += w * p.y;
-        acc.x += w * o.x;
-        acc.y += w * o.y;
-      }
-    const float inv = L > 0.f ? 1.f / L : 0.f;
-    *reinterpret_cast<uint32_t*>(out + ((int64_t)(q0 + row) * Hq + head) * D + c2 * 2) = pack_bf16(acc.x * inv, acc.y * inv);
+    for (int k = 0; k < GROUPS; ++k) {
+      const float2 p = *reinterpret_cast<const float2*>(ml + (k * 64 + row) * 2), o = reinterpret_cast<const float2*>(smem0 + k * RING)[at >> 1];
+      const float w = p.x == -INFINITY ? 0.f : exp2f(p.x - M);  // a group without visible keys
+      L += w * p.y;
+      acc.x += w * o.x;
+      acc.y += w * o.y;
+    }
+    if (S == 1) {
+      store(q0 + row, c2 * 2, L > 0.f ? 1.f / L : 0.f, acc.x, acc.y);
+    } else {
+      reinterpret_cast<float2*>(smem0)[at >> 1] = acc;  // the first group's part, which no other thread reads
+      if (c2 == 0) cml[row] = make_float2(M, L);
+    }
   }
-  if (S > 1) cluster_sync_all();  // nobody leaves while a peer still reads its rows
+  if (S == 1) return;
+  // ---- then rows rank, rank + S, .. from the cluster's CTAs, in order
+  cluster_sync_all();
+  for (int i = threadIdx.x; i < (rows - rank + S - 1) / S * (D / 2); i += GROUPS * 128) {
+    const int row = rank + i / (D / 2) * S, c2 = i % (D / 2);
+    const uint32_t o_at = smem_u32(smem0) + (uint32_t)(row * D + (((c2 >> 2) ^ (row & 7)) << 3) + (c2 & 3) * 2) * 4, ml_at = smem_u32(cml) + row * 8;
+    float2 p[4], o[4];
+    float M = -INFINITY, L = 0.f;
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (r < S) {
+        p[r] = ld_cluster_f2(mapa_shared(ml_at, r));
+        o[r] = ld_cluster_f2(mapa_shared(o_at, r));
+      }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (r < S) M = fmaxf(M, p[r].x);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (r < S) {
+        const float w = p[r].x == -INFINITY ? 0.f : exp2f(p[r].x - M);
+        L += w * p[r].y;
+        acc.x += w * o[r].x;
+        acc.y += w * o[r].y;
+      }
+    store(q0 + row, c2 * 2, L > 0.f ? 1.f / L : 0.f, acc.x, acc.y);
+  }
+  cluster_sync_all();  // nobody leaves while a peer still reads its rows
 }
 
 }  // namespace b200
@@ -1007,12 +1049,25 @@ int launch_few(const CUtensorMap& km, const CUtensorMap& vm, const void* q, int6
 template <int D>
 int launch_prefill(const CUtensorMap& km, const CUtensorMap& vm, const void* q, int64_t q_stride, const int32_t* bt_row,
                    void* out, int S_new, int computed_len, int Hq, int Hkv, float scale, cudaStream_t stream) {
-  auto kern = paged_attn_prefill_kernel<D>;
-  constexpr size_t smem = (size_t)PF_GROUPS * (2 * 2 * BS * D * 2 + 64 * 8 + 32) + 1024;
+  const int tiles = (S_new + 63) / 64, blocks = (computed_len + S_new + BS - 1) / BS, rows = S_new < 64 ? S_new : 64;
+  // One group walks few blocks of keys in less time than four take to meet, which grows with the rows: us, one / four, 32 heads of 128, nothing
+  // cached, 1 row 2.4 / 4.2, 63 rows 4.0 / 8.8; after 300, 1 row 11.4 / 9.7, 33 rows 12.8 / 12.2, 63 rows 13.9 / 14.6; heads of 64, after 96, 1 row
+  // 4.7 / 3.6, 63 rows 5.9 / 5.9, after 32 4.1 / 5.2.  Longer prompts off 16 bytes (the tcgen05 kernel takes the others): tiles of four groups
+  // of 128 columns fill an SM each, so where there are more tiles than SMs one group again, 500 rows of 64 heads 31 / 53.
+  const int few_keys = D == 128 ? 6 + rows / 10 : 3 + rows / 32;
+  if (blocks <= few_keys || (D == 128 && tiles * Hq > sm_count())) {
+    auto kern = paged_attn_prefill_kernel<D, 1>;
+    constexpr size_t smem = (size_t)2 * 2 * BS * D * 2 + 2 * 64 * 8 + 32 + 1024;
+    B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    B200_CUDA_OK(launch_kernel(kern, dim3(tiles, Hq), dim3(128), smem, stream, km, vm, (const __nv_bfloat16*)q, q_stride, bt_row, (__nv_bfloat16*)out,
+                               S_new, computed_len, Hq, Hkv, scale * 1.4426950408889634f));
+    return B200_OK;
+  }
+  auto kern = paged_attn_prefill_kernel<D, PF_GROUPS>;
+  constexpr size_t smem = (size_t)PF_GROUPS * (2 * 2 * BS * D * 2 + 64 * 8 + 32) + 64 * 8 + 1024;
   B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // CTAs of a cluster: while a group has two blocks of keys and the heads leave SMs for them.  S = 1 / 2 / 4, us: 41 tokens after 4096, 32
   // heads of 128 86 / 51 / 35, after 512 20.9 / 17.9 / 17.6, of 64 13.6 / 13.0 / 12.4, after 96 12.1 / 12.8 / 14.4; 40 heads, after 1500 36 / 24 / 32.
-  const int tiles = (S_new + 63) / 64, blocks = (computed_len + S_new + BS - 1) / BS;
   int S = 4;
   while (S > 1 && (tiles * Hq * S > sm_count() || blocks < 2 * PF_GROUPS * S)) S >>= 1;
   B200_CUDA_OK(launch_kernel_cluster(kern, dim3(tiles * S, Hq), dim3(PF_GROUPS * 128), smem, S, stream, km, vm, (const __nv_bfloat16*)q, q_stride,
