@@ -769,32 +769,37 @@ __global__ void __launch_bounds__(GP_THREADS)
     }
 }
 
-// A few outputs per row (a router): a warp takes two rows, its lanes every 32nd 16-byte piece of k, and the 2 NW sums are reduced together by
-// halving.  Tiles of 32 x 32 walk all of k in a dozen CTAs: 304 x 8 x 1024 23.3 us, here 11.9; 304 x 16 23.5 / 13.5.
-template <int NW>
+// A few outputs per row (a router): a warp takes R rows, its lanes every 32nd 16-byte piece of k, and the R NW sums are reduced together by
+// halving -- lanes 16, 8, 4, 2, 1 apart whatever R is, so that a row's sums do not depend on the batch.  Tiles of 32 x 32 walk all of k in a dozen
+// CTAs: 304 x 8 x 1024 23.3 us, here 11.9; 304 x 16 23.5 / 13.5.
+template <int NW, int R>
 __global__ void __launch_bounds__(32) fp32_narrow_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int M, int N, int K,
                                                          float* __restrict__ out, int ldo) {
   griddep_launch();
   griddep_wait();
-  const int lane = threadIdx.x, r0 = blockIdx.x * 2;
-  const float* a0 = a + (int64_t)r0 * lda;
-  const float* a1 = a + (int64_t)(r0 + 1 < M ? r0 + 1 : r0) * lda;
-  float v[2 * NW];
+  constexpr int SUMS = R * NW;
+  const int lane = threadIdx.x, r0 = blockIdx.x * R;
+  const float* ar[R];
 #pragma unroll
-  for (int i = 0; i < 2 * NW; ++i) v[i] = 0.f;
+  for (int r = 0; r < R; ++r) ar[r] = a + (int64_t)(r0 + r < M ? r0 + r : r0) * lda;
+  float v[SUMS];
+#pragma unroll
+  for (int i = 0; i < SUMS; ++i) v[i] = 0.f;
 #pragma unroll 2
   for (int k = lane * 4; k < K; k += 128) {
-    const float4 x = ldf4(a0, k), y = ldf4(a1, k);
+    float4 x[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[r] = ldf4(ar[r], k);
 #pragma unroll
     for (int n = 0; n < NW; ++n) {
       const float4 c = n < N ? ldf4(w, (int64_t)n * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-      v[n] = fmaf(x.w, c.w, fmaf(x.z, c.z, fmaf(x.y, c.y, fmaf(x.x, c.x, v[n]))));
-      v[NW + n] = fmaf(y.w, c.w, fmaf(y.z, c.z, fmaf(y.y, c.y, fmaf(y.x, c.x, v[NW + n]))));
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r * NW + n] = fmaf(x[r].w, c.w, fmaf(x[r].z, c.z, fmaf(x[r].y, c.y, fmaf(x[r].x, c.x, v[r * NW + n]))));
     }
   }
-  int mine = 0, off = 16;  // mine: the sum that this lane ends up with
+  int mine = 0, off = 16;  // mine: the first of the sums that this lane ends up with
 #pragma unroll
-  for (int m = NW; m >= 1; m /= 2, off /= 2) {
+  for (int m = SUMS / 2; m >= (SUMS >= 32 ? SUMS / 32 : 1); m /= 2, off /= 2) {
     const bool up = lane & off;
     mine += up ? m : 0;
 #pragma unroll
@@ -803,10 +808,14 @@ __global__ void __launch_bounds__(32) fp32_narrow_kernel(const float* __restrict
       v[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
     }
   }
+  constexpr int SPARE = SUMS >= 32 ? 1 : 32 / SUMS, LEFT = SUMS >= 32 ? SUMS / 32 : 1;  // lanes of a sum; sums of a lane
 #pragma unroll
-  for (int o = 16 / (2 * NW); o >= 1; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-  const int row = r0 + mine / NW, n = mine % NW;
-  if (lane % (32 / (2 * NW)) == 0 && row < M && n < N) out[(int64_t)row * ldo + n] = v[0];
+  for (int o = SPARE / 2; o >= 1; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+#pragma unroll
+  for (int i = 0; i < LEFT; ++i) {
+    const int row = r0 + (mine + i) / NW, n = (mine + i) % NW;
+    if (lane % SPARE == 0 && row < M && n < N) out[(int64_t)row * ldo + n] = v[i];
+  }
 }
 
 namespace {
@@ -841,8 +850,12 @@ int dense_fp32_linear(int batch, const void* a, int lda, const void* w, int64_t 
   // A row's sums run alike in the two smaller tiles and, where a row has few outputs, in batches of any size: how a prompt is cut changes
   // nothing below the tiles of 64 rows.
   if (N <= 16 && batch == 1 && !gate) {
-    auto kern = N <= 8 ? fp32_narrow_kernel<8> : fp32_narrow_kernel<16>;
-    B200_CUDA_OK(launch_kernel(kern, dim3((M + 1) / 2), dim3(32), 0, st, (const float*)a, lda, (const float*)w, M, N, K, (float*)out, ldo));
+    // rows a warp, 2 / 4 / 8, us: 304 x 16 x 1024 11.5 / 7.4 / 10.5, 4096 x 16 x 2048 41.3 / 16.0 / 23.5, 8192 x 16 x 4096 200 / 104 / 79, 16384 x 16 x 4096
+    // 309 / 205 / 165 (tiles of 32 x 32 before: 19.4, 41.7, 169, 176), 16384 x 8 x 2048 54 / 45 / 57
+    const int r = M < 256 ? 2 : N > 8 && M >= 6000 ? 8 : 4;
+    auto kern = N <= 8 ? (r == 8 ? fp32_narrow_kernel<8, 8> : r == 4 ? fp32_narrow_kernel<8, 4> : fp32_narrow_kernel<8, 2>)
+                       : (r == 8 ? fp32_narrow_kernel<16, 8> : r == 4 ? fp32_narrow_kernel<16, 4> : fp32_narrow_kernel<16, 2>);
+    B200_CUDA_OK(launch_kernel(kern, dim3((M + r - 1) / r), dim3(32), 0, st, (const float*)a, lda, (const float*)w, M, N, K, (float*)out, ldo));
     return B200_OK;
   }
   if (M <= 8) FL_DENSE(8, 32, 8, 1, 4);
