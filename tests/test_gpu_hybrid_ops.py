@@ -795,23 +795,6 @@ def test_ssd_step_sees_parameters_that_the_kernel_ahead_wrote():
         assert torch.equal(y, ops.ssd_scan(xbc, raw, 0, p[:H], p[H:2 * H], p[2 * H:3 * H], want, meta, H, P, N, G)) and torch.equal(s, want)
 
 
-@pytest.mark.parametrize("window", [100, 1 << 30])
-def test_decode_attention_over_a_page_that_is_not_there(window):
-    """A page number below 0 stands for rows of zeros, inside the window too."""
-    from vllm_neuron_b200.hybrid import StepMeta
-
-    ops = _ops()
-    g = torch.Generator(device=DEV).manual_seed(3)
-    G, D, H = 2, 64, 8
-    kp, vp = (torch.randn(10, G, 32, D, generator=g, device=DEV).bfloat16() for _ in range(2))
-    kp[9], vp[9] = 0, 0
-    meta = StepMeta.build([(0, 200, 1), (1, 130, 1)], {0: list(range(1, 8)), 1: list(range(1, 8))}, 32, torch.device(DEV))
-    table = torch.tensor([[1, 2, 3, 4, 5, 9, 7], [2, 9, 1, 9, 3, 4, 5]], dtype=torch.int32, device=DEV)
-    q, sink = torch.randn(2, H * D, generator=g, device=DEV), torch.randn(H, generator=g, device=DEV)
-    want = ops.swa_sink_attn(q, H, kp, vp, table, meta, sink, 0.1, window)
-    assert torch.equal(ops.swa_sink_attn(q, H, kp, vp, torch.where(table == 9, -1, table), meta, sink, 0.1, window), want)
-
-
 def test_allocations_leave_the_interpreter_to_other_threads():
     """A result that has to wait for the device, because cached memory is given back for it, does not hold up other threads' Python."""
     import threading
@@ -905,3 +888,35 @@ def test_a_window_of_no_tokens_beside_a_sink_is_refused():
         meta, table, kp, vp, _, _ = _one_sequence(T, 2, 2, 64, 64, g)
         with pytest.raises(RuntimeError):
             ops.swa_sink_attn(torch.randn(T, 4 * 64, generator=g, device=DEV), 4, kp, vp, table, meta, torch.zeros(4, device=DEV), 0.1, 0)
+
+
+@pytest.mark.parametrize("window", [100, 1 << 30])
+def test_decode_attention_over_a_page_that_is_not_there(window):
+    """A page number below 0 stands for rows of zeros, inside the window too."""
+    from vllm_neuron_b200.hybrid import StepMeta
+
+    ops = _ops()
+    g = torch.Generator(device=DEV).manual_seed(3)
+    G, D, H = 2, 64, 8
+    kp, vp = (torch.randn(10, G, 32, D, generator=g, device=DEV).bfloat16() for _ in range(2))
+    kp[9], vp[9] = 0, 0
+    meta = StepMeta.build([(0, 200, 1), (1, 130, 1)], {0: list(range(1, 8)), 1: list(range(1, 8))}, 32, torch.device(DEV))
+    table = torch.tensor([[1, 2, 3, 4, 5, 9, 7], [2, 9, 1, 9, 3, 4, 5]], dtype=torch.int32, device=DEV)
+    q, sink = torch.randn(2, H * D, generator=g, device=DEV), torch.randn(H, generator=g, device=DEV)
+    want = ops.swa_sink_attn(q, H, kp, vp, table, meta, sink, 0.1, window)
+    assert torch.equal(ops.swa_sink_attn(q, H, kp, vp, torch.where(table == 9, -1, table), meta, sink, 0.1, window), want)
+
+
+@pytest.mark.parametrize("M,N,K", [(3, 40, 64), (9, 40, 64), (33, 100, 60), (8, 33, 128), (70, 65, 100), (20, 30000, 132), (255, 16, 68), (257, 5, 132), (300, 1, 4),
+                                   (6001, 9, 40), (6003, 16, 260), (6003, 8, 128)])
+def test_fp32_linear_on_short_rows_and_of_few_outputs(M, N, K):
+    """Rows of one to four slices in tiles of 8 and 32 rows, wide weights under 32 rows, 2, 4 and 8 rows a warp where a row has few outputs: against 64
+    bits, K roundings of an fp32 sum.  A row's sums do not depend on the batch: its first rows alone give the same bits."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    got = ops.linear_simt(a, w)
+    assert ((got.double() - a.double() @ w.double().T).abs() <= K * 2.0**-24 * (a.abs().double() @ w.abs().double().T)).all()
+    for few in (1, 7, 30):
+        if few < M:
+            assert torch.equal(ops.linear_simt(a[:few], w), got[:few])
