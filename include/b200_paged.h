@@ -205,8 +205,8 @@ int b200_gemm_silu_mul_quant(const void* a, const void* w_gu, void* out_q, float
                              void* stream);
 
 /* qkv projection with RoPE and the KV-cache write fused into its epilogue: b200_gemm (bf16 out, no residual) followed by
- * b200_rope_kv_write on its output, in ONE launch when the decode schedule splits K over a cluster (the token's owner
- * holds whole heads; rotate-half partner = lane ^ D/8), else as the two launches.  Same bits either way: qkv_out keeps
+ * b200_rope_kv_write on its output, in ONE launch for a few tokens (b200_gemm; D a multiple of 32) and when the decode schedule splits K
+ * over a cluster (the token's owner holds whole heads; rotate-half partner = lane ^ D/8), else as the two launches.  Same bits either way: qkv_out keeps
  * rotated q, un-rotated k and v; rotated k and v land in the pools at slot_mapping[t] (slot < 0 skipped).
  * Replaces the qkv linear + rotary + KV scatter inside NxDI's decoder layer (model_loader.py:336-348). */
 int b200_gemm_rope_kv_write(const void* a, const void* w, void* qkv_out, const float* a_scale, const float* w_scale,

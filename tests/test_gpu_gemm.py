@@ -515,3 +515,68 @@ def test_gemm_of_a_few_tokens_sees_scales_and_biases_that_the_kernel_ahead_wrote
     torch.cuda.synchronize()
     for scale, bias, first, both in runs:
         assert torch.equal(first, ops.gemm(x, w, None, scale)) and torch.equal(both, ops.gemm(x, w, None, scale, bias))
+
+
+@pytest.mark.parametrize("kind,m,i,k", [("bf16", 1, 512, 2048), ("bf16", 7, 512, 4096), ("bf16", 8, 96, 5632), ("fp8", 7, 512, 8192), ("int8", 3, 1024, 4096),
+                                        ("int8_wo", 5, 512, 5120), ("int8_wo", 13, 512, 2048), ("int8_wo", 16, 2048, 4608)])
+def test_gemm_silu_mul_of_a_few_tokens(ops, kind, m, i, k):
+    """Sizes at which the linear call takes 16 or 8 warps a CTA and this one four: a row's sum is the same."""
+    test_gemm_silu_mul_matches_unfused(ops, kind, m, i, k, 0)
+
+
+@pytest.mark.parametrize("kind,m", [("bf16", 1), ("bf16", 3), ("bf16", 8), ("fp8", 1), ("fp8", 7), ("int8", 8), ("int8_wo", 3), ("int8_wo", 9), ("int8_wo", 16)])
+@pytest.mark.parametrize("hq,hkv,d,k", [(4, 1, 128, 4096), (8, 2, 64, 272), (3, 1, 96, 2048), (32, 4, 64, 2048), (2, 2, 32, 144)])
+def test_rope_epilogue_of_a_few_tokens(ops, kind, m, hq, hkv, d, k):
+    """Rotation and scatter in the epilogue: the bits of the GEMM and the rotation kernel, and what 64 bits give.  A position past the table is
+    the last one, a slot below 0 is skipped.  Bound: fp32 sums of k products and one bf16 rounding in front of the rotation, one behind it."""
+    g = torch.Generator().manual_seed(m * hq + d)
+    n, bs, nb, max_pos = (hq + 2 * hkv) * d, 32, 4, 64
+    x, w, bias = torch.randn(m, k, generator=g), torch.randn(n, k, generator=g), torch.randn(n, generator=g).bfloat16()
+    x = x.bfloat16() if kind in ("bf16", "int8_wo") else x.clamp(-4, 4).to(torch.float8_e4m3fn) if kind == "fp8" else (20 * x).round().clamp(-127, 127).to(torch.int8)
+    w = w.bfloat16() if kind == "bf16" else w.clamp(-4, 4).to(torch.float8_e4m3fn) if kind == "fp8" else (40 * w).round().clamp(-127, 127).to(torch.int8)
+    xs = torch.rand(m, generator=g) + 0.5 if kind in ("fp8", "int8") else None
+    ws = None if kind == "bf16" else torch.rand(n, generator=g) + 0.5
+    pos, slots = torch.randint(0, max_pos, (m,), generator=g), torch.randperm((nb - 1) * bs, generator=g)[:m] + bs
+    pos[0] = max_pos + 5
+    if m > 1:
+        slots[1] = -1
+    ang = torch.arange(max_pos).float()[:, None] / 10000.0 ** (torch.arange(0, d, 2).float() / d)
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    dev = lambda t: None if t is None else t.cuda()  # noqa: E731
+    pools = [torch.zeros(nb, hkv, bs, d, dtype=torch.bfloat16).cuda() for _ in range(4)]
+    args = (dev(x), dev(w))
+    got = ops.gemm_rope_kv_write(*args, dev(pos), dev(cos), dev(sin), pools[0], pools[1], dev(slots), hq, dev(xs), dev(ws), dev(bias))
+    two = ops.gemm(*args, dev(xs), dev(ws), dev(bias))
+    ops.rope_kv_write(two, dev(pos), dev(cos), dev(sin), pools[2], pools[3], dev(slots), hq)
+    assert torch.equal(got.view(torch.int16), two.view(torch.int16))
+    assert all(torch.equal(pools[i].view(torch.int16), pools[i + 2].view(torch.int16)) for i in (0, 1))
+    a64, w64 = x.double(), w.double()
+    scale = (1 if xs is None else xs.double()[:, None]) * (1 if ws is None else ws.double())
+    want = (a64 @ w64.T * scale + bias.double()).view(m, -1, d)
+    size = (a64.abs() @ w64.abs().T * scale + bias.double().abs()).view(m, -1, d)
+    err = (4 if kind == "int8" else 2 * k + 4) * 2.0**-24 * size + 2.0**-8 * want.abs() * 1.01
+    p = pos.clamp(max=max_pos - 1)
+    c, s = cos.double()[p][:, None], sin.double()[p][:, None]
+
+    def turn(v, c, s):
+        lo, hi = v[..., :d // 2], v[..., d // 2:]
+        return torch.cat([lo * c - hi * s, hi * c + lo * s], -1)
+
+    both = lambda v: torch.cat([v[..., d // 2:], v[..., :d // 2]], -1)  # noqa: E731
+    turned = turn(want, c, s)
+    cc, ss = torch.cat([c, c], -1).abs(), torch.cat([s, s], -1).abs()
+    terr = err * cc + both(err) * ss
+    terr = terr + (turned.abs() + terr) * 2.0**-8 * 1.01 + 2.0**-22 * (want.abs() + both(want).abs())
+    row = got.double().cpu().view(m, -1, d)
+    assert ((row[:, :hq] - turned[:, :hq]).abs() <= terr[:, :hq]).all()
+    assert ((row[:, hq:] - want[:, hq:]).abs() <= err[:, hq:]).all()
+    kp, vp = (t.double().cpu() for t in pools[:2])
+    seen = torch.zeros(nb, bs, dtype=torch.bool)
+    for t in range(m):
+        if slots[t] < 0:
+            continue
+        b, o = divmod(int(slots[t]), bs)
+        seen[b, o] = True
+        assert ((kp[b, :, o] - turned[t, hq:hq + hkv]).abs() <= terr[t, hq:hq + hkv]).all()
+        assert ((vp[b, :, o] - want[t, hq + hkv:]).abs() <= err[t, hq + hkv:]).all()
+    assert not kp.transpose(1, 2)[~seen].any() and not vp.transpose(1, 2)[~seen].any()

@@ -6,9 +6,10 @@
 // as the k slots of its fragments -- a sum does not care which k a slot holds, as long as the tokens' fragments are loaded alike.  No
 // shared memory before the sums meet, no barrier in the loop, and the first PF k-blocks of every warp are in flight BEFORE
 // griddepcontrol.wait: with 16 warps an SM the chip holds 19 MB of the next GEMM's weights while the kernel ahead finishes.
-//   * a CTA takes 16 MT weight rows (MT = 2: gate and up rows of a group, or the two halves of a head, which the epilogue needs together),
-//     its eight warps the k-blocks of 128 bytes in turn; partial sums meet in shared memory in warp order, so results do not depend on timing;
-//   * two accumulators per tile, so a chain of tensor-core sums is a sixteenth of K.
+//   * a CTA takes 16 MT weight rows (MT = 2: gate and up rows of a group, or the two halves of a head, which the epilogue needs together) in
+//     2 to 16 warps.  K is cut into 16 slices, every 16th line of 128 bytes each: a chain of tensor-core sums per slice, and the chains meet in
+//     shared memory in one tree.  16 warps take a slice each, 8 warps two in turn (s and s + 8), fewer warps such pairs one after the other.
+//     So a row's sum does not depend on warps, epilogue or timing: the fused calls give the bits of the linear one followed by what they fuse.
 #include "gemm_small.cuh"
 
 #include <limits.h>
@@ -66,11 +67,13 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
   constexpr bool WO = KIND == KIND_WO8;
   constexpr int THREADS = WARPS * 32;
   constexpr int XE = WO ? 2 : 1;                                            // activation bytes per weight byte
-  constexpr int PF = MT * NT == 4 ? 1 : MT * NT == 2 ? 2 : WO ? 3 : 4;     // k-blocks of a warp in flight: what 128 registers hold
+  constexpr int REDS = WARPS == 16 ? 16 : 8, STEP = REDS;                   // sums that meet, of one slice or two; lines from one of a sum to its next
+  constexpr int SETS = WARPS == 16 ? 1 : 2;                                 // slices that a warp takes in turn
+  constexpr int PF = small_ahead(MT * NT, WO), TURNS = PF % SETS ? PF * SETS : PF;  // lines of a warp in flight: what 128 registers hold
   constexpr int ROWS = 16 * MT, TOK = 8 * NT, PITCH = TOK + 1;
   constexpr int SIDES = EPI == EPI_LINEAR ? 1 : 2;                          // sums that an epilogue item takes
   constexpr int ITEM_ROWS = ROWS / SIDES, ITEMS = ITEM_ROWS * TOK, PER = (ITEMS + THREADS - 1) / THREADS;
-  __shared__ float red[WARPS][ROWS * PITCH];
+  __shared__ float red[REDS][ROWS * PITCH];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
   // first weight row of tile mt
   int row0[MT];
@@ -120,13 +123,25 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
       }
     }
   };
+  constexpr bool BY_LINE = KIND != KIND_F16;  // the second form of the loop below
+  // the line behind kb in a warp's order (nkb or more: none)
+  auto after = [&](int kb) {
+    const int pair = (kb & 7) + WARPS;
+    return WARPS >= 8 || kb + STEP < nkb ? kb + STEP : pair < 8 ? pair : nkb;
+  };
 #pragma unroll
-  for (int s = 0; s < PF; ++s)
-    if (warp + s * WARPS < nkb) load_w(wb[s], warp + s * WARPS);
+  for (int s = 0, k = warp; s < PF; ++s)
+    if (k < nkb) {
+      load_w(wb[s], k);
+      k = BY_LINE ? after(k) : k + STEP;
+    }
   griddep_wait();  // before everything but the weights: scales and biases may be what the kernel ahead has written
 #pragma unroll
-  for (int s = 0; s < PF; ++s)
-    if (warp + s * WARPS < nkb) load_x(xb[s], warp + s * WARPS);
+  for (int s = 0, k = warp; s < PF; ++s)
+    if (k < nkb) {
+      load_x(xb[s], k);
+      k = BY_LINE ? after(k) : k + STEP;
+    }
   // the epilogue's operands of this thread's items, while the products are taken
   float wsc[PER][SIDES], bia[PER][SIDES], asc[PER], res[PER];
   long long pos[PER], slot[PER];
@@ -151,60 +166,98 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
       pos[q] = pos[q] < 0 ? 0 : pos[q] >= ep.rope.max_pos ? ep.rope.max_pos - 1 : pos[q];
     }
   }
-  uint32_t acc[2][MT][NT][4];
+  uint32_t acc[SETS][MT][NT][4];
+  auto clear = [&]() {
 #pragma unroll
-  for (int p = 0; p < 2; ++p)
+    for (int t = 0; t < SETS; ++t)
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[t][mt][nt][e] = 0u;
+  };
+  auto leave = [&](float* to) {  // a slice or a pair (in either order, which a sum does not tell)
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[p][mt][nt][e] = 0u;
-  for (int kb = warp; kb < nkb; kb += PF * WARPS) {
-#pragma unroll
-    for (int s = 0; s < PF; ++s) {
-      const int k = kb + s * WARPS;
-      if (k < nkb) {
-#pragma unroll
-        for (int p = 0; p < 2; ++p)
-#pragma unroll
-          for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) mma_piece<KIND>(acc[p][mt][nt], wb[s][mt][p * 2], wb[s][mt][p * 2 + 1], xb[s][p][nt]);
-        if (k + PF * WARPS < nkb) {
-          load_w(wb[s], k + PF * WARPS);
-          load_x(xb[s], k + PF * WARPS);
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t v = acc[0][mt][nt][e], u = SETS == 2 ? acc[SETS - 1][mt][nt][e] : 0u;
+          to[(mt * 16 + g + (e >= 2 ? 8 : 0)) * PITCH + nt * 8 + 2 * c + (e & 1)] = KIND == KIND_I8 ? __uint_as_float(v + u) : __uint_as_float(v) + __uint_as_float(u);
         }
+  };
+  auto multiply = [&](uint32_t (&d)[MT][NT][4], int st) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) mma_piece<KIND>(d[mt][nt], wb[st][mt][p * 2], wb[st][mt][p * 2 + 1], xb[st][p][nt]);
+  };
+  auto fetch = [&](int st, int k) {
+    load_w(wb[st], k);
+    load_x(xb[st], k);
+  };
+  clear();
+  // Two forms of one order, by what the compiler makes of them.  Chained launches of one token, us, constant offsets / line by line: bf16 4096 x 14336
+  // 20.1 / 22.2, 28672 x 4096 gate and up 42.0 / 44.0; fp8 16.2 / 14.1 and 27.4 / 26.3, int8 weights 512 x 512 1.9 / 1.6, 55296 x 5120 73 / 70.
+  if constexpr (!BY_LINE) {
+    for (int kb = warp; kb < nkb;) {  // a turn's offsets from kb and next are constants
+      int next = kb + TURNS * STEP;
+      const bool end = WARPS < 8 && next >= nkb;  // of a pair; the next one's first lines are fetched meanwhile
+      if (end) next = (kb & 7) + WARPS < 8 ? (kb & 7) + WARPS : nkb;
+#pragma unroll
+      for (int q = 0; q < TURNS; ++q) {
+        const int k = kb + q * STEP, ahead = q < TURNS - PF ? k + PF * STEP : next + (q - TURNS + PF) * STEP;
+        if (k < nkb) multiply(acc[q % SETS], q % PF);
+        if (ahead < nkb) fetch(q % PF, ahead);
       }
+      if (end) {
+        leave(red[kb & 7]);
+        clear();
+      }
+      kb = next;
     }
+  } else {
+    int ahead = warp;
+#pragma unroll
+    for (int s = 0; s < PF; ++s)
+      if (ahead < nkb) ahead = after(ahead);
+    for (int cur = warp; cur < nkb;)
+#pragma unroll
+      for (int q = 0; q < TURNS; ++q)
+        if (cur < nkb) {
+          multiply(acc[q % SETS], q % PF);
+          if (ahead < nkb) {
+            fetch(q % PF, ahead);
+            ahead = after(ahead);
+          }
+          if (WARPS < 8 && cur + STEP >= nkb) {  // the pair's last line
+            leave(red[cur & 7]);
+            clear();
+          }
+          cur = after(cur);
+        }
   }
+  if (WARPS >= 8) leave(red[warp]);
   // Not earlier: CTAs of the next kernels that wait for this one hold registers that its own CTAs still need (a step of TinyLlama, one
   // sequence, 1071 us with this at the top, 776 here; Llama 3.1 8B fp8, 6 layers, 520 and 510)
   griddep_launch();
-  // ---- the warps' sums meet
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int r = mt * 16 + g + (e >= 2 ? 8 : 0), t = nt * 8 + 2 * c + (e & 1);
-        red[warp][r * PITCH + t] = KIND == KIND_I8 ? __int_as_float((int)(acc[0][mt][nt][e] + acc[1][mt][nt][e]))
-                                                   : __uint_as_float(acc[0][mt][nt][e]) + __uint_as_float(acc[1][mt][nt][e]);
-      }
   __syncthreads();
   auto total = [&](int r, int t) {
     if constexpr (KIND == KIND_I8) {
       int v = 0;
 #pragma unroll
-      for (int k = 0; k < WARPS; ++k) v += __float_as_int(red[k][r * PITCH + t]);
+      for (int k = 0; k < REDS; ++k) v += (k & 7) < nkb ? __float_as_int(red[k][r * PITCH + t]) : 0;  // slices without lines were left by nobody
       return (float)v;
     } else {
-      float v[WARPS];  // by halves: log2 roundings
+      float v[REDS];  // by halves: log2 roundings
 #pragma unroll
-      for (int k = 0; k < WARPS; ++k) v[k] = red[k][r * PITCH + t];
+      for (int k = 0; k < REDS; ++k) v[k] = (k & 7) < nkb ? red[k][r * PITCH + t] : 0.f;
 #pragma unroll
-      for (int o = WARPS / 2; o >= 1; o /= 2)
+      for (int o = REDS / 2; o >= 1; o /= 2)
 #pragma unroll
         for (int k = 0; k < o; ++k) v[k] += v[k + o];
       return v[0];

@@ -4,6 +4,8 @@
 
 namespace b200 {
 
+// lines of 128 bytes that a warp has in flight
+__host__ __device__ constexpr int small_ahead(int mma_tiles, bool wo) { return mma_tiles == 4 ? 1 : mma_tiles == 2 ? 2 : wo ? 3 : 4; }
 bool gemm_small_ok(const void* a, const void* w, int epi, int M, int N, int K, int ab_dtype, int head_dim);
 int launch_gemm_small(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, cudaStream_t s);
 

@@ -1445,8 +1445,8 @@ int b200_gemm_rope_kv_write(const void* a, const void* w, void* qkv_out, const f
   B200_REQUIRE(positions && cos_table && sin_table && k_pool && v_pool && slot_mapping, "gemm_rope_kv_write: null pointer");
   B200_REQUIRE(N == (Hq + 2 * Hkv) * D, "gemm_rope_kv_write: N=%d is not (Hq + 2 Hkv) * D = %d", N, (Hq + 2 * Hkv) * D);
   GemmEpilogue ep{a_scale, w_scale, (const __nv_bfloat16*)bias, nullptr, qkv_out, 0, nullptr};
-  // The rotation lives in the split-K owner's epilogue of the decode kernel (a token's whole head in one warp).  Every
-  // other schedule (one CTA per tile, the stream-K prefill kernel, odd head sizes) runs the GEMM, then the RoPE/scatter
+  // The rotation lives in the split-K owner's epilogue of the decode kernel (a token's whole head in one warp) and in that of the kernel
+  // for a few tokens, whose row sums are those of its linear epilogue.  Every other schedule (one CTA per tile, the stream-K prefill kernel, odd head sizes) runs the GEMM, then the RoPE/scatter
   // kernel: same bits either way.
   bool fused = false;
   const bool wide_wo = ab_dtype == B200_INT8_WO && split_k == 0 && gemm_wo_wide(EPI_ROPE, M, N, K);  // its own schedule, without the rotation
