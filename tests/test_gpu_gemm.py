@@ -580,3 +580,10 @@ def test_rope_epilogue_of_a_few_tokens(ops, kind, m, hq, hkv, d, k):
         assert ((kp[b, :, o] - turned[t, hq:hq + hkv]).abs() <= terr[t, hq:hq + hkv]).all()
         assert ((vp[b, :, o] - want[t, hq + hkv:]).abs() <= err[t, hq + hkv:]).all()
     assert not kp.transpose(1, 2)[~seen].any() and not vp.transpose(1, 2)[~seen].any()
+
+
+@pytest.mark.parametrize("m,i,k", [(1, 14336, 4096), (8, 14336, 4096), (5, 9600, 1040), (8, 18688, 512), (3, 512, 256), (7, 512, 128)])
+def test_gemm_silu_mul_quant_of_a_few_tokens(ops, m, i, k):
+    """Token counts that other shapes' GEMMs take to a kernel of their own: the two forms have one order of sums."""
+    test_gemm_silu_mul_quant_fused_equals_two_calls(ops, "fp8", m, i, k)
+    test_gemm_silu_mul_matches_unfused(ops, "fp8", m, i, k, 0)

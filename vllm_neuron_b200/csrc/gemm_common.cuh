@@ -26,7 +26,7 @@ struct KindTraits<KIND_I8> {
 // EPI_ROPE: EPI_LINEAR whose split-K owner epilogue also rotates q/k and scatters k/v (decode kernel, S > 1 only; gemm_small.cu); its own
 // instantiation so the plain linears keep their register budget (80 vs 137)
 // EPI_SILU_QUANT: EPI_SILU_MUL whose CTAs also agree on the per-token amax through a grid-wide barrier and write the
-// quantised activation themselves (decode kernel, S == 1, all CTAs co-resident; b200_gemm_silu_mul_quant)
+// quantised activation themselves (decode kernel, S == 1, all CTAs co-resident; fp8 of a few tokens gemm_small.cu; b200_gemm_silu_mul_quant)
 enum { EPI_LINEAR = 0, EPI_SILU_MUL = 1, EPI_ROPE = 2, EPI_SILU_QUANT = 3 };
 
 struct GemmEpilogue {

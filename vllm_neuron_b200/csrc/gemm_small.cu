@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
       k = BY_LINE ? after(k) : k + STEP;
     }
   // the epilogue's operands of this thread's items, while the products are taken
-  float wsc[PER][SIDES], bia[PER][SIDES], asc[PER], res[PER];
+  float wsc[PER][SIDES], bia[PER][SIDES], asc[PER], res[PER], act[PER];
   long long pos[PER], slot[PER];
   const bool hb = ep.bias != nullptr, hr = EPI == EPI_LINEAR && ep.residual != nullptr;
 #pragma unroll
@@ -277,7 +277,9 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
       const int mm = i < ITEMS ? m : 0;
       const float lo = __bfloat162float(__float2bfloat16_rn(scaled_value(total(r, mm), asc[q], wsc[q][0], hb, bia[q][0], false, 0.f)));
       const float hi = __bfloat162float(__float2bfloat16_rn(scaled_value(total(16 + r, mm), asc[q], wsc[q][1], hb, bia[q][1], false, 0.f)));
-      if constexpr (EPI == EPI_SILU_MUL) {  // whole groups of 32 rows: N is a multiple of 32
+      if constexpr (EPI == EPI_SILU_QUANT) {
+        act[q] = ok ? silu_mul_bf16(lo, hi) : 0.f;
+      } else if constexpr (EPI == EPI_SILU_MUL) {  // whole groups of 32 rows: N is a multiple of 32
         const float v = silu_mul_bf16(lo, hi);
         float x = fabsf(v);
 #pragma unroll
@@ -308,6 +310,48 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
           dst[half] = __float2bfloat16_rn(o2);
         }
       }
+    }
+  }
+  if constexpr (EPI == EPI_SILU_QUANT) {  // the tokens' maxima over the whole grid, as in the decode schedule (gemm_tcgen05.cu) and on its state
+    unsigned int* arrived = reinterpret_cast<unsigned int*>(ep.fq_state + 128);
+    unsigned int* epoch = arrived + 1;
+    const unsigned int e0 = *reinterpret_cast<volatile unsigned int*>(epoch);  // stays until this CTA has arrived
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      const int m = (threadIdx.x + q * THREADS) / ITEM_ROWS;
+      float x = fabsf(act[q]);
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+      if (threadIdx.x % ITEM_ROWS == 0 && m < M) atomicMax(&ep.fq_state[m], ((unsigned long long)(e0 + 1u) << 32) | __float_as_uint(x));
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      if (atomicAdd(arrived, 1u) == gridDim.x - 1) {
+        atomicExch(arrived, 0u);
+        __threadfence();
+        atomicAdd(epoch, 1u);
+      } else {
+        const long long t0 = clock64();
+        unsigned int e;
+        do {
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(e) : "l"(epoch) : "memory");
+          if (clock64() - t0 > 4000000000LL) {  // about 2 s: a grid that is not fully resident must not hang
+            printf("b200: silu-quant grid barrier timeout block %d epoch %u\n", blockIdx.x, e0);
+            __trap();
+          }
+        } while (e == e0);
+      }
+      __threadfence();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      const int i = threadIdx.x + q * THREADS, m = i / ITEM_ROWS, r = i % ITEM_ROWS;
+      if (m >= M) continue;
+      const float amax = __uint_as_float((unsigned int)__ldcg(&ep.fq_state[m])), scale = amax > 0.f ? __fdiv_rn(amax, 448.f) : 1.f;
+      if (blockIdx.x == 0 && r == 0) ep.out_scale[m] = scale;
+      reinterpret_cast<uint8_t*>(ep.out)[(int64_t)m * (N >> 1) + blockIdx.x * 16 + r] = quant_byte<B200_FP8_E4M3>(act[q], scale);
     }
   }
 }
@@ -351,6 +395,24 @@ int launch_gemm_small(const void* a, const void* w, const GemmEpilogue& ep, int 
   if (ab_dtype == B200_FP8_E4M3) return pick_small<KIND_F8F6F4, 1>(a, w, ep, epi, M, N, K, s);
   if (ab_dtype == B200_INT8) return pick_small<KIND_I8, 1>(a, w, ep, epi, M, N, K, s);
   return M <= 8 ? pick_small<KIND_WO8, 1>(a, w, ep, epi, M, N, K, s) : pick_small<KIND_WO8, 2>(a, w, ep, epi, M, N, K, s);
+}
+
+// CTAs of two warps: eight an SM, which holds as many weight rows at once as the decode schedule's tiles, and no other CTA meets the barrier
+bool small_silu_quant_fits(int N) {
+  static const int ctas = [] {
+    auto kern = gemm_small_kernel<KIND_F8F6F4, EPI_SILU_QUANT, 1, 2, 2>;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 64, 0) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    return n * sm_count();
+  }();
+  return N % 32 == 0 && N / 32 <= ctas;
+}
+int launch_gemm_small_silu_quant(const void* a, const void* w, const GemmEpilogue& ep, int M, int N, int K, cudaStream_t s) {
+  return launch_small<KIND_F8F6F4, EPI_SILU_QUANT, 1, 2, 2>(a, w, ep, M, N, K, s);
 }
 
 }  // namespace b200

@@ -8,5 +8,8 @@ namespace b200 {
 __host__ __device__ constexpr int small_ahead(int mma_tiles, bool wo) { return mma_tiles == 4 ? 1 : mma_tiles == 2 ? 2 : wo ? 3 : 4; }
 bool gemm_small_ok(const void* a, const void* w, int epi, int M, int N, int K, int ab_dtype, int head_dim);
 int launch_gemm_small(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, cudaStream_t s);
+// EPI_SILU_QUANT of fp8, for what gemm_small_ok takes and the chip holds at once
+bool small_silu_quant_fits(int N);
+int launch_gemm_small_silu_quant(const void* a, const void* w, const GemmEpilogue& ep, int M, int N, int K, cudaStream_t s);
 
 }  // namespace b200

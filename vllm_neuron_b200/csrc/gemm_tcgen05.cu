@@ -1345,8 +1345,8 @@ namespace {
 // choice for this shape is one CTA per weight tile (S == 1) with the whole grid resident at once: the CTAs meet at a
 // grid-wide barrier, which must never wait for a CTA that has not been scheduled.
 template <int KIND>
-static int launch_silu_quant(const CUtensorMap& wm, const CUtensorMap& am, const GemmEpilogue& ep, int M, int N,
-                             const GemmPlan& p, cudaStream_t s) {
+static int launch_silu_quant(const void* a, const void* w, const CUtensorMap& wm, const CUtensorMap& am, const GemmEpilogue& ep, int M, int N,
+                             int K, const GemmPlan& p, cudaStream_t s) {
   DecodeCfg c;
   int rc = p.bm == 32   ? plan_decode<KIND, 32, EPI_SILU_QUANT>(c, M, p.n_tiles, p.num_kb, 0, false)
            : p.bm == 64 ? plan_decode<KIND, 64, EPI_SILU_QUANT>(c, M, p.n_tiles, p.num_kb, 0, false)
@@ -1356,6 +1356,12 @@ static int launch_silu_quant(const CUtensorMap& wm, const CUtensorMap& am, const
   if (c.S != 1 || p.n_tiles > c.cap_ctas * per_sm) {
     set_last_error("gemm_silu_mul_quant: plan S=%d, %d tiles, capacity %d: not one resident wave", c.S, p.n_tiles,
                    c.cap_ctas * per_sm);
+    return B200_ERR_UNSUPPORTED;
+  }
+  // the sums of the two-call form, for a few tokens those of gemm_small.cu (int8 sums are the same in any order)
+  if (KIND == KIND_F8F6F4 && gemm_small_ok(a, w, EPI_SILU_MUL, M, N, K, B200_FP8_E4M3, 0)) {
+    if (small_silu_quant_fits(N)) return launch_gemm_small_silu_quant(a, w, ep, M, N, K, s);
+    set_last_error("gemm_silu_mul_quant: %d rows of weights are not resident at once", N);
     return B200_ERR_UNSUPPORTED;
   }
   if (p.bm == 32) return launch_decode<KIND, 32, EPI_SILU_QUANT>(wm, am, ep, M, N, p, 0, s);
@@ -1496,8 +1502,8 @@ int b200_gemm_silu_mul_quant(const void* a, const void* w_gu, void* out_q, float
   rc = make_tmap_2d(&am, a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)M, (uint64_t)K, GEMM_BK_BYTES, p.bm);
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  if (ab_dtype == B200_FP8_E4M3) return launch_silu_quant<KIND_F8F6F4>(wm, am, ep, M, N2, p, s);
-  return launch_silu_quant<KIND_I8>(wm, am, ep, M, N2, p, s);
+  if (ab_dtype == B200_FP8_E4M3) return launch_silu_quant<KIND_F8F6F4>(a, w_gu, wm, am, ep, M, N2, K, p, s);
+  return launch_silu_quant<KIND_I8>(a, w_gu, wm, am, ep, M, N2, K, p, s);
 }
 
 int b200_gemm_silu_mul(const void* a, const void* w_gu, void* out_act, const float* a_scale, const float* w_scale,
