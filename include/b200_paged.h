@@ -168,7 +168,7 @@ size_t b200_gemm_workspace_bytes(int M, int N, int K, int ab_dtype, int split_k)
 /* The decode schedule (M <= 128) chosen on the current device for a shape: out6 = {cluster size S, CTAs per SM, weight
  * ring depth, activation ring depth, CTAs the chip holds at once, dynamic shared memory bytes}.  Needs a device.
  * silu_mul selects the epilogue variant planned for: 0 linear, 1 SiLU*mul (b200_gemm_silu_mul), 2 RoPE + KV write
- * (b200_gemm_rope_kv_write).  A few tokens (no rings): S = 1 and 0 bytes.  Weight-only batches on 256 weight rows: the cluster size of the cut tiles; both rings have one depth. */
+ * (b200_gemm_rope_kv_write).  A few tokens (no rings): S = 1, 0 bytes, depths = lines of 128 bytes that a warp has in flight; 2 assumes heads of a multiple of 32.  Weight-only batches on 256 weight rows: the cluster size of the cut tiles; both rings have one depth. */
 int b200_gemm_decode_plan(int M, int N, int K, int ab_dtype, int split_k, int silu_mul, int has_residual, int* out6);
 /* Profiling aid: with a non-NULL device buffer ([#CTAs][8] uint64) every decode-schedule GEMM CTA records %globaltimer
  * at its phase boundaries (tools/gemm_trace.py); NULL (default) switches it off. */

@@ -587,3 +587,12 @@ def test_gemm_silu_mul_quant_of_a_few_tokens(ops, m, i, k):
     """Token counts that other shapes' GEMMs take to a kernel of their own: the two forms have one order of sums."""
     test_gemm_silu_mul_quant_fused_equals_two_calls(ops, "fp8", m, i, k)
     test_gemm_silu_mul_matches_unfused(ops, "fp8", m, i, k, 0)
+
+
+@pytest.mark.parametrize("m,n,k,kind,epi,per_sm,lines", [(1, 2048, 5632, "BF16", 0, 1, 4), (8, 2048, 2048, "BF16", 0, 2, 4), (4, 6144, 4096, "FP8_E4M3", 0, 2, 2),
+                                                         (4, 32000, 2048, "INT8", 0, 4, 2), (2, 6144, 4096, "BF16", 2, 2, 2), (2, 11264, 2048, "BF16", 1, 4, 2),
+                                                         (3, 2048, 8192, "INT8_WO", 0, 1, 3), (16, 2048, 8192, "INT8_WO", 0, 1, 2), (9, 32000, 2048, "INT8_WO", 0, 4, 1)])
+def test_plan_of_a_few_tokens(ops, m, n, k, kind, epi, per_sm, lines):
+    """CTAs an SM holds (16 warps of it) and lines of a warp in flight, by the size of the weights."""
+    got = ops.gemm_decode_plan(m, n, k, getattr(ops, kind), silu_mul=epi)
+    assert list(got.values()) == [1, per_sm, lines, lines, per_sm * torch.cuda.get_device_properties(0).multi_processor_count, 0]

@@ -379,22 +379,38 @@ static int launch_small(const void* a, const void* w, const GemmEpilogue& ep, in
 // CTAs of 16 rows while they fit the chip once (16 warps of one SM share a long row, or 8), then of 32 rows; where those are many, four warps
 // each, so that more of them are in flight and the last wave is short.  Measured, bf16, one token, us: 2048 x 5632 with 16 / 8 warps 5.1 / 6.2,
 // 2048 x 2048 2.6 / 2.5, 4096 x 4096 7.4 / 6.4; 6144 x 4096 16 / 32 rows 11.3 / 10.2; 10272 x 2048 8 / 4 warps 10.2 / 9.2, 32000 x 2048 22.8 / 21.8.
+SmallShape gemm_small_shape(int epi, int M, int N, int K, int ab_dtype) {
+  const int tiles = (N + 15) / 16, sms = sm_count(), nt = M <= 8 ? 1 : 2;
+  const int64_t row = (int64_t)K * (ab_dtype == B200_BF16 ? 2 : 1);
+  SmallShape c{2, 4, 0};
+  if (epi == EPI_ROPE) c.warps = 8;
+  else if (epi == EPI_LINEAR && tiles <= sms && row > 4096) c = {1, 16, 0};
+  else if (epi == EPI_LINEAR && tiles <= 2 * sms) c = {1, 8, 0};
+  else if (epi == EPI_LINEAR && tiles <= 4 * sms) c.warps = 8;
+  c.lines = small_ahead(c.tiles * nt, ab_dtype == B200_INT8_WO);
+  return c;
+}
+
 template <int KIND, int NT>
-static int pick_small(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, cudaStream_t s) {
-  if (epi == EPI_SILU_MUL) return launch_small<KIND, EPI_SILU_MUL, NT, 2, 4>(a, w, ep, M, N, K, s);
-  if (epi == EPI_ROPE) return launch_small<KIND, EPI_ROPE, NT, 2, 8>(a, w, ep, M, N, K, s);
-  const int tiles = (N + 15) / 16, sms = sm_count(), row = K * (KIND == KIND_F16 ? 2 : 1);
-  if (tiles <= sms && row > 4096) return launch_small<KIND, EPI_LINEAR, NT, 1, 16>(a, w, ep, M, N, K, s);
-  if (tiles <= 2 * sms) return launch_small<KIND, EPI_LINEAR, NT, 1, 8>(a, w, ep, M, N, K, s);
-  if (tiles <= 4 * sms) return launch_small<KIND, EPI_LINEAR, NT, 2, 8>(a, w, ep, M, N, K, s);
-  return launch_small<KIND, EPI_LINEAR, NT, 2, 4>(a, w, ep, M, N, K, s);
+static int pick_small(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, cudaStream_t s) {
+  const SmallShape c = gemm_small_shape(epi, M, N, K, ab_dtype);
+#define SMALL_GO(EPI, TILES, WARPS) \
+  if (epi == EPI && c.tiles == TILES && c.warps == WARPS) return launch_small<KIND, EPI, NT, TILES, WARPS>(a, w, ep, M, N, K, s)
+  SMALL_GO(EPI_LINEAR, 1, 16);
+  SMALL_GO(EPI_LINEAR, 1, 8);
+  SMALL_GO(EPI_LINEAR, 2, 8);
+  SMALL_GO(EPI_LINEAR, 2, 4);
+  SMALL_GO(EPI_SILU_MUL, 2, 4);
+  SMALL_GO(EPI_ROPE, 2, 8);
+#undef SMALL_GO
+  return B200_ERR_UNSUPPORTED;
 }
 
 int launch_gemm_small(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, cudaStream_t s) {
-  if (ab_dtype == B200_BF16) return pick_small<KIND_F16, 1>(a, w, ep, epi, M, N, K, s);
-  if (ab_dtype == B200_FP8_E4M3) return pick_small<KIND_F8F6F4, 1>(a, w, ep, epi, M, N, K, s);
-  if (ab_dtype == B200_INT8) return pick_small<KIND_I8, 1>(a, w, ep, epi, M, N, K, s);
-  return M <= 8 ? pick_small<KIND_WO8, 1>(a, w, ep, epi, M, N, K, s) : pick_small<KIND_WO8, 2>(a, w, ep, epi, M, N, K, s);
+  if (ab_dtype == B200_BF16) return pick_small<KIND_F16, 1>(a, w, ep, epi, M, N, K, ab_dtype, s);
+  if (ab_dtype == B200_FP8_E4M3) return pick_small<KIND_F8F6F4, 1>(a, w, ep, epi, M, N, K, ab_dtype, s);
+  if (ab_dtype == B200_INT8) return pick_small<KIND_I8, 1>(a, w, ep, epi, M, N, K, ab_dtype, s);
+  return M <= 8 ? pick_small<KIND_WO8, 1>(a, w, ep, epi, M, N, K, ab_dtype, s) : pick_small<KIND_WO8, 2>(a, w, ep, epi, M, N, K, ab_dtype, s);
 }
 
 // CTAs of two warps: eight an SM, which holds as many weight rows at once as the decode schedule's tiles, and no other CTA meets the barrier

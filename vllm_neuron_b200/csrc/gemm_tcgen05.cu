@@ -1384,10 +1384,11 @@ int b200_gemm_decode_plan(int M, int N, int K, int ab_dtype, int split_k, int si
   if (rc) return rc;
   const int epi = silu_mul == 2 ? EPI_ROPE : silu_mul ? EPI_SILU_MUL : EPI_LINEAR;
   if (split_k == 0 && gemm_small_ok(nullptr, nullptr, epi, M, N, K, ab_dtype, 64)) {  // no cluster, no shared-memory rings
+    const SmallShape c = gemm_small_shape(epi, M, N, K, ab_dtype);
     out6[0] = 1;
-    out6[1] = 2;
-    out6[2] = out6[3] = 2;  // k-blocks of a warp in flight, at least
-    out6[4] = 2 * sm_count();  // at 8 warps
+    out6[1] = 16 / c.warps;
+    out6[2] = out6[3] = c.lines;
+    out6[4] = out6[1] * sm_count();
     out6[5] = 0;
     return B200_OK;
   }
