@@ -57,7 +57,7 @@ def build_bind(force: bool = False) -> str:
     """The extension module beside the library (host code only).  Another torch, Python or compiler flag makes it anew."""
     cmd = _bind_command()
     stamp = os.path.join(HERE, "build", "bind_command.txt")
-    made = " ".join([sys.version, *cmd])
+    made = " ".join([sys.version, *cmd]).replace(HERE, "")  # a copy of the folder is as good
     if not force and os.path.exists(BIND) and all(os.path.getmtime(d) <= os.path.getmtime(BIND) for d in BIND_SOURCES):
         if os.path.exists(stamp) and open(stamp).read() == made:
             return BIND
