@@ -19,7 +19,7 @@
 //   * the weights enter the second product as TWO bf16 terms, hi = bf16(p) in the first 64 columns the scores occupied and
 //     lo = bf16(p - hi) in the other 64 (16 mantissa bits; the scores sit in registers by then), two MMAs per 16 keys;
 //   * a sink (a logit per head, or none) is where the running maximum and the denominator start: 16 heads of 128, window 1024, a prompt of 4096,
-//     78 us (mma.sync kernel, swa_attn_prefill.cu: 271 us);
+//     94 us around the call, weights in two terms (mma.sync kernel, swa_attn_prefill.cu: 276 us);
 //   * sigmoid weights need no maximum and no denominator; rows whose chunk starts after a key step see -inf only, and
 //     the maximum stays -inf without producing NaN.
 #include "hybrid_common.cuh"

@@ -729,7 +729,10 @@ def kv_write_vmix(qkv, k_col0: int, v_col0: int, k_pool, v_pool, slot_mapping, *
 
 
 PREFILL_ATTN_MIN_TOKENS = 16  # longest portion of a step from which the tensor-core attention kernel is used
-PREFILL_TC_MIN_TOKENS = 128   # ... and from which the tcgen05 kernel with its 128-row query tiles is
+# ... and from which the tcgen05 kernel with its 128-row query tiles is.  With a sink, chained launches, us, mma.sync / tcgen05, 16 heads over 4 of 128, window
+# 1024: one portion of 128 tokens 19.1 / 10.9, 256 after 1500 104 / 44, 4096 264 / 76; heads of 64, 128 tokens, window 128 13.9 / 8.3; over 576 steps of
+# one to eight portions and 2 to 64 heads 0.17 to 0.83 of the time.
+PREFILL_TC_MIN_TOKENS = 128
 _SWA_PREFILL_LEGACY = bool(os.environ.get("B200_SWA_PREFILL_LEGACY"))
 
 
