@@ -589,7 +589,7 @@ def test_gemm_silu_mul_quant_of_a_few_tokens(ops, m, i, k):
     test_gemm_silu_mul_matches_unfused(ops, "fp8", m, i, k, 0)
 
 
-@pytest.mark.parametrize("m,n,k,kind,epi,per_sm,lines", [(1, 2048, 5632, "BF16", 0, 1, 4), (8, 2048, 2048, "BF16", 0, 2, 4), (4, 6144, 4096, "FP8_E4M3", 0, 2, 2),
+@pytest.mark.parametrize("m,n,k,kind,epi,per_sm,lines", [(1, 2048, 5632, "BF16", 0, 1, 4), (8, 2048, 2048, "BF16", 0, 2, 4), (1, 4096, 4096, "FP8_E4M3", 0, 1, 2), (4, 6144, 4096, "FP8_E4M3", 0, 2, 2),
                                                          (4, 32000, 2048, "INT8", 0, 4, 2), (2, 6144, 4096, "BF16", 2, 2, 2), (2, 11264, 2048, "BF16", 1, 4, 2),
                                                          (3, 2048, 8192, "INT8_WO", 0, 1, 3), (16, 2048, 8192, "INT8_WO", 0, 1, 2), (9, 32000, 2048, "INT8_WO", 0, 4, 1)])
 def test_plan_of_a_few_tokens(ops, m, n, k, kind, epi, per_sm, lines):

@@ -357,14 +357,14 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
 }
 
 // Which calls the kernel takes: up to 8 tokens all of them, 9 to 16 the weight-only ones.  Chained launches over weights larger than L2, us, decode
-// schedule / here, one token: bf16 2048 x 2048 4.7 / 3.3, 2048 x 5632 8.4 / 6.2, 11264 x 2048 gate and up 12.6 / 10.0, 4096 x 14336 25.3 / 20.3, 28672 x 4096
-// gate and up 44.7 / 41.2; fp8 4.0 / 2.7, 5.8 / 3.9, 8.1 / 7.0, 14.9 / 14.1, 23.2 / 24.2; weight-only 7.1 / 3.0, 11.5 / 4.7, 12.8 / 10.0, 26.1 / 19.2, 38.8 / 34.3.
-// Decode steps at 500 tokens of context, one token: TinyLlama bf16 993 / 621; Llama 3.1 8B, 6 layers, bf16 815 / 699, fp8 549 / 466, 8 tokens weight-only
-// 829 / 651; Qwen2.5 32B, 2 layers, 4 tokens, bf16 675 / 592, fp8 402 / 375 -- with all of a layer's GEMMs on one schedule: a decode-schedule GEMM behind one
+// schedule / here, one token: bf16 2048 x 2048 4.7 / 3.3, 2048 x 5632 8.4 / 6.2, 11264 x 2048 gate and up 12.6 / 10.0, 4096 x 14336 25.3 / 19.4, 28672 x 4096
+// gate and up 44.7 / 41.2; fp8 4.0 / 2.7, 5.8 / 3.9, 8.1 / 7.0, 14.9 / 12.4, 23.2 / 24.2; weight-only 7.1 / 3.0, 11.5 / 4.7, 12.8 / 10.0, 26.1 / 15.8, 38.8 / 34.3.
+// Decode steps at 500 tokens of context, one token: TinyLlama bf16 993 / 620; Llama 3.1 8B, 6 layers, bf16 815 / 689, fp8 549 / 452, 8 tokens weight-only
+// 829 / 629; Qwen2.5 32B, 2 layers, 4 tokens, bf16 675 / 583, fp8 402 / 371 -- with all of a layer's GEMMs on one schedule: a decode-schedule GEMM behind one
 // of these finds no room for its rings.  So weights that alone are slower here (5120 x 27648 fp8 29.8 / 37.5, int8 weights 46 / 56, at 16 tokens 66; 28672 x
 // 4096 fp8 23.2 / 24.2) are left here: with the fp8 28672 x 4096 on the decode schedule the 8B step takes 531.
 // 9 to 16 tokens load twice the fragments a weight: 16 tokens, 8B bf16 820 / 898, fp8 572 / 667; weight-only, whose decode schedule
-// widens in a pass of its own, 847 / 728, TinyLlama 1243 / 779, Qwen 582 / 579.
+// widens in a pass of its own, 847 / 690, TinyLlama 1243 / 768, Qwen 582 / 578.
 bool gemm_small_ok(const void* a, const void* w, int epi, int M, int N, int K, int ab_dtype, int head_dim) {
   const int64_t row = (int64_t)K * (ab_dtype == B200_BF16 ? 2 : 1);
   if (M > (ab_dtype == B200_INT8_WO ? 16 : 8) || row % 16 || (((uintptr_t)a | (uintptr_t)w) & 15) || row * 2 > INT_MAX) return false;
@@ -377,17 +377,17 @@ static int launch_small(const void* a, const void* w, const GemmEpilogue& ep, in
                              (const uint8_t*)w, (const uint8_t*)a, ep, M, N, K));
   return B200_OK;
 }
-// CTAs of 16 rows while they fit the chip once (16 warps of one SM share a long row, or 8), then of 32 rows; where those are many, four warps
-// each, so that more of them are in flight and the last wave is short.  Measured, bf16, one token, us: 2048 x 5632 with 16 / 8 warps 5.1 / 6.2,
-// 2048 x 2048 2.6 / 2.5, 4096 x 4096 7.4 / 6.4; 6144 x 4096 16 / 32 rows 11.3 / 10.2; 10272 x 2048 8 / 4 warps 10.2 / 9.2, 32000 x 2048 22.8 / 21.8.
-// Gate and up rows and the halves of a head come in 32 rows: as many warps a CTA as let all CTAs be resident.  4 tokens, 4 / 8 / 16 warps, 7168 x 4096 gate
+// CTAs of 16 rows while there is an SM for each (16 warps of it share a long row, or 8), then of 32 rows -- gate and up rows and the halves of a head
+// come in 32 -- with as many warps as let all CTAs be resident; where they are many, four each, so that more of them are in flight and the last
+// wave is short.  Measured, bf16, one token, us: 2048 x 5632 with 16 / 8 warps 5.1 / 6.2, 2048 x 2048 2.6 / 2.5; 4096 x 14336 32 rows in 16 warps / 16
+// rows in 8 19.4 / 20.3, fp8 12.4 / 14.1, 16 tokens on int8 weights 19.9 / 25.0; 6144 x 4096 16 / 32 rows 11.3 / 10.2; 10272 x 2048 8 / 4 warps 10.2 / 9.2, 32000 x
+// 2048 22.8 / 21.8.  4 tokens, 4 / 8 / 16 warps, 7168 x 4096 gate
 // and up 14.8 / 12.0 / 12.9 (decode schedule 14.3), 11264 x 2048 10.4 / 12.6 / 12.3; heads of 128, 768 x 4096 12.5 / 7.2 / 5.4 (6.8), 6144 x 4096 14.8 / 11.4 / 12.9.
 SmallShape gemm_small_shape(int epi, int M, int N, int K, int ab_dtype) {
   const int tiles = (N + 15) / 16, sms = sm_count(), nt = M <= 8 ? 1 : 2;
   const int64_t row = (int64_t)K * (ab_dtype == B200_BF16 ? 2 : 1);
   SmallShape c{2, tiles <= 2 * sms ? 16 : tiles <= 4 * sms ? 8 : 4, 0};
-  if (epi == EPI_LINEAR && tiles <= sms && row > 4096) c = {1, 16, 0};
-  else if (epi == EPI_LINEAR && tiles <= 2 * sms) c = {1, 8, 0};
+  if (epi == EPI_LINEAR && tiles <= sms) c = {1, row > 4096 ? 16 : 8, 0};
   c.lines = small_ahead(c.tiles * nt, ab_dtype == B200_INT8_WO);
   return c;
 }
@@ -399,6 +399,7 @@ static int pick_small(const void* a, const void* w, const GemmEpilogue& ep, int 
   if (epi == EPI && c.tiles == TILES && c.warps == WARPS) return launch_small<KIND, EPI, NT, TILES, WARPS>(a, w, ep, M, N, K, s)
   SMALL_GO(EPI_LINEAR, 1, 16);
   SMALL_GO(EPI_LINEAR, 1, 8);
+  SMALL_GO(EPI_LINEAR, 2, 16);
   SMALL_GO(EPI_LINEAR, 2, 8);
   SMALL_GO(EPI_LINEAR, 2, 4);
   SMALL_GO(EPI_SILU_MUL, 2, 16);
