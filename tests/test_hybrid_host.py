@@ -176,6 +176,17 @@ def test_step_parts_are_split_only_where_the_decoded_tokens_are_worth_a_launch()
     assert ops._span(900, 256, 0, 32, 4) == 256 + 644 // 32 + 4 and ops._span(900, 1 << 30, 128, 0, 0) == 128
 
 
+def test_many_decoded_tokens_leave_short_prompts():
+    """64 tokens at 1800 beside 200 new ones, a kv head per query head, pages of whole tiles: 39 us apart and 70 together; other pages as before."""
+    from vllm_neuron_b200 import ops
+    from vllm_neuron_b200.hybrid import StepMeta
+
+    entries = [(0, 0, 200)] + [(1 + i, 1800, 1) for i in range(64)]
+    m = StepMeta.build(entries, {e[0]: list(range(1, 201)) for e in entries}, 32, "cpu")
+    spans = [ops._span(p.max_end, 512, 0, 0, 0) for p in m.parts]
+    assert ops._split_pays(m.parts, 8, 8, 64, 64, False, True, spans) and not ops._split_pays(m.parts, 8, 8, 64, 64, False, True, spans, pages=False)
+
+
 def test_delta_rule_rounds_where_a_chain_is_long_or_the_chip_is_free():
     from vllm_neuron_b200.ops import _delta_rounds
 

@@ -741,15 +741,18 @@ def _span(max_end: int, window: int, chunk: int, pool: int, keep: int) -> int:
     return min(max_end, window, chunk or 1 << 30) + (max(max_end - window, 0) // pool if pool else 0) + keep
 
 
-def _split_pays(parts, num_heads: int, g: int, d: int, dv: int, latent: bool, tc: bool, spans) -> bool:
-    """Whether the decoded tokens of a mixed step are worth launches of their own.  spans: per part, the keys its queries see at most.
+def _split_pays(parts, num_heads: int, g: int, d: int, dv: int, latent: bool, tc: bool, spans, pages: bool = True) -> bool:
+    """Whether the decoded tokens of a mixed step are worth launches of their own.  spans: per part, the keys its queries see at most; pages:
+    the cache's pages are whole tiles of the decode kernel (32 rows).
     In the prompt kernel each of them is a row tile per head (the tcgen05 kernel: per two heads) that walks its keys behind the prompts' own
-    tiles; apart they cost a launch behind the prompts', 14 us, and the decode kernel's time.  The estimate of the first is a list of tiles
-    over the chip's slots: `us` per key and 5 per tile, the last tile's walk on top where there are more tiles than slots, a fifth for
-    sharing the SMs.  Measured, apart / together, us, 16 heads: prompts of 1600, over latents 29 tokens at 1800 366 / 695, 2 356 / 360, 29 at
-    300 317 / 298; window of 512 with sinks, 29 at 1800 111 / 144, 4 97 / 78; full context on tcgen05, 29 at 1800 133 / 143, 4 78 / 56,
-    4 at 300 64 / 46; a prompt of 200 beside one token at 1800, window of 512 43 / 51, 12 heads of 80 45 / 132, at 300 35 / 28.  Over 300 such
-    steps the rule's choice costs 1.6 % more than the better one on average, always apart 8 %, always together 29 %."""
+    tiles; apart they cost a launch behind the prompts' and the decode kernel's time.  The estimate of the first is a list of tiles
+    over the chip's slots: `us` per key and 5 per tile, the last tile's walk on top where there are more tiles than slots, a tenth for
+    sharing the SMs.  The second, over pages of whole tiles: 4 us a launch and 3, the key and value bytes, 8 us for 1000 keys of one token.
+    Measured, apart / together, us, prompts of 1600: 16 heads over 4 of 128, window of 512 with sinks, on tcgen05 29 tokens at 1800 54 / 78, 8 48 / 46,
+    64 at 300 67 / 110, 29 at 300 72 / 66; 8 heads over 8 of 64, 64 at 1800 49 / 109; 200 tokens beside 64 at 1800 39 / 70 (mma.sync kernel 49 / 52).
+    Over 4032 such steps the rule's choice costs 1.1 % more than the better one on average (mma.sync 0.7), always apart 19 (10), always together 38 (64);
+    with the decode kernel's time as it was before its tiles lay on pages 6.0 (4.8).
+    Over latents (29 tokens at 1800 366 / 695, 2 356 / 360, 29 at 300 317 / 298) and other pages: 14 us a launch, a fifth, and that time."""
     us, rows, heads, slots = (0.026, 128, g * -(-num_heads // (2 * g)), 148) if tc else \
         (0.045 + 0.00014 * (d + dv), 64, num_heads, 148 * (4 if dv <= 128 else 2))
     n, keys, tiles, work, walk = 0, 0, 0, 0.0, 0.0
@@ -765,8 +768,11 @@ def _split_pays(parts, num_heads: int, g: int, d: int, dv: int, latent: bool, tc
         return max(walk, last, work / slots + last * max(0.0, 1 - slots / tiles))
 
     alone = max(walk, work / slots + walk * max(0.0, 1 - slots / tiles))
+    together = makespan(tiles + n * heads, work + n * heads * last)
+    if pages and not latent:
+        return 1.1 * together > alone + 4 * (len(parts) - 1) + 3 + keys * (4e-7 * n * g * (d + dv) + 0.008)
     decode = 0.035 * keys * max(1.0, n / 32) if latent else keys * (n * g / 4000 + 0.008)
-    return 1.2 * makespan(tiles + n * heads, work + n * heads * last) > alone + 14 * (len(parts) - 1) + decode
+    return 1.2 * together > alone + 14 * (len(parts) - 1) + decode
 
 
 def swa_sink_attn(q_src, num_heads: int, k_pool, v_pool, block_table, meta, sink, scale: float, window: int,
@@ -810,7 +816,7 @@ def swa_sink_attn(q_src, num_heads: int, k_pool, v_pool, block_table, meta, sink
     if parts:
         tc = _prompt_tc(q_src, k_pool, meta, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool)
         spans = [_span(p.max_end, int(window), int(chunk), pool, int(keep)) for p in parts]
-        if not (tc or _prompt_mma(q_src, k_pool, meta, d, dv)) or not _split_pays(parts, num_heads, g, d, dv, bool(latent_values), tc, spans):
+        if not (tc or _prompt_mma(q_src, k_pool, meta, d, dv)) or not _split_pays(parts, num_heads, g, d, dv, bool(latent_values), tc, spans, bs % 32 == 0):
             parts = None
     for part in parts or [meta]:
         _swa_part(q_src, num_heads, k_pool, v_pool, block_table, part, sink, scale, window, latent_values, chunk, softcap, sigmoid_bias,
