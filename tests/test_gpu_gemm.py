@@ -160,6 +160,22 @@ def test_gemm_pairs_silu_residual_bias(ops, m, n, k):
     _assert_close(ga, a.float().abs().view(m, -1, 16).amax(-1).cpu())
 
 
+# Two token tiles at a time: one such unit a pair, several (three waves), an odd number of token tiles (the last alone), whole waves and the rest one by
+# one, ragged tokens and rows, fewer k-blocks than ring stages and many more
+WIDE_SHAPES = [(300, 10000, 192), (300, 10001, 192), (777, 6144, 1040), (700, 12800, 96), (1030, 16128, 4000), (771, 28416, 4096)]
+
+
+@pytest.mark.parametrize("m,n,k", WIDE_SHAPES)
+@pytest.mark.parametrize("f32", [False, True])
+def test_gemm_pairs_of_two_token_tiles_int8_exact(ops, m, n, k, f32):
+    test_gemm_pairs_int8_exact(ops, m, n, k, f32)
+
+
+@pytest.mark.parametrize("m,n,k", [(777, 6144, 520), (700, 12800, 96)])
+def test_gemm_pairs_of_two_token_tiles_silu_residual_bias(ops, m, n, k):
+    test_gemm_pairs_silu_residual_bias(ops, m, n, k)
+
+
 @pytest.mark.parametrize("kind", ["bf16", "wo"])
 @pytest.mark.parametrize("m,n,k", [(33, 640, 1152), (64, 4096, 2048), (300, 1056, 640)])
 def test_gemm_outputs_on_any_boundary(ops, kind, m, n, k):
@@ -215,6 +231,12 @@ def test_gemm_pairs_bf16_against_64_bits(ops, m, n, k, f32):
     size = x.double().abs() @ w.double().abs().T + bias.double().abs() + res.double().abs()
     got = ops.gemm(x, w, None, None, bias, res, out_dtype=torch.float32 if f32 else torch.bfloat16).double()
     assert ((got - want).abs() <= (k / 16 + 3) * 2.0**-23 * size + (0.0 if f32 else 2.0**-8) * want.abs()).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(257, 1001, 192), (777, 6144, 520)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_gemm_pairs_rows_of_odd_length_and_two_token_tiles(ops, m, n, k, f32):
+    test_gemm_pairs_bf16_against_64_bits(ops, m, n, k, f32)
 
 
 @pytest.mark.parametrize("m,n,k", [(1, 1056, 512), (31, 256, 144), (33, 640, 1152), (64, 992, 256), (65, 256, 128), (128, 1000, 144), (100, 640, 1152), (127, 32, 64), (128, 38144, 256), (96, 5120, 2048),

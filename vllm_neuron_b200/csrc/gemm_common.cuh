@@ -195,10 +195,13 @@ __device__ __forceinline__ void epilogue_chunk_xpose(const GemmEpilogue& ep, con
 bool gemm_wo_wide(int epi, int M, int N, int K);
 int gemm_wo_plan(int epi, int M, int N, int K, int& splits, int& cap_ctas, int& stages, size_t& smem);
 int launch_gemm_wo(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, cudaStream_t stream);
-// Prompt-sized schedule on CTA pairs (gemm_pair.cu): bf16, fp8 and int8 operands.  pair_tokens: tokens of a tile for this shape, 0 where
-// stream-K is the faster schedule.
-int pair_tokens(int M, int N, int K, int ab_dtype);
-int launch_gemm_pair(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, int bt,
+// Prompt-sized schedule on CTA pairs (gemm_pair.cu): bf16, fp8 and int8 operands.  bt: tokens of a tile, 0 where stream-K is the faster
+// schedule; wide: how many units of two token tiles come before those of one.
+struct PairPlan {
+  int bt, wide;
+};
+PairPlan pair_plan(int M, int N, int K, int ab_dtype);
+int launch_gemm_pair(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, PairPlan plan,
                      cudaStream_t stream);
 
 }  // namespace b200

@@ -17,9 +17,11 @@ namespace b200 {
 
 constexpr int GRP_MAX_TILES = 1024;  // row tiles whose schedule fits shared memory
 constexpr int GRP_MAX_ST = 11;
+constexpr int GRP_EPI_WARPS = 8;                      // two per 32-lane group of tensor memory: they share its token chunks
+constexpr int GRP_THREADS = 64 + 32 * GRP_EPI_WARPS;  // + the TMA producer and the MMA issuer
 
 template <bool GLU>
-__global__ void __launch_bounds__(PAIR_THREADS, 1)
+__global__ void __launch_bounds__(GRP_THREADS, 1)
     gemm_group_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap a_map,
                       const __grid_constant__ CUtensorMap a2_map, const int32_t* __restrict__ sorted_ids,
                       const int32_t* __restrict__ tile_expert, const int32_t* __restrict__ num_tiles, int bm, int n_tiles, int num_kb, int nst,
@@ -34,7 +36,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
   __shared__ int32_t sched_n;
   // epilogue scratch, per half of the warps: GLU [2][16][64] exchanged values; then per warp a transposing tile
   __shared__ __align__(16) float xch[GLU ? 2 * 2 * 16 * 64 : 4];
-  __shared__ __align__(16) float xpose[GLU ? PAIR_EPI_WARPS * 16 * 20 : PAIR_EPI_WARPS * XP_WARP_FLOATS];
+  __shared__ __align__(16) float xpose[GLU ? GRP_EPI_WARPS * 16 * 20 : GRP_EPI_WARPS * XP_WARP_FLOATS];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -49,7 +51,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&tfull[s], 1);
-      mbar_init(&tempty[s], 2 * PAIR_EPI_WARPS);
+      mbar_init(&tempty[s], 2 * GRP_EPI_WARPS);
     }
     fence_mbar_init();
     fence_proxy_async();
@@ -263,7 +265,7 @@ static int launch_group(const void* a, const int32_t* sorted_ids, const void* w,
   const int n_tiles = N / (GLU ? GEMM_BN : 2 * GEMM_BN);
   int pairs = sm_count() / 2;
   if ((long long)row_tiles * n_tiles < pairs) pairs = row_tiles * n_tiles;
-  B200_CUDA_OK(launch_kernel_cluster(kern, dim3(2 * pairs), dim3(PAIR_THREADS), RING + 1024, 2, st, wm, am, am2, sorted_ids, tile_expert,
+  B200_CUDA_OK(launch_kernel_cluster(kern, dim3(2 * pairs), dim3(GRP_THREADS), RING + 1024, 2, st, wm, am, am2, sorted_ids, tile_expert,
                                      num_tiles, tile_rows, n_tiles, (K + BK - 1) / BK, nst, stage, out, ldo, N, scatter, limit, act));
   return B200_OK;
 }

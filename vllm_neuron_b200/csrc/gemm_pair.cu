@@ -9,6 +9,9 @@
 // per CTA and k-block in 0.39 us, 84 GB/s per SM, 12.4 TB/s over the chip, whatever the ring depth from 4 stages on (2 stages are
 // slower, and boxes of half the rows, from one or four issuing warps, take 0.53 us).  Pairs are persistent over whole tiles, K is
 // not cut: two accumulators of 256 columns alternate, so a tile's epilogue runs under the next tile's MMAs.
+// Since operand rows are what bounds it, a pair may also take two neighbouring token tiles of one weight tile at once, both accumulators
+// full: 384 rows for 512 tokens instead of twice 256 (figures at pair_plan); the next unit's first token tile runs ahead through the ring (and the
+// ring fills on) while the epilogue drains the other accumulator.  The sums are the same, bit for bit: K goes into one accumulator in one order.
 // Measured against the stream-K schedule that it replaces for these operand kinds (us, B200): bf16 4096 x 10272 x 2048 183 -> 135,
 // 4096 x 2048 x 2048 73 -> 32, 777 x 28672 x 4096 + SiLU 248 -> 175, 333 x 2048 x 2048 71 -> 15; fp8 2048 x 28672 x 4096 + SiLU
 // 316 -> 195, 2048 x 4096 x 14336 145 -> 94 (2.5 PFLOP/s).
@@ -16,22 +19,51 @@
 // grows with the length of a sum that is not cut: K = 4096 4.4e-6 (stream-K 3.7e-6 at 2048 x 4096, where it cuts few tiles, 1.6e-6 at 777 x
 // 2048), K = 14336 1.6e-5 (1.4e-5, 6.0e-6); a quarter to one percent of a bf16 output's own rounding, 1.7e-3.  Spans of four k-blocks added in
 // registers bring 2.4e-7 at any K, take 15 to 60 % longer, and leave the error of every serving step as it is.
+#include <limits.h>
+
 #include <mutex>
 
 #include "gemm_pair.cuh"
 
 namespace b200 {
 
-// Warp roles: 0 = TMA producer (both CTAs), 1 = tensor-memory owner (both) and MMA issuer (leader), 2..9 = epilogue.
+constexpr int PAIR_EPI_WARPS = 16;                     // four per 32-lane group of tensor memory: they share its token chunks
+constexpr int PAIR_THREADS = 64 + 32 * PAIR_EPI_WARPS;  // + the TMA producer and the MMA issuer
+
+// What a pair walks: `wide` units of two neighbouring token tiles of one weight tile, which share its weight rows (both accumulators at
+// once), then the token tiles that are left one by one.
+struct PairUnits {
+  int mt, wide, lone0, units;  // token tiles; wide units; token tiles (weight tile by weight tile) that they cover; all units
+  __host__ __device__ PairUnits(int mt_, int n_tiles, int wide_) : mt(mt_), wide(wide_) {
+    const int u = (mt + 1) / 2, r = wide % u;  // a weight tile's last wide unit holds one token tile where their number is odd
+    lone0 = wide / u * mt + (2 * r < mt ? 2 * r : mt);
+    units = wide + n_tiles * mt - lone0;
+  }
+  // -> weight tile, first token tile, number of token tiles
+  __device__ __forceinline__ void at(int i, int& nt, int& m, int& cnt) const {
+    if (i < wide) {
+      const int u = (mt + 1) / 2;
+      nt = i / u;
+      m = 2 * (i - nt * u);
+      cnt = mt - m < 2 ? 1 : 2;
+    } else {
+      const int t = lone0 + i - wide;
+      nt = t / mt;
+      m = t - nt * mt;
+      cnt = 1;
+    }
+  }
+};
+
+// Warp roles: 0 = TMA producer (both CTAs), 1 = tensor-memory owner (both) and MMA issuer (leader), 2..17 = epilogue.
 template <int KIND, int EPI>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap a_map, GemmEpilogue ep, int M, int N,
-                     int m_tiles, int tiles, int num_kb, int bt, int nst, int w_stream_once) {
+                     PairUnits un, int num_kb, int bt, int nst, int stage, int w_stream_once) {
   using T = KindTraits<KIND>;
   constexpr int BK_ELEMS = GEMM_BK_BYTES / T::ELEM;
   constexpr int W_TILE = GEMM_BN * GEMM_BK_BYTES;
-  const int a_tile = (bt >> 1) * GEMM_BK_BYTES;  // this CTA's half of the tokens
-  const int stage = W_TILE + a_tile;
+  const int a_tile = (bt >> 1) * GEMM_BK_BYTES;  // this CTA's half of a token tile
   const uint32_t idesc = umma_idesc(T::CFMT, T::ABFMT, 2 * GEMM_BN, (uint32_t)bt);
 
   extern __shared__ uint8_t smem_raw[];
@@ -39,7 +71,6 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
   __shared__ uint64_t full[PAIR_MAX_ST], empty[PAIR_MAX_ST], tfull[2], tempty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ __align__(16) float a_s_tile[PAIR_MAX_BT];
-  __shared__ __align__(16) float xpose[PAIR_EPI_WARPS * XP_WARP_FLOATS];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -75,26 +106,29 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
       const uint64_t pol_w = w_stream_once ? policy_evict_first() : policy_evict_last();
       const uint64_t pol_a = policy_evict_last();  // activations are re-read by every pair
       const int n_off = (int)rank * GEMM_BN, m_off = (int)rank * (bt >> 1);
-      // weights do not depend on any kernel of the step: fill the ring with the first tile's before the dependency resolves
+      int nt, mt, cnt;
+      un.at(pair, nt, mt, cnt);
+      // weights do not depend on any kernel of the step: fill the ring with the first unit's before the dependency resolves
       const int npre = num_kb < nst ? num_kb : nst;
       for (int i = 0; i < npre; ++i) {
-        if (rank == 0) mbar_expect_tx(&full[i], 2 * stage);
-        tma_load_2d_pair(smem + (size_t)i * stage, &w_map, mapa_shared(smem_u32(&full[i]), 0), i * BK_ELEMS,
-                         (pair / m_tiles) * 2 * GEMM_BN + n_off, pol_w);
+        if (rank == 0) mbar_expect_tx(&full[i], 2 * (W_TILE + cnt * a_tile));
+        tma_load_2d_pair(smem + (size_t)i * stage, &w_map, mapa_shared(smem_u32(&full[i]), 0), i * BK_ELEMS, nt * 2 * GEMM_BN + n_off, pol_w);
       }
       griddep_wait();
       int i = 0, s = 0, ph = 1;  // first pass over the ring: the stages are free (a parity-1 wait on a fresh barrier returns at once)
-      for (int tile = pair; tile < tiles; tile += pairs) {
-        const int n0 = (tile / m_tiles) * 2 * GEMM_BN + n_off, m0 = (tile % m_tiles) * bt + m_off;
+      for (int unit = pair; unit < un.units; unit += pairs) {
+        un.at(unit, nt, mt, cnt);
+        const int n0 = nt * 2 * GEMM_BN + n_off, m0 = mt * bt + m_off;
         for (int kb = 0; kb < num_kb; ++kb, ++i) {
           const uint32_t bar = mapa_shared(smem_u32(&full[s]), 0);
           uint8_t* ws = smem + (size_t)s * stage;
           if (i >= npre) {
             mbar_wait(&empty[s], ph);
-            if (rank == 0) mbar_expect_tx(&full[s], 2 * stage);
+            if (rank == 0) mbar_expect_tx(&full[s], 2 * (W_TILE + cnt * a_tile));
             tma_load_2d_pair(ws, &w_map, bar, kb * BK_ELEMS, n0, pol_w);
           }
           tma_load_2d_pair(ws + W_TILE, &a_map, bar, kb * BK_ELEMS, m0, pol_a);
+          if (cnt == 2) tma_load_2d_pair(ws + W_TILE + a_tile, &a_map, bar, kb * BK_ELEMS, m0 + bt, pol_a);
           if (++s == nst) {
             s = 0;
             ph ^= 1;
@@ -105,20 +139,49 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
     __syncwarp();
   } else if (warp == 1) {
     if (rank == 0) {
-      int s = 0, ph = 0, seg = 0;
-      for (int tile = pair; tile < tiles; tile += pairs, ++seg) {
+      int s = 0, ph = 0, seg = 0, nt, mt, cnt;
+      // the MMAs of token tile h of the unit whose operands lie in stage `st`
+      auto mma = [&](int st, int h, uint32_t acc, bool first) {
+        const uint32_t wa = smem_u32(smem + (size_t)st * stage), aa = wa + W_TILE + h * a_tile;
+#pragma unroll
+        for (int kk = 0; kk < GEMM_BK_BYTES / 32; ++kk)  // UMMA_K = 32 bytes of K
+          umma_ss_pair<KIND>(acc, umma_desc_sw128(wa + kk * 32), umma_desc_sw128(aa + kk * 32), idesc, (uint32_t)(!first || kk != 0));
+      };
+      for (int unit = pair; unit < un.units; unit += pairs) {
+        un.at(unit, nt, mt, cnt);
         const int as = seg & 1;
         if (seg >= 2) mbar_wait(&tempty[as], ((seg >> 1) - 1) & 1);
         tc_fence_after();
-        const uint32_t acc = tmem_base + (uint32_t)(as * PAIR_MAX_BT);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const uint32_t acc = tmem_base + (uint32_t)(as * PAIR_MAX_BT), acc2 = tmem_base + (uint32_t)((as ^ 1) * PAIR_MAX_BT);
+        // of a wide unit the first token tile runs ahead through the ring while the epilogue still drains the other accumulator
+        int ahead = 0, s2 = s;
+        if (cnt == 2) {
+          for (; ahead < num_kb && ahead < nst; ++ahead) {
+            mbar_wait(&full[s], ph);
+            tc_fence_after();
+            if (lane == 0) mma(s, 0, acc, ahead == 0);
+            __syncwarp();
+            if (++s == nst) {
+              s = 0;
+              ph ^= 1;
+            }
+          }
+          if (seg >= 1) mbar_wait(&tempty[as ^ 1], (((seg + 1) >> 1) - 1) & 1);
+          tc_fence_after();
+          if (lane == 0)
+            for (int k = 0; k < ahead; ++k) {
+              mma(s2, 1, acc2, k == 0);
+              tc_commit_pair(&empty[s2]);
+              if (++s2 == nst) s2 = 0;
+            }
+          __syncwarp();
+        }
+        for (int kb = ahead; kb < num_kb; ++kb) {
           mbar_wait(&full[s], ph);
           tc_fence_after();
           if (lane == 0) {
-            const uint32_t wa = smem_u32(smem + (size_t)s * stage), aa = wa + W_TILE;
-#pragma unroll
-            for (int kk = 0; kk < GEMM_BK_BYTES / 32; ++kk)  // UMMA_K = 32 bytes of K
-              umma_ss_pair<KIND>(acc, umma_desc_sw128(wa + kk * 32), umma_desc_sw128(aa + kk * 32), idesc, (uint32_t)((kb | kk) != 0));
+            mma(s, 0, acc, kb == 0);
+            if (cnt == 2) mma(s, 1, acc2, false);
             tc_commit_pair(&empty[s]);
           }
           __syncwarp();
@@ -127,48 +190,68 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
             ph ^= 1;
           }
         }
-        if (lane == 0) tc_commit_pair(&tfull[as]);
+        if (lane == 0) {
+          tc_commit_pair(&tfull[as]);
+          if (cnt == 2) tc_commit_pair(&tfull[as ^ 1]);
+        }
         __syncwarp();
+        seg += cnt;
       }
     }
   } else {
-    const int lg = warp & 3, half = (warp - 2) >> 2;
+    const int lg = warp & 3, quarter = (warp - 2) >> 2;
     const int et = threadIdx.x - 64;
-    float* xp = xpose + (warp - 2) * XP_WARP_FLOATS;
+    const bool scaled = KIND == KIND_I8 || ep.a_scale || ep.w_scale, by_two = epilogue_by_two(ep, EPI == EPI_LINEAR ? N : N >> 1);
+    const bool ahead = EPI == EPI_LINEAR && ep.residual && by_two && !ep.out_f32;  // residuals are loaded before the accumulators are there
     griddep_wait();
-    int seg = 0;
-    for (int tile = pair; tile < tiles; tile += pairs, ++seg) {
-      const int as = seg & 1;
-      const int m0 = (tile % m_tiles) * bt;
-      const int n0w = (tile / m_tiles) * 2 * GEMM_BN + (int)rank * GEMM_BN + lg * 32;
-      const int n = n0w + lane;
-      named_bar_sync(1, 32 * PAIR_EPI_WARPS);  // the previous tile's readers of a_s_tile are done
-      if (et < bt) a_s_tile[et] = (ep.a_scale && m0 + et < M) ? ep.a_scale[m0 + et] : 1.f;
-      const float w_sc = (ep.w_scale && n < N) ? ep.w_scale[n] : 1.f;
-      const float bias_v = (ep.bias && n < N) ? __bfloat162float(ep.bias[n]) : 0.f;
-      named_bar_sync(1, 32 * PAIR_EPI_WARPS);
-      mbar_wait(&tfull[as], (seg >> 1) & 1);
-      __syncwarp();  // lanes may leave the wait one by one; tcgen05.ld wants them together
-      tc_fence_after();
-      const uint32_t acc = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(as * PAIR_MAX_BT);
-      // the two warps of a lane group take alternate pairs of 16-token chunks
-#pragma unroll 1
-      for (int c0 = half * 32; c0 < bt; c0 += 64) {
-        uint32_t v0[16], v1[16];
-        tmem_ld_32x32b_x16(acc + c0, v0);
-        tmem_ld_32x32b_x16(acc + c0 + 16, v1);
-        tmem_ld_wait();
-        float f[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) f[j] = KIND == KIND_I8 ? (float)(int32_t)v0[j] : __uint_as_float(v0[j]);
-        if (m0 + c0 < M) epilogue_chunk_xpose<EPI>(ep, f, m0 + c0, c0, M, n0w, N, lane, a_s_tile, w_sc, bias_v, xp);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) f[j] = KIND == KIND_I8 ? (float)(int32_t)v1[j] : __uint_as_float(v1[j]);
-        if (m0 + c0 + 16 < M) epilogue_chunk_xpose<EPI>(ep, f, m0 + c0 + 16, c0 + 16, M, n0w, N, lane, a_s_tile, w_sc, bias_v, xp);
-      }
+    // this warp has read what it takes of an accumulator: the MMAs may write it again while the last chunk is finished
+    auto give_back = [&](int as) {
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty[as]), 0));
+      if (lane == 0) mbar_arrive_cluster_relaxed(mapa_shared(smem_u32(&tempty[as]), 0));
+    };
+    int seg = 0, nt, mt, cnt;
+    for (int unit = pair; unit < un.units; unit += pairs) {
+      un.at(unit, nt, mt, cnt);
+      const int n0w = nt * 2 * GEMM_BN + (int)rank * GEMM_BN + lg * 32;
+      const int n = n0w + lane;
+      for (int h = 0; h < cnt; ++h, ++seg) {
+        const int as = seg & 1;
+        const int m0 = (mt + h) * bt;
+        named_bar_sync(1, 32 * PAIR_EPI_WARPS);  // the previous tile's readers of a_s_tile are done
+        if (et < bt) a_s_tile[et] = (ep.a_scale && m0 + et < M) ? ep.a_scale[m0 + et] : 1.f;
+        const float w_sc = (ep.w_scale && n < N) ? ep.w_scale[n] : 1.f;
+        const float bias_v = (ep.bias && n < N) ? __bfloat162float(ep.bias[n]) : 0.f;
+        named_bar_sync(1, 32 * PAIR_EPI_WARPS);
+        uint32_t r[8] = {};
+        int c0 = quarter * 16;
+        if (ahead && c0 < bt) epilogue_residual(ep, r, m0 + c0, M, n, N, lane & 1);
+        mbar_wait(&tfull[as], (seg >> 1) & 1);
+        __syncwarp();  // lanes may leave the wait one by one; tcgen05.ld wants them together
+        tc_fence_after();
+        const uint32_t acc = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(as * PAIR_MAX_BT);
+        // the four warps of a lane group take every fourth chunk of 16 tokens
+        uint32_t v[16];
+        if (c0 < bt) tmem_ld_32x32b_x16(acc + c0, v);
+        else give_back(as);
+#pragma unroll 1
+        for (; c0 < bt; c0 += 64) {
+          tmem_ld_wait16(v);
+          float f[16];
+          uint32_t q[8];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) f[j] = KIND == KIND_I8 ? (float)(int32_t)v[j] : __uint_as_float(v[j]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) q[j] = r[j];
+          if (c0 + 64 < bt) {
+            tmem_ld_32x32b_x16(acc + c0 + 64, v);
+            if (ahead) epilogue_residual(ep, r, m0 + c0 + 64, M, n, N, lane & 1);
+          } else {
+            give_back(as);
+          }
+          epilogue_chunk_lanes<EPI>(ep, f, q, m0 + c0, M, n0w, N, lane, a_s_tile + c0, w_sc, bias_v, scaled, by_two);
+        }
+      }
     }
   }
   tc_fence_before();
@@ -179,10 +262,11 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
 
 namespace {
 
-constexpr size_t PAIR_SMEM_RING = 232448 - 1024 - (PAIR_MAX_BT * 4 + PAIR_EPI_WARPS * XP_WARP_FLOATS * 4 + 512);
+constexpr size_t PAIR_SMEM_RING = 232448 - 1024 - (PAIR_MAX_BT * 4 + 512);
 
-int pair_stages(int bt) {
-  int n = (int)(PAIR_SMEM_RING / (size_t)(GEMM_BN * GEMM_BK_BYTES + (bt / 2) * GEMM_BK_BYTES));
+int pair_stage_bytes(int bt, bool wide) { return (GEMM_BN + (wide ? bt : bt / 2)) * GEMM_BK_BYTES; }
+int pair_stages(int stage) {
+  int n = (int)(PAIR_SMEM_RING / (size_t)stage);
   return n > PAIR_MAX_ST ? PAIR_MAX_ST : n;
 }
 
@@ -216,7 +300,7 @@ int max_pairs(int& out) {
 }
 
 template <int KIND, int EPI>
-int launch_pair(const void* a, const void* w, const GemmEpilogue& ep, int M, int N, int K, int bt, cudaStream_t stream) {
+int launch_pair(const void* a, const void* w, const GemmEpilogue& ep, int M, int N, int K, int bt, int wide, cudaStream_t stream) {
   constexpr int EB = KindTraits<KIND>::ELEM, BK = GEMM_BK_BYTES / EB;
   const CUtensorMapDataType dt = EB == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
   int pairs = 0;
@@ -227,54 +311,70 @@ int launch_pair(const void* a, const void* w, const GemmEpilogue& ep, int M, int
   if (rc) return rc;
   rc = make_tmap_2d(&am, a, dt, EB, (uint64_t)K, (uint64_t)M, (uint64_t)K * EB, BK, bt / 2);
   if (rc) return rc;
-  const int m_tiles = (M + bt - 1) / bt, n_tiles = (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN), tiles = m_tiles * n_tiles;
-  const int used = tiles < pairs ? tiles : pairs;
+  const int m_tiles = (M + bt - 1) / bt, n_tiles = (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN), stage = pair_stage_bytes(bt, wide > 0);
+  const PairUnits un(m_tiles, n_tiles, wide);
+  const int used = un.units < pairs ? un.units : pairs;
   B200_CUDA_OK(launch_kernel_cluster(gemm_pair_kernel<KIND, EPI>, dim3(2 * used), dim3(PAIR_THREADS), PAIR_SMEM_RING + 1024, 2, stream, wm,
-                                     am, ep, M, N, m_tiles, tiles, (K + BK - 1) / BK, bt, pair_stages(bt), m_tiles == 1 ? 1 : 0));
+                                     am, ep, M, N, un, (K + BK - 1) / BK, bt, pair_stages(stage), stage, m_tiles == 1 ? 1 : 0));
   return B200_OK;
 }
 
 }  // namespace
 
-// Tokens of a tile.  A wave of tiles costs its k-blocks -- 640 clocks up to 128 tokens, from there 3 for each of the 128 + bt/2 operand
-// rows (measured: 0.336 us at 96 and 128 tokens, 0.358 at 192, 0.428 at 256) -- plus filling the ring, draining the last accumulator and
-// the launch; so the widest tile wins unless a narrower one saves a wave or the padding of the last token tile.  Measured (us, 74 pairs):
-//   4096 x 10272 x 2048 bf16: bt 256 134.8, 224 149.2, 192 160.7, 128 212.6;  3688 x 2048 x 2048: 256 31.2, 192 41.8;
-//   1636 x 2048 x 2048: 192 18.6, 256 19.3, 128 28.5;  333 x 2048 x 2048: 64 15.2, 256 17.8;  777 x 4096 x 4096: 224 29.9, 192 50.8.
-// 0: stream-K (gemm_tcgen05.cu) takes the call.  It cuts K, which pays where few tiles walk a long K or a nearly empty wave follows a full
+// Tokens of a tile, and whether a pair takes two token tiles at once.  A wave of tiles costs its k-blocks -- 3 clocks for each of the 128 + bt/2
+// operand rows, no less than at 128 tokens -- plus filling the ring, draining the last accumulator and the launch; so the widest tile wins unless a narrower one saves a
+// wave or the padding of the last token tile.  Two at once cost 520 + 2.2 bt clocks a k-block, both accumulators' epilogue at the end and some of it
+// between waves; the waves that would not fill go one by one where that ends sooner.  Fitted to and checked against 645 measured calls (bf16, fp8,
+// SiLU and fp32 outputs, 129 to 4096 tokens, 14 weights, 11 to 13 plans each, L2 flushed): the choice is 0.3 % slower than the best plan on average, 12 % at
+// most, and 0.940 of one by one on average; 0.97 or less in 325 calls, over 1.03 in six (600 x 55296 x 5120 + SiLU 343 / 313 us).
+// Measured (us, one by one / two at once, bf16): 777 x 6144 x 4096 63.5 / 50.0, 777 x 28672 x 4096 196 / 160, 2048 x 28672 x 4096 363 / 311, fp8 201 /
+// 182, 4096 x 10272 x 2048 158 / 138, fp32 141 / 129.
+// bt = 0: stream-K (gemm_tcgen05.cu) takes the call.  It cuts K, which pays where few tiles walk a long K or a nearly empty wave follows a full
 // one: about 25 us, 0.52 for each k-block of 128 x 256 of an SM's share, and 8 for every CTA that adds to one tile.  Measured (us, pairs /
 // stream-K, bf16): 129 x 5120 x 27648 152 / 106, 256 158 / 115, 320 158 / 156, 512 164 / 173, 777 327 / 292, 1290 400 / 447;
 // 300 x 1024 x 28672 155 / 123, 1400 157 / 122; 200 x 8192 x 28672 175 / 139, 300 170 / 240; 129 x 4096 x 14336 80 / 85, 1200 161 / 158.
 // Over 700 measured calls (bf16 and fp8, 129 to 4096 tokens) the rule takes the slower side by more than 5 % in seven, by 13 % at most, and
 // never leaves a faster pair schedule.
-int pair_tokens(int M, int N, int K, int ab_dtype) {
+PairPlan pair_plan(int M, int N, int K, int ab_dtype) {
   const int eb = ab_dtype == B200_BF16 ? 2 : 1, sms = sm_count();
   const int pairs = sms / 2, num_kb = (K * eb + GEMM_BK_BYTES - 1) / GEMM_BK_BYTES, n_tiles = (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN);
   long long best_cost = 0;
-  int best = 0;
-  for (int bt = PAIR_MAX_BT; bt >= 64; bt -= 32) {
-    const long long tiles = (long long)((M + bt - 1) / bt) * n_tiles, waves = (tiles + pairs - 1) / pairs;
-    const long long cost = waves * ((long long)num_kb * (bt <= 128 ? 640 : 3 * (GEMM_BN + bt / 2)) + 2500 + 10 * bt);
-    if (!best || cost < best_cost) {
-      best = bt;
+  PairPlan best{0, 0};
+  auto offer = [&](int bt, int wide, long long cost) {
+    if (!best.bt || cost < best_cost) {
+      best = PairPlan{bt, wide};
       best_cost = cost;
+    }
+  };
+  for (int bt = PAIR_MAX_BT; bt >= 64; bt -= 32) {
+    const int mt = (M + bt - 1) / bt;
+    const long long lone_cost = (long long)num_kb * 3 * (GEMM_BN + (bt > 128 ? bt : 128) / 2) + 2600 + 7 * bt;
+    offer(bt, 0, ((long long)mt * n_tiles + pairs - 1) / pairs * lone_cost);
+    if (mt < 2 || bt < 128) continue;
+    const long long wide_cost = (long long)num_kb * (2600 + 11 * bt) / 5 + 3700 + 34 * bt, all = (long long)((mt + 1) / 2) * n_tiles;
+    if (all > INT_MAX) continue;
+    for (const long long wide : {all, all / pairs * pairs}) {  // wide to the end, or whole waves of it and the rest one by one
+      if (!wide) continue;
+      const PairUnits un(mt, n_tiles, (int)wide);
+      const long long waves = (wide + pairs - 1) / pairs;
+      offer(bt, (int)wide, waves * wide_cost + (waves - 1) * 4100 + (un.units - wide + pairs - 1) / pairs * lone_cost);
     }
   }
   const double sk_tiles = (double)((M + 255) / 256) * ((N + GEMM_BN - 1) / GEMM_BN), shared = sms / sk_tiles;
   const double stream_k_us = 25.0 + 0.52 * sk_tiles * num_kb / sms + 8.0 * (shared > 1.0 ? shared : 1.0);
-  return stream_k_us * 1850.0 < (double)best_cost ? 0 : best;  // clocks at 1.85 GHz
+  return stream_k_us * 1850.0 < (double)best_cost ? PairPlan{0, 0} : best;  // clocks at 1.85 GHz
 }
 
-int launch_gemm_pair(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, int bt,
+int launch_gemm_pair(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, PairPlan p,
                      cudaStream_t s) {
   if (ab_dtype == B200_BF16)
-    return epi == EPI_SILU_MUL ? launch_pair<KIND_F16, EPI_SILU_MUL>(a, w, ep, M, N, K, bt, s)
-                               : launch_pair<KIND_F16, EPI_LINEAR>(a, w, ep, M, N, K, bt, s);
+    return epi == EPI_SILU_MUL ? launch_pair<KIND_F16, EPI_SILU_MUL>(a, w, ep, M, N, K, p.bt, p.wide, s)
+                               : launch_pair<KIND_F16, EPI_LINEAR>(a, w, ep, M, N, K, p.bt, p.wide, s);
   if (ab_dtype == B200_FP8_E4M3)
-    return epi == EPI_SILU_MUL ? launch_pair<KIND_F8F6F4, EPI_SILU_MUL>(a, w, ep, M, N, K, bt, s)
-                               : launch_pair<KIND_F8F6F4, EPI_LINEAR>(a, w, ep, M, N, K, bt, s);
-  return epi == EPI_SILU_MUL ? launch_pair<KIND_I8, EPI_SILU_MUL>(a, w, ep, M, N, K, bt, s)
-                             : launch_pair<KIND_I8, EPI_LINEAR>(a, w, ep, M, N, K, bt, s);
+    return epi == EPI_SILU_MUL ? launch_pair<KIND_F8F6F4, EPI_SILU_MUL>(a, w, ep, M, N, K, p.bt, p.wide, s)
+                               : launch_pair<KIND_F8F6F4, EPI_LINEAR>(a, w, ep, M, N, K, p.bt, p.wide, s);
+  return epi == EPI_SILU_MUL ? launch_pair<KIND_I8, EPI_SILU_MUL>(a, w, ep, M, N, K, p.bt, p.wide, s)
+                             : launch_pair<KIND_I8, EPI_LINEAR>(a, w, ep, M, N, K, p.bt, p.wide, s);
 }
 
 }  // namespace b200

@@ -1294,8 +1294,8 @@ int gemm_common(const void* a, const void* w, const GemmEpilogue& ep, int epi, i
   if (wide) return launch_gemm_wo(a, w, ep, epi, M, N, K, (cudaStream_t)stream);
   // prompt-sized batches run on CTA pairs; stream-K keeps the shapes where cutting K is faster, the weight-only kind, whose tiles are widened
   // on the way, and calls that cap its CTAs
-  if (const int bt = !p.decode && !wo && split_k == 0 ? pair_tokens(M, N, K, ab_dtype) : 0)
-    return launch_gemm_pair(a, w, ep, epi, M, N, K, ab_dtype, bt, (cudaStream_t)stream);
+  if (const PairPlan plan = !p.decode && !wo && split_k == 0 ? pair_plan(M, N, K, ab_dtype) : PairPlan{0, 0}; plan.bt)
+    return launch_gemm_pair(a, w, ep, epi, M, N, K, ab_dtype, plan, (cudaStream_t)stream);
   CUtensorMapDataType dt = eb == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
   int bk = GEMM_BK_BYTES / eb;
   CUtensorMap wm, am;
