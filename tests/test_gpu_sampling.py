@@ -52,6 +52,21 @@ def test_topk_candidates_at_the_ends_of_its_paths(ops, v):
     assert np.array_equal(val.cpu().numpy(), wv) and np.array_equal(idx.cpu().numpy(), wi)
 
 
+@pytest.mark.parametrize("b,v,pitch", [(5, 16383, 16383), (5, 16384, 16384), (5, 16387, 16387), (3, 40001, 40004), (80, 16390, 16392), (160, 16384, 16384)])
+def test_topk_candidates_of_rows_cut_by_clusters(ops, b, v, pitch):
+    """Eight, four and two CTAs a row, rows that do not start on 16 bytes; kinds of rows as above, and one whose values differ in their last bits only."""
+    x = torch.zeros(b, pitch)
+    x[:, :v] = _logits(b, v, v)
+    x[1, :v] = x[1, :v].sort().values
+    x[2, :v] = x[2, 0] * (1 + torch.arange(v) % 7 * 2.0**-23)
+    if b > 4:
+        x[3, torch.randperm(v, generator=torch.Generator().manual_seed(v))[40:]] = -float("inf")
+        x[4, :v:13] = x[4, :v].max()
+    val, idx = ops.topk_candidates(x.cuda()[:, :v])
+    wv, wi = S.topk_candidates_ref(x[:, :v].contiguous().numpy())
+    assert np.array_equal(val.cpu().numpy(), wv) and np.array_equal(idx.cpu().numpy(), wi)
+
+
 def test_constant_row_keeps_the_lowest_indices(ops):
     x = torch.zeros(2, 5000)
     val, idx = ops.topk_candidates(x.cuda())

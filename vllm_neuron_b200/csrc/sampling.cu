@@ -3,9 +3,12 @@
 // temperature 0 => top_k 1).  Two kernels:
 //   topk_candidates_kernel : one CTA per row; the 256 largest fp32 logits of the (local) vocab shard, exactly,
 //                            sorted by (value desc, index asc); ties broken towards the LOWER index like argmax_kernel.
+//   topk_cluster_kernel    : the same for long rows, eight CTAs a row.
 //   sample_candidates_kernel: merges the candidate lists of all TP shards of a row, applies top-k / temperature / top-p and
 //                            draws with the caller's uniform u[row] by inverse CDF (fp32, sequential, fixed order).
 // Both are HBM/L2-bound integer+compare work (the logits row was just written by the lm_head GEMM); no tensor cores.
+#include <limits.h>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -13,9 +16,11 @@ namespace b200 {
 constexpr int SAMPLE_K = 256;        // candidates per (row, shard): the reference's _MAX_NEURON_SAMPLING_TOP_K (RUNNER:74)
 constexpr int TOPK_THREADS = 1024;
 constexpr int EQ_CAP = 1024;
-constexpr int LIST_CAP = 4096;       // elements at or above the threshold that are sorted directly
 constexpr int LIST_ALL = 1024;       // rows of so few logits are sorted whole
-constexpr int LIST_MIN_V = 64000;    // rows from which a threshold and the few that reach it beat the radix select
+constexpr int CL_CTAS = 8;           // CTAs of a long row, at most
+constexpr int CL_GROUPS = 1024;      // disjoint groups of a long row whose maxima give the threshold
+constexpr int CL_CAP = 2048;         // elements at or above it that are sorted directly
+constexpr int CL_MIN_V = 16384;      // rows from which that beats the radix select (and 512 of the groups hold something)
 
 // monotone map fp32 -> uint32 (larger float <=> larger key); -0 < +0 is irrelevant here
 __device__ __forceinline__ uint32_t f2key(float x) {
@@ -53,95 +58,27 @@ __device__ __forceinline__ unsigned long long pack_cand(uint32_t key, uint32_t i
   return ((unsigned long long)key << 32) | (unsigned long long)(0xffffffffu - idx);
 }
 
-// LIST: with the two passes below (the list's shared memory is L1 that the radix select would keep the row in: 48000 logits 44 us without
-// it, 50 with)
-template <bool LIST>
-__global__ void __launch_bounds__(TOPK_THREADS)
-    topk_candidates_kernel(const float* __restrict__ logits, int64_t row_stride, float* __restrict__ cand_val,
-                           int64_t* __restrict__ cand_idx, int V, int64_t idx_offset) {
-  griddep_launch();
-  griddep_wait();
+// sorted composite keys -> this row's candidates
+__device__ __forceinline__ void write_candidates(const unsigned long long* __restrict__ keys, int K, float* __restrict__ cand_val,
+                                                 int64_t* __restrict__ cand_idx, int64_t idx_offset) {
+  for (int j = threadIdx.x; j < SAMPLE_K; j += blockDim.x) {
+    const unsigned long long c = keys[j];
+    const bool ok = j < K;
+    cand_val[j] = ok ? key2f((uint32_t)(c >> 32)) : -INFINITY;
+    cand_idx[j] = ok ? idx_offset + (int64_t)(0xffffffffu - (uint32_t)c) : -1;
+  }
+}
+
+// the row's candidates by radix select, TOPK_THREADS threads
+__device__ __noinline__ void topk_radix_row(const float* __restrict__ r, int V, float* __restrict__ cand_val, int64_t* __restrict__ cand_idx,
+                                            int64_t idx_offset) {
   __shared__ unsigned int hist[256];
   __shared__ unsigned long long cand[SAMPLE_K];
   __shared__ unsigned int eq_idx[EQ_CAP];
   __shared__ unsigned int s_prefix, s_need, s_cnt, s_eq_cnt, s_eq_total;
   __shared__ unsigned int warp_tot[TOPK_THREADS / 32];
-  const float* r = logits + (int64_t)blockIdx.x * row_stride;
   const int tid = threadIdx.x;
   const int K = V < SAMPLE_K ? V : SAMPLE_K;
-
-  // ---- two passes over the row: the least of 256 disjoint groups' maxima is a threshold that at least 256 elements reach (about 1400
-  // of a row in no particular order, whatever its length); they are listed and sorted.  Rows that put more than LIST_CAP elements there
-  // (long runs of ties, sorted rows, rows masked almost everywhere) go through the radix select below, and give the list up when it is
-  // full; so do rows in between: sorting 2048 or 4096 elements takes 25 or 47 us, whatever the length.  Radix select / list (us, 8 rows):
-  // 1000 logits 26 / 13, 2000 26 / 24, 4096 26 / 47, 32000 42 / 30 to 52, 50257 44 / 56, 65536 60 / 34 to 57, 128256 91 / 41 to 64.
-  if constexpr (LIST) {
-    __shared__ unsigned long long list[LIST_CAP];
-    __shared__ unsigned int group_min[TOPK_THREADS / 32];
-    const bool vec = (row_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
-    const int V4 = vec ? V / 4 : 0;
-    const float4* r4 = reinterpret_cast<const float4*>(r);
-    uint32_t thr = 0;
-    if (V > LIST_ALL) {
-      uint32_t mx = 0;
-#pragma unroll 4
-      for (int i = tid; i < V4; i += TOPK_THREADS) {
-        const float4 x = r4[i];
-        mx = max(max(max(f2key(x.x), f2key(x.y)), max(f2key(x.z), f2key(x.w))), mx);
-      }
-      for (int i = 4 * V4 + tid; i < V; i += TOPK_THREADS) mx = max(mx, f2key(r[i]));
-      mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));  // four threads make a group
-      mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-      mx = __reduce_min_sync(0xffffffffu, mx);
-      if ((tid & 31) == 0) group_min[tid >> 5] = mx;
-    }
-    if (tid == 0) s_cnt = 0;
-    __syncthreads();
-    if (V > LIST_ALL) thr = __reduce_min_sync(0xffffffffu, group_min[tid & 31]);
-    auto take = [&](float x, int i) {
-      const uint32_t k = f2key(x);
-      if (k >= thr) {
-        const unsigned at = atomicAdd(&s_cnt, 1u);
-        if (at < LIST_CAP) list[at] = pack_cand(k, (uint32_t)i);
-      }
-    };
-    auto take4 = [&](float4 x, int i) {
-      take(x.x, 4 * i);
-      take(x.y, 4 * i + 1);
-      take(x.z, 4 * i + 2);
-      take(x.w, 4 * i + 3);
-    };
-    int i4 = tid;
-    for (; i4 + 7 * TOPK_THREADS < V4 && *(volatile unsigned int*)&s_cnt <= LIST_CAP; i4 += 8 * TOPK_THREADS) {
-      float4 x[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] = r4[i4 + j * TOPK_THREADS];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) take4(x[j], i4 + j * TOPK_THREADS);
-    }
-    if (*(volatile unsigned int*)&s_cnt <= LIST_CAP) {
-#pragma unroll 4
-      for (; i4 < V4; i4 += TOPK_THREADS) take4(r4[i4], i4);
-    }
-    for (int i = 4 * V4 + tid; i < V; i += TOPK_THREADS) take(r[i], i);
-    __syncthreads();
-    const int cnt = (int)s_cnt;
-    if (cnt <= LIST_CAP) {
-      int n2 = SAMPLE_K;
-      while (n2 < cnt) n2 <<= 1;
-      for (int i = cnt + tid; i < n2; i += TOPK_THREADS) list[i] = 0ull;
-      __syncthreads();
-      bitonic_sort_desc(list, n2);
-      for (int j = tid; j < SAMPLE_K; j += TOPK_THREADS) {
-        const unsigned long long c = list[j];
-        const bool ok = j < K;
-        cand_val[(int64_t)blockIdx.x * SAMPLE_K + j] = ok ? key2f((uint32_t)(c >> 32)) : -INFINITY;
-        cand_idx[(int64_t)blockIdx.x * SAMPLE_K + j] = ok ? idx_offset + (int64_t)(0xffffffffu - (uint32_t)c) : -1;
-      }
-      return;
-    }
-  }
-
   // ---- radix select of the K-th largest key: 4 passes of 8 bits, most significant first
   if (tid == 0) {
     s_prefix = 0;
@@ -230,12 +167,131 @@ __global__ void __launch_bounds__(TOPK_THREADS)
   for (int j = K + tid; j < SAMPLE_K; j += TOPK_THREADS) cand[j] = 0ull;  // V < 256: pad (sorts last)
   __syncthreads();
   bitonic_sort_desc(cand, SAMPLE_K);
-  for (int j = tid; j < SAMPLE_K; j += TOPK_THREADS) {
-    const unsigned long long c = cand[j];
-    const bool ok = j < K;
-    cand_val[(int64_t)blockIdx.x * SAMPLE_K + j] = ok ? key2f((uint32_t)(c >> 32)) : -INFINITY;
-    cand_idx[(int64_t)blockIdx.x * SAMPLE_K + j] = ok ? idx_offset + (int64_t)(0xffffffffu - (uint32_t)c) : -1;
+  write_candidates(cand, K, cand_val, cand_idx, idx_offset);
+}
+
+__global__ void __launch_bounds__(TOPK_THREADS)
+    topk_candidates_kernel(const float* __restrict__ logits, int64_t row_stride, float* __restrict__ cand_val,
+                           int64_t* __restrict__ cand_idx, int V, int64_t idx_offset) {
+  griddep_launch();
+  griddep_wait();
+  const float* r = logits + (int64_t)blockIdx.x * row_stride;
+  cand_val += (int64_t)blockIdx.x * SAMPLE_K;
+  cand_idx += (int64_t)blockIdx.x * SAMPLE_K;
+  if (V > LIST_ALL) {
+    topk_radix_row(r, V, cand_val, cand_idx, idx_offset);
+    return;
   }
+  __shared__ unsigned long long list[LIST_ALL];
+  int n2 = SAMPLE_K;
+  while (n2 < V) n2 <<= 1;
+  for (int i = threadIdx.x; i < n2; i += TOPK_THREADS) list[i] = i < V ? pack_cand(f2key(r[i]), (uint32_t)i) : 0ull;
+  __syncthreads();
+  bitonic_sort_desc(list, n2);
+  write_candidates(list, V < SAMPLE_K ? V : SAMPLE_K, cand_val, cand_idx, idx_offset);
+}
+
+// bitonic_sort_desc of n <= TOPK_THREADS keys, one a thread: steps within a warp are shuffles, the others (10 of 45 at n = 512) one barrier
+// each, by turns through the two halves of buf [2 n]; the sorted keys end in buf[0 .. n)
+__device__ __forceinline__ void bitonic_sort_lanes(unsigned long long* buf, int n) {
+  const int tid = threadIdx.x;
+  unsigned long long a = tid < n ? buf[tid] : 0ull;
+  int turn = 1;
+  for (int k = 2; k <= n; k <<= 1) {
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      unsigned long long b;
+      if (j >= 32) {
+        unsigned long long* x = buf + (turn ? n : 0);
+        turn ^= 1;
+        if (tid < n) x[tid] = a;
+        __syncthreads();
+        b = tid < n ? x[tid ^ j] : 0ull;
+      } else {
+        b = __shfl_xor_sync(0xffffffffu, a, j);
+      }
+      const bool larger = ((tid & k) == 0) == ((tid & j) == 0);
+      a = (a > b) == larger ? a : b;
+    }
+  }
+  __syncthreads();
+  if (tid < n) buf[tid] = a;
+  __syncthreads();
+}
+
+// Long rows: a cluster of eight CTAs (fewer where rows are many: those of all rows are resident together) cuts a row.  The 256th largest of 1024 disjoint groups' maxima is a threshold that at least 256 elements reach
+// (about 300 of a row in no particular order, whatever its length; the groups are strided, so runs of large neighbours spread over them).
+// Every CTA finds it from all the maxima (a bit at a time, one barrier each), lists the elements of its slice that reach it with the first CTA,
+// and that one sorts them.  Rows that put more than CL_CAP elements there (long runs of ties, rows masked almost everywhere) go through the radix
+// select, as do shorter rows.  Bound by the latency of the steps: two passes over the slice (the second from L1), two cluster barriers, 32 counts,
+// the sort.  Measured (us with the events around it, one CTA a row / now): one row of 128256 70 / 20, 23 rows 70 / 27, 128 rows 72 / 36; 16384: 35 / 16, 35 / 23,
+// 37 / 25; 200 rows, two waves: 113 / 61.
+__global__ void __launch_bounds__(TOPK_THREADS)
+    topk_cluster_kernel(const float* __restrict__ logits, int64_t row_stride, float* __restrict__ cand_val, int64_t* __restrict__ cand_idx, int V,
+                        int64_t idx_offset) {
+  __shared__ uint32_t group_max[CL_GROUPS];
+  __shared__ unsigned long long list[CL_CAP];
+  __shared__ unsigned int s_cnt;
+  const int tid = threadIdx.x, rank = (int)cluster_ctarank(), ctas = (int)cluster_nctarank();  // a power of two
+  const int64_t row = blockIdx.x / ctas;
+  const float* r = logits + row * row_stride;
+  if (tid == 0) s_cnt = 0;
+  griddep_launch();
+  griddep_wait();
+  const bool vec = (row_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+  const int V4 = vec ? V / 4 : 0, lo4 = (int)((int64_t)V4 * rank / ctas), hi4 = (int)((int64_t)V4 * (rank + 1) / ctas);
+  const int rest = V - 4 * V4, lo = 4 * V4 + (int)((int64_t)rest * rank / ctas), hi = 4 * V4 + (int)((int64_t)rest * (rank + 1) / ctas);
+  const float4* r4 = reinterpret_cast<const float4*>(r);
+  uint32_t mx = 0;
+#pragma unroll 4
+  for (int i = lo4 + tid; i < hi4; i += TOPK_THREADS) {
+    const float4 x = r4[i];
+    mx = max(max(max(f2key(x.x), f2key(x.y)), max(f2key(x.z), f2key(x.w))), mx);
+  }
+  for (int i = lo + tid; i < hi; i += TOPK_THREADS) mx = max(mx, f2key(r[i]));
+  for (int o = 1; o < ctas; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));  // as many threads as CTAs make a group ...
+  // ... and each of them tells one CTA
+  st_cluster_f32(mapa_shared(smem_u32(&group_max[(rank * TOPK_THREADS + tid) / ctas]), tid & (ctas - 1)), __uint_as_float(mx));
+  cluster_sync_all();  // the maxima are everywhere, the first CTA's count is 0
+  const uint32_t mine = group_max[tid];
+  uint32_t thr = 0;
+  for (int b = 31; b >= 8; --b) {  // to 15 bits of mantissa: a few more elements for a quarter of the barriers
+    const uint32_t t = thr | (1u << b);
+    if (__syncthreads_count(mine >= t) >= SAMPLE_K) thr = t;
+  }
+  const uint32_t cnt0 = mapa_shared(smem_u32(&s_cnt), 0), list0 = mapa_shared(smem_u32(list), 0);
+  auto take = [&](float x, int i) {
+    const uint32_t k = f2key(x);
+    if (k >= thr) {
+      uint32_t at;
+      asm volatile("atom.shared::cluster.add.u32 %0, [%1], 1;\n" : "=r"(at) : "r"(cnt0) : "memory");
+      if (at < CL_CAP) asm volatile("st.shared::cluster.u64 [%0], %1;\n" ::"r"(list0 + 8 * at), "l"(pack_cand(k, (uint32_t)i)) : "memory");
+    }
+  };
+#pragma unroll 4
+  for (int i = lo4 + tid; i < hi4; i += TOPK_THREADS) {
+    const float4 x = r4[i];
+    take(x.x, 4 * i);
+    take(x.y, 4 * i + 1);
+    take(x.z, 4 * i + 2);
+    take(x.w, 4 * i + 3);
+  }
+  for (int i = lo + tid; i < hi; i += TOPK_THREADS) take(r[i], i);
+  cluster_sync_all();  // the list is whole; nobody reaches into another CTA from here on
+  if (rank != 0) return;
+  cand_val += row * SAMPLE_K;
+  cand_idx += row * SAMPLE_K;
+  const int cnt = (int)s_cnt;
+  if (cnt > CL_CAP) {
+    topk_radix_row(r, V, cand_val, cand_idx, idx_offset);
+    return;
+  }
+  int n2 = SAMPLE_K;
+  while (n2 < cnt) n2 <<= 1;
+  for (int i = cnt + tid; i < n2; i += TOPK_THREADS) list[i] = 0ull;
+  __syncthreads();
+  if (n2 <= TOPK_THREADS) bitonic_sort_lanes(list, n2);
+  else bitonic_sort_desc(list, n2);
+  write_candidates(list, SAMPLE_K, cand_val, cand_idx, idx_offset);
 }
 
 // cand_val / cand_idx: [groups][B][256] (one group per TP shard, each sorted descending; -inf / -1 padding).
@@ -439,9 +495,14 @@ int b200_topk_candidates(const float* logits, int64_t row_stride, float* cand_va
   B200_REQUIRE(logits && cand_val && cand_idx, "topk_candidates: null pointer");
   B200_REQUIRE(V > 0 && idx_offset >= 0 && idx_offset + V <= 0xffffffffll, "topk_candidates: bad V / idx_offset");
   if (B <= 0) return B200_OK;
-  const bool list = V <= LIST_ALL || V >= LIST_MIN_V;
-  B200_CUDA_OK(launch_kernel(list ? topk_candidates_kernel<true> : topk_candidates_kernel<false>, dim3(B), dim3(TOPK_THREADS), 0,
-                             (cudaStream_t)stream, logits, row_stride, cand_val, cand_idx, V, idx_offset));
+  int ctas = CL_CTAS;  // two CTAs fit an SM: a wave, where rows are not too many for it
+  while (ctas > 2 && (int64_t)B * ctas > 2 * sm_count()) ctas /= 2;
+  if (V >= CL_MIN_V && B <= INT_MAX / ctas)
+    B200_CUDA_OK(launch_kernel_cluster(topk_cluster_kernel, dim3(B * ctas), dim3(TOPK_THREADS), 0, ctas, (cudaStream_t)stream, logits, row_stride,
+                                       cand_val, cand_idx, V, idx_offset));
+  else
+    B200_CUDA_OK(launch_kernel(topk_candidates_kernel, dim3(B), dim3(TOPK_THREADS), 0, (cudaStream_t)stream, logits, row_stride, cand_val, cand_idx,
+                               V, idx_offset));
   return B200_OK;
 }
 
