@@ -45,6 +45,23 @@ def test_rmsnorm_quant(ops, kind):
     assert torch.equal(q.cpu().view(torch.uint8), qw.view(torch.uint8))
 
 
+@pytest.mark.parametrize("h", [64, 2048, 2056, 4096, 5120, 8192])
+@pytest.mark.parametrize("kind", [None, "fp8", "int8"])
+def test_rmsnorm_of_many_rows_has_the_bits_of_few(ops, h, kind):
+    """512 rows and more may take half the threads a row: the same bits as in calls of fewer rows, and near the reference."""
+    g = torch.Generator(device="cuda").manual_seed(h)
+    x = (torch.randn((513, h), generator=g, device="cuda") * 3).bfloat16()
+    w = (1 + 0.1 * torch.randn(h, generator=g, device="cuda")).bfloat16()
+    kw = {} if kind is None else {"quant": kind, "want_bf16": True}
+    many = ops.rmsnorm(x, w, 1e-5, **kw)
+    few = [ops.rmsnorm(x[a:b], w, 1e-5, **kw) for a, b in ((0, 300), (300, 513))]
+    if kind is None:
+        many, few = [many], [[f] for f in few]
+    for m, parts in zip(many, zip(*few)):
+        assert torch.equal(m.view(torch.uint8), torch.cat(parts).view(torch.uint8))
+    _ulp_close(many[-1][:64], kv_ref.rmsnorm_ref(x[:64].cpu(), w.cpu(), 1e-5), 0.99)
+
+
 @pytest.mark.parametrize("kind", ["fp8", "int8"])
 def test_quantize_per_token_bit_exact(ops, kind):
     g = torch.Generator().manual_seed(8)

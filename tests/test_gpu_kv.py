@@ -131,6 +131,11 @@ def test_rope_kv_write_bit_exact(ops, hq, hkv, d, t):
     assert torch.equal(device_to_logical_pool(vd).cpu().view(torch.int16), vp.view(torch.int16))
 
 
+@pytest.mark.parametrize("hq,hkv,d,t", [(104, 8, 128, 3), (33, 3, 64, 5), (6, 2, 96, 9), (3, 1, 16, 2)])
+def test_rope_kv_write_of_wide_rows_and_other_head_sizes(ops, hq, hkv, d, t):
+    test_rope_kv_write_bit_exact(ops, hq, hkv, d, t)
+
+
 def test_decode_meta_speculative_slots_match_golden(ops, golden_index):
     """num_spec = k: slot_mapping [B, k] = slots[0] + i, the reference's EAGLE / fused-speculation rows (model_runner.py:825-830)."""
     n = 0
