@@ -705,6 +705,25 @@ def test_short_prompt_rows_take_the_small_kernel(m, n, k, short):
     assert ((got.double() - want).abs() <= k * 2.0**-23 * (a.double().abs() @ w.double().abs().T)).all()
 
 
+@pytest.mark.parametrize("T,W,off", [(1, 4, 0), (5, 1028, 0), (2, 4100, 0), (700, 132, 0), (4, 30, 0), (3, 64, 1), (3, 64, 2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_embedding_and_tanh_norm_in_vectors(T, W, off, dtype):
+    """Rows of whole vectors, rows that are none (30), tables and inputs that start one or two elements behind a boundary; token ids outside the
+    vocabulary take its ends.  One rounding of the product; the norm two, of tanh's 2 ulp, plus the rounding to the output type."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(T * W + off)
+    table = torch.randn(11 * W + off, generator=g).to(dtype)[off:].view(11, W)
+    tokens = torch.randint(-2, 13, (T,), generator=g, dtype=torch.int32)
+    placed = torch.empty(11 * W + off, dtype=dtype, device=DEV)[off:].view(11, W).copy_(table)
+    want = table.float()[tokens.long().clamp(0, 10)] * 0.37
+    assert torch.equal(ops.embed_scale(tokens.to(DEV), placed, 0.37).cpu(), want)
+    x, w, b = torch.randn(T, W, generator=g), torch.randn(W, generator=g), torch.randn(W, generator=g)
+    xd = torch.empty(T * W + off, device=DEV)[off:].view(T, W).copy_(x)
+    got = ops.dyt_norm(xd, w.to(DEV), b.to(DEV), 1.1, dtype).double().cpu()
+    ref = torch.tanh(1.1 * x.double()) * w.double() + b.double()
+    assert ((got - ref).abs() <= 2.0**-21 * (w.abs() + b.abs()).double() + (2.0**-8 if dtype == torch.bfloat16 else 0.0) * ref.abs()).all()
+
+
 @pytest.mark.parametrize("T,W", [(1, 4), (3, 1028), (2, 4096), (5, 4100), (700, 132), (4, 30)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_row_kernels_in_vectors(T, W, dtype):

@@ -17,6 +17,22 @@ __global__ void embed_scale_kernel(const int32_t* __restrict__ tokens, const WT*
   for (int i = threadIdx.x; i < W; i += blockDim.x) out[(int64_t)t * W + i] = ldf(table, (int64_t)tok * W + i) * scale;
 }
 
+// four columns at a time (4096 x 2048 from bf16: 19.7 -> 9.9 us)
+template <typename WT>
+__global__ void embed_scale_vec_kernel(const int32_t* __restrict__ tokens, const WT* __restrict__ table, float* __restrict__ out, int W, int V,
+                                       float scale) {
+  griddep_launch();
+  griddep_wait();
+  const int t = blockIdx.x;
+  int tok = tokens[t];
+  tok = tok < 0 ? 0 : (tok >= V ? V - 1 : tok);
+#pragma unroll 2
+  for (int i = threadIdx.x * 4; i < W; i += blockDim.x * 4) {
+    const float4 v = ldf4(table, (int64_t)tok * W + i);
+    *reinterpret_cast<float4*>(out + (int64_t)t * W + i) = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+  }
+}
+
 template <typename OT>
 __global__ void dyt_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float alpha,
                            OT* __restrict__ out, int W, int64_t total) {
@@ -25,6 +41,23 @@ __global__ void dyt_kernel(const float* __restrict__ x, const float* __restrict_
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(i % W);
     stf(out, i, tanhf(alpha * x[i]) * w[c] + b[c]);
+  }
+}
+
+// the same, four columns a thread, which walks down the rows (4096 x 2048 to bf16: 24.0 -> 9.0 us)
+template <typename OT>
+__global__ void dyt_vec_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, float alpha,
+                               OT* __restrict__ out, int W, int T) {
+  griddep_launch();
+  griddep_wait();
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (c >= W) return;
+  const float4 u = ldf4(w, c), v = ldf4(b, c);
+#pragma unroll 2
+  for (int t = blockIdx.y; t < T; t += gridDim.y) {
+    const float4 r = ldf4(x, (int64_t)t * W + c);
+    stf4(out, (int64_t)t * W + c, make_float4(tanhf(alpha * r.x) * u.x + v.x, tanhf(alpha * r.y) * u.y + v.y, tanhf(alpha * r.z) * u.z + v.z,
+                                              tanhf(alpha * r.w) * u.w + v.w));
   }
 }
 
@@ -50,11 +83,14 @@ __global__ void dyt_residual_kernel(float* __restrict__ x, const float* __restri
 
 // The same four columns at a time: a thread keeps its columns' weights and walks down the rows, so that nothing is divided and every access
 // is a vector (4096 x 2048 with expert rows: 57 -> 29 us on average over a layer; one scalar and a 64-bit division per element before).
-template <typename OT>
-__global__ void dyt_residual_vec_kernel(float* __restrict__ x, const float* __restrict__ y, int nsum, const float* __restrict__ y2,
+// NS: nsum where it is known at compile time (0: any), so that two rows' loads go out together (4096 x 2048, one
+// row of y: 18.3 us, at its bytes).
+template <typename OT, int NS>
+__global__ void dyt_residual_vec_kernel(float* __restrict__ x, const float* __restrict__ y, int nsum_, const float* __restrict__ y2,
                                         const float* __restrict__ w1, const float* __restrict__ b1, float a1,
                                         const float* __restrict__ w2, const float* __restrict__ b2, float a2, OT* __restrict__ out2,
                                         int W, int T) {
+  const int nsum = NS ? NS : nsum_;
   griddep_launch();
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   griddep_wait();  // before the weights too: they may be what the kernel ahead has written
@@ -209,6 +245,12 @@ int b200_embed_scale(const int32_t* tokens, const void* table, int table_dtype, 
                      void* stream) {
   B200_REQUIRE(tokens && table && out, "embed_scale: null pointer");
   if (T <= 0) return B200_OK;
+  if (W % 4 == 0 && vec4_ok(table, table_dtype == B200_BF16 ? 2 : 4) && vec4_ok(out)) {
+    B200_DISPATCH_ELEM(table_dtype, WT,
+                       B200_CUDA_OK(launch_kernel(embed_scale_vec_kernel<WT>, dim3(T), dim3(vec_threads(W / 4)), 0, (cudaStream_t)stream, tokens,
+                                                  (const WT*)table, out, W, V, scale)));
+    return B200_OK;
+  }
   B200_DISPATCH_ELEM(table_dtype, WT,
                      B200_CUDA_OK(launch_kernel(embed_scale_kernel<WT>, dim3(T), dim3(256), 0, (cudaStream_t)stream, tokens,
                                                 (const WT*)table, out, W, V, scale)));
@@ -220,6 +262,13 @@ int b200_dyt_norm(const float* x, const float* w, const float* b, float alpha, v
   B200_REQUIRE(x && w && b && out, "dyt_norm: null pointer");
   if (T <= 0) return B200_OK;
   const int64_t total = (int64_t)T * W;
+  if (W % 4 == 0 && vec4_ok(x) && vec4_ok(w) && vec4_ok(b) && vec4_ok(out, out_dtype == B200_BF16 ? 2 : 4)) {
+    const int th = vec_threads(W / 4);
+    B200_DISPATCH_ELEM(out_dtype, OT,
+                       B200_CUDA_OK(launch_kernel(dyt_vec_kernel<OT>, vec_grid(W / 4, th, T), dim3(th), 0, (cudaStream_t)stream, x, w, b, alpha,
+                                                  (OT*)out, W, T)));
+    return B200_OK;
+  }
   B200_DISPATCH_ELEM(out_dtype, OT,
                      B200_CUDA_OK(launch_kernel(dyt_kernel<OT>, dim3(flat_grid(total, 256)), dim3(256), 0, (cudaStream_t)stream,
                                                 x, w, b, alpha, (OT*)out, W, total)));
@@ -236,7 +285,10 @@ int b200_dyt_residual(float* x, const float* y, int nsum, const float* y2, const
   if (W % 4 == 0 && vec4_ok(x) && vec4_ok(y) && vec4_ok(y2) && vec4_ok(w1) && vec4_ok(b1) && vec4_ok(w2) && vec4_ok(b2) && vec4_ok(out2, oes)) {
     const int th = vec_threads(W / 4);
     B200_DISPATCH_ELEM(out_dtype, OT,
-                       B200_CUDA_OK(launch_kernel(dyt_residual_vec_kernel<OT>, vec_grid(W / 4, th, T), dim3(th), 0, (cudaStream_t)stream, x,
+                       B200_CUDA_OK(launch_kernel(nsum == 1   ? dyt_residual_vec_kernel<OT, 1>
+                                                  : nsum == 2 ? dyt_residual_vec_kernel<OT, 2>
+                                                              : dyt_residual_vec_kernel<OT, 0>,
+                                                  vec_grid(W / 4, th, T), dim3(th), 0, (cudaStream_t)stream, x,
                                                   y, nsum, y2, w1, b1, alpha1, w2, b2, alpha2, (OT*)out2, W, T)));
     return B200_OK;
   }

@@ -64,6 +64,10 @@ __device__ __forceinline__ void stf4<__nv_bfloat16>(__nv_bfloat16* p, int64_t i,
   *reinterpret_cast<uint2*>(p + i) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
 }
 __device__ __forceinline__ float4 ldf4(const float* p, int64_t i) { return *reinterpret_cast<const float4*>(p + i); }
+__device__ __forceinline__ float4 ldf4(const __nv_bfloat16* p, int64_t i) {
+  const uint2 v = *reinterpret_cast<const uint2*>(p + i);
+  return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+}
 // whether rows of these tensors (pitches and offsets in elements, multiples of 4) are whole aligned vectors of four
 inline bool vec4_ok(const void* p, int elem_bytes = 4) { return ((uintptr_t)p & (4 * elem_bytes - 1)) == 0; }
 
