@@ -601,6 +601,10 @@ int b200_latent_q_prep(const float* q, int ldq, int H, int D, int R, int rot_n, 
 int b200_latent_attn_decode(const float* q, int ldq, const void* pool, const int32_t* block_table, int64_t bt_stride,
                             const int32_t* tok_row, const int32_t* tok_pos, const float* sink, float scale, int window, void* out,
                             int T, int H, int D, int Dv, int block_size, void* stream);
+/* the same, a token's keys shared by `splits` CTAs (1, 2, 4 or 8) */
+int b200_latent_attn_decode_split(const float* q, int ldq, const void* pool, const int32_t* block_table, int64_t bt_stride,
+                                  const int32_t* tok_row, const int32_t* tok_pos, const float* sink, float scale, int window, void* out,
+                                  int T, int H, int D, int Dv, int block_size, int splits, void* stream);
 
 /* ---------------------------------------------------------------- hyper-connections
  * The residual stream of a token is S copies (x fp32 [T][S][W], S <= 32).  hyper_embed: every copy = table[token];

@@ -402,3 +402,38 @@ def test_batched_per_head_linear_with_sigmoid_gate():
         typed = torch.zeros((T, B * N), dtype=dtype, device=DEV)
         ops.batched_linear(a.to(DEV), w.to(DEV), typed, a_batch_stride=K, out_batch_stride=N, gate=gate.to(DEV)[:, 2:])
         _close(typed.view(T, B, N), want * torch.sigmoid(gate[:, 2:].double())[:, :, None], max(tol, 1e-2 if dtype == torch.bfloat16 else 0))
+
+
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
+@pytest.mark.parametrize("H,C,R,window,sinks", [(16, 256, 64, 1 << 30, False), (20, 128, 32, 1 << 30, True), (5, 64, 16, 300, True)])
+def test_attention_over_cached_latents_shared_by_a_cluster(H, C, R, window, sinks, splits):
+    """One token each at 1 to 1100 keys, so that CTAs of a cluster get several rounds of tiles, one, a part of a tile or no key at all.  Bound: the weights and
+    the output are rounded to bf16."""
+    from vllm_neuron_b200 import _cabi
+
+    g = torch.Generator().manual_seed(H + splits)
+    n = [1, 31, 33, 256, 257, 700, 1100]
+    D, T = C + R, len(n)
+    bt, at = torch.zeros(T, 35, dtype=torch.int32), 1
+    for i, c in enumerate(n):
+        k = -(-c // 32)
+        bt[i, :k] = torch.arange(at, at + k)
+        at += k
+    pool = torch.randn(at, 32, D, generator=g).bfloat16()
+    q, sink = torch.randn(T, H, D, generator=g), torch.randn(H, generator=g) + 3
+    scale = D ** -0.5
+    out = torch.empty(T, H, C, dtype=torch.bfloat16, device=DEV)
+    d = lambda x: x.to(DEV)  # noqa: E731
+    qd, pd, btd, rows, pos, sd = d(q), d(pool), d(bt), d(torch.arange(T, dtype=torch.int32)), d(torch.tensor(n, dtype=torch.int32) - 1), d(sink)
+    rc = _cabi.load().b200_latent_attn_decode_split(qd.data_ptr(), H * D, pd.data_ptr(), btd.data_ptr(), bt.shape[1], rows.data_ptr(), pos.data_ptr(),
+                                                    sd.data_ptr() if sinks else None, scale, window, out.data_ptr(), T, H, D, C, 32, splits,
+                                                    _ops()._stream())
+    assert rc == 0
+    for i, c in enumerate(n):
+        keys = pool[bt[i, :-(-c // 32)].long()].view(-1, D)[max(0, c - window):c].double()
+        z = q[i].bfloat16().double() @ keys.T * scale
+        if sinks:
+            z = torch.cat([z, sink.double()[:, None]], 1)
+        w = torch.softmax(z, 1)[:, :keys.shape[0]]
+        want, size = w @ keys[:, :C], w @ keys[:, :C].abs()
+        assert ((out[i].double().cpu() - want).abs() <= 2.0**-8 * want.abs() + 2.0**-8 * size + 1e-6).all()

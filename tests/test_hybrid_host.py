@@ -193,3 +193,10 @@ def test_delta_rule_rounds_where_a_chain_is_long_or_the_chip_is_free():
     assert _delta_rounds(4096, 4096, 16, 128, 128) and _delta_rounds(300, 331, 8, 64, 64) and _delta_rounds(17, 4 * 17, 8, 64, 64)
     assert not _delta_rounds(17, 20 * 17, 8, 64, 64) and not _delta_rounds(130, 32 * 130, 8, 64, 64) and _delta_rounds(300, 6000, 8, 64, 64)
     assert not _delta_rounds(17, 20 * 17, 8, 128, 128) and _delta_rounds(40, 64 * 40, 8, 128, 128) and _delta_rounds(8, 64 * 8, 8, 128, 128)
+
+
+def test_latent_splits_while_there_are_keys_to_share_and_clusters_fit():
+    from vllm_neuron_b200.ops import _latent_splits
+
+    assert [_latent_splits(1, 16, k) for k in (200, 257, 600, 1025)] == [1, 2, 4, 8]
+    assert [_latent_splits(t, 16, 4000) for t in (9, 16, 30, 37, 68, 100)] == [8, 4, 4, 2, 2, 1] and _latent_splits(15, 40, 4000) == 2

@@ -15,7 +15,10 @@
 //     take the visible keys in tiles of 32 round-robin (each warp gathers its tile into its own shared-memory buffer with
 //     cp.async, S = Q K^T and O += P V on mma.sync m16n8k16 with the values read from the leading columns of the same
 //     tile, fp32 online softmax per warp) and merge through shared memory.  With a window the walk starts at its first key; a sink
-//     starts every warp's maximum and, in warp 0 alone, the denominator.
+//     starts every warp's maximum and, in the first warp alone, the denominator.  Few tokens leave most SMs idle (a CTA takes one whole), and a
+//     warp then walks its tiles one after the other, copy and products: so a token's keys may be shared by the CTAs of a cluster, whose
+//     merged parts meet through distributed shared memory (29 tokens at 1800, 16 heads over rows
+//     of 320: 80 -> 45 us, one at 2000 84 -> 35).
 #include <math.h>
 
 #include "hybrid_common.cuh"
@@ -104,7 +107,9 @@ __global__ void __launch_bounds__(256)
   __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(la_sm);                       // [16][ldk]
   __nv_bfloat16* Kt = Qs + 16 * ldk + (size_t)warp * LD_KEYS * ldk;                   // this warp's [32][ldk]
   float* ml = reinterpret_cast<float*>(Qs + 16 * ldk + (size_t)nw * LD_KEYS * ldk);   // [nw][16][2]
-  const int t = blockIdx.x, h0 = blockIdx.y * 16;
+  const int S = (int)cluster_nctarank(), rank = (int)cluster_ctarank();
+  float* part = ml + nw * 32;  // S > 1: this CTA's O [16][Dv], then its maxima and denominators [16][2]
+  const int t = blockIdx.x / S, h0 = blockIdx.y * 16;
   const int pos = tok_pos[t];
   const int32_t* bt = block_table + (int64_t)tok_row[t] * bt_stride;
   for (int i = threadIdx.x; i < 16 * (D / 2); i += blockDim.x) {
@@ -117,7 +122,7 @@ __global__ void __launch_bounds__(256)
   const int r_lo = lane >> 2;
   const int lo = pos - window + 1 > 0 ? pos - window + 1 : 0;  // the first visible key
   float m_lo = sink && h0 + r_lo < H ? sink[h0 + r_lo] : -INFINITY, m_hi = sink && h0 + r_lo + 8 < H ? sink[h0 + r_lo + 8] : -INFINITY;
-  const bool count_sink = sink && warp == 0 && (lane & 3) == 0;  // the sink's 1 in the denominator, once per row
+  const bool count_sink = sink && warp == 0 && rank == 0 && (lane & 3) == 0;  // the sink's 1 in the denominator, once per row
   float l_lo = count_sink && h0 + r_lo < H ? 1.0f : 0.f, l_hi = count_sink && h0 + r_lo + 8 < H ? 1.0f : 0.f;
   float o[2 * DV16M][4];
 #pragma unroll
@@ -125,7 +130,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int c = 0; c < 4; ++c) o[j][c] = 0.f;
   const int kch = D / 8;  // 16-byte chunks per cache row
-  for (int j0 = lo + LD_KEYS * warp; j0 <= pos; j0 += LD_KEYS * nw) {
+  for (int j0 = lo + LD_KEYS * (warp + nw * rank); j0 <= pos; j0 += LD_KEYS * nw * S) {
     // ---- this warp's 32 cache rows -> its buffer (rows past the token's position are zeros)
     const int jm = j0 + lane;
     const int64_t myrow = jm <= pos ? (int64_t)bt[jm / bs] * bs + (jm % bs) : -1;
@@ -244,12 +249,46 @@ __global__ void __launch_bounds__(256)
     for (int w = 0; w < nw; ++w) mt = fmaxf(mt, ml[(w * 16 + r) * 2]);
     float lt = 0.f, v = 0.f;
     for (int w = 0; w < nw; ++w) {
-      const float f = __expf(ml[(w * 16 + r) * 2] - mt);  // a warp without keys holds O = 0, m = -inf or the sink, l = 0 (1: the sink)
+      const float f = mt > -INFINITY ? __expf(ml[(w * 16 + r) * 2] - mt) : 0.f;  // a warp without keys holds O = 0, m = -inf or the sink, l = 0 (1: the sink)
       lt += ml[(w * 16 + r) * 2 + 1] * f;
       v += O0[w * wstride + r * Dv + d] * f;
     }
+    if (S > 1) {
+      part[r * Dv + d] = v;
+      if (d == 0) part[16 * Dv + 2 * r] = mt, part[16 * Dv + 2 * r + 1] = lt;
+    } else {
+      out[((int64_t)t * H + h0 + r) * Dv + d] = __float2bfloat16_rn(v / lt);
+    }
+  }
+  if (S == 1) return;
+  cluster_sync_all();  // every CTA's part is there
+  const uint32_t mine = smem_u32(part);
+  auto peer = [&](int q, int i) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(mapa_shared(mine, (uint32_t)q) + 4u * (uint32_t)i) : "memory");
+    return v;
+  };
+  for (int i = rank * blockDim.x + threadIdx.x; i < 16 * Dv; i += S * blockDim.x) {
+    const int r = i / Dv, d = i - r * Dv;
+    if (h0 + r >= H) continue;
+    float m[8], l[8], o[8], mt = -INFINITY;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < S) {
+        m[q] = peer(q, 16 * Dv + 2 * r), l[q] = peer(q, 16 * Dv + 2 * r + 1), o[q] = peer(q, i);
+        mt = fmaxf(mt, m[q]);
+      }
+    float lt = 0.f, v = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < S) {
+        const float f = __expf(m[q] - mt);
+        lt += l[q] * f;
+        v += o[q] * f;
+      }
     out[((int64_t)t * H + h0 + r) * Dv + d] = __float2bfloat16_rn(v / lt);
   }
+  cluster_sync_all();  // nobody leaves while another reads its part
 }
 
 }  // namespace b200
@@ -283,35 +322,50 @@ int b200_latent_q_prep(const float* q, int ldq, int H, int D, int R, int rot_n, 
   return B200_OK;
 }
 
-int b200_latent_attn_decode(const float* q, int ldq, const void* pool, const int32_t* block_table, int64_t bt_stride,
+static int latent_attn_decode(const float* q, int ldq, const void* pool, const int32_t* block_table, int64_t bt_stride,
                             const int32_t* tok_row, const int32_t* tok_pos, const float* sink, float scale, int window, void* out,
-                            int T, int H, int D, int Dv, int block_size, void* stream) {
+                            int T, int H, int D, int Dv, int block_size, int splits, void* stream) {
   B200_REQUIRE(q && pool && block_table && tok_row && tok_pos && out, "latent_attn_decode: null pointer");
   B200_REQUIRE(window >= 1, "latent_attn_decode: window %d", window);
+  B200_REQUIRE(splits == 1 || splits == 2 || splits == 4 || splits == 8, "latent_attn_decode: %d splits", splits);
   if (D % 16 || Dv % 16 || Dv > 256 || Dv > D || D > 1024 || (ldq & 1) || ((uintptr_t)q & 7) || H < 1) {
     set_last_error("latent_attn_decode: row width %d / value width %d need multiples of 16 (values <= 256)", D, Dv);
     return B200_ERR_UNSUPPORTED;
   }
   if (T <= 0) return B200_OK;
   int nw = 8;
-  auto bytes = [&](int w) { return (size_t)(16 + w * LD_KEYS) * (D + 8) * 2 + (size_t)w * 16 * 2 * 4; };
+  auto bytes = [&](int w) {
+    return (size_t)(16 + w * LD_KEYS) * (D + 8) * 2 + (size_t)w * 16 * 2 * 4 + (splits > 1 ? (size_t)(16 * Dv + 32) * 4 : 0);
+  };
   while (nw > 1 && bytes(nw) > 200 * 1024) nw >>= 1;
   const size_t smem = bytes(nw);
-  dim3 grid(T, (H + 15) / 16);
+  dim3 grid(T * splits, (H + 15) / 16);
   typedef __nv_bfloat16 BT;
 #define LAD_LAUNCH(M)                                                                                                          \
   do {                                                                                                                         \
     if (smem > 48 * 1024)                                                                                                      \
       B200_CUDA_OK(cudaFuncSetAttribute(latent_attn_decode_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    B200_CUDA_OK(launch_kernel(latent_attn_decode_kernel<M>, grid, dim3(nw * 32), smem, (cudaStream_t)stream, q, ldq,          \
-                               (const BT*)pool, block_table, bt_stride, tok_row, tok_pos, sink, scale, window, (BT*)out, H, D, \
-                               Dv, block_size));                                                                               \
+    B200_CUDA_OK(launch_kernel_cluster(latent_attn_decode_kernel<M>, grid, dim3(nw * 32), smem, splits, (cudaStream_t)stream, q, ldq,    \
+                                       (const BT*)pool, block_table, bt_stride, tok_row, tok_pos, sink, scale, window, (BT*)out, H, D, \
+                                       Dv, block_size));                                                                               \
   } while (0)
   if (Dv <= 64) LAD_LAUNCH(4);
   else if (Dv <= 128) LAD_LAUNCH(8);
   else LAD_LAUNCH(16);
 #undef LAD_LAUNCH
   return B200_OK;
+}
+
+int b200_latent_attn_decode(const float* q, int ldq, const void* pool, const int32_t* block_table, int64_t bt_stride,
+                            const int32_t* tok_row, const int32_t* tok_pos, const float* sink, float scale, int window, void* out,
+                            int T, int H, int D, int Dv, int block_size, void* stream) {
+  return latent_attn_decode(q, ldq, pool, block_table, bt_stride, tok_row, tok_pos, sink, scale, window, out, T, H, D, Dv, block_size, 1, stream);
+}
+
+int b200_latent_attn_decode_split(const float* q, int ldq, const void* pool, const int32_t* block_table, int64_t bt_stride,
+                                  const int32_t* tok_row, const int32_t* tok_pos, const float* sink, float scale, int window, void* out,
+                                  int T, int H, int D, int Dv, int block_size, int splits, void* stream) {
+  return latent_attn_decode(q, ldq, pool, block_table, bt_stride, tok_row, tok_pos, sink, scale, window, out, T, H, D, Dv, block_size, splits, stream);
 }
 
 }  // extern "C"

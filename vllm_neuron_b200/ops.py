@@ -839,6 +839,18 @@ def _prompt_mma(q, k_pool, meta, d, dv) -> bool:
             and d <= 512 and dv <= 256 and q.stride(0) % 2 == 0)
 
 
+def _latent_splits(tokens: int, heads: int, keys: int) -> int:
+    """CTAs that share a token's keys in latent attention: while there are rounds of tiles to share (8 warps of 32 keys) and the clusters of all tokens
+    and groups of 16 heads are resident together, a CTA an SM (clusters of 4 and 8 leave some free).  us, 16 heads over rows of 320, one CTA / two / four /
+    eight: one token at 2000 84 / 59 / 43 / 35, at 200 33 / 37 / 35 / 35; 16 tokens at 2000 84 / 59 / 43 / 66; 29 at 1800 80 / 59 / 45 / 66; 37 at 1500 70 / 53
+    / 72; 64 at 2000 84 / 62 / 84; 100 at 1000 55 / 84."""
+    ctas = tokens * -(-heads // 16)
+    n = 1
+    while n < 8 and 256 * n < keys and 2 * n * ctas <= {1: 136, 2: 120, 4: 72}[n]:
+        n *= 2
+    return n
+
+
 def _swa_part(q_src, num_heads, k_pool, v_pool, block_table, meta, sink, scale, window, latent_values, chunk, softcap, sigmoid_bias, out_f32,
               split_p, pool, pool_args, keep, out, g, bs, d, dv, v_pitch, v_div):
     """The sequences of `meta` (a step, or a StepPart of one) through the kernel that suits them.  Prompt kernels index the step's rows
@@ -877,10 +889,11 @@ def _swa_part(q_src, num_heads, k_pool, v_pool, block_table, meta, sink, scale, 
             and dv <= 256 and q_src.stride(0) % 2 == 0):
         # attention over cached latents, decode-sized steps: the heads of a token are the rows of a tensor-core tile
         with _k("latent_attn_decode"):
-            check(_lib().b200_latent_attn_decode(q_src, q_src.stride(0), k_pool, block_table,
-                                                       block_table.stride(0), meta.tok_row, meta.tok_pos, sink,
-                                                       float(scale), int(window), out, t, num_heads, d, dv, bs),
-                  "b200_latent_attn_decode")
+            splits = _latent_splits(t, num_heads, _span(getattr(meta, "max_end", 0) or 0, int(window), 0, 0, 0))
+            check(_lib().b200_latent_attn_decode_split(q_src, q_src.stride(0), k_pool, block_table,
+                                                             block_table.stride(0), meta.tok_row, meta.tok_pos, sink,
+                                                             float(scale), int(window), out, t, num_heads, d, dv, bs, splits),
+                  "b200_latent_attn_decode_split")
         return
     # decode-sized steps, fp32 pools and odd head sizes.  Long contexts at small batch: several CTAs share a (token, kv head)'s keys, so that
     # every SM has its CTAs
