@@ -437,3 +437,44 @@ def test_attention_over_cached_latents_shared_by_a_cluster(H, C, R, window, sink
         w = torch.softmax(z, 1)[:, :keys.shape[0]]
         want, size = w @ keys[:, :C], w @ keys[:, :C].abs()
         assert ((out[i].double().cpu() - want).abs() <= 2.0**-8 * want.abs() + 2.0**-8 * size + 1e-6).all()
+
+
+@pytest.mark.parametrize("window,sinks", [(1 << 30, False), (1 << 30, True), (100, True), (1, False)])
+@pytest.mark.parametrize("H,C,R", [(3, 256, 64), (2, 256, 16), (4, 128, 32), (1, 128, 0)])
+def test_prompt_portions_over_cached_latents_on_tensor_memory(H, C, R, window, sinks):
+    """Portions that end inside a tile, a page and a key step or on their borders, from position 0 or further on, a decoded token between them; rows of
+    the pages past a sequence's end hold NaN.  Bound: the weights and the output are rounded to bf16."""
+    ops, g = _ops(), torch.Generator().manual_seed(H)
+    ent = [(0, 0, 128), (1, 0, 1), (2, 31, 129), (3, 300, 17), (4, 64, 64), (5, 1, 300)]
+    D, T, at, rows, scale = C + R, sum(n for _, _, n in ent), 1, {}, (C + R) ** -0.5
+    for r, p, n in ent:
+        rows[r] = list(range(at, at + -(-(p + n) // 32)))
+        at += len(rows[r])
+    pool = torch.full((at, 1, 32, D), float("nan"), dtype=torch.bfloat16)
+    pool[0] = 0
+    for r, p, n in ent:
+        flat = pool[rows[r]].view(-1, D)
+        flat[:p + n] = torch.randn(p + n, D, generator=g).bfloat16()
+        pool[rows[r]] = flat.view(-1, 1, 32, D)
+    bt = torch.zeros(len(ent), max(map(len, rows.values())), dtype=torch.int32)
+    for r in rows:
+        bt[r, :len(rows[r])] = torch.tensor(rows[r])
+    q, sink = torch.randn(T, H, D, generator=g), torch.randn(H, generator=g) + 3
+    m, out = _meta(ent, rows, 32), torch.empty(T, H, C, dtype=torch.bfloat16, device=DEV)
+    qd, pd, bd, sd = q.view(T, -1).to(DEV), pool.to(DEV), bt.to(DEV), sink.to(DEV) if sinks else None
+    lib = ops._lib()
+    assert lib.b200_latent_attn_prefill_tc_supported(D, C, 32)
+    ops.check(lib.b200_latent_attn_prefill_tc(qd, H * D, pd, at, bd, bd.stride(0), m.seq_start, m.seq_slot, m.seq_pos0, len(ent), m.max_new, sd, scale,
+                                              window, out, H, D, C, 32), "b200_latent_attn_prefill_tc")
+    t = 0
+    for r, p, n in ent:
+        keys = pool[rows[r]].view(-1, D)[:p + n].double()
+        z = torch.einsum("thd,kd->htk", q[t:t + n].bfloat16().double(), keys) * scale
+        i, j = torch.arange(p, p + n)[:, None], torch.arange(p + n)[None]
+        z = z.masked_fill((j > i) | (j <= i - window), float("-inf"))
+        if sinks:
+            z = torch.cat([z, sink.double()[:, None, None].expand(H, n, 1)], 2)
+        w = torch.softmax(z, 2)[:, :, :p + n]
+        want, size = torch.einsum("htk,kc->thc", w, keys[:, :C]), torch.einsum("htk,kc->thc", w, keys[:, :C].abs())
+        assert ((out[t:t + n].double().cpu() - want).abs() <= 2.0**-8 * want.abs() + 2.0**-8 * size + 1e-6).all()
+        t += n

@@ -134,6 +134,8 @@ SIGNATURES = {
     "b200_latent_q_prep": (_i, [_p, _i, _i, _i, _i, _i, _i, _p, _p, _p, _p, _i, _p, _i, _p]),
     "b200_latent_attn_decode": (_i, [_p, _i, _p, _p, _i64, _p, _p, _p, _f, _i, _p, _i, _i, _i, _i, _i, _p]),
     "b200_latent_attn_decode_split": (_i, [_p, _i, _p, _p, _i64, _p, _p, _p, _f, _i, _p, _i, _i, _i, _i, _i, _i, _p]),
+    "b200_latent_attn_prefill_tc": (_i, [_p, _i, _p, _i, _p, _i64, _p, _p, _p, _i, _i, _p, _f, _i, _p, _i, _i, _i, _i, _p]),
+    "b200_latent_attn_prefill_tc_supported": (_i, [_i, _i, _i]),
     # hyper-connections: several copies of the residual stream mixed around every sublayer
     "b200_hyper_embed": (_i, [_p, _p, _i, _p, _i, _p, _p, _f, _p, _i, _i, _i, _p]),
     "b200_hyper_residual": (_i, [_p, _i, _p, _i, _p, _i, _p, _p, _p, _p, _p, _f, _i, _p, _i, _i, _i, _p]),

@@ -14,7 +14,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200_paged.so")
 SOURCES = ["host.cu", "kv_ops.cu", "paged_attn.cu", "paged_attn_prefill_tc.cu", "gemm_tcgen05.cu", "gemm_pair.cu", "gemm_group.cu", "gemm_wo.cu", "gemm_small.cu", "tp_allreduce.cu", "sampling.cu",
            "dyt_norm.cu", "ssm_scan.cu", "ssm_segment.cu", "swa_attn.cu", "swa_attn_prefill.cu", "swa_attn_prefill_tc.cu", "moe.cu", "rms_norm.cu", "delta_rule.cu",
-           "latent_attn.cu", "gated_scan.cu", "selective_scan.cu", "hyper_conn.cu"]
+           "latent_attn.cu", "latent_attn_prefill_tc.cu", "gated_scan.cu", "selective_scan.cu", "hyper_conn.cu"]
 HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "gemm_common.cuh"), os.path.join(CSRC, "gemm_pair.cuh"), os.path.join(CSRC, "gemm_group.cuh"), os.path.join(CSRC, "gemm_small.cuh"), os.path.join(CSRC, "hybrid_common.cuh"), os.path.join(CSRC, "ssm_common.cuh"), os.path.join(os.path.dirname(HERE), "include", "b200_paged.h")]
 # the library's functions on torch tensors, for ops.py: good for the Python in its name and the torch that its attribute `torch` names
 BIND = os.path.join(HERE, "_b200_bind" + sysconfig.get_config_var("EXT_SUFFIX"))

@@ -132,7 +132,7 @@ PyMethodDef methods[] = {
     FN(b200_gated_scan_prep), FN(b200_gather_logprobs), FN(b200_gemm), FN(b200_gemm_rope_kv_write), FN(b200_gemm_silu_mul),
     FN(b200_gemm_silu_mul_quant), FN(b200_gemm_workspace_bytes), FN(b200_glu), FN(b200_grouped_linear), FN(b200_head_rmsnorm_gate),
     FN(b200_hyper_embed), FN(b200_hyper_residual), FN(b200_kv_pool_mean), FN(b200_kv_write), FN(b200_kv_write_vmix),
-    FN(b200_latent_attn_decode), FN(b200_latent_attn_decode_split), FN(b200_latent_kv_write), FN(b200_latent_q_prep), FN(b200_matrix_memory_gates), FN(b200_matrix_memory_out),
+    FN(b200_latent_attn_decode), FN(b200_latent_attn_decode_split), FN(b200_latent_attn_prefill_tc), FN(b200_latent_attn_prefill_tc_supported), FN(b200_latent_kv_write), FN(b200_latent_q_prep), FN(b200_matrix_memory_gates), FN(b200_matrix_memory_out),
     FN(b200_matrix_memory_scan), FN(b200_moe_align), FN(b200_moe_gather_scale), FN(b200_moe_tile_rows), FN(b200_moe_topk),
     FN(b200_moe_topk_grouped), FN(b200_paged_attn_decode), FN(b200_paged_attn_decode_workspace_bytes), FN(b200_paged_attn_prefill),
     FN(b200_poly_norm), FN(b200_postln_residual), FN(b200_qk_norm_rope_kv_write), FN(b200_quantize_per_token), FN(b200_remask_spec_output),

@@ -314,7 +314,7 @@ def _kenetar_floors(name, t, keys_per_query, kv_tokens, nseq):
     att = (2.0 * t * la["heads"] * keys_per_query * (row + la["kv_rank"]),
            2.0 * kv_tokens * row + t * la["heads"] * (4 * row + 2 * la["kv_rank"]))
     return {
-        "swa_sink_attn_prefill[latent]": att, "swa_sink_attn[latent]": att, "latent_attn_decode": att,
+        "swa_sink_attn_prefill[latent]": att, "swa_sink_attn_prefill_tc[latent]": att, "swa_sink_attn[latent]": att, "latent_attn_decode": att,
         "delta_scan": (8.0 * t * d["heads"] * d["dim"] * d["vdim"],
                        t * (4 * c + 4 * hp) + 8.0 * nseq * d["heads"] * d["dim"] * d["vdim"]),
         "delta_prep": (0.0, t * 16.0 * d["kv_heads"] * d["dim"]),

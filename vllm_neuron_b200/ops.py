@@ -752,9 +752,10 @@ def _split_pays(parts, num_heads: int, g: int, d: int, dv: int, latent: bool, tc
     64 at 300 67 / 110, 29 at 300 72 / 66; 8 heads over 8 of 64, 64 at 1800 49 / 109; 200 tokens beside 64 at 1800 39 / 70 (mma.sync kernel 49 / 52).
     Over 4032 such steps the rule's choice costs 1.1 % more than the better one on average (mma.sync 0.7), always apart 19 (10), always together 38 (64);
     with the decode kernel's time as it was before its tiles lay on pages 6.0 (4.8).
-    Over latents (29 tokens at 1800 366 / 695, 2 356 / 360, 29 at 300 317 / 298) and other pages: 14 us a launch, a fifth, and that time."""
-    us, rows, heads, slots = (0.026, 128, g * -(-num_heads // (2 * g)), 148) if tc else \
-        (0.045 + 0.00014 * (d + dv), 64, num_heads, 148 * (4 if dv <= 128 else 2))
+    Over other pages: 14 us a launch, a fifth, and the decode kernel's time.  Over latents that kernel takes 17 us and more for the width of the rows, and
+    the rounds of a cluster's keys; rows of 320, prompt of 600, us apart / together: 2 tokens at 200 58 / 31, 29 at 1800 71 / 182, 64 at 300 63 / 125."""
+    us, rows, heads, slots = (0.0195, 128, num_heads, 148 * (2 if dv <= 128 else 1)) if tc and latent else \
+        (0.026, 128, g * -(-num_heads // (2 * g)), 148) if tc else (0.045 + 0.00014 * (d + dv), 64, num_heads, 148 * (4 if dv <= 128 else 2))
     n, keys, tiles, work, walk = 0, 0, 0, 0.0, 0.0
     for p, span in zip(parts, spans):
         if p.max_new < PREFILL_ATTN_MIN_TOKENS:
@@ -771,8 +772,10 @@ def _split_pays(parts, num_heads: int, g: int, d: int, dv: int, latent: bool, tc
     together = makespan(tiles + n * heads, work + n * heads * last)
     if pages and not latent:
         return 1.1 * together > alone + 4 * (len(parts) - 1) + 3 + keys * (4e-7 * n * g * (d + dv) + 0.008)
-    decode = 0.035 * keys * max(1.0, n / 32) if latent else keys * (n * g / 4000 + 0.008)
-    return 1.2 * together > alone + 14 * (len(parts) - 1) + decode
+    if latent:
+        splits = _latent_splits(n, num_heads, keys)
+        return together > alone + 8 * (len(parts) - 1) + 0.044 * d + 3 + 9e-5 * d * keys / splits * -(-n * -(-num_heads // 16) * splits // 148)
+    return 1.2 * together > alone + 14 * (len(parts) - 1) + keys * (n * g / 4000 + 0.008)
 
 
 def swa_sink_attn(q_src, num_heads: int, k_pool, v_pool, block_table, meta, sink, scale: float, window: int,
@@ -814,7 +817,8 @@ def swa_sink_attn(q_src, num_heads: int, k_pool, v_pool, block_table, meta, sink
     # decoded tokens beside prompt portions: each kind on its own kernel where that pays, in one launch of the prompt kernel otherwise
     parts = getattr(meta, "parts", None)
     if parts:
-        tc = _prompt_tc(q_src, k_pool, meta, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool)
+        tc = _latent_tc(q_src, k_pool, meta, d, dv, bs, chunk, softcap, sigmoid_bias, out_f32) if latent_values else \
+            _prompt_tc(q_src, k_pool, meta, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool)
         spans = [_span(p.max_end, int(window), int(chunk), pool, int(keep)) for p in parts]
         if not (tc or _prompt_mma(q_src, k_pool, meta, d, dv)) or not _split_pays(parts, num_heads, g, d, dv, bool(latent_values), tc, spans, bs % 32 == 0):
             parts = None
@@ -837,6 +841,15 @@ def _prompt_mma(q, k_pool, meta, d, dv) -> bool:
     """Shorter prompt portions in bf16 serving: the mma.sync kernel."""
     return (k_pool.dtype == torch.bfloat16 and meta.max_new >= PREFILL_ATTN_MIN_TOKENS and d % 16 == 0 and dv % 16 == 0
             and d <= 512 and dv <= 256 and q.stride(0) % 2 == 0)
+
+
+def _latent_tc(q, k_pool, meta, d, dv, bs, chunk, softcap, sigmoid_bias, out_f32) -> bool:
+    """Prompt portions over cached latents, bf16 rows of up to 64 columns beside the 128 or 256 value columns, pages of 32 tokens: the tcgen05
+    kernel.  From the shortest portion on: us, 16 heads over rows of 320, mma.sync / here: 16 tokens 20 / 14, at 1800 227 / 47, 128 41 / 18, 1000 162 / 39,
+    1600 310 / 51, 512 at 4000 549 / 107; rows of 160: 16 16 / 12, 1600 184 / 51."""
+    return bool(not (chunk or softcap or out_f32) and sigmoid_bias is None and k_pool.dtype == torch.bfloat16 and meta.max_new >= PREFILL_ATTN_MIN_TOKENS
+                and q.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0 and k_pool.data_ptr() % 16 == 0
+                and _lib().b200_latent_attn_prefill_tc_supported(d, dv, bs))
 
 
 def _latent_splits(tokens: int, heads: int, keys: int) -> int:
@@ -875,6 +888,13 @@ def _swa_part(q_src, num_heads, k_pool, v_pool, block_table, meta, sink, scale, 
                                                              1 if split_p else 0, int(window) if window < (1 << 30) else 0,
                                                              int(keep), sink),
                   "b200_swa_attn_prefill_tc_sink")
+        return
+    if latent_values and _latent_tc(q_all, k_pool, meta, d, dv, bs, chunk, softcap, sigmoid_bias, out_f32):
+        with _k("swa_sink_attn_prefill_tc" + tag):
+            check(_lib().b200_latent_attn_prefill_tc(q_all, q_all.stride(0), k_pool, k_pool.shape[0], block_table, block_table.stride(0),
+                                                           meta.seq_start, meta.seq_slot, meta.seq_pos0, meta.num_seqs, meta.max_new, sink,
+                                                           float(scale), int(window), out_all, num_heads, d, dv, bs),
+                  "b200_latent_attn_prefill_tc")
         return
     if _prompt_mma(q_all, k_pool, meta, d, dv):
         with _k("swa_sink_attn_prefill" + tag):
