@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(GRP_THREADS, 1)
   __shared__ __align__(16) float xch[GLU ? 2 * 2 * 16 * 64 : 4];
   __shared__ __align__(16) float xpose[GLU ? GRP_EPI_WARPS * 16 * 20 : GRP_EPI_WARPS * XP_WARP_FLOATS];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   if (warp == 0 && lane == 0) {
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(GRP_THREADS, 1)
   const int rows_e = GLU ? 2 * outs : outs;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t pol_w = policy_evict_first(), pol_a = policy_evict_last();
       int i = 0, s = 0, ph = 1;
       for (int tile = pair; tile < tiles; tile += pairs) {
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(GRP_THREADS, 1)
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (rank == 0) {
+    if (rank == 0 && elect_one()) {
       int s = 0, ph = 0, seg = 0;
       for (int tile = pair; tile < tiles; tile += pairs, ++seg) {
         const int as = seg & 1, cnt = (sched[tile / n_tiles] & 1) ? 2 * bm : bm;
@@ -142,23 +142,20 @@ __global__ void __launch_bounds__(GRP_THREADS, 1)
         for (int kb = 0; kb < num_kb; ++kb) {
           mbar_wait(&full[s], ph);
           tc_fence_after();
-          if (lane == 0) {
-            const uint32_t wa = smem_u32(smem + (size_t)s * stage), aa = wa + W_TILE;
+          const uint32_t wa = smem_u32(smem + (size_t)s * stage), aa = wa + W_TILE;
 #pragma unroll
-            for (int kk = 0; kk < GEMM_BK_BYTES / 32; ++kk)
-              umma_ss_pair<KIND_F16>(acc, umma_desc_sw128(wa + kk * 32), umma_desc_sw128(aa + kk * 32), idesc, (uint32_t)((kb | kk) != 0));
-            tc_commit_pair(&empty[s]);
-          }
-          __syncwarp();
+          for (int kk = 0; kk < GEMM_BK_BYTES / 32; ++kk)
+            umma_ss_pair<KIND_F16>(acc, umma_desc_sw128(wa + kk * 32), umma_desc_sw128(aa + kk * 32), idesc, (uint32_t)((kb | kk) != 0));
+          tc_commit_pair(&empty[s]);
           if (++s == nst) {
             s = 0;
             ph ^= 1;
           }
         }
-        if (lane == 0) tc_commit_pair(&tfull[as]);
-        __syncwarp();
+        tc_commit_pair(&tfull[as]);
       }
     }
+    __syncwarp();
   } else {
     const int lg = warp & 3, half = (warp - 2) >> 2;
     int seg = 0;

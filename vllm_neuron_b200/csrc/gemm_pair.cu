@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
   __shared__ uint32_t tmem_slot;
   __shared__ __align__(16) float a_s_tile[PAIR_MAX_BT];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
   const uint32_t tmem_base = tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t pol_w = w_stream_once ? policy_evict_first() : policy_evict_last();
       const uint64_t pol_a = policy_evict_last();  // activations are re-read by every pair
       const int n_off = (int)rank * GEMM_BN, m_off = (int)rank * (bt >> 1);
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (rank == 0) {
+    if (rank == 0 && elect_one()) {
       int s = 0, ph = 0, seg = 0, nt, mt, cnt;
       // the MMAs of token tile h of the unit whose operands lie in stage `st`
       auto mma = [&](int st, int h, uint32_t acc, bool first) {
@@ -159,8 +159,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
           for (; ahead < num_kb && ahead < nst; ++ahead) {
             mbar_wait(&full[s], ph);
             tc_fence_after();
-            if (lane == 0) mma(s, 0, acc, ahead == 0);
-            __syncwarp();
+            mma(s, 0, acc, ahead == 0);
             if (++s == nst) {
               s = 0;
               ph ^= 1;
@@ -168,36 +167,29 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
           }
           if (seg >= 1) mbar_wait(&tempty[as ^ 1], (((seg + 1) >> 1) - 1) & 1);
           tc_fence_after();
-          if (lane == 0)
-            for (int k = 0; k < ahead; ++k) {
-              mma(s2, 1, acc2, k == 0);
-              tc_commit_pair(&empty[s2]);
-              if (++s2 == nst) s2 = 0;
-            }
-          __syncwarp();
+          for (int k = 0; k < ahead; ++k) {
+            mma(s2, 1, acc2, k == 0);
+            tc_commit_pair(&empty[s2]);
+            if (++s2 == nst) s2 = 0;
+          }
         }
         for (int kb = ahead; kb < num_kb; ++kb) {
           mbar_wait(&full[s], ph);
           tc_fence_after();
-          if (lane == 0) {
-            mma(s, 0, acc, kb == 0);
-            if (cnt == 2) mma(s, 1, acc2, false);
-            tc_commit_pair(&empty[s]);
-          }
-          __syncwarp();
+          mma(s, 0, acc, kb == 0);
+          if (cnt == 2) mma(s, 1, acc2, false);
+          tc_commit_pair(&empty[s]);
           if (++s == nst) {
             s = 0;
             ph ^= 1;
           }
         }
-        if (lane == 0) {
-          tc_commit_pair(&tfull[as]);
-          if (cnt == 2) tc_commit_pair(&tfull[as ^ 1]);
-        }
-        __syncwarp();
+        tc_commit_pair(&tfull[as]);
+        if (cnt == 2) tc_commit_pair(&tfull[as ^ 1]);
         seg += cnt;
       }
     }
+    __syncwarp();
   } else {
     const int lg = warp & 3, quarter = (warp - 2) >> 2;
     const int et = threadIdx.x - 64;

@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(KIND == KIND_WO8 ? GEMM_THREADS + 128 : GEMM_T
   float* a_s_tile = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(fix_flag + 1) + 15) & ~uintptr_t(15));  // [BM]
   float* xpose = a_s_tile + BM;  // [4 epilogue warps][16][XP_PITCH]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int P = gridDim.x, c = blockIdx.x;
   const long long U = (long long)tiles * num_kb;
   const long long u0 = span_begin(U, P, c), u1 = span_begin(U, P, c + 1);
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(KIND == KIND_WO8 ? GEMM_THREADS + 128 : GEMM_T
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0 && u1 > u0) {
+    if (u1 > u0 && elect_one()) {
       const uint64_t pol_w = w_stream_once ? policy_evict_first() : policy_evict_last();
       const uint64_t pol_a = policy_evict_last();  // activations are re-read by every CTA
       const int total = (int)(u1 - u0);
@@ -243,21 +243,21 @@ __global__ void __launch_bounds__(KIND == KIND_WO8 ? GEMM_THREADS + 128 : GEMM_T
       }
     }
   } else if (warp == 1) {
-    int i = 0, seg = 0;
-    for (long long u = u0; u < u1; ++seg) {
-      const int kb0 = (int)(u % num_kb);
-      const long long left = u1 - u;
-      const int nk = left < (long long)(num_kb - kb0) ? (int)left : num_kb - kb0;
-      const int as = seg & 1;
-      if (seg >= 2) mbar_wait(&tempty[as], ((seg >> 1) - 1) & 1);
-      tc_fence_after();
-      const uint32_t acc = tmem_base + (uint32_t)(as * BM);
-      for (int k = 0; k < nk; ++k, ++i) {
-        const int s = i % NSTAGES;
-        mbar_wait(&full[s], (i / NSTAGES) & 1);
-        if constexpr (WO) mbar_wait(&full_cvt[s], (i / NSTAGES) & 1);
+    if (elect_one()) {
+      int i = 0, seg = 0;
+      for (long long u = u0; u < u1; ++seg) {
+        const int kb0 = (int)(u % num_kb);
+        const long long left = u1 - u;
+        const int nk = left < (long long)(num_kb - kb0) ? (int)left : num_kb - kb0;
+        const int as = seg & 1;
+        if (seg >= 2) mbar_wait(&tempty[as], ((seg >> 1) - 1) & 1);
         tc_fence_after();
-        if (lane == 0) {
+        const uint32_t acc = tmem_base + (uint32_t)(as * BM);
+        for (int k = 0; k < nk; ++k, ++i) {
+          const int s = i % NSTAGES;
+          mbar_wait(&full[s], (i / NSTAGES) & 1);
+          if constexpr (WO) mbar_wait(&full_cvt[s], (i / NSTAGES) & 1);
+          tc_fence_after();
           const uint32_t wa = smem_u32(smem + (size_t)s * STAGE);
           const uint32_t aa = wa + W_TILE;
 #pragma unroll
@@ -265,12 +265,11 @@ __global__ void __launch_bounds__(KIND == KIND_WO8 ? GEMM_THREADS + 128 : GEMM_T
             umma_ss<MK>(acc, umma_desc_sw128(wa + kk * 32), umma_desc_sw128(aa + kk * 32), IDESC, (uint32_t)((k | kk) != 0));
           tc_commit(&empty[s]);  // smem slot is free once these MMAs retire
         }
-        __syncwarp();
+        tc_commit(&tfull[as]);
+        u += nk;
       }
-      if (lane == 0) tc_commit(&tfull[as]);
-      __syncwarp();
-      u += nk;
     }
+    __syncwarp();
   } else if (WO && warp >= 6) {
     // weight-only: warps 6..9 widen raw int8 weight tiles into the bf16 operand half of each stage
     const int ct = threadIdx.x - 192;  // 0..127
@@ -585,7 +584,7 @@ __global__ void __launch_bounds__(KIND == KIND_WO8 ? WO_THREADS : DEC_THREADS, K
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(red_full + 1);
   float* stage = reinterpret_cast<float*>(smem);  // [BM][128] fp32 partial, aliases the (dead) ring after the last MMA
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int n_tile = blockIdx.x / S;
   const int kb0 = (int)((long long)num_kb * r / S), kb1 = (int)((long long)num_kb * (r + 1) / S);
   const int nk = kb1 - kb0;
@@ -633,7 +632,7 @@ __global__ void __launch_bounds__(KIND == KIND_WO8 ? WO_THREADS : DEC_THREADS, K
   float w4[4] = {1.f, 1.f, 1.f, 1.f}, b4[4] = {0.f, 0.f, 0.f, 0.f};  // S > 1: rows 4*t4 + e
 
   if (warp == 0) {
-    if (lane == 0 && nk > 0) {
+    if (nk > 0 && elect_one()) {
       const uint64_t pol_w = policy_evict_first();  // every weight byte is read once per step
       const int npre = nk < nst ? nk : nst;
       // weights do not depend on any kernel of the step: fill the ring with W tiles before the dependency resolves
@@ -674,15 +673,15 @@ __global__ void __launch_bounds__(KIND == KIND_WO8 ? WO_THREADS : DEC_THREADS, K
     }
     __syncwarp();  // lanes 1..31 park here
   } else if (warp == 1) {
-    int s = 0, ph = 0;
-    int t = 0, pht = 0;  // weight-only: TMEM weight slot / its parity
-    for (int i = 0; i < nk; ++i) {
-      mbar_wait(&full_w[WO ? t : s], WO ? pht : ph);
-      if (trace && lane == 0 && i < 8) trace[(size_t)gridDim.x * 8 + (size_t)blockIdx.x * 16 + i] = globaltimer_ns();
-      mbar_wait(&full_a[s], ph);
-      if (trace && lane == 0 && i < 8) trace[(size_t)gridDim.x * 8 + (size_t)blockIdx.x * 16 + 8 + i] = globaltimer_ns();
-      tc_fence_after();
-      if (lane == 0) {
+    if (elect_one()) {
+      int s = 0, ph = 0;
+      int t = 0, pht = 0;  // weight-only: TMEM weight slot / its parity
+      for (int i = 0; i < nk; ++i) {
+        mbar_wait(&full_w[WO ? t : s], WO ? pht : ph);
+        if (trace && i < 8) trace[(size_t)gridDim.x * 8 + (size_t)blockIdx.x * 16 + i] = globaltimer_ns();
+        mbar_wait(&full_a[s], ph);
+        if (trace && i < 8) trace[(size_t)gridDim.x * 8 + (size_t)blockIdx.x * 16 + 8 + i] = globaltimer_ns();
+        tc_fence_after();
         if (i == 0) B200_STAMP(2);
         const uint32_t aa = smem_u32(a_ring + (size_t)s * A_TILE);
         if constexpr (WO) {
@@ -702,22 +701,21 @@ __global__ void __launch_bounds__(KIND == KIND_WO8 ? WO_THREADS : DEC_THREADS, K
           tc_commit(&empty_a[s]);
           tc_commit(&empty_w[s]);
         }
+        if (++s == nst) {
+          s = 0;
+          ph ^= 1;
+        }
+        if (++t == NW) {
+          t = 0;
+          pht ^= 1;
+        }
       }
-      __syncwarp();
-      if (++s == nst) {
-        s = 0;
-        ph ^= 1;
-      }
-      if (++t == NW) {
-        t = 0;
-        pht ^= 1;
-      }
+      tc_commit(tfull);
     }
-    if (lane == 0) tc_commit(tfull);
     __syncwarp();
   } else if (warp == AP_WARP) {
     // ---- activation producer: everything it loads was written by the previous kernel of the stream
-    if (lane == 0 && nk > 0) {
+    if (nk > 0 && elect_one()) {
       const uint64_t pol_a = policy_evict_last();  // activations are re-read by every tile
       griddep_wait();
       B200_STAMP(1);

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(WOX_THREADS, 1)
   __shared__ uint64_t full_raw[WOX_MAX_ST], empty_raw[WOX_MAX_ST], full_a[WOX_MAX_ST], empty_a[WOX_MAX_ST], full_w[SLOTS], empty_w[SLOTS], tfull;
   __shared__ uint32_t tmem_slot;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int S = (int)cluster_nctarank(), r = (int)cluster_ctarank();
   const int n_tile = tile0 + (int)blockIdx.x / S;
   const int kb0 = (int)((long long)num_kb * r / S), nk = (int)((long long)num_kb * (r + 1) / S) - kb0;
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(WOX_THREADS, 1)
 
   if (warp == 0) {
     // raw weights: nothing of the step writes them, so they start before the dependency resolves
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t pol = policy_evict_first();
       int s = 0, ph = 1;
       for (int i = 0; i < nk; ++i) {
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(WOX_THREADS, 1)
     }
     __syncwarp();
   } else if (warp == 2 + WOX_CONV) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t pol = policy_evict_last();
       griddep_wait();
       int s = 0, ph = 1;
@@ -135,15 +135,15 @@ __global__ void __launch_bounds__(WOX_THREADS, 1)
     }
     __syncwarp();
   } else if (warp == 1) {
-    int s = 0, ph = 0, t = 0, pht = 0;
-    for (int i = 0; i < nk; ++i) {
-      mbar_wait(&full_a[s], ph);
-      const uint32_t aa = smem_u32(smem + (size_t)s * STAGE + WOX_RAW);
+    if (elect_one()) {
+      int s = 0, ph = 0, t = 0, pht = 0;
+      for (int i = 0; i < nk; ++i) {
+        mbar_wait(&full_a[s], ph);
+        const uint32_t aa = smem_u32(smem + (size_t)s * STAGE + WOX_RAW);
 #pragma unroll
-      for (int kh = 0; kh < 2; ++kh) {
-        mbar_wait(&full_w[t], pht);
-        tc_fence_after();
-        if (lane == 0) {
+        for (int kh = 0; kh < 2; ++kh) {
+          mbar_wait(&full_w[t], pht);
+          tc_fence_after();
 #pragma unroll
           for (int half = 0; half < 2; ++half)
 #pragma unroll
@@ -152,19 +152,18 @@ __global__ void __launch_bounds__(WOX_THREADS, 1)
                           IDESC, (uint32_t)((i | kh | kk) != 0));
           tc_commit(&empty_w[t]);
           if (kh == 1) tc_commit(&empty_a[s]);
+          if (++t == (int)SLOTS) {
+            t = 0;
+            pht ^= 1;
+          }
         }
-        __syncwarp();
-        if (++t == (int)SLOTS) {
-          t = 0;
-          pht ^= 1;
+        if (++s == nst) {
+          s = 0;
+          ph ^= 1;
         }
       }
-      if (++s == nst) {
-        s = 0;
-        ph ^= 1;
-      }
+      tc_commit(&tfull);
     }
-    if (lane == 0) tc_commit(&tfull);
     __syncwarp();
   } else {
     // widening: a thread owns one weight row of the tile, the two groups of eight warps alternate between stages.

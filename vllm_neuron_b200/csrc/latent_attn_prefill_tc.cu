@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
 #pragma unroll
     for (int c = 0; c < CH; ++c) tma_load_2d(dst + c * LP_KCH, &k_map, &k_full[s], c * 64, blk * LP_BLK);
   };
-  if ((warp == 5 || warp == 6) && lane == 0)
+  if ((warp == 5 || warp == 6) && elect_one())
     for (int it = 0; it < min(ST, niter); ++it) load_keys(it);
   __syncwarp();
   // q tile, all threads: fp32 rows -> bf16, K-major 128B swizzle; four pieces of 8 columns in flight a thread (128 rows of 320: 20 pieces each)
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
   }
 
   if (warp == 5 || warp == 6) {
-    if (lane == 0)
+    if (elect_one())
       for (int it = ST; it < niter; ++it) load_keys(it);
     __syncwarp();
   } else if (warp == 4) {

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
   uint64_t* o_full = p_ready + 2;                    // 2
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int G = Hq / Hkv, pairs = (G + 1) >> 1;
   const int kvh = blockIdx.x / pairs, pr = blockIdx.x - kvh * pairs;
   const int head0 = kvh * G + 2 * pr;
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
   asm volatile("setmaxnreg.dec.sync.aligned.u32 56;\n");
   if (warp == 9 || warp == 10) {
     // ---------------------------------------------------------------- K (warp 9) / V (warp 10) producer
-    if (lane == 0) {
+    if (elect_one()) {
       const CUtensorMap* map = warp == 9 ? &k_map : &v_map;
       uint8_t* ring = warp == 9 ? k_s : v_s;
       uint64_t* full = warp == 9 ? k_full : v_full;
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
     __syncwarp();
   } else if (warp == 8) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, (uint32_t)(ntile * TILE));
       for (int t = 0; t < ntile; ++t)
 #pragma unroll

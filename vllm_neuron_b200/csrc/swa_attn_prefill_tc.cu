@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1)
   uint64_t* o_full = p_ready + 2;                    // 2
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   if (warp == 8 && lane == 0) {
     tma_prefetch_desc(&k_map);
     tma_prefetch_desc(&v_map);
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;\n");
     if (warp == 9 || warp == 10) {
       // ---------------------------------------------------------------- K (warp 9) / V (warp 10) producer
-      if (lane == 0) {
+      if (elect_one()) {
         const bool is_k = warp == 9;
         const CUtensorMap* map = is_k ? &k_map : &v_map;
         uint8_t* ring = is_k ? k_s : v_s;
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1)
       __syncwarp();
     } else if (warp == 8) {
       // ---------------------------------------------------------------- MMA issuer
-      if (lane == 0) {
+      if (elect_one()) {
         auto issue_s = [&](int t, int s) {
           const uint32_t qa = smem_u32(q_s + t * TQ), ka = smem_u32(k_s + (size_t)s * TK + (MAPS ? t * NHK * HALFK : 0));
           constexpr int PER = KROW / 32;  // 16-column MMA steps per row piece
