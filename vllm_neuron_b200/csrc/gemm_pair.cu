@@ -313,20 +313,19 @@ int launch_pair(const void* a, const void* w, const GemmEpilogue& ep, int M, int
 
 }  // namespace
 
-// Tokens of a tile, and whether a pair takes two token tiles at once.  A wave of tiles costs its k-blocks -- 3 clocks for each of the 128 + bt/2
-// operand rows, no less than at 128 tokens -- plus filling the ring, draining the last accumulator and the launch; so the widest tile wins unless a narrower one saves a
-// wave or the padding of the last token tile.  Two at once cost 520 + 2.2 bt clocks a k-block, both accumulators' epilogue at the end and some of it
-// between waves; the waves that would not fill go one by one where that ends sooner.  Fitted to and checked against 645 measured calls (bf16, fp8,
-// SiLU and fp32 outputs, 129 to 4096 tokens, 14 weights, 11 to 13 plans each, L2 flushed): the choice is 0.3 % slower than the best plan on average, 12 % at
-// most, and 0.940 of one by one on average; 0.97 or less in 325 calls, over 1.03 in six (600 x 55296 x 5120 + SiLU 343 / 313 us).
-// Measured (us, one by one / two at once, bf16): 777 x 6144 x 4096 63.5 / 50.0, 777 x 28672 x 4096 196 / 160, 2048 x 28672 x 4096 363 / 311, fp8 201 /
-// 182, 4096 x 10272 x 2048 158 / 138, fp32 141 / 129.
-// bt = 0: stream-K (gemm_tcgen05.cu) takes the call.  It cuts K, which pays where few tiles walk a long K or a nearly empty wave follows a full
-// one: about 25 us, 0.52 for each k-block of 128 x 256 of an SM's share, and 8 for every CTA that adds to one tile.  Measured (us, pairs /
-// stream-K, bf16): 129 x 5120 x 27648 152 / 106, 256 158 / 115, 320 158 / 156, 512 164 / 173, 777 327 / 292, 1290 400 / 447;
-// 300 x 1024 x 28672 155 / 123, 1400 157 / 122; 200 x 8192 x 28672 175 / 139, 300 170 / 240; 129 x 4096 x 14336 80 / 85, 1200 161 / 158.
-// Over 700 measured calls (bf16 and fp8, 129 to 4096 tokens) the rule takes the slower side by more than 5 % in seven, by 13 % at most, and
-// never leaves a faster pair schedule.
+// Tokens of a tile, and whether a pair takes two token tiles at once.  A wave of tiles costs its k-blocks -- 320 + 0.625 bt clocks each, the operands'
+// way into shared memory and the MMAs' issue -- plus filling the ring, draining the last accumulator and the launch; so the widest tile wins unless
+// a narrower one saves a wave or the padding of the last token tile.  Two at once cost 250 + 2.75 bt clocks a k-block, both accumulators' epilogue at the
+// end and some of it between waves; the waves that would not fill go one by one where that ends sooner.  Fitted to and checked against 560 measured
+// calls (bf16, fp8, SiLU and fp32 outputs, 129 to 4096 tokens, 14 weights, 11 to 17 plans each, L2 flushed): the choice is 0.6 % slower than the best
+// plan on average, 14 % at most, and 0.966 of what the constants from before the MMAs were issued by an elected lane chose; 0.97 or less in 203
+// calls, over 1.03 in four (1.05 at most).
+// Measured (us, those constants / now, bf16): 777 x 6144 x 4096 50.0 / 39.2, 777 x 28672 x 4096 144 / 132, 2048 tokens of an fp8 prompt step 4265 / 4127.
+// bt = 0: stream-K (gemm_tcgen05.cu) takes the call.  It cuts K, which pays where few tiles walk a very long K: about 25 us, 0.52 for each
+// k-block of 128 x 256 of an SM's share, and 8 for every CTA that adds to one tile.  Measured (us, pairs / stream-K, bf16): 129 x 2048 x 53248
+// 213 / 139, 300 x 2048 x 53248 215 / 174, 512 x 2560 x 53248 221 / 209, 1290 x 512 x 53248 217 / 154; 129 x 5120 x 27648 121 / 111, 256 123 / 121;
+// 300 x 1024 x 28672 119 / 125, 1400 150 / 148; 129 x 8192 x 28672 131 / 139.  Over 390 measured calls (bf16 and fp8, 129 to 2000 tokens) the rule
+// takes the slower side by more than 5 % in two, by 9 % at most.
 PairPlan pair_plan(int M, int N, int K, int ab_dtype) {
   const int eb = ab_dtype == B200_BF16 ? 2 : 1, sms = sm_count();
   const int pairs = sms / 2, num_kb = (K * eb + GEMM_BK_BYTES - 1) / GEMM_BK_BYTES, n_tiles = (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN);
@@ -340,16 +339,16 @@ PairPlan pair_plan(int M, int N, int K, int ab_dtype) {
   };
   for (int bt = PAIR_MAX_BT; bt >= 64; bt -= 32) {
     const int mt = (M + bt - 1) / bt;
-    const long long lone_cost = (long long)num_kb * 3 * (GEMM_BN + (bt > 128 ? bt : 128) / 2) + 2600 + 7 * bt;
+    const long long lone_cost = (long long)num_kb * 5 * (512 + bt) / 8 + 4000 + 6 * bt;
     offer(bt, 0, ((long long)mt * n_tiles + pairs - 1) / pairs * lone_cost);
     if (mt < 2 || bt < 128) continue;
-    const long long wide_cost = (long long)num_kb * (2600 + 11 * bt) / 5 + 3700 + 34 * bt, all = (long long)((mt + 1) / 2) * n_tiles;
+    const long long wide_cost = (long long)num_kb * (1000 + 11 * bt) / 4 + 2700 + 50 * bt, all = (long long)((mt + 1) / 2) * n_tiles;
     if (all > INT_MAX) continue;
     for (const long long wide : {all, all / pairs * pairs}) {  // wide to the end, or whole waves of it and the rest one by one
       if (!wide) continue;
       const PairUnits un(mt, n_tiles, (int)wide);
       const long long waves = (wide + pairs - 1) / pairs;
-      offer(bt, (int)wide, waves * wide_cost + (waves - 1) * 4100 + (un.units - wide + pairs - 1) / pairs * lone_cost);
+      offer(bt, (int)wide, waves * wide_cost + (waves - 1) * 2500 + (un.units - wide + pairs - 1) / pairs * lone_cost);
     }
   }
   const double sk_tiles = (double)((M + 255) / 256) * ((N + GEMM_BN - 1) / GEMM_BN), shared = sms / sk_tiles;
