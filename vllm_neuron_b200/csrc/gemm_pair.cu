@@ -321,11 +321,11 @@ int launch_pair(const void* a, const void* w, const GemmEpilogue& ep, int M, int
 // plan on average, 14 % at most, and 0.966 of what the constants from before the MMAs were issued by an elected lane chose; 0.97 or less in 203
 // calls, over 1.03 in four (1.05 at most).
 // Measured (us, those constants / now, bf16): 777 x 6144 x 4096 50.0 / 39.2, 777 x 28672 x 4096 144 / 132, 2048 tokens of an fp8 prompt step 4265 / 4127.
-// bt = 0: stream-K (gemm_tcgen05.cu) takes the call.  It cuts K, which pays where few tiles walk a very long K: about 25 us, 0.52 for each
-// k-block of 128 x 256 of an SM's share, and 8 for every CTA that adds to one tile.  Measured (us, pairs / stream-K, bf16): 129 x 2048 x 53248
-// 213 / 139, 300 x 2048 x 53248 215 / 174, 512 x 2560 x 53248 221 / 209, 1290 x 512 x 53248 217 / 154; 129 x 5120 x 27648 121 / 111, 256 123 / 121;
-// 300 x 1024 x 28672 119 / 125, 1400 150 / 148; 129 x 8192 x 28672 131 / 139.  Over 390 measured calls (bf16 and fp8, 129 to 2000 tokens) the rule
-// takes the slower side by more than 5 % in two, by 9 % at most.
+// bt = 0: stream-K (gemm_tcgen05.cu) takes the call.  It cuts K, which pays where few tiles walk a very long K: about 18 us, 0.52 for each
+// k-block of 128 x 256 of an SM's share, 7.5 for every CTA that adds to one tile and 0.03 a token; a pair's walk takes at least 500 clocks a k-block.
+// Measured (us, pairs / stream-K, bf16): 129 x 2048 x 53248 213 / 139, 300 x 2048 x 53248 215 / 174, 512 x 2560 x 53248 221 / 209, 1290 x 512 x 53248
+// 217 / 154; 129 x 5120 x 27648 121 / 111, 256 123 / 121; 300 x 1024 x 28672 119 / 125, 1400 150 / 148; 129 x 8192 x 28672 131 / 139.  Over 398 measured
+// calls (bf16 and fp8, 129 to 2000 tokens) the rule takes the slower side by more than 4 % in two, by 5 % at most.
 PairPlan pair_plan(int M, int N, int K, int ab_dtype) {
   const int eb = ab_dtype == B200_BF16 ? 2 : 1, sms = sm_count();
   const int pairs = sms / 2, num_kb = (K * eb + GEMM_BK_BYTES - 1) / GEMM_BK_BYTES, n_tiles = (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN);
@@ -352,8 +352,9 @@ PairPlan pair_plan(int M, int N, int K, int ab_dtype) {
     }
   }
   const double sk_tiles = (double)((M + 255) / 256) * ((N + GEMM_BN - 1) / GEMM_BN), shared = sms / sk_tiles;
-  const double stream_k_us = 25.0 + 0.52 * sk_tiles * num_kb / sms + 8.0 * (shared > 1.0 ? shared : 1.0);
-  return stream_k_us * 1850.0 < (double)best_cost ? PairPlan{0, 0} : best;  // clocks at 1.85 GHz
+  const double stream_k_us = 18.0 + 0.52 * sk_tiles * num_kb / sms + 7.5 * (shared > 1.0 ? shared : 1.0) + 0.03 * M;
+  const double pair_cost = (double)best_cost, walk = 500.0 * num_kb + 5000.0;  // one wave's walk from memory
+  return stream_k_us * 1850.0 < (pair_cost > walk ? pair_cost : walk) ? PairPlan{0, 0} : best;  // clocks at 1.85 GHz
 }
 
 int launch_gemm_pair(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, PairPlan p,
