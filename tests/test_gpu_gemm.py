@@ -233,6 +233,18 @@ def test_gemm_pairs_bf16_against_64_bits(ops, m, n, k, f32):
     assert ((got - want).abs() <= (k / 16 + 3) * 2.0**-23 * size + (0.0 if f32 else 2.0**-8) * want.abs()).all()
 
 
+@pytest.mark.parametrize("kind", ["bf16", "fp8"])
+def test_gemm_rope_kv_write_of_a_decode_batch_on_pairs(ops, kind):
+    test_gemm_rope_kv_write_matches_two_launches(ops, kind, 100, 64, 8, 128, 2048, 0)
+
+
+@pytest.mark.parametrize("m,n,k", [(17, 10272, 2048), (64, 9473, 520), (65, 10272, 2048), (128, 18944, 1032)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_gemm_decode_batches_on_pairs(ops, m, n, k, f32):
+    """Up to 128 tokens against rows that fill a wave of pairs, or miss it by one, and a K of a part of a block."""
+    test_gemm_pairs_bf16_against_64_bits(ops, m, n, k, f32)
+
+
 @pytest.mark.parametrize("m,n,k", [(257, 1001, 192), (777, 6144, 520)])
 @pytest.mark.parametrize("f32", [False, True])
 def test_gemm_pairs_rows_of_odd_length_and_two_token_tiles(ops, m, n, k, f32):

@@ -357,6 +357,24 @@ PairPlan pair_plan(int M, int N, int K, int ab_dtype) {
   return stream_k_us * 1850.0 < (pair_cost > walk ? pair_cost : walk) ? PairPlan{0, 0} : best;  // clocks at 1.85 GHz
 }
 
+// Decode-sized batches on CTA pairs: the decode schedule cuts K over clusters, so every SM reads weights whatever N is, and pays for the partial sums; pairs
+// walk the whole K, which takes no longer where their tiles fill the waves, or where K is short.  A wave of pairs is bound by its k-blocks (0.247 us each) or by its weights
+// (5.9 TB/s), behind 9.5 us of launch, first loads and epilogue; the decode schedule takes 12 us and 5.7 TB/s up to 64 tokens, 15 us and 5.0 TB/s
+// above, where its tile of 128 tokens halves the ring.  The pairs have to win by a twentieth, above 64 tokens by 0.15: they have no rotating epilogue, and a qkv
+// projection that they take needs another launch (b200_gemm_rope_kv_write keeps the bits of the two calls).  Measured, us, decode schedule / pairs, L2 flushed: bf16 64 x 10272 x 2048 22.5 / 18.5, 128 30.7 /
+// 20.5; 64 x 55296 x 5120 113 / 101, 128 131 / 103; 64 x 28672 x 4096 55.3 / 55.3, 128 63.5 / 55.4; 128 x 4096 x 4096 24.6 / 26.6, 64 x 8192 x 28672 94 / 121;
+// fp8 128 x 6144 x 4096 24.5 / 20.5, 64 18.5 / 18.4.  Over 160 such calls (17 to 128 tokens, 16 weights) the choice costs 0.4 % more than the better one.
+bool pair_takes_decode(int M, int N, int K, int ab_dtype) {
+  const double row = (double)K * (ab_dtype == B200_BF16 ? 2 : 1), steps = 0.247 * ((row + GEMM_BK_BYTES - 1) / GEMM_BK_BYTES);
+  const int pairs = sm_count() / 2, tiles = (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN), rest = tiles % pairs;
+  auto wave = [&](int n) {
+    const double bytes = n * (2.0 * GEMM_BN) * row / 5.9e6;
+    return n == 0 ? 0.0 : bytes > steps ? bytes : steps;
+  };
+  const double pair_us = 9.5 + (tiles / pairs) * wave(pairs) + wave(rest);
+  return M <= 64 ? pair_us < 0.95 * (12.0 + N * row / 5.7e6) : pair_us < 0.85 * (15.0 + N * row / 5.0e6);
+}
+
 int launch_gemm_pair(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, PairPlan p,
                      cudaStream_t s) {
   if (ab_dtype == B200_BF16)

@@ -1290,9 +1290,9 @@ int gemm_common(const void* a, const void* w, const GemmEpilogue& ep, int epi, i
   // decode-sized batches of the weight-only kind: 256 weight rows per CTA (narrow weights, and calls that name their K splits, keep the
   // 128-row schedule)
   if (wide) return launch_gemm_wo(a, w, ep, epi, M, N, K, (cudaStream_t)stream);
-  // prompt-sized batches run on CTA pairs; stream-K keeps the shapes where cutting K is faster, the weight-only kind, whose tiles are widened
-  // on the way, and calls that cap its CTAs
-  if (const PairPlan plan = !p.decode && !wo && split_k == 0 ? pair_plan(M, N, K, ab_dtype) : PairPlan{0, 0}; plan.bt)
+  // prompt-sized batches run on CTA pairs, and decode-sized ones where those are faster; stream-K keeps the shapes where cutting K is faster, the
+  // weight-only kind, whose tiles are widened on the way, and calls that cap its CTAs
+  if (const PairPlan plan = !wo && split_k == 0 && (!p.decode || (epi != EPI_ROPE && pair_takes_decode(M, N, K, ab_dtype))) ? pair_plan(M, N, K, ab_dtype) : PairPlan{0, 0}; plan.bt)
     return launch_gemm_pair(a, w, ep, epi, M, N, K, ab_dtype, plan, (cudaStream_t)stream);
   CUtensorMapDataType dt = eb == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
   int bk = GEMM_BK_BYTES / eb;
@@ -1451,11 +1451,12 @@ int b200_gemm_rope_kv_write(const void* a, const void* w, void* qkv_out, const f
   B200_REQUIRE(N == (Hq + 2 * Hkv) * D, "gemm_rope_kv_write: N=%d is not (Hq + 2 Hkv) * D = %d", N, (Hq + 2 * Hkv) * D);
   GemmEpilogue ep{a_scale, w_scale, (const __nv_bfloat16*)bias, nullptr, qkv_out, 0, nullptr};
   // The rotation lives in the split-K owner's epilogue of the decode kernel (a token's whole head in one warp) and in that of the kernel
-  // for a few tokens, whose row sums are those of its linear epilogue.  Every other schedule (one CTA per tile, the stream-K prefill kernel, odd head sizes) runs the GEMM, then the RoPE/scatter
-  // kernel: same bits either way.
+  // for a few tokens, whose row sums are those of its linear epilogue.  Every other schedule (one CTA per tile, CTA pairs, the stream-K prefill kernel, odd head
+  // sizes) runs the GEMM, then the RoPE/scatter kernel: same bits either way.
   bool fused = false;
   const bool wide_wo = ab_dtype == B200_INT8_WO && split_k == 0 && gemm_wo_wide(EPI_ROPE, M, N, K);  // its own schedule, without the rotation
-  if (M <= 128 && !wide_wo && (D == 64 || D == 128) && N % GEMM_BN == 0 && max_pos > 0 &&
+  const bool on_pairs = split_k == 0 && ab_dtype != B200_INT8_WO && K > 0 && pair_takes_decode(M, N, K, ab_dtype);  // the linear call's schedule
+  if (M <= 128 && !wide_wo && !on_pairs && (D == 64 || D == 128) && N % GEMM_BN == 0 && max_pos > 0 &&
       (ab_dtype == B200_BF16 || ab_dtype == B200_FP8_E4M3 || ab_dtype == B200_INT8 || ab_dtype == B200_INT8_WO)) {
     int plan6[6];
     if (b200_gemm_decode_plan(M, N, K, ab_dtype, split_k, 2, 0, plan6) == B200_OK && plan6[0] > 1) fused = true;
