@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
   uint64_t* v_full = k_empty + PF_ST;
   uint64_t* v_empty = v_full + PF_ST;
   uint64_t* s_full = v_empty + PF_ST;                // 2 (per tile)
-  uint64_t* p_ready = s_full + 2;                    // 2
-  uint64_t* o_full = p_ready + 2;                    // 2
+  uint64_t* p_ready = s_full + 2;                    // 2 x 2 (per tile, half of the step's keys)
+  uint64_t* o_full = p_ready + 4;                    // 2
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -123,7 +123,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
     }
     for (int t = 0; t < 2; ++t) {
       mbar_init(&s_full[t], 1);
-      mbar_init(&p_ready[t], 4);  // one arrival per softmax warp of the tile
+      mbar_init(&p_ready[2 * t], 4);  // one arrival per softmax warp of the tile
+      mbar_init(&p_ready[2 * t + 1], 4);
       mbar_init(&o_full[t], 1);
     }
     fence_mbar_init();
@@ -185,12 +186,14 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
         }
         tc_commit(&s_full[t]);
       };
-      auto issue_pv = [&](int t, int s, int j) {
+      auto issue_pv = [&](int t, int s, int j, int half) {
         const uint32_t va = smem_u32(v_s + (size_t)s * TILE);
 #pragma unroll
-        for (int kk = 0; kk < PF_BN / 16; ++kk)  // 16 tokens per UMMA_K: two 8-row groups of the [token][d] tile
+        for (int k4 = 0; k4 < PF_BN / 32; ++k4) {
+          const int kk = half * (PF_BN / 32) + k4;  // 16 tokens per UMMA_K: two 8-row groups of the [token][d] tile
           umma_ts_f16(tmem_base + 256u + (uint32_t)t * 128u, tmem_base + (uint32_t)t * 128u + (uint32_t)kk * 8u,
                       umma_desc_mn_sw128(va + kk * 2048, HALF, 1024), IDESC_PV, (uint32_t)((j | kk) != 0));
+        }
       };
       mbar_wait(q_full, 0);
       mbar_wait(&k_full[0], 0);
@@ -202,9 +205,12 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
         const bool more = j + 1 < nsteps;
         mbar_wait(&v_full[s], (uint32_t)(j / PF_ST) & 1u);
         for (int t = 0; t < ntile; ++t) {
-          mbar_wait(&p_ready[t], (uint32_t)j & 1u);
-          tc_fence_after();
-          issue_pv(t, s, j);
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            mbar_wait(&p_ready[2 * t + half], (uint32_t)j & 1u);
+            tc_fence_after();
+            issue_pv(t, s, j, half);
+          }
           if (t == ntile - 1) tc_commit(&v_empty[s]);
           if (more) {
             if (t == 0) {
@@ -285,27 +291,32 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
       // p = 2^(s*scale - m), row sum on four independent chains, bf16 P over the first 64 columns S occupied
       float l4[4] = {0.f, 0.f, 0.f, 0.f};
       const float neg_m = -m_used;
-      uint32_t pk[PF_BN / 2];
+      // The products of the first 64 keys run while the other weights are made; they were behind them when an MMA took 95 clocks to issue.  32 heads of
+      // 128 over 8, one hand-over / two: 4096 tokens 133 / 128 us, 777 behind 3104 68.1 / 65.5, 128 at 16384 243 / 231
 #pragma unroll
-      for (int i = 0; i < PF_BN; i += 4) {
-        const float p0 = ex2_approx(fmaf(__uint_as_float(sv[i]), scale_log2, neg_m));
-        const float p1 = ex2_approx(fmaf(__uint_as_float(sv[i + 1]), scale_log2, neg_m));
-        const float p2 = ex2_approx(fmaf(__uint_as_float(sv[i + 2]), scale_log2, neg_m));
-        const float p3 = ex2_approx(fmaf(__uint_as_float(sv[i + 3]), scale_log2, neg_m));
-        l4[0] += p0;
-        l4[1] += p1;
-        l4[2] += p2;
-        l4[3] += p3;
-        pk[i >> 1] = pack_bf16(p0, p1);
-        pk[(i >> 1) + 1] = pack_bf16(p2, p3);
+      for (int half = 0; half < 2; ++half) {
+        uint32_t pk[PF_BN / 4];
+#pragma unroll
+        for (int e = 0; e < PF_BN / 2; e += 4) {
+          const int i = half * (PF_BN / 2) + e;
+          const float p0 = ex2_approx(fmaf(__uint_as_float(sv[i]), scale_log2, neg_m));
+          const float p1 = ex2_approx(fmaf(__uint_as_float(sv[i + 1]), scale_log2, neg_m));
+          const float p2 = ex2_approx(fmaf(__uint_as_float(sv[i + 2]), scale_log2, neg_m));
+          const float p3 = ex2_approx(fmaf(__uint_as_float(sv[i + 3]), scale_log2, neg_m));
+          l4[0] += p0;
+          l4[1] += p1;
+          l4[2] += p2;
+          l4[3] += p3;
+          pk[e >> 1] = pack_bf16(p0, p1);
+          pk[(e >> 1) + 1] = pack_bf16(p2, p3);
+        }
+        tmem_st_32x32b_x32(s_addr + half * 32, pk);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_ready[2 * t + half]);
       }
       l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
-      tmem_st_32x32b_x32(s_addr, *reinterpret_cast<uint32_t(*)[32]>(&pk[0]));
-      tmem_st_32x32b_x32(s_addr + 32, *reinterpret_cast<uint32_t(*)[32]>(&pk[32]));
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_ready[t]);
     }
     // epilogue: O / l -> bf16 rows
     mbar_wait(&o_full[t], 0);
