@@ -10,7 +10,7 @@
 // kernel which these portions took before (3.19e-3 / 3.03e-3 relative, now 2.93e-3).
 // What bounds it: the products of a step, 20 score MMAs of 6 KB of operands from shared memory at 320 columns (~950 clocks) and 8 of the values
 // (512), then a step's weights on the way (1100 clocks, beside the next scores).  16 heads, rows of 320, 1600 tokens: 310 us on mma.sync, here 51; 16 tokens
-// at 1800 227 / 47.  Before all threads laid down the queries and the output went through shared memory 96, before the elected lane 63.
+// at 1800 227 / 45.  Before all threads laid down the queries and the output went through shared memory 96, before the elected lane 63.
 // Steps of 64 keys: 80 KB of queries and three stages of 40 KB fill the shared memory at 320 columns; 128 keys would leave one stage.
 // Rows of up to 192 columns: two stages, so that two CTAs share an SM.
 #include "common.cuh"
@@ -94,8 +94,8 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
   uint64_t* k_full = reinterpret_cast<uint64_t*>(k_s + ST * KST);  // ST
   uint64_t* k_empty = k_full + ST;   // ST
   uint64_t* s_full = k_empty + ST;   // 2
-  uint64_t* p_ready = s_full + 2;    // 2
-  uint64_t* o_done = p_ready + 2;    // 1: the products of a step
+  uint64_t* p_ready = s_full + 2;    // 2 x 2 (buffer, half of the step's keys)
+  uint64_t* o_done = p_ready + 4;    // 1: the products of a step
   uint64_t* o_full = o_done + 1;     // 1: those of all steps (a waiter may be two steps behind o_done here, which its parity cannot tell)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 1);
 
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
     if (lane == 0) {
       tma_prefetch_desc(&k_map);
       for (int s = 0; s < ST; ++s) mbar_init(&k_full[s], 2), mbar_init(&k_empty[s], 1);
-      for (int b = 0; b < 2; ++b) mbar_init(&s_full[b], 1), mbar_init(&p_ready[b], 4);
+      for (int b = 0; b < 2; ++b) mbar_init(&s_full[b], 1), mbar_init(&p_ready[2 * b], 4), mbar_init(&p_ready[2 * b + 1], 4);
       mbar_init(o_done, 1);
       mbar_init(o_full, 1);
       fence_mbar_init();
@@ -185,11 +185,13 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
       if (niter > 1) issue_s(1);
       for (int it = 0; it < niter; ++it) {
         const int s = it % ST;
-        mbar_wait(&p_ready[it & 1], (uint32_t)(it >> 1) & 1u);
-        tc_fence_after();
         const uint32_t va = smem_u32(k_s + s * KST), p = tmem + (uint32_t)(it & 1) * LP_BN;
 #pragma unroll
         for (int kk = 0; kk < LP_BN / 16; ++kk) {  // 16 keys: two 8-row groups of the [key][column] pieces
+          if ((kk & 1) == 0) {
+            mbar_wait(&p_ready[2 * (it & 1) + (kk >> 1)], (uint32_t)(it >> 1) & 1u);
+            tc_fence_after();
+          }
           const uint64_t vd = lp_desc_mn(va + kk * 2048);
           umma_ts_f16(tmem + O_COL, p + (uint32_t)kk * 8u, vd, IDESC_PV, (uint32_t)((it | kk) != 0));
           umma_ts_f16(tmem + O_COL, p + 32u + (uint32_t)kk * 8u, vd, IDESC_PV, 1u);
@@ -281,12 +283,12 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
         }
         lp_st_x16(s_addr + c * 16, hi);
         lp_st_x16(s_addr + 32 + c * 16, lo);
+        tmem_st_wait();  // the products of the first 32 keys run while the other weights are made (512 tokens at 4000, 16 heads of 320: 98.4 -> 95.5 us)
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_ready[2 * (it & 1) + c]);
       }
       l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_ready[it & 1]);
     }
     // ------------------------------------------------------------------ O / l -> rows of the output
     mbar_wait(o_full, 0);
@@ -326,7 +328,7 @@ static int lp_launch(const CUtensorMap& km, const float* q, int ldq, const int32
                      const int32_t* seq_slot, const int32_t* seq_pos0, int B, int max_new, void* out, int H, int D, float scale, int window,
                      const float* sink, cudaStream_t stream) {
   auto kern = latent_prefill_tc_kernel<C, ST>;
-  const size_t smem = (size_t)(C / 64 + 1) * (LP_QCH + ST * LP_KCH) + 128 + 1024;
+  const size_t smem = (size_t)(C / 64 + 1) * (LP_QCH + ST * LP_KCH) + 256 + 1024;
   static bool attr_done = false;
   if (!attr_done) {
     B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
