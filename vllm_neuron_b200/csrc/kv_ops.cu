@@ -445,6 +445,7 @@ __device__ __forceinline__ void argmax_take(float& best, int& bi, float x, int i
 __global__ void __launch_bounds__(ARGMAX_THREADS) argmax_kernel(const float* __restrict__ logits, int64_t row_stride,
                                                                 float* __restrict__ out_val, int64_t* __restrict__ out_idx,
                                                                 int V, int64_t idx_offset) {
+  cluster_arrive_relaxed();  // "this CTA runs": waited for before the first store into another CTA, under the scan of the slice
   griddep_launch();
   griddep_wait();
   __shared__ float sv[32];
@@ -483,6 +484,7 @@ __global__ void __launch_bounds__(ARGMAX_THREADS) argmax_kernel(const float* __r
     si[w] = bi;
   }
   __syncthreads();
+  cluster_wait();  // every CTA of the cluster runs: rank 0's shared memory may be written
   if (w == 0) {
     constexpr int NW = ARGMAX_THREADS / 32;
     best = l < NW ? sv[l] : -INFINITY;

@@ -235,6 +235,8 @@ __global__ void __launch_bounds__(TOPK_THREADS)
   const int64_t row = blockIdx.x / ctas;
   const float* r = logits + row * row_stride;
   if (tid == 0) s_cnt = 0;
+  __syncwarp();
+  cluster_arrive_relaxed();  // "this CTA runs": waited for before the first store into another CTA, under the pass over the row
   griddep_launch();
   griddep_wait();
   const bool vec = (row_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
@@ -249,6 +251,7 @@ __global__ void __launch_bounds__(TOPK_THREADS)
   }
   for (int i = lo + tid; i < hi; i += TOPK_THREADS) mx = max(mx, f2key(r[i]));
   for (int o = 1; o < ctas; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));  // as many threads as CTAs make a group ...
+  cluster_wait();  // every CTA of the cluster runs: its shared memory may be written
   // ... and each of them tells one CTA
   st_cluster_f32(mapa_shared(smem_u32(&group_max[(rank * TOPK_THREADS + tid) / ctas]), tid & (ctas - 1)), __uint_as_float(mx));
   cluster_sync_all();  // the maxima are everywhere, the first CTA's count is 0
