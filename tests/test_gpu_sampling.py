@@ -67,6 +67,20 @@ def test_topk_candidates_of_rows_cut_by_clusters(ops, b, v, pitch):
     assert np.array_equal(val.cpu().numpy(), wv) and np.array_equal(idx.cpu().numpy(), wi)
 
 
+@pytest.mark.parametrize("v", [16385, 40000, 128256])
+def test_topk_candidates_around_a_full_list(ops, v):
+    """Rows that put 1023, 1024 (the list's size), 1025 and almost all of their elements at the threshold, masked ones among them."""
+    x = _logits(7, v, v)
+    order = torch.randperm(v, generator=torch.Generator().manual_seed(v))
+    for row, n in enumerate((1023, 1024, 1025)):
+        x[row, order[:n]] = 20.0
+    for row, (n, low) in enumerate(((40, -float("inf")), (255, -float("inf")), (300, torch.finfo(torch.float32).min), (0, 1.0)), 3):
+        x[row, order[n:]] = low
+    val, idx = ops.topk_candidates(x.cuda())
+    wv, wi = S.topk_candidates_ref(x.numpy())
+    assert np.array_equal(val.cpu().numpy(), wv) and np.array_equal(idx.cpu().numpy(), wi)
+
+
 def test_constant_row_keeps_the_lowest_indices(ops):
     x = torch.zeros(2, 5000)
     val, idx = ops.topk_candidates(x.cuda())

@@ -19,7 +19,7 @@ constexpr int EQ_CAP = 1024;
 constexpr int LIST_ALL = 1024;       // rows of so few logits are sorted whole
 constexpr int CL_CTAS = 8;           // CTAs of a long row, at most
 constexpr int CL_GROUPS = 1024;      // disjoint groups of a long row whose maxima give the threshold
-constexpr int CL_CAP = 2048;         // elements at or above it that are sorted directly
+constexpr int CL_CAP = TOPK_THREADS; // elements at or above it that are sorted directly, one a thread
 constexpr int CL_MIN_V = 16384;      // rows from which that beats the radix select (and 512 of the groups hold something)
 
 // monotone map fp32 -> uint32 (larger float <=> larger key); -0 < +0 is irrelevant here
@@ -218,18 +218,62 @@ __device__ __forceinline__ void bitonic_sort_lanes(unsigned long long* buf, int 
   __syncthreads();
 }
 
+// the elements of the row whose keys are above v -> list (CL_CAP of them at most), their number -> *cnt (0 before; more than CL_CAP: too many)
+__device__ __noinline__ void list_above(const float* __restrict__ r, int V4, int V, uint32_t v, unsigned long long* list, unsigned int* cnt) {
+  const float4* r4 = reinterpret_cast<const float4*>(r);
+  bool full = false;
+  auto take = [&](float x, int i) {
+    const uint32_t k = f2key(x);
+    if (k > v && !full) {
+      const uint32_t at = atomicAdd(cnt, 1u);
+      if (at < CL_CAP) list[at] = pack_cand(k, (uint32_t)i);
+      else full = true;
+    }
+  };
+#pragma unroll 4
+  for (int i = threadIdx.x; i < V4; i += TOPK_THREADS) {
+    const float4 x = r4[i];
+    take(x.x, 4 * i);
+    take(x.y, 4 * i + 1);
+    take(x.z, 4 * i + 2);
+    take(x.w, 4 * i + 3);
+  }
+  for (int i = 4 * V4 + threadIdx.x; i < V; i += TOPK_THREADS) take(r[i], i);
+  __syncthreads();
+}
+
+// list[have .. SAMPLE_K) = the first elements whose key is v, in the order of their indices (there are enough of them)
+__device__ __noinline__ void fill_with_ties(const float* __restrict__ r, int V, uint32_t v, unsigned long long* list, int have) {
+  __shared__ int warp_hits[TOPK_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int b = 0; b < V && have < SAMPLE_K; b += TOPK_THREADS) {
+    const int i = b + threadIdx.x;
+    const bool hit = i < V && f2key(r[i]) == v;
+    const uint32_t m = __ballot_sync(0xffffffffu, hit);
+    if (lane == 0) warp_hits[warp] = __popc(m);
+    __syncthreads();
+    const int w = warp_hits[lane], at = have + (int)__reduce_add_sync(0xffffffffu, lane < warp ? w : 0) + __popc(m & ((1u << lane) - 1));
+    if (hit && at < SAMPLE_K) list[at] = pack_cand(v, (uint32_t)i);
+    have += (int)__reduce_add_sync(0xffffffffu, w);
+    __syncthreads();
+  }
+}
+
 // Long rows: a cluster of eight CTAs (fewer where rows are many: those of all rows are resident together) cuts a row.  The 256th largest of 1024 disjoint groups' maxima is a threshold that at least 256 elements reach
 // (about 300 of a row in no particular order, whatever its length; the groups are strided, so runs of large neighbours spread over them).
 // Every CTA finds it from all the maxima (a bit at a time, one barrier each), lists the elements of its slice that reach it with the first CTA,
-// and that one sorts them.  Rows that put more than CL_CAP elements there (long runs of ties, rows masked almost everywhere) go through the radix
-// select, as do shorter rows.  Bound by the latency of the steps: two passes over the slice (the second from L1), two cluster barriers, 32 counts,
-// the sort.  Measured (us with the events around it, one CTA a row / now): one row of 128256 70 / 20, 23 rows 70 / 27, 128 rows 72 / 36; 16384: 35 / 16, 35 / 23,
-// 37 / 25; 200 rows, two waves: 113 / 61.
-__global__ void __launch_bounds__(TOPK_THREADS)
+// and that one sorts them.  Rows that put more than CL_CAP elements there (rows masked almost everywhere, long runs of ties) have that many at the
+// 256th largest maximum itself: the first CTA then lists the elements above it, and the first of those that equal it fill the list up.  Where those
+// above are too many as well (their groups hold many large elements) the row goes through the radix select, as do shorter rows.  Bound by the latency
+// of the steps: two passes over the slice (the second from L1), two cluster barriers, 24 counts, the sort; 32 registers, so that two CTAs share an SM.
+// Measured (us with the events around it, one CTA a row / now): one row of 128256 45 / 19, 23 rows 71 / 26, 128 rows 72 / 36; 16384: 39 / 18, 43 / 24, 42 / 25; 200
+// rows, two waves: 110 / 54.  Masked but for 40 elements, one CTA a row / all listed, then the radix select / now: 23 rows of 128256 102 / 164 / 40, 32000 39 / 70 /
+// 29, 16384 33 / 50 / 28.
+__global__ void __launch_bounds__(TOPK_THREADS, 2)
     topk_cluster_kernel(const float* __restrict__ logits, int64_t row_stride, float* __restrict__ cand_val, int64_t* __restrict__ cand_idx, int V,
                         int64_t idx_offset) {
   __shared__ uint32_t group_max[CL_GROUPS];
-  __shared__ unsigned long long list[CL_CAP];
+  __shared__ unsigned long long list[2 * CL_CAP];  // the elements listed, and room for the sort
   __shared__ unsigned int s_cnt;
   const int tid = threadIdx.x, rank = (int)cluster_ctarank(), ctas = (int)cluster_nctarank();  // a power of two
   const int64_t row = blockIdx.x / ctas;
@@ -262,12 +306,14 @@ __global__ void __launch_bounds__(TOPK_THREADS)
     if (__syncthreads_count(mine >= t) >= SAMPLE_K) thr = t;
   }
   const uint32_t cnt0 = mapa_shared(smem_u32(&s_cnt), 0), list0 = mapa_shared(smem_u32(list), 0);
+  bool full = false;  // a thread that finds no place left walks no further
   auto take = [&](float x, int i) {
     const uint32_t k = f2key(x);
-    if (k >= thr) {
+    if (k >= thr && !full) {
       uint32_t at;
       asm volatile("atom.shared::cluster.add.u32 %0, [%1], 1;\n" : "=r"(at) : "r"(cnt0) : "memory");
       if (at < CL_CAP) asm volatile("st.shared::cluster.u64 [%0], %1;\n" ::"r"(list0 + 8 * at), "l"(pack_cand(k, (uint32_t)i)) : "memory");
+      else full = true;
     }
   };
 #pragma unroll 4
@@ -283,17 +329,30 @@ __global__ void __launch_bounds__(TOPK_THREADS)
   if (rank != 0) return;
   cand_val += row * SAMPLE_K;
   cand_idx += row * SAMPLE_K;
-  const int cnt = (int)s_cnt;
+  int cnt = (int)s_cnt;
   if (cnt > CL_CAP) {
-    topk_radix_row(r, V, cand_val, cand_idx, idx_offset);
-    return;
+    for (int b = 7; b >= 0; --b) {  // the rest of the bits: thr is the 256th largest maximum
+      const uint32_t t = thr | (1u << b);
+      if (__syncthreads_count(mine >= t) >= SAMPLE_K) thr = t;
+    }
+    if (tid == 0) s_cnt = 0;
+    __syncthreads();
+    list_above(r, V4, V, thr, list, &s_cnt);
+    cnt = (int)s_cnt;
+    if (cnt > CL_CAP) {
+      topk_radix_row(r, V, cand_val, cand_idx, idx_offset);
+      return;
+    }
+    if (cnt < SAMPLE_K) {
+      fill_with_ties(r, V, thr, list, cnt);
+      cnt = SAMPLE_K;
+    }
   }
   int n2 = SAMPLE_K;
   while (n2 < cnt) n2 <<= 1;
   for (int i = cnt + tid; i < n2; i += TOPK_THREADS) list[i] = 0ull;
   __syncthreads();
-  if (n2 <= TOPK_THREADS) bitonic_sort_lanes(list, n2);
-  else bitonic_sort_desc(list, n2);
+  bitonic_sort_lanes(list, n2);
   write_candidates(list, SAMPLE_K, cand_val, cand_idx, idx_offset);
 }
 
