@@ -158,7 +158,8 @@ int b200_paged_attn_prefill(const void* q, int64_t q_token_stride, const void* k
  *   shape from occupancy queries and a latency/bandwidth model (b200_gemm_decode_plan reports it).
  *   Weight-only batches (INT8_WO) of wide weights take 256 weight rows per CTA instead where split_k is 0.  M <= 8 (INT8_WO: 16) with split_k = 0:
  *   CTAs of 16 or 32 weight rows whose warps share K and multiply out of registers (gemm_small.cu).  Weights whose tiles of 256 rows fill
- *   the waves of CTA pairs go there with split_k = 0 (bf16, fp8 and int8; b200_gemm_decode_plan still reports the schedule of this paragraph).
+ *   the waves of CTA pairs go there with split_k = 0 (bf16, fp8 and int8) where this schedule would not cut K, so that the sums are the same
+ *   (b200_gemm_decode_plan still reports the schedule of this paragraph).
  * M > 128 (prefill), split_k = 0: CTA pairs, each on whole tiles of 256 weight rows x 64 to 256 tokens; where few tiles walk a long K, and for
  *   INT8_WO, the schedule of an explicit split_k:
  *   persistent stream-K over min(split_k, #SM) CTAs (0 = one per SM), each an equal share of the (tile, k-block) space; tiles cut by a share

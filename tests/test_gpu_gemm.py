@@ -245,6 +245,18 @@ def test_gemm_decode_batches_on_pairs(ops, m, n, k, f32):
     test_gemm_pairs_bf16_against_64_bits(ops, m, n, k, f32)
 
 
+@pytest.mark.parametrize("m,n,k", [(41, 10272, 2048), (64, 12288, 4096), (17, 16032, 4096), (100, 6144, 4096)])
+@pytest.mark.parametrize("kind", ["bf16", "fp8"])
+def test_gemm_decode_batches_cut_k_as_their_plan_says(ops, kind, m, n, k):
+    """The sums of a call that names no split are those of the split that the plan reports: a longer sum would lose more low bits."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    dt = torch.bfloat16 if kind == "bf16" else torch.float8_e4m3fn
+    a, w = torch.randn(m, k, generator=g, device="cuda").to(dt), torch.randn(n, k, generator=g, device="cuda").to(dt)
+    split = ops.gemm_decode_plan(m, n, k, ops._ab_dtype(a))["split"]
+    assert m > 64 or split > 1
+    assert torch.equal(ops.gemm(a, w, out_dtype=torch.float32), ops.gemm(a, w, out_dtype=torch.float32, split_k=split))
+
+
 @pytest.mark.parametrize("m,n,k", [(257, 1001, 192), (777, 6144, 520)])
 @pytest.mark.parametrize("f32", [False, True])
 def test_gemm_pairs_rows_of_odd_length_and_two_token_tiles(ops, m, n, k, f32):

@@ -201,7 +201,7 @@ struct PairPlan {
   int bt, wide;
 };
 PairPlan pair_plan(int M, int N, int K, int ab_dtype);
-bool pair_takes_decode(int M, int N, int K, int ab_dtype);  // up to 128 tokens: whether the pairs are faster than the decode schedule
+bool pair_takes_decode(int M, int N, int K, int ab_dtype);  // up to 128 tokens: whether the pairs are faster than the decode schedule that walks all of K
 int launch_gemm_pair(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, PairPlan plan,
                      cudaStream_t stream);
 

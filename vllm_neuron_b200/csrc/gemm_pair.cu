@@ -357,13 +357,13 @@ PairPlan pair_plan(int M, int N, int K, int ab_dtype) {
   return stream_k_us * 1850.0 < (pair_cost > walk ? pair_cost : walk) ? PairPlan{0, 0} : best;  // clocks at 1.85 GHz
 }
 
-// Decode-sized batches on CTA pairs: the decode schedule cuts K over clusters, so every SM reads weights whatever N is, and pays for the partial sums; pairs
-// walk the whole K, which takes no longer where their tiles fill the waves, or where K is short.  A wave of pairs is bound by its k-blocks (0.247 us each) or by its weights
-// (5.9 TB/s), behind 9.5 us of launch, first loads and epilogue; the decode schedule takes 12 us and 5.7 TB/s up to 64 tokens, 15 us and 5.0 TB/s
-// above, where its tile of 128 tokens halves the ring.  The pairs have to win by a twentieth, above 64 tokens by 0.15: they have no rotating epilogue, and a qkv
-// projection that they take needs another launch (b200_gemm_rope_kv_write keeps the bits of the two calls).  Measured, us, decode schedule / pairs, L2 flushed: bf16 64 x 10272 x 2048 22.5 / 18.5, 128 30.7 /
-// 20.5; 64 x 55296 x 5120 113 / 101, 128 131 / 103; 64 x 28672 x 4096 55.3 / 55.3, 128 63.5 / 55.4; 128 x 4096 x 4096 24.6 / 26.6, 64 x 8192 x 28672 94 / 121;
-// fp8 128 x 6144 x 4096 24.5 / 20.5, 64 18.5 / 18.4.  Over 160 such calls (17 to 128 tokens, 16 weights) the choice costs 0.4 % more than the better one.
+// Decode-sized batches whose K the decode schedule does not cut (decode_on_pairs asks for that: bf16, fp8 and int8, 9 to 128 tokens, every epilogue but the
+// rotating one).  A wave of pairs is bound by its k-blocks (0.247 us each) or by its weights (5.9 TB/s), behind 9.5 us of launch, first loads and epilogue; the
+// decode schedule takes 12 us and 5.7 TB/s up to 64 tokens, 15 us and 5.0 TB/s above, where its tile of 128 tokens halves the ring.  The pairs have to
+// win by a twentieth, above 64 tokens by 0.15.  Measured, us, decode schedule / pairs, L2 flushed: bf16 128 x 10272 x 2048 32.8 / 20.5, 64 x 55296 x 5120
+// 119 / 101, 12 tokens 115 / 100, SiLU 128 139 / 102, 64 x 28672 x 4096 57.3 / 55.3, 128 fp32 63.5 / 57.3, 80 x 12288 x 4096 47.1 / 28.7; fp8 41 x 32000 x 2048
+// 24.6 / 22.5, 128 x 28672 x 4096 SiLU 43.0 / 34.8; int8 64 x 49152 x 2048 38.9 / 28.7.  Over 492 such calls (20 weights, 12 to 128 tokens, linear, fp32 and
+// SiLU outputs) the rule never takes the slower side by more than 3 %.
 bool pair_takes_decode(int M, int N, int K, int ab_dtype) {
   const double row = (double)K * (ab_dtype == B200_BF16 ? 2 : 1), steps = 0.247 * ((row + GEMM_BK_BYTES - 1) / GEMM_BK_BYTES);
   const int pairs = sm_count() / 2, tiles = (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN), rest = tiles % pairs;

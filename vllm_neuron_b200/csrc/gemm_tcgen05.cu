@@ -1262,6 +1262,34 @@ int launch_rope(const CUtensorMap& wm, const CUtensorMap& am, const GemmEpilogue
   return launch_decode<KIND, 128, EPI_ROPE>(wm, am, ep, M, N, p, split_k, stream);
 }
 
+template <int KIND, int EPI>
+int query_plan(DecodeCfg& c, const GemmPlan& p, int M, int split_k, bool resid) {
+  if (p.bm == 32) return plan_decode<KIND, 32, EPI>(c, M, p.n_tiles, p.num_kb, split_k, resid);
+  if (p.bm == 64) return plan_decode<KIND, 64, EPI>(c, M, p.n_tiles, p.num_kb, split_k, resid);
+  return plan_decode<KIND, 128, EPI>(c, M, p.n_tiles, p.num_kb, split_k, resid);
+}
+template <int EPI>
+int query_plan(DecodeCfg& c, const GemmPlan& p, int M, int ab_dtype, int split_k, bool resid) {
+  return ab_dtype == B200_BF16       ? query_plan<KIND_F16, EPI>(c, p, M, split_k, resid)
+         : ab_dtype == B200_FP8_E4M3 ? query_plan<KIND_F8F6F4, EPI>(c, p, M, split_k, resid)
+         : ab_dtype == B200_INT8_WO  ? query_plan<KIND_WO8, EPI>(c, p, M, split_k, resid)
+                                     : query_plan<KIND_I8, EPI>(c, p, M, split_k, resid);
+}
+int query_plan(DecodeCfg& c, const GemmPlan& p, int epi, int M, int ab_dtype, int split_k, bool resid) {
+  return epi == EPI_ROPE       ? query_plan<EPI_ROPE>(c, p, M, ab_dtype, split_k, resid)
+         : epi == EPI_SILU_MUL ? query_plan<EPI_SILU_MUL>(c, p, M, ab_dtype, split_k, resid)
+                               : query_plan<EPI_LINEAR>(c, p, M, ab_dtype, split_k, resid);
+}
+
+// Whether a decode-sized call runs on CTA pairs: where those are faster, and only where the decode schedule would not cut K either, so that the sums are
+// the same bit for bit.  The tensor cores cut the low bits of a sum at every 16 products, so a longer sum is a less precise one (fp32 outputs against 64
+// bits, cut as the decode schedule cuts / whole: 41 x 10272 x 2048 bf16 0.6e-6 / 2.1e-6, 41 x 12288 x 4096 2.1e-6 / 4.4e-6, fp8 7.5e-8 / 1.0e-7).
+bool decode_on_pairs(const GemmPlan& p, int epi, int M, int N, int K, int ab_dtype, int split_k, bool resid) {
+  DecodeCfg c;
+  return ab_dtype != B200_INT8_WO && split_k == 0 && epi != EPI_ROPE && pair_takes_decode(M, N, K, ab_dtype) &&
+         query_plan(c, p, epi, M, ab_dtype, 0, resid) == B200_OK && c.S == 1;
+}
+
 int gemm_common(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype,
                 int split_k, void* workspace, size_t workspace_bytes, void* stream) {
   B200_REQUIRE(a && w && ep.out, "gemm: null pointer");
@@ -1292,7 +1320,8 @@ int gemm_common(const void* a, const void* w, const GemmEpilogue& ep, int epi, i
   if (wide) return launch_gemm_wo(a, w, ep, epi, M, N, K, (cudaStream_t)stream);
   // prompt-sized batches run on CTA pairs, and decode-sized ones where those are faster; stream-K keeps the shapes where cutting K is faster, the
   // weight-only kind, whose tiles are widened on the way, and calls that cap its CTAs
-  if (const PairPlan plan = !wo && split_k == 0 && (!p.decode || (epi != EPI_ROPE && pair_takes_decode(M, N, K, ab_dtype))) ? pair_plan(M, N, K, ab_dtype) : PairPlan{0, 0}; plan.bt)
+  const bool on_pairs = p.decode ? decode_on_pairs(p, epi, M, N, K, ab_dtype, split_k, ep.residual != nullptr) : !wo && split_k == 0;
+  if (const PairPlan plan = on_pairs ? pair_plan(M, N, K, ab_dtype) : PairPlan{0, 0}; plan.bt)
     return launch_gemm_pair(a, w, ep, epi, M, N, K, ab_dtype, plan, (cudaStream_t)stream);
   CUtensorMapDataType dt = eb == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
   int bk = GEMM_BK_BYTES / eb;
@@ -1326,15 +1355,6 @@ int gemm_common(const void* a, const void* w, const GemmEpilogue& ep, int epi, i
   return dispatch_gemm<KIND_I8, EPI_SILU_MUL>(wm, am, ep, workspace, M, N, p, split_k, s);
 }
 
-}  // namespace
-
-namespace {
-template <int KIND, int EPI>
-int query_plan(DecodeCfg& c, int bm, int M, int n_tiles, int num_kb, int split_k, bool resid) {
-  if (bm == 32) return plan_decode<KIND, 32, EPI>(c, M, n_tiles, num_kb, split_k, resid);
-  if (bm == 64) return plan_decode<KIND, 64, EPI>(c, M, n_tiles, num_kb, split_k, resid);
-  return plan_decode<KIND, 128, EPI>(c, M, n_tiles, num_kb, split_k, resid);
-}
 }  // namespace
 
 namespace {
@@ -1399,23 +1419,7 @@ int b200_gemm_decode_plan(int M, int N, int K, int ab_dtype, int split_k, int si
     return rc;
   }
   DecodeCfg c{};
-  const bool r = has_residual != 0;
-  if (silu_mul == 2) {  // the qkv GEMM with the RoPE / KV-write epilogue
-    rc = ab_dtype == B200_BF16 ? query_plan<KIND_F16, EPI_ROPE>(c, p.bm, M, p.n_tiles, p.num_kb, split_k, r)
-         : ab_dtype == B200_FP8_E4M3 ? query_plan<KIND_F8F6F4, EPI_ROPE>(c, p.bm, M, p.n_tiles, p.num_kb, split_k, r)
-         : ab_dtype == B200_INT8_WO  ? query_plan<KIND_WO8, EPI_ROPE>(c, p.bm, M, p.n_tiles, p.num_kb, split_k, r)
-                                     : query_plan<KIND_I8, EPI_ROPE>(c, p.bm, M, p.n_tiles, p.num_kb, split_k, r);
-  } else if (silu_mul) {
-    rc = ab_dtype == B200_BF16 ? query_plan<KIND_F16, EPI_SILU_MUL>(c, p.bm, M, p.n_tiles, p.num_kb, split_k, r)
-         : ab_dtype == B200_FP8_E4M3 ? query_plan<KIND_F8F6F4, EPI_SILU_MUL>(c, p.bm, M, p.n_tiles, p.num_kb, split_k, r)
-         : ab_dtype == B200_INT8_WO  ? query_plan<KIND_WO8, EPI_SILU_MUL>(c, p.bm, M, p.n_tiles, p.num_kb, split_k, r)
-                                     : query_plan<KIND_I8, EPI_SILU_MUL>(c, p.bm, M, p.n_tiles, p.num_kb, split_k, r);
-  } else {
-    rc = ab_dtype == B200_BF16 ? query_plan<KIND_F16, EPI_LINEAR>(c, p.bm, M, p.n_tiles, p.num_kb, split_k, r)
-         : ab_dtype == B200_FP8_E4M3 ? query_plan<KIND_F8F6F4, EPI_LINEAR>(c, p.bm, M, p.n_tiles, p.num_kb, split_k, r)
-         : ab_dtype == B200_INT8_WO  ? query_plan<KIND_WO8, EPI_LINEAR>(c, p.bm, M, p.n_tiles, p.num_kb, split_k, r)
-                                     : query_plan<KIND_I8, EPI_LINEAR>(c, p.bm, M, p.n_tiles, p.num_kb, split_k, r);
-  }
+  rc = query_plan(c, p, epi, M, ab_dtype, split_k, has_residual != 0);
   if (rc) return rc;
   out6[0] = c.S;
   out6[1] = c.smem > SMEM_TWO_PER_SM ? 1 : 2;
@@ -1455,8 +1459,7 @@ int b200_gemm_rope_kv_write(const void* a, const void* w, void* qkv_out, const f
   // sizes) runs the GEMM, then the RoPE/scatter kernel: same bits either way.
   bool fused = false;
   const bool wide_wo = ab_dtype == B200_INT8_WO && split_k == 0 && gemm_wo_wide(EPI_ROPE, M, N, K);  // its own schedule, without the rotation
-  const bool on_pairs = split_k == 0 && ab_dtype != B200_INT8_WO && K > 0 && pair_takes_decode(M, N, K, ab_dtype);  // the linear call's schedule
-  if (M <= 128 && !wide_wo && !on_pairs && (D == 64 || D == 128) && N % GEMM_BN == 0 && max_pos > 0 &&
+  if (M <= 128 && !wide_wo && (D == 64 || D == 128) && N % GEMM_BN == 0 && max_pos > 0 &&
       (ab_dtype == B200_BF16 || ab_dtype == B200_FP8_E4M3 || ab_dtype == B200_INT8 || ab_dtype == B200_INT8_WO)) {
     int plan6[6];
     if (b200_gemm_decode_plan(M, N, K, ab_dtype, split_k, 2, 0, plan6) == B200_OK && plan6[0] > 1) fused = true;
