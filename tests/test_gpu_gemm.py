@@ -257,6 +257,15 @@ def test_gemm_decode_batches_cut_k_as_their_plan_says(ops, kind, m, n, k):
     assert torch.equal(ops.gemm(a, w, out_dtype=torch.float32), ops.gemm(a, w, out_dtype=torch.float32, split_k=split))
 
 
+@pytest.mark.parametrize("m,n,k", [(129, 3584, 18944), (512, 1024, 28672), (256, 8192, 28672)])
+def test_gemm_prompts_against_a_long_k_keep_the_cut_sums(ops, m, n, k):
+    """Few tiles that walk a long K: the sums are those of stream-K over every SM, not one long sum a tile."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a, w = torch.randn(m, k, generator=g, device="cuda").bfloat16(), torch.randn(n, k, generator=g, device="cuda").bfloat16()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert torch.equal(ops.gemm(a, w, out_dtype=torch.float32), ops.gemm(a, w, out_dtype=torch.float32, split_k=sms))
+
+
 @pytest.mark.parametrize("m,n,k", [(257, 1001, 192), (777, 6144, 520)])
 @pytest.mark.parametrize("f32", [False, True])
 def test_gemm_pairs_rows_of_odd_length_and_two_token_tiles(ops, m, n, k, f32):

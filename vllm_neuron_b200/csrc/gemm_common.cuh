@@ -195,12 +195,13 @@ __device__ __forceinline__ void epilogue_chunk_xpose(const GemmEpilogue& ep, con
 bool gemm_wo_wide(int epi, int M, int N, int K);
 int gemm_wo_plan(int epi, int M, int N, int K, int& splits, int& cap_ctas, int& stages, size_t& smem);
 int launch_gemm_wo(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, cudaStream_t stream);
-// Prompt-sized schedule on CTA pairs (gemm_pair.cu): bf16, fp8 and int8 operands.  bt: tokens of a tile, 0 where stream-K is the faster
-// schedule; wide: how many units of two token tiles come before those of one.
+// Schedule on CTA pairs (gemm_pair.cu): bf16, fp8 and int8 operands.  bt: tokens of a tile; wide: how many units of two token tiles come before those
+// of one.
 struct PairPlan {
   int bt, wide;
 };
 PairPlan pair_plan(int M, int N, int K, int ab_dtype);
+bool stream_k_keeps(int M, int N, int K, int ab_dtype);     // prompt-sized calls: whether stream-K takes them instead
 bool pair_takes_decode(int M, int N, int K, int ab_dtype);  // up to 128 tokens: whether the pairs are faster than the decode schedule that walks all of K
 int launch_gemm_pair(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, PairPlan plan,
                      cudaStream_t stream);

@@ -321,11 +321,6 @@ int launch_pair(const void* a, const void* w, const GemmEpilogue& ep, int M, int
 // plan on average, 14 % at most, and 0.966 of what the constants from before the MMAs were issued by an elected lane chose; 0.97 or less in 203
 // calls, over 1.03 in four (1.05 at most).
 // Measured (us, those constants / now, bf16): 777 x 6144 x 4096 50.0 / 39.2, 777 x 28672 x 4096 144 / 132, 2048 tokens of an fp8 prompt step 4265 / 4127.
-// bt = 0: stream-K (gemm_tcgen05.cu) takes the call.  It cuts K, which pays where few tiles walk a very long K: about 18 us, 0.52 for each
-// k-block of 128 x 256 of an SM's share, 7.5 for every CTA that adds to one tile and 0.03 a token; a pair's walk takes at least 500 clocks a k-block.
-// Measured (us, pairs / stream-K, bf16): 129 x 2048 x 53248 213 / 139, 300 x 2048 x 53248 215 / 174, 512 x 2560 x 53248 221 / 209, 1290 x 512 x 53248
-// 217 / 154; 129 x 5120 x 27648 121 / 111, 256 123 / 121; 300 x 1024 x 28672 119 / 125, 1400 150 / 148; 129 x 8192 x 28672 131 / 139.  Over 398 measured
-// calls (bf16 and fp8, 129 to 2000 tokens) the rule takes the slower side by more than 4 % in two, by 5 % at most.
 PairPlan pair_plan(int M, int N, int K, int ab_dtype) {
   const int eb = ab_dtype == B200_BF16 ? 2 : 1, sms = sm_count();
   const int pairs = sms / 2, num_kb = (K * eb + GEMM_BK_BYTES - 1) / GEMM_BK_BYTES, n_tiles = (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN);
@@ -351,10 +346,28 @@ PairPlan pair_plan(int M, int N, int K, int ab_dtype) {
       offer(bt, (int)wide, waves * wide_cost + (waves - 1) * 2500 + (un.units - wide + pairs - 1) / pairs * lone_cost);
     }
   }
+  return best;
+}
+
+// Whether a prompt-sized call stays with stream-K (gemm_tcgen05.cu), which cuts K: few tiles against a long K, or a nearly empty wave behind a full one.  Its
+// time is about 25 us, 0.52 for each k-block of 128 x 256 of an SM's share and 8 for every CTA that adds to one tile; a wave of pairs stands here with the cost
+// that it had while an MMA took 95 clocks to issue (640 clocks a k-block up to 128 tokens, from there 3 for each of the 128 + bt / 2 operand rows).  With
+// today's costs the pairs would take more calls, up to 0.6 of the time, but they walk all of K in one accumulator, and the tensor cores cut the low bits
+// of a sum at every 16 products, so a sum that stream-K cuts would lose more of them.  Measured, bf16, us and error of fp32 outputs against 64 bits, stream-K /
+// pairs: 129 x 3584 x 18944 107 / 86, 0.36e-5 / 2.2e-5; 129 x 8192 x 28672 139 / 135, 1.2e-5 / 3.3e-5; 512 x 1024 x 28672 135 / 127, 0.32e-5 / 3.3e-5;
+// 777 x 5120 x 27648 305 / 186, 2.3e-5 / 3.2e-5; fp8 4096 x 32000 x 2048 406 / 180, 7.05e-8 / 7.07e-8.
+bool stream_k_keeps(int M, int N, int K, int ab_dtype) {
+  const int eb = ab_dtype == B200_BF16 ? 2 : 1, sms = sm_count();
+  const int pairs = sms / 2, num_kb = (K * eb + GEMM_BK_BYTES - 1) / GEMM_BK_BYTES, n_tiles = (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN);
+  long long pair_cost = LLONG_MAX;
+  for (int bt = PAIR_MAX_BT; bt >= 64; bt -= 32) {
+    const long long tiles = (long long)((M + bt - 1) / bt) * n_tiles, waves = (tiles + pairs - 1) / pairs;
+    const long long cost = waves * ((long long)num_kb * (bt <= 128 ? 640 : 3 * (GEMM_BN + bt / 2)) + 2500 + 10 * bt);
+    if (cost < pair_cost) pair_cost = cost;
+  }
   const double sk_tiles = (double)((M + 255) / 256) * ((N + GEMM_BN - 1) / GEMM_BN), shared = sms / sk_tiles;
-  const double stream_k_us = 18.0 + 0.52 * sk_tiles * num_kb / sms + 7.5 * (shared > 1.0 ? shared : 1.0) + 0.03 * M;
-  const double pair_cost = (double)best_cost, walk = 500.0 * num_kb + 5000.0;  // one wave's walk from memory
-  return stream_k_us * 1850.0 < (pair_cost > walk ? pair_cost : walk) ? PairPlan{0, 0} : best;  // clocks at 1.85 GHz
+  const double stream_k_us = 25.0 + 0.52 * sk_tiles * num_kb / sms + 8.0 * (shared > 1.0 ? shared : 1.0);
+  return stream_k_us * 1850.0 < (double)pair_cost;  // clocks at 1.85 GHz
 }
 
 // Decode-sized batches whose K the decode schedule does not cut (decode_on_pairs asks for that: bf16, fp8 and int8, 9 to 128 tokens, every epilogue but the
@@ -363,7 +376,7 @@ PairPlan pair_plan(int M, int N, int K, int ab_dtype) {
 // win by a twentieth, above 64 tokens by 0.15.  Measured, us, decode schedule / pairs, L2 flushed: bf16 128 x 10272 x 2048 32.8 / 20.5, 64 x 55296 x 5120
 // 119 / 101, 12 tokens 115 / 100, SiLU 128 139 / 102, 64 x 28672 x 4096 57.3 / 55.3, 128 fp32 63.5 / 57.3, 80 x 12288 x 4096 47.1 / 28.7; fp8 41 x 32000 x 2048
 // 24.6 / 22.5, 128 x 28672 x 4096 SiLU 43.0 / 34.8; int8 64 x 49152 x 2048 38.9 / 28.7.  Over 492 such calls (20 weights, 12 to 128 tokens, linear, fp32 and
-// SiLU outputs) the rule never takes the slower side by more than 3 %.
+// SiLU outputs) none that goes to the pairs is slower there by more than 3 %.
 bool pair_takes_decode(int M, int N, int K, int ab_dtype) {
   const double row = (double)K * (ab_dtype == B200_BF16 ? 2 : 1), steps = 0.247 * ((row + GEMM_BK_BYTES - 1) / GEMM_BK_BYTES);
   const int pairs = sm_count() / 2, tiles = (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN), rest = tiles % pairs;

@@ -1318,11 +1318,10 @@ int gemm_common(const void* a, const void* w, const GemmEpilogue& ep, int epi, i
   // decode-sized batches of the weight-only kind: 256 weight rows per CTA (narrow weights, and calls that name their K splits, keep the
   // 128-row schedule)
   if (wide) return launch_gemm_wo(a, w, ep, epi, M, N, K, (cudaStream_t)stream);
-  // prompt-sized batches run on CTA pairs, and decode-sized ones where those are faster; stream-K keeps the shapes where cutting K is faster, the
+  // prompt-sized batches run on CTA pairs, and decode-sized ones where those are faster; stream-K keeps the shapes whose sums it cuts to advantage, the
   // weight-only kind, whose tiles are widened on the way, and calls that cap its CTAs
-  const bool on_pairs = p.decode ? decode_on_pairs(p, epi, M, N, K, ab_dtype, split_k, ep.residual != nullptr) : !wo && split_k == 0;
-  if (const PairPlan plan = on_pairs ? pair_plan(M, N, K, ab_dtype) : PairPlan{0, 0}; plan.bt)
-    return launch_gemm_pair(a, w, ep, epi, M, N, K, ab_dtype, plan, (cudaStream_t)stream);
+  if (p.decode ? decode_on_pairs(p, epi, M, N, K, ab_dtype, split_k, ep.residual != nullptr) : !wo && split_k == 0 && !stream_k_keeps(M, N, K, ab_dtype))
+    return launch_gemm_pair(a, w, ep, epi, M, N, K, ab_dtype, pair_plan(M, N, K, ab_dtype), (cudaStream_t)stream);
   CUtensorMapDataType dt = eb == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
   int bk = GEMM_BK_BYTES / eb;
   CUtensorMap wm, am;
