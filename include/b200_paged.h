@@ -158,8 +158,7 @@ int b200_paged_attn_prefill(const void* q, int64_t q_token_stride, const void* k
  *   shape from occupancy queries and a latency/bandwidth model (b200_gemm_decode_plan reports it).
  *   Weight-only batches (INT8_WO) of wide weights take 256 weight rows per CTA instead where split_k is 0.  M <= 8 (INT8_WO: 16) with split_k = 0:
  *   CTAs of 16 or 32 weight rows whose warps share K and multiply out of registers (gemm_small.cu).  Weights whose tiles of 256 rows fill
- *   the waves of CTA pairs go there with split_k = 0 (bf16, fp8 and int8) where this schedule would not cut K, so that the sums are the same
- *   (b200_gemm_decode_plan still reports the schedule of this paragraph).
+ *   the waves of CTA pairs go there with split_k = 0 (bf16, fp8 and int8) where this schedule would not cut K, so that the sums are the same.
  * M > 128 (prefill), split_k = 0: CTA pairs, each on whole tiles of 256 weight rows x 64 to 256 tokens; where few tiles walk a long K, and for
  *   INT8_WO, the schedule of an explicit split_k:
  *   persistent stream-K over min(split_k, #SM) CTAs (0 = one per SM), each an equal share of the (tile, k-block) space; tiles cut by a share
@@ -170,8 +169,12 @@ size_t b200_gemm_workspace_bytes(int M, int N, int K, int ab_dtype, int split_k)
 /* The decode schedule (M <= 128) chosen on the current device for a shape: out6 = {cluster size S, CTAs per SM, weight
  * ring depth, activation ring depth, CTAs the chip holds at once, dynamic shared memory bytes}.  Needs a device.
  * silu_mul selects the epilogue variant planned for: 0 linear, 1 SiLU*mul (b200_gemm_silu_mul), 2 RoPE + KV write
- * (b200_gemm_rope_kv_write).  A few tokens (no rings): S = 1, 0 bytes, depths = lines of 128 bytes that a warp has in flight; 2 assumes heads of a multiple of 32.  Weight-only batches on 256 weight rows: the cluster size of the cut tiles; both rings have one depth. */
+ * (b200_gemm_rope_kv_write).  A few tokens (no rings): S = 1, 0 bytes, depths = lines of 128 bytes that a warp has in flight; 2 assumes heads of a multiple of 32.  Weight-only batches on 256 weight rows: the cluster size of the cut tiles; both rings have one depth.
+ * CTA pairs: S = 1, one CTA per SM, both rings one depth. */
 int b200_gemm_decode_plan(int M, int N, int K, int ab_dtype, int split_k, int silu_mul, int has_residual, int* out6);
+/* Calls of any M with split_k = 0: out4 = {tokens of a tile, units of two token tiles, all units that the CTA pairs share, ring depth}, zeros where
+ * another schedule takes the call.  silu_mul 0 or 1 as above.  Needs a device. */
+int b200_gemm_pair_plan(int M, int N, int K, int ab_dtype, int silu_mul, int has_residual, int* out4);
 /* Profiling aid: with a non-NULL device buffer ([#CTAs][8] uint64) every decode-schedule GEMM CTA records %globaltimer
  * at its phase boundaries (tools/gemm_trace.py); NULL (default) switches it off. */
 void b200_gemm_set_trace(void* device_buf);

@@ -651,3 +651,19 @@ def test_plan_of_a_few_tokens(ops, m, n, k, kind, epi, per_sm, lines):
     """CTAs an SM holds (16 warps of it) and lines of a warp in flight, by the size of the weights."""
     got = ops.gemm_decode_plan(m, n, k, getattr(ops, kind), silu_mul=epi)
     assert list(got.values()) == [1, per_sm, lines, lines, per_sm * torch.cuda.get_device_properties(0).multi_processor_count, 0]
+
+
+@pytest.mark.parametrize("m,n,k,kind,epi,on", [(64, 55296, 5120, "BF16", 0, True), (128, 12288, 4096, "FP8_E4M3", 2, True), (100, 28672, 4096, "INT8", 1, True), (64, 4096, 4096, "BF16", 0, False),
+                                               (41, 12288, 4096, "FP8_E4M3", 2, False), (64, 128256, 4096, "INT8_WO", 0, False)])
+def test_plan_of_decode_batches_on_pairs(ops, m, n, k, kind, epi, on):
+    """The plan of a call that the CTA pairs take is theirs: one CTA an SM, no cut of K, a ring of their stages of 128 rows of weights and their tokens."""
+    dt = getattr(ops, kind)
+    got, pair = ops.gemm_decode_plan(m, n, k, dt, silu_mul=epi), ops.gemm_pair_plan(m, n, k, dt, silu_mul=epi == 1)
+    assert (pair["tokens"] > 0) == on
+    if on:
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        assert pair["wide"] == 0 and pair["units"] == -(-m // pair["tokens"]) * -(-n // 256)
+        assert (got["split"], got["ctas_per_sm"], got["w_stages"], got["a_stages"], got["cap_ctas"]) == (1, 1, pair["stages"], pair["stages"], sms // 2 * 2)
+        assert got["smem"] >= pair["stages"] * (128 + pair["tokens"] // 2) * 128
+    else:
+        assert ops.gemm_decode_plan(m, n, k, dt, split_k=got["split"], silu_mul=epi) == got or kind == "INT8_WO"

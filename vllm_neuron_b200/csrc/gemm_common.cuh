@@ -203,6 +203,7 @@ struct PairPlan {
 PairPlan pair_plan(int M, int N, int K, int ab_dtype);
 bool stream_k_keeps(int M, int N, int K, int ab_dtype);     // prompt-sized calls: whether stream-K takes them instead
 bool pair_takes_decode(int M, int N, int K, int ab_dtype);  // up to 128 tokens: whether the pairs are faster than the decode schedule that walks all of K
+void pair_shape(int M, int N, PairPlan plan, int& units, int& stages, size_t& smem);  // what the pairs walk, their ring and shared memory
 int launch_gemm_pair(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype, PairPlan plan,
                      cudaStream_t stream);
 

@@ -313,6 +313,12 @@ int launch_pair(const void* a, const void* w, const GemmEpilogue& ep, int M, int
 
 }  // namespace
 
+void pair_shape(int M, int N, PairPlan p, int& units, int& stages, size_t& smem) {
+  units = PairUnits((M + p.bt - 1) / p.bt, (N + 2 * GEMM_BN - 1) / (2 * GEMM_BN), p.wide).units;
+  stages = pair_stages(pair_stage_bytes(p.bt, p.wide > 0));
+  smem = PAIR_SMEM_RING + 1024;
+}
+
 // Tokens of a tile, and whether a pair takes two token tiles at once.  A wave of tiles costs its k-blocks -- 320 + 0.625 bt clocks each, the operands'
 // way into shared memory and the MMAs' issue -- plus filling the ring, draining the last accumulator and the launch; so the widest tile wins unless
 // a narrower one saves a wave or the padding of the last token tile.  Two at once cost 250 + 2.75 bt clocks a k-block, both accumulators' epilogue at the

@@ -1289,6 +1289,12 @@ bool decode_on_pairs(const GemmPlan& p, int epi, int M, int N, int K, int ab_dty
   return ab_dtype != B200_INT8_WO && split_k == 0 && epi != EPI_ROPE && pair_takes_decode(M, N, K, ab_dtype) &&
          query_plan(c, p, epi, M, ab_dtype, 0, resid) == B200_OK && c.S == 1;
 }
+// Prompt-sized batches run on CTA pairs, and decode-sized ones where those are faster; stream-K keeps the shapes whose sums it cuts to advantage, the
+// weight-only kind, whose tiles are widened on the way, and calls that cap its CTAs.
+bool gemm_on_pairs(const GemmPlan& p, int epi, int M, int N, int K, int ab_dtype, int split_k, bool resid) {
+  if (p.decode) return decode_on_pairs(p, epi, M, N, K, ab_dtype, split_k, resid);
+  return ab_dtype != B200_INT8_WO && split_k == 0 && !stream_k_keeps(M, N, K, ab_dtype);
+}
 
 int gemm_common(const void* a, const void* w, const GemmEpilogue& ep, int epi, int M, int N, int K, int ab_dtype,
                 int split_k, void* workspace, size_t workspace_bytes, void* stream) {
@@ -1318,9 +1324,7 @@ int gemm_common(const void* a, const void* w, const GemmEpilogue& ep, int epi, i
   // decode-sized batches of the weight-only kind: 256 weight rows per CTA (narrow weights, and calls that name their K splits, keep the
   // 128-row schedule)
   if (wide) return launch_gemm_wo(a, w, ep, epi, M, N, K, (cudaStream_t)stream);
-  // prompt-sized batches run on CTA pairs, and decode-sized ones where those are faster; stream-K keeps the shapes whose sums it cuts to advantage, the
-  // weight-only kind, whose tiles are widened on the way, and calls that cap its CTAs
-  if (p.decode ? decode_on_pairs(p, epi, M, N, K, ab_dtype, split_k, ep.residual != nullptr) : !wo && split_k == 0 && !stream_k_keeps(M, N, K, ab_dtype))
+  if (gemm_on_pairs(p, epi, M, N, K, ab_dtype, split_k, ep.residual != nullptr))
     return launch_gemm_pair(a, w, ep, epi, M, N, K, ab_dtype, pair_plan(M, N, K, ab_dtype), (cudaStream_t)stream);
   CUtensorMapDataType dt = eb == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
   int bk = GEMM_BK_BYTES / eb;
@@ -1420,12 +1424,40 @@ int b200_gemm_decode_plan(int M, int N, int K, int ab_dtype, int split_k, int si
   DecodeCfg c{};
   rc = query_plan(c, p, epi, M, ab_dtype, split_k, has_residual != 0);
   if (rc) return rc;
+  // (a qkv projection whose K is not cut runs as the linear call and the rotation's own launch)
+  if (decode_on_pairs(p, epi == EPI_ROPE && c.S == 1 ? EPI_LINEAR : epi, M, N, K, ab_dtype, split_k, has_residual != 0)) {
+    int units;
+    size_t smem;
+    pair_shape(M, N, pair_plan(M, N, K, ab_dtype), units, out6[2], smem);
+    out6[0] = out6[1] = 1;
+    out6[3] = out6[2];
+    out6[4] = sm_count() & ~1;
+    out6[5] = (int)smem;
+    return B200_OK;
+  }
   out6[0] = c.S;
   out6[1] = c.smem > SMEM_TWO_PER_SM ? 1 : 2;
   out6[2] = c.nst;
   out6[3] = c.nst;
   out6[4] = c.cap_ctas;
   out6[5] = (int)c.smem;
+  return B200_OK;
+}
+
+int b200_gemm_pair_plan(int M, int N, int K, int ab_dtype, int silu_mul, int has_residual, int* out4) {
+  B200_REQUIRE(out4 && M > 0 && N > 0 && K > 0, "gemm_pair_plan: bad arguments");
+  B200_REQUIRE(ab_dtype == B200_BF16 || ab_dtype == B200_FP8_E4M3 || ab_dtype == B200_INT8 || ab_dtype == B200_INT8_WO, "gemm_pair_plan: bad dtype");
+  GemmPlan p;
+  int rc = plan_gemm(p, M, N, K, ab_dtype, 0);
+  if (rc) return rc;
+  const int epi = silu_mul ? EPI_SILU_MUL : EPI_LINEAR;
+  out4[0] = out4[1] = out4[2] = out4[3] = 0;
+  if (gemm_small_ok(nullptr, nullptr, epi, M, N, K, ab_dtype, 0) || !gemm_on_pairs(p, epi, M, N, K, ab_dtype, 0, has_residual != 0)) return B200_OK;
+  const PairPlan plan = pair_plan(M, N, K, ab_dtype);
+  size_t smem;
+  out4[0] = plan.bt;
+  out4[1] = plan.wide;
+  pair_shape(M, N, plan, out4[2], out4[3], smem);
   return B200_OK;
 }
 

@@ -299,6 +299,15 @@ def gemm_decode_plan(m, n, k, ab_dtype, split_k=0, silu_mul=False, has_residual=
     return dict(zip(("split", "ctas_per_sm", "w_stages", "a_stages", "cap_ctas", "smem"), list(out)))
 
 
+def gemm_pair_plan(m, n, k, ab_dtype, silu_mul=False, has_residual=False) -> dict:
+    """What the CTA pairs take of a GEMM that names no split: tokens of a tile (0: another schedule runs), units of two token tiles, all units."""
+    import ctypes
+
+    out = (ctypes.c_int * 4)()
+    check(_cabi.load().b200_gemm_pair_plan(m, n, k, ab_dtype, int(silu_mul), int(has_residual), out), "b200_gemm_pair_plan")
+    return dict(zip(("tokens", "wide", "units", "stages"), list(out)))
+
+
 def gemm_workspace_bytes(m, n, k, ab_dtype, split_k=0) -> int:
     return int(_lib().b200_gemm_workspace_bytes(m, n, k, ab_dtype, split_k))
 
