@@ -160,8 +160,7 @@ def test_gemm_pairs_silu_residual_bias(ops, m, n, k):
     _assert_close(ga, a.float().abs().view(m, -1, 16).amax(-1).cpu())
 
 
-# Two token tiles at a time: one such unit a pair, several (three waves), an odd number of token tiles (the last alone), whole waves and the rest one by
-# one, ragged tokens and rows, fewer k-blocks than ring stages and many more
+# More of both: two token tiles a unit (777 x 6144), several tiles a pair, ragged tokens and rows, fewer k-blocks than ring stages and many more
 WIDE_SHAPES = [(300, 10000, 192), (300, 10001, 192), (777, 6144, 1040), (700, 12800, 96), (1030, 16128, 4000), (771, 28416, 4096)]
 
 
@@ -169,6 +168,44 @@ WIDE_SHAPES = [(300, 10000, 192), (300, 10001, 192), (777, 6144, 1040), (700, 12
 @pytest.mark.parametrize("f32", [False, True])
 def test_gemm_pairs_of_two_token_tiles_int8_exact(ops, m, n, k, f32):
     test_gemm_pairs_int8_exact(ops, m, n, k, f32)
+
+
+# Units of two token tiles: (m, n, k in int8, waves of them, whether lone tiles follow, whether the token tiles are odd in number, so that a weight tile's last
+# unit holds one).  With several waves a pair's next unit starts while the epilogue still reads the accumulator of its second tile.  As many k-blocks as
+# ring stages and more; none of these plans has fewer.
+WIDE_PLANS = [(258, 12851, 720, 1, False, False), (784, 5588, 672, 1, False, True), (258, 19046, 736, 1, True, False), (770, 9717, 752, 1, True, True), (261, 37770, 1792, 2, False, False),
+              (1063, 15187, 3984, 2, True, False), (1541, 9389, 10752, 2, False, True), (1038, 15811, 10608, 2, True, True), (577, 31692, 4752, 3, True, False)]
+
+
+def _wide_plan(ops, m, n, k, kind):
+    plan = ops.gemm_pair_plan(m, n, k, kind)
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    return -(-plan["wide"] // pairs), plan["units"] > plan["wide"], -(-m // plan["tokens"]) % 2 == 1
+
+
+@pytest.mark.parametrize("m,n,k,waves,lone,odd", WIDE_PLANS)
+@pytest.mark.parametrize("f32", [False, True])
+def test_gemm_pairs_units_of_two_token_tiles_int8_exact(ops, m, n, k, waves, lone, odd, f32):
+    """Bounds as in test_gemm_pairs_int8_exact; the plan is the one that the shape stands for."""
+    assert _wide_plan(ops, m, n, k, ops.INT8) == (waves, lone, odd)
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    r = lambda *s: torch.randint(-127, 128, s, generator=g, dtype=torch.int8, device="cuda")  # noqa: E731
+    x, w, xs, ws = r(m, k), r(n, k), torch.rand(m, generator=g, device="cuda") + 0.5, torch.rand(n, generator=g, device="cuda") + 0.5
+    want = x.double() @ w.double().T * xs.double()[:, None] * ws.double()
+    got = ops.gemm(x, w, xs, ws, out_dtype=torch.float32 if f32 else torch.bfloat16).double()
+    assert ((got - want).abs() <= want.abs() * (2.0**-22 if f32 else 2.0**-8)).all()
+
+
+@pytest.mark.parametrize("m,n,k,waves,lone,odd", [(770, 9728, 376, 1, True, True), (258, 19072, 368, 1, True, False), (261, 37792, 896, 2, False, False)])
+def test_gemm_pairs_units_of_two_token_tiles_silu_residual_bias(ops, m, n, k, waves, lone, odd):
+    assert _wide_plan(ops, m, n, k, ops.BF16) == (waves, lone, odd)
+    test_gemm_pairs_silu_residual_bias(ops, m, n, k)
+
+
+@pytest.mark.parametrize("f32", [False, True])
+def test_gemm_pairs_units_of_two_token_tiles_rows_of_odd_length(ops, f32):
+    assert _wide_plan(ops, 258, 12851, 360, ops.BF16) == (1, False, False)
+    test_gemm_pairs_bf16_against_64_bits(ops, 258, 12851, 360, f32)
 
 
 @pytest.mark.parametrize("m,n,k", [(777, 6144, 520), (700, 12800, 96)])
