@@ -441,7 +441,7 @@ def test_attention_over_cached_latents_shared_by_a_cluster(H, C, R, window, sink
 
 @pytest.mark.parametrize("window,sinks", [(1 << 30, False), (1 << 30, True), (100, True), (1, False)])
 @pytest.mark.parametrize("H,C,R", [(3, 256, 64), (2, 256, 16), (4, 128, 32), (1, 128, 0)])
-def test_prompt_portions_over_cached_latents_on_tensor_memory(H, C, R, window, sinks):
+def test_prompt_portions_over_cached_latents_on_tensor_memory(H, C, R, window, sinks, first_seen=lambda p: 0):
     """Portions that end inside a tile, a page and a key step or on their borders, from position 0 or further on, a decoded token between them; rows of
     the pages past a sequence's end hold NaN.  Bound: the weights and the output are rounded to bf16."""
     ops, g = _ops(), torch.Generator().manual_seed(H)
@@ -455,6 +455,7 @@ def test_prompt_portions_over_cached_latents_on_tensor_memory(H, C, R, window, s
     for r, p, n in ent:
         flat = pool[rows[r]].view(-1, D)
         flat[:p + n] = torch.randn(p + n, D, generator=g).bfloat16()
+        flat[:first_seen(p)] = float("nan")
         pool[rows[r]] = flat.view(-1, 1, 32, D)
     bt = torch.zeros(len(ent), max(map(len, rows.values())), dtype=torch.int32)
     for r in rows:
@@ -469,6 +470,7 @@ def test_prompt_portions_over_cached_latents_on_tensor_memory(H, C, R, window, s
     t = 0
     for r, p, n in ent:
         keys = pool[rows[r]].view(-1, D)[:p + n].double()
+        keys[:first_seen(p)] = 0
         z = torch.einsum("thd,kd->htk", q[t:t + n].bfloat16().double(), keys) * scale
         i, j = torch.arange(p, p + n)[:, None], torch.arange(p + n)[None]
         z = z.masked_fill((j > i) | (j <= i - window), float("-inf"))
@@ -478,3 +480,10 @@ def test_prompt_portions_over_cached_latents_on_tensor_memory(H, C, R, window, s
         want, size = torch.einsum("htk,kc->thc", w, keys[:, :C]), torch.einsum("htk,kc->thc", w, keys[:, :C].abs())
         assert ((out[t:t + n].double().cpu() - want).abs() <= 2.0**-8 * want.abs() + 2.0**-8 * size + 1e-6).all()
         t += n
+
+
+@pytest.mark.parametrize("window", [1, 40, 100])
+@pytest.mark.parametrize("H,C,R", [(2, 256, 64), (2, 128, 32)])
+def test_prompt_portions_over_cached_latents_do_not_read_ahead_of_the_window(H, C, R, window):
+    """Rows ahead of the window of a sequence's first new query hold NaN, in pages wholly ahead of it too: they are in the first step of 64 keys."""
+    test_prompt_portions_over_cached_latents_on_tensor_memory(H, C, R, window, True, lambda p: max(0, p - window + 1))

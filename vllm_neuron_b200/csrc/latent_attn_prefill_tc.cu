@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
     const uint32_t lanes = tmem + ((uint32_t)(warp * 32) << 16);
     const uint32_t o_addr = lanes + O_COL;
     const int qpos = pos0 + q0 + row;
-    const int klo = first_key(qpos), klo_last = first_key(pos0 + q0 + LP_BM - 1);
+    const int klo = first_key(qpos), klo_first = first_key(pos0 + q0), klo_last = first_key(pos0 + q0 + LP_BM - 1);
     constexpr float LOG2E = 1.4426950408889634f;
     const float sl = scale * LOG2E;
     // a sink is a key without a value: the running maximum starts at its logit (not scaled), the denominator at its 1
@@ -228,12 +228,14 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
 #pragma unroll
         for (int i = 0; i < LP_BN; ++i)
           if (k0 + i > qpos || k0 + i < klo) sv[i] = 0xff800000u;
-        if (k0 + LP_BN > kv_end) {  // rows past the tile's keys are values with weight 0: whatever the page holds there must be finite
+        // keys that no row of the tile sees -- past the tile's last, ahead of the first row's window -- are values with weight 0: whatever their pages hold
+        // there must be finite
+        const int head = klo_first - k0, tail = kv_end - k0;  // the step's seen keys are head .. tail - 1
+        if (head > 0 || tail < LP_BN) {
           uint8_t* ks = k_s + (it % ST) * KST;
-          const int first = kv_end - k0, n16 = (LP_BN - first) * 8;
-          for (int idx = row; idx < (C / 64) * n16; idx += 128) {
-            const int c = idx / n16, r = idx - c * n16;
-            *reinterpret_cast<uint4*>(ks + c * LP_KCH + first * 128 + r * 16) = make_uint4(0u, 0u, 0u, 0u);
+          for (int idx = row; idx < (C / 64) * LP_BN * 8; idx += 128) {
+            const int c = idx / (LP_BN * 8), r = idx - c * (LP_BN * 8), key = r >> 3;
+            if (key < head || key >= tail) *reinterpret_cast<uint4*>(ks + c * LP_KCH + r * 16) = make_uint4(0u, 0u, 0u, 0u);
           }
           fence_proxy_async();
         }
