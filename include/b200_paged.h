@@ -612,7 +612,7 @@ int b200_latent_attn_decode_split(const float* q, int ldq, const void* pool, con
                                   int T, int H, int D, int Dv, int block_size, int splits, void* stream);
 /* Latent attention of prompt portions on tcgen05, bf16 pools of pages of 32 tokens: sequence s brings query rows [seq_start[s],
  * seq_start[s+1]) of q (fp32 [T][H][D], pitch ldq) from position seq_pos0[s] on and sees its block-table row seq_slot[s]; values are the
- * first Dv columns of the D.  Dv 128 or 256, Dv <= D <= Dv + 64, D a multiple of 16, ldq of 4, q and out 16-byte aligned, else
+ * first Dv columns of the D.  Dv 128 or 256, Dv <= D <= Dv + 64, D a multiple of 16, ldq of 4, q and out 16-byte aligned, scale > 0, else
  * B200_ERR_UNSUPPORTED (_supported tells for the sizes).  window >= 1; out bf16 [T][H][Dv]. */
 int b200_latent_attn_prefill_tc_supported(int D, int Dv, int block_size);
 int b200_latent_attn_prefill_tc(const float* q, int ldq, const void* pool, int num_blocks, const int32_t* block_table, int64_t bt_stride,

@@ -487,3 +487,20 @@ def test_prompt_portions_over_cached_latents_on_tensor_memory(H, C, R, window, s
 def test_prompt_portions_over_cached_latents_do_not_read_ahead_of_the_window(H, C, R, window):
     """Rows ahead of the window of a sequence's first new query hold NaN, in pages wholly ahead of it too: they are in the first step of 64 keys."""
     test_prompt_portions_over_cached_latents_on_tensor_memory(H, C, R, window, True, lambda p: max(0, p - window + 1))
+
+
+@pytest.mark.parametrize("scale", [-0.06, 0.0])
+def test_prompt_portions_over_cached_latents_of_any_scale(scale):
+    """A scale that turns the order of the scores round, and one that makes them all alike.  Bound: the weights and the output are rounded to bf16."""
+    ops, g = _ops(), torch.Generator().manual_seed(3)
+    H, C, D, n = 4, 128, 160, 150
+    blocks = {0: _pages(n, 32)}
+    pool = torch.randn(len(blocks[0]) + 1, 1, 32, D, generator=g).bfloat16()
+    bt = torch.tensor([blocks[0]], dtype=torch.int32)
+    q = torch.randn(n, H, D, generator=g) * 4
+    out = ops.swa_sink_attn(q.view(n, -1).to(DEV), H, pool.to(DEV), None, bt.to(DEV), _meta([(0, 0, n)], blocks, 32), None, scale, 1 << 30, latent_values=C)
+    keys = pool[blocks[0]].view(-1, D)[:n].double()
+    z = torch.einsum("thd,kd->htk", q.bfloat16().double(), keys) * scale
+    w = torch.softmax(z.masked_fill(torch.ones(n, n).triu(1).bool(), float("-inf")), 2)
+    want, size = torch.einsum("htk,kc->thc", w, keys[:, :C]), torch.einsum("htk,kc->thc", w, keys[:, :C].abs())
+    assert ((out.view(n, H, C).double().cpu() - want).abs() <= 2.0**-8 * want.abs() + 2.0**-8 * size + 1e-6).all()

@@ -358,8 +358,8 @@ int b200_latent_attn_prefill_tc(const float* q, int ldq, const void* pool, int n
   B200_REQUIRE(window >= 1, "latent_attn_prefill_tc: window %d", window);
   B200_REQUIRE(q && pool && block_table && seq_start && seq_slot && seq_pos0 && out, "latent_attn_prefill_tc: null pointer");
   B200_REQUIRE(H > 0, "latent_attn_prefill_tc: %d query heads", H);
-  if (!b200_latent_attn_prefill_tc_supported(D, C, block_size) || (ldq & 3) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15)) {
-    set_last_error("latent_attn_prefill_tc: rows of %d columns with %d values or the layout of q have no kernel", D, C);
+  if (!b200_latent_attn_prefill_tc_supported(D, C, block_size) || !(scale > 0.f) || (ldq & 3) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15)) {
+    set_last_error("latent_attn_prefill_tc: rows of %d columns with %d values, a scale of %g or the layout of q have no kernel", D, C, (double)scale);
     return B200_ERR_UNSUPPORTED;
   }
   if (B <= 0 || max_new <= 0) return B200_OK;

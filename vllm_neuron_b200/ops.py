@@ -826,7 +826,7 @@ def swa_sink_attn(q_src, num_heads: int, k_pool, v_pool, block_table, meta, sink
     # decoded tokens beside prompt portions: each kind on its own kernel where that pays, in one launch of the prompt kernel otherwise
     parts = getattr(meta, "parts", None)
     if parts:
-        tc = _latent_tc(q_src, k_pool, meta, d, dv, bs, chunk, softcap, sigmoid_bias, out_f32) if latent_values else \
+        tc = _latent_tc(q_src, k_pool, meta, d, dv, bs, scale, chunk, softcap, sigmoid_bias, out_f32) if latent_values else \
             _prompt_tc(q_src, k_pool, meta, d, dv, bs, v_div, latent_values, softcap, sigmoid_bias, pool)
         spans = [_span(p.max_end, int(window), int(chunk), pool, int(keep)) for p in parts]
         if not (tc or _prompt_mma(q_src, k_pool, meta, d, dv)) or not _split_pays(parts, num_heads, g, d, dv, bool(latent_values), tc, spans, bs % 32 == 0):
@@ -852,11 +852,11 @@ def _prompt_mma(q, k_pool, meta, d, dv) -> bool:
             and d <= 512 and dv <= 256 and q.stride(0) % 2 == 0)
 
 
-def _latent_tc(q, k_pool, meta, d, dv, bs, chunk, softcap, sigmoid_bias, out_f32) -> bool:
+def _latent_tc(q, k_pool, meta, d, dv, bs, scale, chunk, softcap, sigmoid_bias, out_f32) -> bool:
     """Prompt portions over cached latents, bf16 rows of up to 64 columns beside the 128 or 256 value columns, pages of 32 tokens: the tcgen05
-    kernel.  From the shortest portion on: us, 16 heads over rows of 320, mma.sync / here: 16 tokens 20 / 14, at 1800 227 / 47, 128 41 / 18, 1000 162 / 39,
+    kernel (positive scales: it scales a row's largest score, not the scores).  From the shortest portion on: us, 16 heads over rows of 320, mma.sync / here: 16 tokens 20 / 14, at 1800 227 / 47, 128 41 / 18, 1000 162 / 39,
     1600 310 / 51, 512 at 4000 549 / 107; rows of 160: 16 16 / 12, 1600 184 / 51."""
-    return bool(not (chunk or softcap or out_f32) and sigmoid_bias is None and k_pool.dtype == torch.bfloat16 and meta.max_new >= PREFILL_ATTN_MIN_TOKENS
+    return bool(not (chunk or softcap or out_f32) and scale > 0 and sigmoid_bias is None and k_pool.dtype == torch.bfloat16 and meta.max_new >= PREFILL_ATTN_MIN_TOKENS
                 and q.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0 and k_pool.data_ptr() % 16 == 0
                 and _lib().b200_latent_attn_prefill_tc_supported(d, dv, bs))
 
@@ -898,7 +898,7 @@ def _swa_part(q_src, num_heads, k_pool, v_pool, block_table, meta, sink, scale, 
                                                              int(keep), sink),
                   "b200_swa_attn_prefill_tc_sink")
         return
-    if latent_values and _latent_tc(q_all, k_pool, meta, d, dv, bs, chunk, softcap, sigmoid_bias, out_f32):
+    if latent_values and _latent_tc(q_all, k_pool, meta, d, dv, bs, scale, chunk, softcap, sigmoid_bias, out_f32):
         with _k("swa_sink_attn_prefill_tc" + tag):
             check(_lib().b200_latent_attn_prefill_tc(q_all, q_all.stride(0), k_pool, k_pool.shape[0], block_table, block_table.stride(0),
                                                            meta.seq_start, meta.seq_slot, meta.seq_pos0, meta.num_seqs, meta.max_new, sink,
