@@ -504,3 +504,19 @@ def test_prompt_portions_over_cached_latents_of_any_scale(scale):
     w = torch.softmax(z.masked_fill(torch.ones(n, n).triu(1).bool(), float("-inf")), 2)
     want, size = torch.einsum("htk,kc->thc", w, keys[:, :C]), torch.einsum("htk,kc->thc", w, keys[:, :C].abs())
     assert ((out.view(n, H, C).double().cpu() - want).abs() <= 2.0**-8 * want.abs() + 2.0**-8 * size + 1e-6).all()
+
+
+def test_attention_over_cached_latents_one_cta_a_token():
+    """The entry point without splits is that of one: the same bits."""
+    from vllm_neuron_b200 import _cabi
+
+    g = torch.Generator(device=DEV).manual_seed(1)
+    T, H, C, D, bs = 3, 5, 64, 80, 16
+    pool = torch.randn(T * 4, bs, D, generator=g, device=DEV).bfloat16()
+    bt = torch.arange(T * 4, dtype=torch.int32, device=DEV).view(T, 4)
+    q, rows, pos = torch.randn(T, H * D, generator=g, device=DEV), torch.arange(T, dtype=torch.int32, device=DEV), torch.tensor([0, 17, 63], dtype=torch.int32, device=DEV)
+    outs = [torch.zeros(T, H * C, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    lib, stream = _cabi.load(), _ops()._stream()
+    args = lambda out: (q.data_ptr(), H * D, pool.data_ptr(), bt.data_ptr(), 4, rows.data_ptr(), pos.data_ptr(), None, D ** -0.5, 1 << 30, out.data_ptr(), T, H, D, C, bs)  # noqa: E731
+    assert lib.b200_latent_attn_decode(*args(outs[0]), stream) == 0 and lib.b200_latent_attn_decode_split(*args(outs[1]), 1, stream) == 0
+    assert outs[0].any() and torch.equal(*outs)
