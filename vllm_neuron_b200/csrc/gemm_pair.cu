@@ -217,15 +217,14 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
         named_bar_sync(1, 32 * PAIR_EPI_WARPS);
         uint32_t r[8] = {};
         int c0 = quarter * 16;
-        if (ahead && c0 < bt) epilogue_residual(ep, r, m0 + c0, M, n, N, lane & 1);
+        if (ahead) epilogue_residual(ep, r, m0 + c0, M, n, N, lane & 1);
         mbar_wait(&tfull[as], (seg >> 1) & 1);
         __syncwarp();  // lanes may leave the wait one by one; tcgen05.ld wants them together
         tc_fence_after();
         const uint32_t acc = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(as * PAIR_MAX_BT);
         // the four warps of a lane group take every fourth chunk of 16 tokens
         uint32_t v[16];
-        if (c0 < bt) tmem_ld_32x32b_x16(acc + c0, v);
-        else give_back(as);
+        tmem_ld_32x32b_x16(acc + c0, v);  // bt >= 64: each of the four has a chunk
 #pragma unroll 1
         for (; c0 < bt; c0 += 64) {
           tmem_ld_wait16(v);
