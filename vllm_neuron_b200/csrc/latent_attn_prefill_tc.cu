@@ -26,41 +26,6 @@ constexpr int LP_BLK = 32;        // tokens per page
 constexpr int LP_THREADS = 256;   // warps 0-3 weights, 4 MMA, 5 and 6 load a page of a step each
 constexpr int LP_QCH = LP_BM * 128, LP_KCH = LP_BN * 128;  // 64 columns of the query tile / of a step's keys
 
-// MN-major, 128B-swizzled operand: 64 contiguous elements of N per row, 8 K-rows per 1024 B atom
-__device__ __forceinline__ uint64_t lp_desc_mn(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((LP_KCH >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((1024 >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-__device__ __forceinline__ void lp_ld_x32(uint32_t taddr, uint32_t* v) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]),
-        "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]),
-        "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void lp_st_x16(uint32_t taddr, const uint32_t* v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16};\n" ::"r"(taddr),
-      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
-      "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-      : "memory");
-}
-__device__ __forceinline__ float lp_ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // C: value columns; rows of D = 16 n columns, C <= D <= C + 64.  ST: stages of keys.
 template <int C, int ST>
 __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
@@ -192,7 +157,7 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
             mbar_wait(&p_ready[2 * (it & 1) + (kk >> 1)], (uint32_t)(it >> 1) & 1u);
             tc_fence_after();
           }
-          const uint64_t vd = lp_desc_mn(va + kk * 2048);
+          const uint64_t vd = umma_desc_mn_sw128(va + kk * 2048, LP_KCH, 1024);
           umma_ts_f16(tmem + O_COL, p + (uint32_t)kk * 8u, vd, IDESC_PV, (uint32_t)((it | kk) != 0));
           umma_ts_f16(tmem + O_COL, p + 32u + (uint32_t)kk * 8u, vd, IDESC_PV, 1u);
         }
@@ -221,8 +186,8 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
       mbar_wait(&s_full[it & 1], (uint32_t)(it >> 1) & 1u);
       tc_fence_after();
       uint32_t sv[LP_BN];
-      lp_ld_x32(s_addr, &sv[0]);
-      lp_ld_x32(s_addr + 32, &sv[32]);
+      tmem_ld_32x32b_x32(s_addr, &sv[0]);
+      tmem_ld_32x32b_x32(s_addr + 32, &sv[32]);
       tmem_ld_wait();
       if (masked) {
 #pragma unroll
@@ -251,7 +216,7 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
       // lazy maximum: move it (and pay the O read-modify-write) only when it grew by more than 2^8
       const bool grow = m_new > m_used + 8.f;
       if (__any_sync(0xffffffffu, grow)) {
-        const float alpha = grow ? lp_ex2(m_used - m_new) : 1.f;  // m_used = -inf -> 0
+        const float alpha = grow ? ex2_approx(m_used - m_new) : 1.f;  // m_used = -inf -> 0
         if (grow) m_used = m_new;
         l *= alpha;
         if (it > 0) {
@@ -260,11 +225,11 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
 #pragma unroll 1
           for (int c = 0; c < C / 32; ++c) {
             uint32_t v[32];
-            lp_ld_x32(o_addr + c * 32, v);
+            tmem_ld_32x32b_x32(o_addr + c * 32, v);
             tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-            tmem_st_32x32b_x32(o_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+            tmem_st_32x32b_x32(o_addr + c * 32, v);
           }
           tmem_st_wait();
         }
@@ -276,15 +241,15 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
         uint32_t hi[16], lo[16];
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          const float p0 = lp_ex2(fmaf(__uint_as_float(sv[c * 32 + i]), sl, neg_m));
-          const float p1 = lp_ex2(fmaf(__uint_as_float(sv[c * 32 + i + 1]), sl, neg_m));
+          const float p0 = ex2_approx(fmaf(__uint_as_float(sv[c * 32 + i]), sl, neg_m));
+          const float p1 = ex2_approx(fmaf(__uint_as_float(sv[c * 32 + i + 1]), sl, neg_m));
           l4[(i >> 1) & 3] += p0 + p1;
           const uint32_t h = pack_bf16(p0, p1);
           hi[i >> 1] = h;
           lo[i >> 1] = pack_bf16(p0 - __uint_as_float(h << 16), p1 - __uint_as_float(h & 0xffff0000u));
         }
-        lp_st_x16(s_addr + c * 16, hi);
-        lp_st_x16(s_addr + 32 + c * 16, lo);
+        tmem_st_32x32b_x16(s_addr + c * 16, hi);
+        tmem_st_32x32b_x16(s_addr + 32 + c * 16, lo);
         tmem_st_wait();  // the products of the first 32 keys run while the other weights are made (512 tokens at 4000, 16 heads of 320: 98.4 -> 95.5 us)
         tc_fence_before();
         __syncwarp();
@@ -302,7 +267,7 @@ __global__ void __launch_bounds__(LP_THREADS, C <= 128 ? 2 : 1)
 #pragma unroll 1
     for (int c = 0; c < C / 32; ++c) {
       uint32_t v[32];
-      lp_ld_x32(o_addr + c * 32, v);
+      tmem_ld_32x32b_x32(o_addr + c * 32, v);
       tmem_ld_wait();
 #pragma unroll
       for (int i = 0; i < 32; i += 8)

@@ -37,16 +37,6 @@ constexpr int TP_BLK = 32;   // tokens per page
 constexpr int TP_HALF = TP_BN * 128;  // one [128 rows x 128 B] operand half = 16 KB
 enum { TP_SOFTMAX = 0, TP_CAPPED = 1, TP_SIGMOID = 2 };
 
-// MN-major, 128B-swizzled operand: 64 contiguous elements of M/N per row, 8 K-rows per 1024 B atom
-__device__ __forceinline__ uint64_t tp_desc_mn_sw128(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
 // K-major, 64B-swizzled operand tile: rows of 64 B, 8-row groups 512 B apart
 __device__ __forceinline__ uint64_t tp_desc_sw64(uint32_t smem_addr) {
   uint64_t d = 0;
@@ -57,31 +47,6 @@ __device__ __forceinline__ uint64_t tp_desc_sw64(uint32_t smem_addr) {
   d |= (uint64_t)4 << 61;  // SWIZZLE_64B
   return d;
 }
-__device__ __forceinline__ void tp_ld_x32(uint32_t taddr, uint32_t* v) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]),
-        "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]),
-        "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tp_st_x16(uint32_t taddr, const uint32_t* v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16};\n" ::"r"(taddr),
-      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
-      "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-      : "memory");
-}
-__device__ __forceinline__ float tp_ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
-  return y;
-}
-
 template <int DK, int DV, int KIND, bool MAPS>
 __global__ void __launch_bounds__(TP_THREADS, 1)
     swa_prefill_tc_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
@@ -245,7 +210,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1)
 #pragma unroll
           for (int k4 = 0; k4 < TP_BN / 32; ++k4) {
             const int kk = half * (TP_BN / 32) + k4;  // 16 keys per UMMA_K: two 8-row groups of the [token][d] tile
-            const uint64_t vd = tp_desc_mn_sw128(va + kk * 2048, TP_HALF, 1024);
+            const uint64_t vd = umma_desc_mn_sw128(va + kk * 2048, TP_HALF, 1024);
             umma_ts_f16(o_t, p_t + (uint32_t)kk * 8u, vd, IDESC_PV, (uint32_t)((it | kk) != 0));
             if (split_p) umma_ts_f16(o_t, p_t + 64u + (uint32_t)kk * 8u, vd, IDESC_PV, 1u);
           }
@@ -331,15 +296,15 @@ __global__ void __launch_bounds__(TP_THREADS, 1)
         const bool masked = k0 + TP_BN - 1 > pos0 + q0 || k0 < klo_last;  // some key of the step is hidden from some row
         uint32_t sv[TP_BN];
         auto load_scores = [&]() {
-          tp_ld_x32(s_addr, &sv[0]);
-          tp_ld_x32(s_addr + 32, &sv[32]);
-          tp_ld_x32(s_addr + 64, &sv[64]);
-          tp_ld_x32(s_addr + 96, &sv[96]);
+          tmem_ld_32x32b_x32(s_addr, &sv[0]);
+          tmem_ld_32x32b_x32(s_addr + 32, &sv[32]);
+          tmem_ld_32x32b_x32(s_addr + 64, &sv[64]);
+          tmem_ld_32x32b_x32(s_addr + 96, &sv[96]);
           tmem_ld_wait();
           if (KIND == TP_CAPPED) {
 #pragma unroll
             for (int i = 0; i < TP_BN; ++i)
-              sv[i] = __float_as_uint(capl - __fdividef(2.0f * capl, 1.0f + tp_ex2(__uint_as_float(sv[i]) * cap_arg)));
+              sv[i] = __float_as_uint(capl - __fdividef(2.0f * capl, 1.0f + ex2_approx(__uint_as_float(sv[i]) * cap_arg)));
           }
           if (masked) {
 #pragma unroll
@@ -363,18 +328,18 @@ __global__ void __launch_bounds__(TP_THREADS, 1)
           // lazy maximum: move it (and pay the O read-modify-write) only when it grew by more than 2^8
           const bool grow = m_new > m_used + 8.f;
           if (__any_sync(0xffffffffu, grow)) {
-            const float alpha = grow ? tp_ex2(m_used - m_new) : 1.f;  // m_used = -inf -> 0
+            const float alpha = grow ? ex2_approx(m_used - m_new) : 1.f;  // m_used = -inf -> 0
             if (grow) m_used = m_new;
             l *= alpha;
             if (it > 0) {  // rare after the first steps: the score registers are given up for the O tile and loaded again
 #pragma unroll 1
               for (int c = 0; c < DV / 32; ++c) {
                 uint32_t v[32];
-                tp_ld_x32(o_addr + c * 32, v);
+                tmem_ld_32x32b_x32(o_addr + c * 32, v);
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-                tmem_st_32x32b_x32(o_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+                tmem_st_32x32b_x32(o_addr + c * 32, v);
               }
               tmem_st_wait();
               load_scores();
@@ -391,21 +356,22 @@ __global__ void __launch_bounds__(TP_THREADS, 1)
             const float s0 = __uint_as_float(sv[c * 32 + i]), s1 = __uint_as_float(sv[c * 32 + i + 1]);
             float p0, p1;
             if (KIND == TP_SIGMOID) {  // 1 / (1 + 2^-(s + b)); a hidden key's -inf gives 1 / inf = 0
-              p0 = __fdividef(1.0f, 1.0f + tp_ex2(-fmaf(s0, sl, sb_log2)));
-              p1 = __fdividef(1.0f, 1.0f + tp_ex2(-fmaf(s1, sl, sb_log2)));
+              p0 = __fdividef(1.0f, 1.0f + ex2_approx(-fmaf(s0, sl, sb_log2)));
+              p1 = __fdividef(1.0f, 1.0f + ex2_approx(-fmaf(s1, sl, sb_log2)));
             } else {
-              p0 = tp_ex2(fmaf(s0, sl, neg_m));
-              p1 = tp_ex2(fmaf(s1, sl, neg_m));
+              p0 = ex2_approx(fmaf(s0, sl, neg_m));
+              p1 = ex2_approx(fmaf(s1, sl, neg_m));
               l4[(i >> 1) & 3] += p0 + p1;
             }
             const uint32_t h = pack_bf16(p0, p1);
             hi[i >> 1] = h;
             lo[i >> 1] = pack_bf16(p0 - __uint_as_float(h << 16), p1 - __uint_as_float(h & 0xffff0000u));
           }
-          tp_st_x16(s_addr + c * 16, hi);
-          if (split_p) tp_st_x16(s_addr + 64 + c * 16, lo);
+          tmem_st_32x32b_x16(s_addr + c * 16, hi);
+          if (split_p) tmem_st_32x32b_x16(s_addr + 64 + c * 16, lo);
           // the products of the first 64 keys run while the other weights are made: us, one hand-over / two, prompts of 2500, 77 and 1111: two maps
-          // over 128 values 114 / 111, capped 77.4 / 75.5, sigmoid 76.0 / 71.5
+          // over 128 values 114 / 111, capped 77.4 / 75.5, sigmoid 76.0 / 71.5; 16 heads over 4 of 128, 4096 tokens plain 87 / 86, capped 160 / 155, sigmoid 116 / 108;
+          // of 64 plain 77 / 77, capped 150 / 152.  (The register cap makes it spill: 20 to 60 bytes a thread stored, 64 to 216 loaded; before 0 to 20 and 0 to 40.)
           if (c & 1) {
             tmem_st_wait();
             tc_fence_before();
@@ -424,7 +390,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1)
 #pragma unroll 1
       for (int c = 0; c < DV / 32; ++c) {
         uint32_t v[32];
-        tp_ld_x32(o_addr + c * 32, v);
+        tmem_ld_32x32b_x32(o_addr + c * 32, v);
         tmem_ld_wait();
         if (ok && out_f32) {
           float* dst = reinterpret_cast<float*>(out) + o_off + c * 32;
