@@ -70,7 +70,7 @@ __device__ __forceinline__ float silu_mul_bf16(float g, float u) {
   return __bfloat162float(__float2bfloat16_rn(silu_f32(g) * u));
 }
 
-// Prompt epilogue (stream-K and CTA pairs) of one 16-token chunk, transposed through a per-warp shared-memory tile so that global
+// Prompt epilogue (stream-K; the CTA pairs have their own in gemm_pair.cuh) of one 16-token chunk, transposed through a per-warp shared-memory tile so that global
 // memory sees 16-byte vectors instead of one 2-byte element per lane:
 //   TMEM hands lane l the weight row n0w + l of 16 tokens; the warp writes the scaled values (a_scale, w_scale, bias
 //   applied, fp32) as xp[token][row] (pitch XP_PITCH floats), then lane (token = l / 4 + 8 it, rows 8 (l % 4) ..) adds the

@@ -1,4 +1,4 @@
-// Weight GEMM of prompt-sized batches (M > 128) on CTA pairs:
+// Weight GEMM on CTA pairs: prompt-sized batches (M > 128) but those that stream_k_keeps, and decode-sized ones that pair_takes_decode:
 //
 //   out[m][n] = (sum_k a[m][k] w[n][k]) * a_scale[m] * w_scale[n] + bias[n] + residual[m][n]
 //

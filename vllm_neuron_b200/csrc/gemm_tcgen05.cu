@@ -15,7 +15,8 @@
 //    fp32 partial, slice by slice, into the peer that owns those weight rows (st.shared::cluster), one cluster barrier,
 //    then each CTA adds the slices in fixed rank order (bit-reproducible) and runs the epilogue for its 128/S rows.
 //    No global workspace, no atomics, no second kernel.  CTAs are sized (<= 105 KB smem, <= 64 TMEM columns) so that
-//    two are resident per SM: the prologue/epilogue of one overlaps the streaming of the other.
+//    two are resident per SM: the prologue/epilogue of one overlaps the streaming of the other.  Calls that would take S = 1 and whose tiles fill the
+//    waves of CTA pairs run there (gemm_pair.cu).
 //  * PREFILL (M > 128): CTA pairs (gemm_pair.cu) for bf16, fp8 and int8 operands.  For the weight-only kind, long K against few tiles and
 //    calls that cap the CTAs persistent stream-K, one CTA per SM; the flattened (tile, k-block) space is cut into equal
 //    contiguous spans; a tile cut by a span boundary is finished by whichever contributor arrives last (partials parked
