@@ -278,8 +278,21 @@ def test_gemm_rope_kv_write_of_a_decode_batch_on_pairs(ops, kind):
 @pytest.mark.parametrize("m,n,k", [(17, 10272, 2048), (64, 9473, 520), (65, 10272, 2048), (128, 18944, 1032)])
 @pytest.mark.parametrize("f32", [False, True])
 def test_gemm_decode_batches_on_pairs(ops, m, n, k, f32):
-    """Up to 128 tokens against rows that fill a wave of pairs, or miss it by one, and a K of a part of a block."""
+    """Up to 128 tokens against rows that fill a wave of pairs, or miss it by one, and a K of a part of a block, whichever schedule takes them."""
     test_gemm_pairs_bf16_against_64_bits(ops, m, n, k, f32)
+
+
+@pytest.mark.parametrize("m,n,k", [(9, 49153, 2048), (16, 55296, 1032), (17, 49152, 2040), (64, 49001, 1032), (65, 10272, 2048), (97, 18945, 520), (128, 18944, 1032)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_gemm_decode_batches_that_the_pairs_take(ops, m, n, k, f32):
+    """9 to 128 tokens, rows of odd length, a last k-block that is not whole; every one of these runs on the pairs."""
+    assert ops.gemm_pair_plan(m, n, k, ops.BF16, has_residual=True)["tokens"] > 0
+    test_gemm_pairs_bf16_against_64_bits(ops, m, n, k, f32)
+
+
+def test_gemm_rope_kv_write_of_a_decode_batch_has_its_linear_call_on_pairs(ops):
+    for kind in (ops.BF16, ops.FP8_E4M3):
+        assert ops.gemm_pair_plan(100, 80 * 128, 2048, kind)["tokens"] > 0
 
 
 @pytest.mark.parametrize("m,n,k", [(41, 10272, 2048), (64, 12288, 4096), (17, 16032, 4096), (100, 6144, 4096)])
